@@ -34,6 +34,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 namespace mdg {
 
 constexpr int kErrCapacity = 1;
@@ -216,6 +218,13 @@ __device__ __forceinline__ void warp_max_to(unsigned long long *addr, double v) 
     const unsigned long long mine = (unsigned long long)__double_as_longlong(v);
     if (mine > cur) atomicMax(addr, mine);
   }
+}
+
+// The error flag as one lane of the warp read it: the lanes of an atom must
+// agree on whether they take its row (they exchange values), and the flag
+// can be raised by another block at any time.  All lanes must call.
+__device__ __forceinline__ int warp_error(const Status *st) {
+  return __shfl_sync(0xffffffffu, *(volatile const int *)&st->error, 0);
 }
 
 // Fixed order block sum written to partials[blockIdx.x * nsum + k].
@@ -913,13 +922,14 @@ __global__ void __launch_bounds__(BLOCK) k_permute(Arrays a, Box b, int n, int4 
     a.cell_tmp[s] = a.cell[o];
     a.q_old[s] = q;
     const double x[3] = {q.x, q.y, q.z};
-    a.mult[s] = (unsigned char)border_bits(x, b, &m);
+    const int strips = border_bits(x, b, &m);
+    a.mult[s] = (unsigned char)strips;
     // FP32 coordinates for the list prefilter (x in box coordinates, y and z
-    // relative to the cell) and the packed cell coordinates
+    // relative to the cell), with the strip bits, and the packed cell coordinates
     const int c = a.cell_tmp[s];
     const int cx = c % b.ms[0], cy = (c / b.ms[0]) % b.ms[1], cz = c / (b.ms[0] * b.ms[1]);
     const int gz = cz + b.z0;  // global layer (the local one in a slab)
-    a.qloc[s] = make_float4((float)q.x, (float)(q.y - cy * b.cs[1]), (float)(q.z - gz * b.cs[2]), 0.f);
+    a.qloc[s] = make_float4((float)q.x, (float)(q.y - cy * b.cs[1]), (float)(q.z - gz * b.cs[2]), __int_as_float(strips));
     a.cxyz[s] = pack_cell(cx, cy, cz);
     if (pack) {
       // the coming step's first-drift positions for the fused FP32 NVE pass
@@ -984,7 +994,7 @@ __device__ __forceinline__ bool band_test(const double4 *__restrict__ q, int i, 
 // and the lanes file the ones they keep in slot order through a ballot over
 // the atom's lanes, so the row is the same for every lane count; cnt stays
 // equal on all of them.
-template <bool NEED, bool SELF, int BTPA, bool PIPE, typename Emit>
+template <bool NEED, bool SELF, int BTPA, typename Emit>
 __device__ __forceinline__ void build_range(const float4 *__restrict__ qloc, const double4 *__restrict__ q,
                                             const unsigned char *__restrict__ mult, int beg, int end, float bx,
                                             float by, float bz, int need, int shift, const Box &b, int i, int &cnt,
@@ -1010,34 +1020,21 @@ __device__ __forceinline__ void build_range(const float4 *__restrict__ qloc, con
       if (SELF) keep = keep && j != i;
       return keep;
     };
-    // PIPE: the next four candidates' loads are issued before this four's
-    // tests (four more float4 registers)
     int j = beg;
     float4 n0, n1, n2, n3;
-    if (PIPE && j + 4 <= end) {
+    if (j + 4 <= end) {
       n0 = __ldg(qloc + j);
       n1 = __ldg(qloc + j + 1);
       n2 = __ldg(qloc + j + 2);
       n3 = __ldg(qloc + j + 3);
     }
     for (; j + 4 <= end; j += 4) {
-      float4 l0, l1, l2, l3;
-      if (PIPE) {
-        l0 = n0;
-        l1 = n1;
-        l2 = n2;
-        l3 = n3;
-        if (j + 8 <= end) {
-          n0 = __ldg(qloc + j + 4);
-          n1 = __ldg(qloc + j + 5);
-          n2 = __ldg(qloc + j + 6);
-          n3 = __ldg(qloc + j + 7);
-        }
-      } else {
-        l0 = __ldg(qloc + j);
-        l1 = __ldg(qloc + j + 1);
-        l2 = __ldg(qloc + j + 2);
-        l3 = __ldg(qloc + j + 3);
+      const float4 l0 = n0, l1 = n1, l2 = n2, l3 = n3;
+      if (j + 8 <= end) {
+        n0 = __ldg(qloc + j + 4);
+        n1 = __ldg(qloc + j + 5);
+        n2 = __ldg(qloc + j + 6);
+        n3 = __ldg(qloc + j + 7);
       }
       float r0, r1, r2, r3;
       bool k0 = prefilter(j, l0, r0), k1 = prefilter(j + 1, l1, r1), k2 = prefilter(j + 2, l2, r2),
@@ -1103,13 +1100,12 @@ __device__ __forceinline__ void build_range(const float4 *__restrict__ qloc, con
 // rows in (dz, dy) order, then x order across the row's cells -- the cells
 // in dx order, as a 27-cell walk visits them.  Returns the partners found
 // (entries beyond the capacity are counted, not filed).
-template <bool SLAB = false, int BTPA = 1, bool PIPE = true, typename Emit>
+template <int BTPA, typename Emit>
 __device__ __forceinline__ int build_rows(const Box &b, const float4 *__restrict__ qloc,
                                           const double4 *__restrict__ q, const unsigned char *__restrict__ mult,
                                           const int *__restrict__ tab, int pc, int i, Emit &emit) {
   const float4 li = qloc[i];
-  const int cx = pc & 2047, cy = (pc >> 11) & 2047, lz = pc >> 22;
-  const int cz = SLAB ? b.z0 + lz : lz;  // global layer
+  const int cx = pc & 2047, cy = (pc >> 11) & 2047, cz = pc >> 22;
   const int ms0 = b.ms[0], ms1 = b.ms[1], ms2 = b.ms[2];
   const float hi = b.sl2_hi;
   const int mx = ms0 * kXSub;
@@ -1136,13 +1132,6 @@ __device__ __forceinline__ int build_rows(const Box &b, const float4 *__restrict
     const double sz = zc == 1 ? -b.L[2] : (zc == 2 ? b.L[2] : 0.0);
     const float bz = (float)((z - cz) * b.cs[2] + sz) - li.z;
     const float gz = dz == 0 ? 0.f : (dz < 0 ? li.z : csz - li.z);
-    // the layer's block of trim-table rows: the global layer in a single
-    // domain; in a slab an owned local layer or one of the two ghost blocks
-    int blk = z;
-    if (SLAB) {
-      const int nl = lz + dz;
-      blk = nl < 0 ? b.nzl : (nl >= b.nzl ? b.nzl + 1 : nl);
-    }
     for (int dy = -1; dy <= 1; dy++) {
       const float gy = dy == 0 ? 0.f : (dy < 0 ? li.y : csy - li.y);
       const float g2 = fmaf(gy, gy, gz * gz);
@@ -1160,26 +1149,331 @@ __device__ __forceinline__ int build_rows(const Box &b, const float4 *__restrict
       if (y < 0) { y += ms1; yc = 1; } else if (y >= ms1) { y -= ms1; yc = 2; }
       const double sy = yc == 1 ? -b.L[1] : (yc == 2 ? b.L[1] : 0.0);
       const float by = (float)((y - cy) * b.cs[1] + sy) - li.y;
-      const int *xr = tab + (size_t)(blk * ms1 + y) * (mx + 1);
+      const int *xr = tab + (size_t)(z * ms1 + y) * (mx + 1);
       const int yz = (yc << 2) | (zc << 4);
       if (vlo < 0)  // through the -x face: the row's last cells, image shift -L
-        build_range<true, false, BTPA, PIPE>(qloc, q, mult, xr[vlo + mx], xr[mx], bxm, by, bz,
+        build_range<true, false, BTPA>(qloc, q, mult, xr[vlo + mx], xr[mx], bxm, by, bz,
                                        needed_strips(-b.L[0], sy, sz), 1 | yz, b, i, cnt, emit);
       {
         const int a0 = max(vlo, 0), a1 = min(vhi, mx);
         const int beg = xr[a0], end = xr[a1];
         const int need = needed_strips(0.0, sy, sz);
         if (dz == 0 && dy == 0)
-          build_range<false, true, BTPA, PIPE>(qloc, q, mult, beg, end, bx0, by, bz, 0, yz, b, i, cnt, emit);
+          build_range<false, true, BTPA>(qloc, q, mult, beg, end, bx0, by, bz, 0, yz, b, i, cnt, emit);
         else if (need)
-          build_range<true, false, BTPA, PIPE>(qloc, q, mult, beg, end, bx0, by, bz, need, yz, b, i, cnt, emit);
+          build_range<true, false, BTPA>(qloc, q, mult, beg, end, bx0, by, bz, need, yz, b, i, cnt, emit);
         else
-          build_range<false, false, BTPA, PIPE>(qloc, q, mult, beg, end, bx0, by, bz, 0, yz, b, i, cnt, emit);
+          build_range<false, false, BTPA>(qloc, q, mult, beg, end, bx0, by, bz, 0, yz, b, i, cnt, emit);
       }
       if (vhi > mx)  // through the +x face: the row's first cells, image shift +L
-        build_range<true, false, BTPA, PIPE>(qloc, q, mult, xr[0], xr[vhi - mx], bxp, by, bz,
+        build_range<true, false, BTPA>(qloc, q, mult, xr[0], xr[vhi - mx], bxp, by, bz,
                                        needed_strips(b.L[0], sy, sz), 2 | yz, b, i, cnt, emit);
     }
+  }
+  return cnt;
+}
+
+// ---- rows of a warp's atoms, one lane per atom
+// What a lane's row walk needs of its box (the replica's own in an ensemble).
+struct RowGeom {
+  double L[3], cs0, inv_cs0, sl2;
+  float csy, csz, lo, hi;  // cell edges along y and z; the FP32 prefilter band
+  int ms[3], z0, nzl;
+};
+
+__device__ __forceinline__ RowGeom row_geom(const Box &b) {
+  return RowGeom{{b.L[0], b.L[1], b.L[2]}, b.cs[0],   b.inv_cs[0], b.sl2, (float)b.cs[1], (float)b.cs[2], b.sl2_lo,
+                 b.sl2_hi,  {b.ms[0], b.ms[1], b.ms[2]}, b.z0, b.nzl};
+}
+
+// Strip bits an image shift needs (needed_strips), from its code (shift_of):
+// code 1 (-L) needs the high strip, code 2 (+L) the low one.
+__device__ __forceinline__ int strips_of(int code) { return ((code & 0x15) << 1) | ((code & 0x2a) >> 1); }
+
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Candidates of one run that a warp stages at a time, and words of found
+// partners that a lane keeps before they go to the list.
+constexpr int kRunStage = 128, kRowWords = 16;
+
+// Shared memory of one warp's row walk.
+struct WarpRows {
+  float4 xy[kRunStage / 2];  // staged candidates in pairs: x0, x1, y0, y1
+  float2 zz[kRunStage / 2];  //                             z0, z1
+  // column l: lane l's words, 32 candidates each: partners as bits (the first
+  // candidate at bit 31) and the first candidate's slot
+  uint2 word[kRowWords][32];
+};
+
+// The exact test of candidate j of atom i (within_search_exact) through the
+// y and z images of the row (code yz, see shift_of) and the minimum image in
+// x.  A candidate near SearchLength is less than half the box away in x, so
+// that image is the one it was staged for; it must also lie in cells cx - 1
+// .. cx + 1 as the reference's search sees them, which a walk past the lane's
+// own window does not promise.
+static __device__ __noinline__ bool band_test_row(const RowGeom &g, const double4 *__restrict__ q, int i, int j, int cx,
+                                           int yz) {
+  const double4 qi = q[i], qj = q[j];
+  const double t = qj.x - qi.x;
+  const int xc = t > 0.5 * g.L[0] ? 1 : (t < -0.5 * g.L[0] ? 2 : 0);
+  const int cj = cell_coord(qj.x, g.inv_cs0, g.ms[0]) + (xc == 1 ? -g.ms[0] : (xc == 2 ? g.ms[0] : 0));
+  if (cj < cx - 1 || cj > cx + 1) return false;
+  return within_search_exact(qi, qj, shift_of(xc, 0, g.L), shift_of(yz, 1, g.L), shift_of(yz, 2, g.L), g.sl2);
+}
+
+// The full Verlet rows of a warp's 32 atoms, one lane each: build_rows' rows
+// entry for entry (the same 9 runs of slots in the same order, the same FP32
+// prefilter, ghost-existence rule and exact test of the band).  All 32 lanes
+// call; lanes without an atom pass active = false and any valid slot i.
+// owner tells lanes of different systems apart.
+//
+// build_rows is bound by the L1 data path, its latency and its branches: every
+// lane loads its own candidates (32 addresses a load, two thirds of the lanes
+// busy), about 38 instructions a candidate, and files each partner with a
+// scattered 4-byte store.  Here the lanes of one x-row of cells walk together
+// (slots are in cell order, so a warp's atoms are of one x-row, or of a few,
+// which take turns):
+// - the run of slots that their windows cover is staged in shared memory by
+//   coalesced loads, already moved through the x face where the run wraps,
+//   with the images that the reference never builds put out of reach, so the
+//   walk tests neither;
+// - every lane walks as many candidates as the longest window, from its own
+//   window's start: candidates outside the window lie out of reach in x and
+//   fail the test, so the walk has no bound to test; four consecutive lanes of
+//   one cell walk the union of their windows and read one address;
+// - packed FP32 instructions take two candidates, and a candidate's verdict
+//   is the sign of r^2 - hi shifted into a word: 8 instructions a candidate
+//   and no branch.  Words with a candidate in the band (the sign of
+//   (r^2 - hi)(r^2 - lo)) take the exact test for all their partners;
+// - the words are turned into entries at the end, all lanes at the same
+//   entry, so that 32 stores fill a 128-byte line of the list.
+// On the 256,000-atom liquid the kernel takes 152 us against 235 us (300
+// warp instructions an atom against 470, issue 65% against 57%); a rebuild of
+// the 2.05M-atom liquid 1.13 ms against 2.05 ms.  64 registers (32 warps an
+// SM, a few spills outside the walk) against 80: 1.13 and 1.17 ms; partners
+// filed one by one in a shared-memory ring instead of words: 1.6 ms.
+template <bool SLAB>
+__device__ __forceinline__ int build_rows_warp(const RowGeom &g, const float4 *__restrict__ qloc,
+                                               const double4 *__restrict__ q, const int *__restrict__ tab, int owner,
+                                               int pc, int i, bool active, WarpRows &sm, int *__restrict__ nbr,
+                                               int stride, int maxnb) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int kNoSlot = 1 << 30;  // above every slot; differences with slots stay in range
+  const int lane = threadIdx.x & 31;
+  const float4 li = qloc[i];
+  const int cx = pc & 2047;
+  const int mx = g.ms[0] * kXSub, vbase = (cx - 1) * kXSub;
+  // x_i in sub-bins from the lower face of cell cx - 1
+  const double qx = q[i].x;
+  const double per_bin = kXSub / g.cs0;
+  const float ubin = (float)((qx - (cx - 1) * g.cs0) * per_bin), per_binf = (float)per_bin;
+  const float2 bx = make_float2((float)(-qx), (float)(-qx));
+  // lanes 4k .. 4k + 3 of one cell of one system
+  const int key = active ? pc : -1;  // no packed cell is -1
+  const int k1 = __shfl_xor_sync(kAll, key, 1), k2 = __shfl_xor_sync(kAll, key, 2);
+  const int o1 = __shfl_xor_sync(kAll, owner, 1), o2 = __shfl_xor_sync(kAll, owner, 2);
+  const int s1 = active && key == k1 && owner == o1, s2 = active && key == k2 && owner == o2;
+  const int s12 = __shfl_xor_sync(kAll, s1, 2);  // the other pair's
+  const bool quad = s1 && s2 && s12;
+  int cnt = 0;  // entries in the list
+
+  // one turn per x-row of cells among the lanes' atoms
+  for (unsigned left = __ballot_sync(kAll, active); left;) {
+    const int lead = __ffs(left) - 1;
+    const unsigned row = (unsigned)__shfl_sync(kAll, pc, lead) >> 11;
+    const int row_owner = __shfl_sync(kAll, owner, lead);
+    const bool on = active && ((unsigned)pc >> 11) == row && owner == row_owner;
+    left &= ~__ballot_sync(kAll, on);
+    // a candidate is kept when r^2 - hi < 0: never on the other lanes
+    const float2 nhi = on ? make_float2(-g.hi, -g.hi) : make_float2(1.f, 1.f);
+    const float2 nlo = on ? make_float2(-g.lo, -g.lo) : make_float2(1.f, 1.f);
+    const int cy = (int)(row & 2047u), lz = (int)(row >> 11);
+    // the row's geometry, from the turn's own lanes
+    const int ms1 = __shfl_sync(kAll, g.ms[1], lead), ms2 = __shfl_sync(kAll, g.ms[2], lead);
+    const int rmx = __shfl_sync(kAll, mx, lead);
+    const float Lx = __shfl_sync(kAll, (float)g.L[0], lead);
+    const int *rtab = (const int *)__shfl_sync(kAll, (unsigned long long)tab, lead);
+    const int cz = SLAB ? g.z0 + lz : lz;  // global layer
+    int nw = 0, fresh = 0;                 // the lane's words, and the partners in them
+
+    // the words' partners into the list
+    auto flush = [&]() {
+      const int mine = min(fresh, maxnb - cnt), n = __reduce_max_sync(kAll, mine);
+      int *dst = nbr + (size_t)cnt * stride + i;
+      const uint2 *w = &sm.word[0][lane];
+      uint2 m = make_uint2(0u, 0u);
+      for (int t = 0; t < n; t++, dst += stride) {
+        if (t < mine) {
+          if (m.x == 0u) {  // the next word (none is empty)
+            m = *w;
+            w += 32;
+          }
+          const int b = __clz(m.x);
+          *dst = (int)m.y + b;
+          m.x ^= 0x80000000u >> b;
+        }
+      }
+      cnt += fresh;
+      nw = fresh = 0;
+    };
+
+#pragma unroll 1
+    for (int r = 0; r < 9; r++) {
+      const int dz = r / 3 - 1, dy = r % 3 - 1;
+      int z = cz + dz, y = cy + dy, yz = 0;  // yz: the run's image shift along y and z (shift_of's code)
+      if (z < 0) { z += ms2; yz = 1 << 4; } else if (z >= ms2) { z -= ms2; yz = 2 << 4; }
+      if (y < 0) { y += ms1; yz |= 1 << 2; } else if (y >= ms1) { y -= ms1; yz |= 2 << 2; }
+      int blk = z;
+      if (SLAB) {
+        const int nl = lz + dz;
+        blk = nl < 0 ? g.nzl : (nl >= g.nzl ? g.nzl + 1 : nl);
+      }
+      // the lane's window [wl, wh) in sub-bins of the 3 kXSub bins of cells
+      // cx - 1 .. cx + 1 (build_rows' windows; empty when out of reach)
+      const float gz = dz == 0 ? 0.f : (dz < 0 ? li.z : g.csz - li.z);
+      const float gy = dy == 0 ? 0.f : (dy < 0 ? li.y : g.csy - li.y);
+      const float g2 = fmaf(gy, gy, gz * gz);
+      const float reach = sqrt_approx(fmaxf(g.hi - g2, 0.f)) * per_binf;
+      const bool out = !on || g2 > g.hi;
+      int wl = out ? 3 * kXSub : max((int)floorf(ubin - reach - 1e-3f), 0);
+      int wh = out ? 0 : min((int)floorf(ubin + reach + 1e-3f) + 1, 3 * kXSub);
+#pragma unroll
+      for (int o = 1; o <= 2; o <<= 1) {
+        const int lo2 = __shfl_xor_sync(kAll, wl, o), hi2 = __shfl_xor_sync(kAll, wh, o);
+        if (quad) {
+          wl = min(wl, lo2);
+          wh = max(wh, hi2);
+        }
+      }
+      // as slots [e0, e1) of the row continued through its x faces: slots
+      // below x0 are those of the row's end (image shift -L), slots from x1
+      // on those of its start (+L)
+      const int *xr = rtab + (size_t)(blk * ms1 + y) * (rmx + 1);
+      const int x0 = xr[0], x1 = xr[rmx], nrow = x1 - x0;
+      int e0 = kNoSlot, e1 = -kNoSlot;
+      if (wl < wh) {
+        const int b0 = vbase + wl, b1 = vbase + wh;
+        e0 = b0 < 0 ? xr[b0 + rmx] - nrow : xr[b0];
+        e1 = b1 > rmx ? xr[b1 - rmx] + nrow : xr[b1];
+        if (e0 >= e1) {
+          e0 = kNoSlot;
+          e1 = -kNoSlot;
+        }
+      }
+      const int c0 = __reduce_min_sync(kAll, e0), c1 = __reduce_max_sync(kAll, e1);
+      const bool wraps = c0 < x0 || c1 > x1, plain = !wraps && yz == 0;
+      const float byf = (float)dy * g.csy - li.y, bzf = (float)dz * g.csz - li.z;
+      const float2 by = make_float2(byf, byf), bz = make_float2(bzf, bzf);
+      for (int c = c0; c < c1; c += kRunStage) {
+        const int total = min(c1 - c, kRunStage);
+        __syncwarp();  // the last walk has read the stage
+        if (plain) {
+          for (int t = 2 * lane; t < ((total + 3) & ~3); t += 64) {
+            const float4 *p = qloc + c + t;
+            float4 l0 = make_float4(1e18f, 0.f, 0.f, 0.f), l1 = l0;
+            if (t < total) l0 = __ldg(p);
+            if (t + 1 < total) l1 = __ldg(p + 1);
+            sm.xy[t >> 1] = make_float4(l0.x, l1.x, l0.y, l1.y);
+            sm.zz[t >> 1] = make_float2(l0.z, l1.z);
+          }
+        } else {
+          for (int t = 2 * lane; t < ((total + 3) & ~3); t += 64) {
+            float4 p[2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+              p[u] = make_float4(1e18f, 0.f, 0.f, 0.f);
+              if (t + u < total) {
+                int s = c + t + u, code = yz;
+                float sx = 0.f;
+                if (s < x0) {
+                  s += nrow;
+                  sx = -Lx;
+                  code |= 1;
+                } else if (s >= x1) {
+                  s -= nrow;
+                  sx = Lx;
+                  code |= 2;
+                }
+                const int need = strips_of(code);
+                p[u] = __ldg(qloc + s);
+                p[u].x = (__float_as_int(p[u].w) & need) == need ? p[u].x + sx : 1e18f;
+              }
+            }
+            sm.xy[t >> 1] = make_float4(p[0].x, p[1].x, p[0].y, p[1].y);
+            sm.zz[t >> 1] = make_float2(p[0].z, p[1].z);
+          }
+        }
+        __syncwarp();
+        // the lane's part of the stage, from an even candidate; the longest
+        // one sets the warp's walk, and starts move down to end in the stage
+        const int f0 = max(e0, c), f1 = min(e1, c + total);
+        int st = f0 < f1 ? (f0 - c) & ~1 : 0;
+        const int trip = (__reduce_max_sync(kAll, f0 < f1 ? f1 - c - st : 0) + 3) & ~3;
+        st = min(st, ((total + 3) & ~3) - trip);
+        const float4 *pxy = sm.xy + (st >> 1);
+        const float2 *pzz = sm.zz + (st >> 1);
+        for (int k = 0; k < trip; k += 32, st += 32) {
+          unsigned m = 0u, band = 0u;
+          const int kn = min(trip - k, 32);
+#pragma unroll 2
+          for (int u = 0; u < kn; u += 4, pxy += 2, pzz += 2) {
+            const float4 a0 = pxy[0], a1 = pxy[1];
+            const float2 z0 = pzz[0], z1 = pzz[1];
+            const float2 ex0 = __fadd2_rn(make_float2(a0.x, a0.y), bx), ey0 = __fadd2_rn(make_float2(a0.z, a0.w), by);
+            const float2 ex1 = __fadd2_rn(make_float2(a1.x, a1.y), bx), ey1 = __fadd2_rn(make_float2(a1.z, a1.w), by);
+            const float2 ez0 = __fadd2_rn(z0, bz), ez1 = __fadd2_rn(z1, bz);
+            const float2 r0 = __ffma2_rn(ex0, ex0, __ffma2_rn(ey0, ey0, __fmul2_rn(ez0, ez0)));
+            const float2 r1 = __ffma2_rn(ex1, ex1, __ffma2_rn(ey1, ey1, __fmul2_rn(ez1, ez1)));
+            const float2 h0 = __fadd2_rn(r0, nhi), h1 = __fadd2_rn(r1, nhi);
+            const float2 b0 = __fmul2_rn(h0, __fadd2_rn(r0, nlo)), b1 = __fmul2_rn(h1, __fadd2_rn(r1, nlo));
+            m = __funnelshift_l(__float_as_uint(h0.x), m, 1);
+            m = __funnelshift_l(__float_as_uint(h0.y), m, 1);
+            m = __funnelshift_l(__float_as_uint(h1.x), m, 1);
+            m = __funnelshift_l(__float_as_uint(h1.y), m, 1);
+            band |= __float_as_uint(b0.x) | __float_as_uint(b0.y);
+            band |= __float_as_uint(b1.x) | __float_as_uint(b1.y);
+          }
+          m <<= 32 - kn;
+          const int first = c + st;  // virtual slot of bit 31
+          const int self = i - first;
+          if (r == 4 && self >= 0 && self < 32) m &= ~(0x80000000u >> self);
+          if (__any_sync(kAll, (int)(band & 0x80000000u))) {
+            // some candidate of some lane in the band: exact test of that
+            // lane's partners
+            if (band >> 31)
+              for (unsigned left2 = m; left2;) {
+                const int b = __clz(left2);
+                left2 &= ~(0x80000000u >> b);
+                int s = first + b;
+                s += s < x0 ? nrow : (s >= x1 ? -nrow : 0);
+                if (!band_test_row(g, q, i, s, cx, yz)) m &= ~(0x80000000u >> b);
+              }
+          }
+          if (!wraps) {
+            if (m) sm.word[nw++][lane] = make_uint2(m, (unsigned)first);
+          } else {
+            // the run wraps: the slots before, in and after the row in words
+            // of their own
+            const int h0 = x0 - first, h1 = x1 - first;
+            const unsigned lt0 = h0 <= 0 ? 0u : (h0 >= 32 ? 0xffffffffu : ~(0xffffffffu >> h0));
+            const unsigned lt1 = h1 <= 0 ? 0u : (h1 >= 32 ? 0xffffffffu : ~(0xffffffffu >> h1));
+            if (m & lt0) sm.word[nw++][lane] = make_uint2(m & lt0, (unsigned)(first + nrow));
+            if (m & lt1 & ~lt0) sm.word[nw++][lane] = make_uint2(m & lt1 & ~lt0, (unsigned)first);
+            if (m & ~lt1) sm.word[nw++][lane] = make_uint2(m & ~lt1, (unsigned)(first - nrow));
+          }
+          fresh += __popc(m);
+          if (__any_sync(kAll, nw > kRowWords - 3)) flush();
+        }
+      }
+    }
+    flush();
+    // padded with the atom itself to a multiple of 4
+    if (on)
+      for (int k = cnt; (k & 3) && k < maxnb; k++) nbr[(size_t)k * stride + i] = i;
   }
   return cnt;
 }
@@ -1196,19 +1490,48 @@ __device__ __forceinline__ int stage_shift_atom(const int4 *plan, int npl, int j
   return plan[lo].w - plan[lo].z;
 }
 
-// Rebuild 6/6: full Verlet list, one thread per atom (build_rows).  Each
+// Longest row and list entries of a warp's atoms (cnt: a lane's row, 0 for
+// none).  All lanes must call.
+__device__ __forceinline__ void count_rows(Status *st, int cnt) {
+  const int wmax = __reduce_max_sync(0xffffffffu, cnt);
+  const int wsum = __reduce_add_sync(0xffffffffu, cnt);
+  if ((threadIdx.x & 31) == 0 && wsum) {
+    atomicMax(&st->max_row, wmax);
+    atomicAdd((unsigned long long *)&st->list_entries, (unsigned long long)wsum);
+  }
+}
+
+// Rebuild 6/6: full Verlet list, one thread per atom (build_rows_warp) or
+// BTPA of them (build_rows; also the rows that carry stage indices).  Each
 // candidate is first tested in FP32; only candidates whose FP32 r^2 falls in
 // a band around SearchLength^2 -- wider than the FP32 error bound, which
 // mdg_create derives from the box -- are decided by the exact FP64 test, so
 // the pair set is the reference's bit for bit.  Rows are padded with the
 // atom's own index to a multiple of 4.
 template <int BLOCK, bool STAGE, bool SLAB = false, int BTPA = 1>
-__global__ void __launch_bounds__(BLOCK) k_build(Arrays a, Box b, int n) {
-  static_assert(!(STAGE && SLAB), "staged rows are single-domain only");
+__global__ void __launch_bounds__(BLOCK, !STAGE && BTPA == 1 ? 1024 / BLOCK : 0) k_build(Arrays a, Box b, int n) {
+  static_assert(!SLAB || (!STAGE && BTPA == 1), "slabs: one lane per atom, rows not staged");
   static_assert(!STAGE || BTPA == 1, "staged rows are built one lane per atom");
   const int t = blockIdx.x * BLOCK + threadIdx.x;
   const int i = t / BTPA, sub = t % BTPA;
   int cnt = 0;
+  if (!STAGE && BTPA == 1) {
+    __shared__ WarpRows rows[STAGE || BTPA > 1 ? 1 : BLOCK / 32];
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    // the lanes of a warp walk together: they agree on the error flag
+    if (t - l < n && !warp_error(a.st)) {
+      const bool active = i < n;
+      const int ii = active ? i : n - 1;
+      cnt = build_rows_warp<SLAB>(row_geom(b), a.qloc, a.q, a.xsub, 0, a.cxyz[ii], ii, active, rows[w], a.nbr, a.stride,
+                                  a.maxnb);
+      if (active) {
+        a.nnbr[i] = min(cnt, a.maxnb);
+        if (cnt > a.maxnb) atomicOr(&a.st->error, kErrCapacity);
+      }
+    }
+    count_rows(a.st, cnt);
+    return;
+  }
   // STAGE: also the rows as stage indices (FP32-mixed staged force), from
   // the block's stage plan, see k_stage_plan
   __shared__ int4 plan[STAGE ? kStageRanges : 1];
@@ -1255,7 +1578,7 @@ __global__ void __launch_bounds__(BLOCK) k_build(Arrays a, Box b, int n) {
         stage_entry(a.nbr16, stride, i, k, v, g0, g1);
       }
     };
-    cnt = build_rows<SLAB, BTPA>(b, a.qloc, a.q, a.mult, a.xsub, a.cxyz[i], i, emit);
+    cnt = build_rows<BTPA>(b, a.qloc, a.q, a.mult, a.xsub, a.cxyz[i], i, emit);
     if (sub == 0) a.nnbr[i] = min(cnt, maxnb);
     if (cnt > maxnb) {
       if (sub == 0) atomicOr(&a.st->error, kErrCapacity);
@@ -1272,12 +1595,7 @@ __global__ void __launch_bounds__(BLOCK) k_build(Arrays a, Box b, int n) {
     }
   }
   if (sub != 0) cnt = 0;  // the atom's row is counted once
-  const int wmax = __reduce_max_sync(0xffffffffu, cnt);
-  const int wsum = __reduce_add_sync(0xffffffffu, cnt);
-  if ((threadIdx.x & 31) == 0 && wsum) {
-    atomicMax(&a.st->max_row, wmax);
-    atomicAdd((unsigned long long *)&a.st->list_entries, (unsigned long long)wsum);
-  }
+  count_rows(a.st, cnt);
 }
 
 // Before a build: clear the build counters.
@@ -1899,13 +2217,6 @@ __device__ __forceinline__ void fp32_row_global(const Arrays &a, const Box &b, c
   Fx += (double)fx;  // the last chunk when it holds one group (else +0)
   Fy += (double)fy;
   Fz += (double)fz;
-}
-
-// The error flag as one lane of the warp read it: the lanes of an atom must
-// agree on whether they take its row (they exchange values), and the flag
-// can be raised by another block at any time.  All lanes must call.
-__device__ __forceinline__ int warp_error(const Status *st) {
-  return __shfl_sync(0xffffffffu, *(volatile const int *)&st->error, 0);
 }
 
 // Sum of one value per atom over a block's BLOCK / TPA atoms (consecutive

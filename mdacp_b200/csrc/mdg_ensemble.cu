@@ -163,6 +163,18 @@ __device__ __forceinline__ void rep_add(long long *slot_base, size_t stride_byte
   }
 }
 
+// Longest row into the replica's status, one atomic per warp as rep_max.
+__device__ __forceinline__ void rep_max_row(const Ens &e, int r, int cnt, bool active) {
+  const int rr = active ? r : -1;
+  const int r0 = __shfl_sync(0xffffffffu, rr, 0);
+  if (__all_sync(0xffffffffu, rr == r0) && r0 >= 0) {
+    const int m = __reduce_max_sync(0xffffffffu, cnt);
+    if ((threadIdx.x & 31) == 0) atomicMax(&e.rs[r0].max_row, m);
+  } else if (active) {
+    atomicMax(&e.rs[r].max_row, cnt);
+  }
+}
+
 // Index k of the work-list replica that holds work item g (the largest k
 // with prefix[k] <= g; nk >= 1).
 __device__ __forceinline__ int work_find(const int *prefix, int nk, int g) {
@@ -478,10 +490,12 @@ __device__ __forceinline__ int permute_atom(const Ens &e, int r, int s) {
   e.q_old[s] = q;
   const double x[3] = {q.x, q.y, q.z};
   int m = 1;
-  e.mult[s] = (unsigned char)border_bits(x, b, &m);
+  const int strips = border_bits(x, b, &m);
+  e.mult[s] = (unsigned char)strips;
   const int c = cg - rep.cell_off;
   const int cx = c % rep.ms[0], cy = (c / rep.ms[0]) % rep.ms[1], cz = c / (rep.ms[0] * rep.ms[1]);
-  e.qloc[s] = make_float4((float)q.x, (float)(q.y - cy * rep.cs[1]), (float)(q.z - cz * rep.cs[2]), 0.f);
+  e.qloc[s] = make_float4((float)q.x, (float)(q.y - cy * rep.cs[1]), (float)(q.z - cz * rep.cs[2]),
+                          __int_as_float(strips));
   e.cxyz[s] = pack_cell(cx, cy, cz);
   return m;
 }
@@ -513,21 +527,44 @@ __global__ void __launch_bounds__(kEB) ke_copy_back(Ens e) {
   }
 }
 
-// One atom's row of the list build, as the single-system build makes it
-// (build_rows: same rows in the same order); all-pairs with the minimum
-// image for small replicas.  Returns the entries kept.
-__device__ __forceinline__ int ens_build_row(const Ens &e, int i) {
-  const int r = e.rep_of[i];
-  RepStatus &st = e.rs[r];
-  const Rep rep = e.rep[r];
+// Row of atom i of a small replica (an axis shorter than three cells): every
+// other atom of the replica in slot order, through its minimum image (unique:
+// L > 2 SearchLength).  An FP32 minimum image on the prefilter coordinates
+// (which are box coordinates here, the replica being one cell) drops the far
+// atoms; its band is 1e-4 SL^2 plus the rounding of coordinates up to the
+// box lengths (each of the three differences is off by less than 4 u L, u =
+// 2^-24, and 2 SL of that reaches r^2).  The others take the exact test.
+// Returns the entries found.  Four candidates are loaded at a time; the FP64
+// test of every candidate that this replaced took 74 us for 24 replicas of up to
+// 3,000 atoms on a B200 (one block's lanes walk 500 candidates each, so the
+// launch waits for that chain).
+__device__ __forceinline__ int small_row(const Ens &e, const Rep &rep, int i) {
   const int maxnb = e.maxnb, stride = e.stride;
+  const double4 qi = e.q[i];
+  const float4 li = e.qloc[i];
+  const float lx = (float)rep.L[0], ly = (float)rep.L[1], lz = (float)rep.L[2];
+  const float ix = 1.f / lx, iy = 1.f / ly, iz = 1.f / lz;
+  const float hi = (float)(rep.sl2 * 1.0001 + 16.0 / 16777216.0 * (rep.L[0] + rep.L[1] + rep.L[2]) * rep.sl);
+  const int end = rep.atom_off + rep.n;
   int cnt = 0;
-  if (rep.small) {
-    const double4 qi = e.q[i];
-    for (int j = rep.atom_off; j < rep.atom_off + rep.n; j++) {
-      if (j == i) continue;
+  for (int j0 = rep.atom_off; j0 < end; j0 += 4) {
+    float4 l[4];
+    bool near[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) l[u] = e.qloc[min(j0 + u, end - 1)];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      float dx = l[u].x - li.x, dy = l[u].y - li.y, dz = l[u].z - li.z;
+      dx = fmaf(-lx, rintf(dx * ix), dx);
+      dy = fmaf(-ly, rintf(dy * iy), dy);
+      dz = fmaf(-lz, rintf(dz * iz), dz);
+      near[u] = j0 + u < end && j0 + u != i && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= hi;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (!near[u]) continue;
+      const int j = j0 + u;
       const double4 qj = e.q[j];
-      // the minimum-image shift per axis (unique: L > 2 SearchLength)
       const double tx = qj.x - qi.x, ty = qj.y - qi.y, tz = qj.z - qi.z;
       const double sx = tx > rep.hL[0] ? -rep.L[0] : (tx < -rep.hL[0] ? rep.L[0] : 0.0);
       const double sy = ty > rep.hL[1] ? -rep.L[1] : (ty < -rep.hL[1] ? rep.L[1] : 0.0);
@@ -538,31 +575,42 @@ __device__ __forceinline__ int ens_build_row(const Ens &e, int i) {
       if (cnt < maxnb) e.nbr[(size_t)cnt * stride + i] = j;
       cnt++;
     }
-  } else {
-    auto emit = [&](int j, int k) {
-      if (k < maxnb) e.nbr[(size_t)k * stride + i] = j;
-    };
-    // without the load pipeline: it takes ke_build from 72 to 152 registers
-    cnt = build_rows<false, 1, false>(box_of(e, rep), e.qloc, e.q, e.mult, e.xsub + rep.tab_off, e.cxyz[i], i, emit);
   }
-  e.nnbr[i] = min(cnt, maxnb);
-  if (cnt > maxnb) {
-    atomicOr(e.error, kErrCapacity);
-  } else {
-    for (int k = cnt; k < ((cnt + 3) & ~3); k++) e.nbr[(size_t)k * stride + i] = i;
-  }
-  atomicMax(&st.max_row, cnt);
-  return min(cnt, maxnb);
+  for (int k = cnt; k < ((cnt + 3) & ~3) && k < maxnb; k++) e.nbr[(size_t)k * stride + i] = i;
+  return cnt;
 }
 
-__global__ void __launch_bounds__(kEF) ke_build(Ens e) {
+// Rows of the rebuilding replicas' atoms (rebuild work list), as the
+// single-system build makes them (build_rows_warp; small_row for replicas
+// narrower than three cells); a warp's 32 atoms may belong to several
+// replicas.  Block-uniform sweeps, so every lane reaches the warp's votes.
+__global__ void __launch_bounds__(kEF, 768 / kEF) ke_build(Ens e) {
+  __shared__ WarpRows rows[kEF / 32];
+  const int w = threadIdx.x >> 5;
   const int total = e.wb.count[1];
+  if (total == 0 || __shfl_sync(0xffffffffu, *(volatile const int *)e.error, 0)) return;
   for (int base = blockIdx.x * kEF; base < total; base += gridDim.x * kEF) {
     const int g = base + threadIdx.x;
-    const bool active = g < total && !*e.error;
-    int r = 0, kept = 0;
-    if (active) kept = ens_build_row(e, work_atom(e, e.wb, g, &r));
-    rep_add(&e.rs[0].list_entries, sizeof(RepStatus), r, kept, active);
+    if (base + w * 32 >= total) return;  // whole warps leave together
+    const bool active = g < total;
+    int r = 0;
+    const int i = work_atom(e, e.wb, min(g, total - 1), &r);
+    const Rep &rep = e.rep[r];
+    const bool cells = active && !rep.small;
+    int cnt = 0;
+    if (__any_sync(0xffffffffu, cells)) {
+      const RowGeom geom{{rep.L[0], rep.L[1], rep.L[2]}, rep.cs[0], rep.inv_cs[0], rep.sl2, (float)rep.cs[1],
+                         (float)rep.cs[2], rep.sl2_lo, rep.sl2_hi, {rep.ms[0], rep.ms[1], rep.ms[2]}, 0, rep.ms[2]};
+      cnt = build_rows_warp<false>(geom, e.qloc, e.q, e.xsub + rep.tab_off, r, e.cxyz[i], i, cells, rows[w], e.nbr,
+                                   e.stride, e.maxnb);
+    }
+    if (active && rep.small) cnt = small_row(e, rep, i);
+    if (active) {
+      e.nnbr[i] = min(cnt, e.maxnb);
+      if (cnt > e.maxnb) atomicOr(e.error, kErrCapacity);
+    }
+    rep_max_row(e, r, cnt, active);
+    rep_add(&e.rs[0].list_entries, sizeof(RepStatus), r, min(cnt, e.maxnb), active);
   }
 }
 
