@@ -148,7 +148,7 @@ cudaError_t dalloc(T **p, size_t count) {
 }
 
 void free_arrays(Arrays &a) {
-  void *ptrs[] = {a.q, a.v, a.q_old, a.qfix, a.qfix2, a.qloc, a.cxyz, a.xsub, a.ids, a.type, a.cell, a.nbr, a.nnbr, a.cell_count,
+  void *ptrs[] = {a.q, a.v, a.q_old, a.qfix, a.qfix2, a.pz, a.pz2, a.qloc, a.cxyz, a.xsub, a.ids, a.type, a.cell, a.nbr, a.nnbr, a.cell_count,
                   a.cell_start, a.slot, a.perm, a.perm2, a.q_tmp, a.v_tmp, a.v_lag, a.ids_tmp, a.type_tmp,
                   a.cell_tmp, a.mult, a.cand, a.partials, a.st, a.stage_rng, a.stage_n, a.nbr16, a.disp2};
   for (void *p : ptrs)
@@ -255,6 +255,10 @@ double step_lag(const mdg_handle *h) {
 // Pairlist rebuild (MDManager::MakePairList).
 // pack: where to put the coming step's first-drift positions after the
 // rebuild (the fused FP32 NVE step), or nullptr.
+int4 *fix_buffer(mdg_handle *h, int k) { return k ? h->a.qfix2 : h->a.qfix; }
+// The z array of a packed copy (null: fixed-point).
+double *fix_z(const mdg_handle *h, const int4 *buf) { return buf == h->a.qfix2 ? h->a.pz2 : h->a.pz; }
+
 // Kernels of one rebuild (launch_build).
 int build_kernels(const mdg_handle *h) { return (h->ncell <= kScanSingleCells ? 9 : 11) + (h->a.stage_cap > 0 ? 1 : 0); }
 
@@ -291,7 +295,7 @@ void launch_build(mdg_handle *h, cudaStream_t s, int4 *pack = nullptr) {
   }
   k_scatter<kBlock><<<blocks_for(n, kBlock), kBlock, 0, s>>>(a, n);
   k_sort_cells<<<blocks_for(h->ncell * 32, kBlock), kBlock, 0, s>>>(a, h->box, h->ncell);
-  k_permute<kBlock><<<blocks_for(n, kBlock), kBlock, 0, s>>>(a, h->box, n, pack);
+  k_permute<kBlock><<<blocks_for(n, kBlock), kBlock, 0, s>>>(a, h->box, n, pack, pack ? fix_z(h, pack) : nullptr);
   k_copy_back<kBlock><<<blocks_for(n, kBlock), kBlock, 0, s>>>(a, n);
   if (a.stage_cap > 0) {
     static_assert(kForceBlock == kStageBlock, "the build writes stage rows per force block");
@@ -303,12 +307,9 @@ void launch_build(mdg_handle *h, cudaStream_t s, int4 *pack = nullptr) {
   k_build_done<<<1, 32, 0, s>>>(a, h->box);
 }
 
-// The FP32-mixed NVE step runs as one force pass per step (both half
-// drifts fused, the next step's fixed-point copy packed into the other
-// buffer).
-bool fused_step(const mdg_handle *h) {
-  return h->prm.precision == MDG_FP32_MIXED && h->prm.thermostat == MDG_NVE && h->ext.kind == 0;
-}
+// The NVE step runs as one force pass per step (both half drifts fused, the
+// next step's positions packed into the other buffer).
+bool fused_step(const mdg_handle *h) { return h->prm.thermostat == MDG_NVE && h->ext.kind == 0; }
 
 // The executor pass after a step (nothing when none is set); returns kernels.
 int launch_external(mdg_handle *h, cudaStream_t s) {
@@ -320,7 +321,6 @@ int launch_external(mdg_handle *h, cudaStream_t s) {
   return 3;
 }
 
-int4 *fix_buffer(mdg_handle *h, int k) { return k ? h->a.qfix2 : h->a.qfix; }
 
 // Dynamic shared memory of every staged force instantiation.
 template <int MODE>
@@ -362,9 +362,31 @@ void launch_fp32(mdg_handle *h, cudaStream_t s, const Thermo &th, int drift, con
     k_force_fp32<kThreads, MODE, 0, TPA><<<nb, kThreads, 0, s>>>(h->a, h->box, n, th, qf, nullptr);
 }
 
+int fp64_blocks(int n) { return blocks_for(n * fp64_lanes(n), kForceBlock); }
+
+template <int MODE, int TPA>
+void launch_fp64(mdg_handle *h, cudaStream_t s, const Thermo &th, int drift, const int4 *qf, int4 *qf_next) {
+  const int n = h->n, nb = fp64_blocks(n);
+  const PosSplit pos{reinterpret_cast<const double2 *>(qf), fix_z(h, qf)};
+  if constexpr (MODE == kKick) {
+    if (drift == 2) {
+      k_force_fp64<kForceBlock, MODE, 2, TPA><<<nb, kForceBlock, 0, s>>>(h->a, h->box, n, th, pos, qf_next,
+                                                                          fix_z(h, qf_next));
+      return;
+    }
+  }
+  if constexpr (MODE == kKick || MODE == kKickNoseHoover) {
+    if (drift) {
+      k_force_fp64<kForceBlock, MODE, 1, TPA><<<nb, kForceBlock, 0, s>>>(h->a, h->box, n, th, pos, nullptr, nullptr);
+      return;
+    }
+  }
+  k_force_fp64<kForceBlock, MODE, 0, TPA><<<nb, kForceBlock, 0, s>>>(h->a, h->box, n, th, pos, nullptr, nullptr);
+}
+
 // drift: 1 also applies the second half drift in the same pass, 2 the whole
-// fused NVE step reading qf and packing into qf_next (FP32-mixed only);
-// returns false when the caller still has to launch the second drift.
+// fused NVE step reading qf and packing into qf_next; returns whether the
+// second drift was made.
 template <int MODE>
 bool launch_force_mode(mdg_handle *h, cudaStream_t s, const Thermo &th, int drift = 0, const int4 *qf = nullptr,
                        int4 *qf_next = nullptr) {
@@ -388,8 +410,12 @@ bool launch_force_mode(mdg_handle *h, cudaStream_t s, const Thermo &th, int drif
     else launch_fp32<MODE, 1>(h, s, th, drift, qf, qf_next);
     return drift != 0;
   }
-  k_force_fp64<kForceBlock, MODE><<<nb, kForceBlock, 0, s>>>(h->a, h->box, n, th);
-  return false;
+  switch (fp64_lanes(n)) {
+    case 8: launch_fp64<MODE, 8>(h, s, th, drift, qf, qf_next); break;
+    case 4: launch_fp64<MODE, 4>(h, s, th, drift, qf, qf_next); break;
+    default: launch_fp64<MODE, 1>(h, s, th, drift, qf, qf_next);
+  }
+  return drift != 0;
 }
 
 Thermo thermo_of(const mdg_handle *h) {
@@ -430,7 +456,7 @@ int launch_step_tail(mdg_handle *h, cudaStream_t s, cudaEvent_t ev_start, cudaEv
     rec(ev_stop);
     return 1;
   }
-  launch_drift(h, s, fix, 0);
+  launch_drift(h, s, true, 0);
   launches++;
   if (h->prm.thermostat == MDG_NOSE_HOOVER) {
     const int nbk = blocks_for(n, kBlock);
@@ -440,7 +466,7 @@ int launch_step_tail(mdg_handle *h, cudaStream_t s, cudaEvent_t ev_start, cudaEv
     // the second drift does not read zeta, so it may precede the zeta update
     const bool drifted = launch_force_mode<kKickNoseHoover>(h, s, th, 1);
     rec(ev_stop);
-    k_zeta<1024><<<1, 1024, 0, s>>>(h->a, h->box, blocks_for(n, kForceBlock), n,
+    k_zeta<1024><<<1, 1024, 0, s>>>(h->a, h->box, fix ? blocks_for(n, kForceBlock) : fp64_blocks(n), n,
                                      h->prm.aimed_temperature, h->prm.heatbath_tau);
     launches += 4;
     if (!drifted) {
@@ -791,7 +817,8 @@ int persistent_grid(mdg_handle *h) {
 bool use_persistent(mdg_handle *h) {
   // the staged force pass (stage_atoms) runs as graph steps: the persistent
   // pass gathers from global memory
-  if (!fused_step(h) || h->prm.step_mode == MDG_STEPS_GRAPHS || h->a.stage_cap > 0) return false;
+  if (!fused_step(h) || h->prm.precision != MDG_FP32_MIXED || h->prm.step_mode == MDG_STEPS_GRAPHS || h->a.stage_cap > 0)
+    return false;
   const int tpa = persistent_tpa(h);
   const int g = persistent_grid(h);
   if (g <= 0) return false;
@@ -859,7 +886,7 @@ mdg_status build_rebuild_graph(mdg_handle *h) {
 mdg_status run_persistent(mdg_handle *h, long long target, Status *st) {
   mdg_status r;
   if (h->fix_buf < 0) {
-    k_pack_half<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n, h->a.qfix);
+    k_pack_half<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n, h->a.qfix, h->a.pz);
     h->kernel_launches++;
     h->fix_buf = 0;
   }
@@ -986,12 +1013,14 @@ mdg_status mdg_create(const mdg_params *prm, mdg_handle **out) {
   const int cap = h->cap;
   a.stride = (cap + 31) / 32 * 32;
   a.maxnb = 0;
-  h->partial_cap = (size_t)blocks_for(cap, kForceBlock) * 3 + 64;
+  h->partial_cap = (size_t)blocks_for(cap, kForceBlock / 8) * 3 + 64;  // 16 atoms a block at least, 3 sums
   if (e == cudaSuccess) e = dalloc(&a.q, cap);
   if (e == cudaSuccess) e = dalloc(&a.v, cap);
   if (e == cudaSuccess) e = dalloc(&a.q_old, cap);
   if (e == cudaSuccess) e = dalloc(&a.qfix, cap);
   if (e == cudaSuccess) e = dalloc(&a.qfix2, cap);
+  if (e == cudaSuccess && prm->precision == MDG_FP64) e = dalloc(&a.pz, cap);
+  if (e == cudaSuccess && prm->precision == MDG_FP64) e = dalloc(&a.pz2, cap);
   if (e == cudaSuccess) e = dalloc(&a.qloc, cap);
   if (e == cudaSuccess) e = dalloc(&a.cxyz, cap);
   if (e == cudaSuccess) e = dalloc(&a.xsub, trim_table_size(b));
@@ -1219,7 +1248,7 @@ mdg_status mdg_update_position_half(mdg_handle *h) {
   h->fix_buf = -1;  // q, v or the fixed-point copy change outside the fused step
   h->obs_lag = 0.0;
   if (h->n == 0) return MDG_OK;
-  launch_drift(h, h->stream, h->prm.precision == MDG_FP32_MIXED, 0);
+  launch_drift(h, h->stream, true, 0);
   CUDA_TRY(h, cudaGetLastError());
   return MDG_OK;
 }
@@ -1231,8 +1260,7 @@ mdg_status mdg_calculate_force(mdg_handle *h) {
   h->obs_lag = 0.0;
   if (h->n == 0) return MDG_OK;
   if ((r = ensure_list(h))) return r;
-  if (h->prm.precision == MDG_FP32_MIXED)
-    k_pack_fix<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n);
+  k_pack_fix<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n);
   launch_force_mode<kKick>(h, h->stream, thermo_of(h));
   CUDA_TRY(h, cudaGetLastError());
   return MDG_OK;
@@ -1458,7 +1486,7 @@ mdg_status mdg_calculate(mdg_handle *h, int nsteps) {
     if (left <= 0) break;
     if (fused_step(h) && h->fix_buf != 0) {
       // the graph's first step reads buffer 0
-      k_pack_half<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n, h->a.qfix);
+      k_pack_half<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n, h->a.qfix, h->a.pz);
       h->kernel_launches++;
       h->fix_buf = 0;
     }
@@ -1512,8 +1540,7 @@ mdg_status mdg_forces(mdg_handle *h, double *f4) {
   if (h->n == 0) return MDG_OK;
   if (!f4) return MDG_ERR_INVALID_ARGUMENT;
   if ((r = ensure_list(h))) return r;
-  if (h->prm.precision == MDG_FP32_MIXED)
-    k_pack_fix<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n);
+  k_pack_fix<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n);
   launch_force_mode<kForceOut>(h, h->stream, thermo_of(h));
   CUDA_TRY(h, cudaGetLastError());
   CUDA_TRY(h, cudaMemcpyAsync(f4, h->a.v_tmp, sizeof(double4) * h->n, cudaMemcpyDeviceToHost, h->stream));
@@ -1527,9 +1554,13 @@ mdg_status mdg_observe(mdg_handle *h, double *ke, double *pe, double *virial) {
   double out[3] = {0.0, 0.0, 0.0};
   if (h->n > 0) {
     if ((r = ensure_list(h))) return r;
-    const int nb = blocks_for(h->n, kBlock);
+    const int nb = fp64_blocks(h->n);
     const double lag = h->observer_mode ? h->obs_lag : 0.0;
-    k_observe<kBlock><<<nb, kBlock, 0, h->stream>>>(h->a, h->box, h->n, lag);
+    switch (fp64_lanes(h->n)) {
+      case 8: k_observe<kForceBlock, 8><<<nb, kForceBlock, 0, h->stream>>>(h->a, h->box, h->n, lag); break;
+      case 4: k_observe<kForceBlock, 4><<<nb, kForceBlock, 0, h->stream>>>(h->a, h->box, h->n, lag); break;
+      default: k_observe<kForceBlock, 1><<<nb, kForceBlock, 0, h->stream>>>(h->a, h->box, h->n, lag);
+    }
     k_final_sum<256, 3><<<1, 256, 0, h->stream>>>(h->a.partials, nb, h->d_sums);
     CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaMemcpyAsync(out, h->d_sums, sizeof out, cudaMemcpyDeviceToHost, h->stream));
@@ -1549,7 +1580,12 @@ mdg_status mdg_pair_counts(mdg_handle *h, int64_t *within_cutoff, int64_t *list_
     if ((r = ensure_list(h))) return r;
     unsigned long long *d = reinterpret_cast<unsigned long long *>(h->d_sums);
     CUDA_TRY(h, cudaMemsetAsync(d, 0, 2 * sizeof(unsigned long long), h->stream));
-    k_count_pairs<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n, d);
+    const int nb = fp64_blocks(h->n);
+    switch (fp64_lanes(h->n)) {
+      case 8: k_count_pairs<kForceBlock, 8><<<nb, kForceBlock, 0, h->stream>>>(h->a, h->box, h->n, d); break;
+      case 4: k_count_pairs<kForceBlock, 4><<<nb, kForceBlock, 0, h->stream>>>(h->a, h->box, h->n, d); break;
+      default: k_count_pairs<kForceBlock, 1><<<nb, kForceBlock, 0, h->stream>>>(h->a, h->box, h->n, d);
+    }
     CUDA_TRY(h, cudaGetLastError());
     CUDA_TRY(h, cudaMemcpyAsync(c, d, sizeof c, cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));

@@ -128,6 +128,7 @@ struct Arrays {
   double4 *q, *v, *q_old;
   int4 *qfix;
   int4 *qfix2;        // second fixed-point buffer: the fused NVE step reads one and writes the other
+  double *pz, *pz2;   // FP64 handles: z of the packed positions whose (x, y) are qfix, qfix2 as double2; null otherwise
   float4 *qloc;       // FP32 coordinates at the last build (list prefilter): x global, y z cell-local
   int *cxyz;          // packed cell coordinates of each slot at the last build
   int *xsub;          // x sub-bin starts of every cell and row ends (list-build trim table)
@@ -172,6 +173,22 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
+
+// a / b for normal b: one Newton step on the hardware's approximate
+// reciprocal, then the quotient corrected by its residual with fused
+// multiply-adds (P. W. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990).  The reciprocal is good to about
+// 2^-40, so the quotient before its last rounding is to about 2^-80: the
+// correctly rounded one but for some 10^-8 of the operands, where it is its
+// neighbour.  Unlike the operator it has no branch for unusual operands, so
+// the quotients of several pairs overlap.
+__device__ __forceinline__ double quotient(double a, double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+  y = fma(y, fma(-b, y, 1.0), y);
+  const double q = a * y;
+  return fma(fma(-b, q, a), y, q);
+}
 
 // The skin budget's cost of one step, 2 vmax dt, each operation separately
 // rounded as in PairList::IsPairListExpired (src/pairlist.cc:25-65), so
@@ -259,6 +276,22 @@ __device__ __forceinline__ int fixed_coord(double x, double L) {
   u -= floor(u);
   const long long k = __double2ll_rn(u * 4294967296.0);
   return (int)(unsigned int)(unsigned long long)k;
+}
+
+// Position (x, y, z) of atom i into a packed copy: fixed-point, or with a z
+// array (FP64 handles) as (x, y) and z apart.  The FP64 pair kernels gather 24
+// bytes a partner from the split copy: in a double4 array the 16-byte halves
+// of consecutive atoms fall on every other 16-byte column of the L1's data
+// banks and z on every fourth, which made the gathers' bank conflicts the
+// bound of the pass.
+__device__ __forceinline__ void pack_position(int4 *out, double *out_z, int i, double x, double y, double z,
+                                              const double L[3]) {
+  if (out_z) {
+    reinterpret_cast<double2 *>(out)[i] = make_double2(x, y);
+    out_z[i] = z;
+  } else {
+    out[i] = make_int4(fixed_coord(x, L[0]), fixed_coord(y, L[1]), fixed_coord(z, L[2]), 0);
+  }
 }
 
 // Minimum-image ghost coordinate as the reference forms it: the copy of
@@ -909,7 +942,7 @@ __device__ __forceinline__ int border_bits(const double x[3], const Box &b, int 
 // Rebuild 5/6: gather into cell order (temporary arrays), snapshot q_old
 // (PairList::Init), ghost-strip membership and the total copy count.
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_permute(Arrays a, Box b, int n, int4 *pack) {
+__global__ void __launch_bounds__(BLOCK) k_permute(Arrays a, Box b, int n, int4 *pack, double *pack_z) {
   const int s = blockIdx.x * BLOCK + threadIdx.x;
   int m = 0;
   if (s < n && !a.st->error) {
@@ -932,12 +965,11 @@ __global__ void __launch_bounds__(BLOCK) k_permute(Arrays a, Box b, int n, int4 
     a.qloc[s] = make_float4((float)q.x, (float)(q.y - cy * b.cs[1]), (float)(q.z - gz * b.cs[2]), __int_as_float(strips));
     a.cxyz[s] = pack_cell(cx, cy, cz);
     if (pack) {
-      // the coming step's first-drift positions for the fused FP32 NVE pass
+      // the coming step's first-drift positions for the fused NVE pass
       const double4 v = a.v[o];
       const double dt2 = b.dt * 0.5;
-      pack[s] = make_int4(fixed_coord(dadd(q.x, dmul(v.x, dt2)), b.L[0]),
-                          fixed_coord(dadd(q.y, dmul(v.y, dt2)), b.L[1]),
-                          fixed_coord(dadd(q.z, dmul(v.z, dt2)), b.L[2]), 0);
+      pack_position(pack, pack_z, s, dadd(q.x, dmul(v.x, dt2)), dadd(q.y, dmul(v.y, dt2)), dadd(q.z, dmul(v.z, dt2)),
+                    b.L);
     }
   }
   const int tot = __reduce_add_sync(0xffffffffu, m);
@@ -1641,7 +1673,7 @@ static __global__ void k_build_done(Arrays a, Box b) {
 }
 
 // q += v dt/2 (ForceCalculator::UpdatePositionHalf, src/fcalculator.cc:17-30);
-// FIX also writes the fixed-point copy used by the FP32-mixed force.
+// FIX also writes the packed copy that the force pass reads.
 template <int BLOCK, bool FIX>
 __global__ void __launch_bounds__(BLOCK) k_drift(Arrays a, Box b, int n, int track_vmax) {
   const int i = blockIdx.x * BLOCK + threadIdx.x;
@@ -1654,8 +1686,7 @@ __global__ void __launch_bounds__(BLOCK) k_drift(Arrays a, Box b, int n, int tra
     q.y = dadd(q.y, dmul(v.y, dt2));
     q.z = dadd(q.z, dmul(v.z, dt2));
     a.q[i] = q;
-    if (FIX) a.qfix[i] = make_int4(fixed_coord(q.x, b.L[0]), fixed_coord(q.y, b.L[1]),
-                                   fixed_coord(q.z, b.L[2]), 0);
+    if (FIX) pack_position(a.qfix, a.pz, i, q.x, q.y, q.z, b.L);
     if (track_vmax) {
       v2 = dadd(dadd(dmul(v.x, v.x), dmul(v.y, v.y)), dmul(v.z, v.z));
       if (!isfinite(v2) || !isfinite(q.x + q.y + q.z)) atomicOr(&a.st->error, kErrNonFinite);
@@ -1774,25 +1805,24 @@ __global__ void __launch_bounds__(BLOCK) k_density(Arrays a, Box b, int n, doubl
 }
 
 // Packs q + v dt/2 (the coming step's first half drift) into out without
-// moving atoms: the fixed-point copy the fused NVE force pass reads.
+// moving atoms: the copy the fused NVE force pass reads.
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_pack_half(Arrays a, Box b, int n, int4 *out) {
+__global__ void __launch_bounds__(BLOCK) k_pack_half(Arrays a, Box b, int n, int4 *out, double *out_z) {
   const int i = blockIdx.x * BLOCK + threadIdx.x;
   if (i >= n || a.st->error) return;
   const double4 q = a.q[i];
   const double4 v = a.v[i];
   const double dt2 = b.dt * 0.5;
-  out[i] = make_int4(fixed_coord(dadd(q.x, dmul(v.x, dt2)), b.L[0]), fixed_coord(dadd(q.y, dmul(v.y, dt2)), b.L[1]),
-                     fixed_coord(dadd(q.z, dmul(v.z, dt2)), b.L[2]), 0);
+  pack_position(out, out_z, i, dadd(q.x, dmul(v.x, dt2)), dadd(q.y, dmul(v.y, dt2)), dadd(q.z, dmul(v.z, dt2)), b.L);
 }
 
-// Writes the fixed-point copy of q without moving atoms.
+// Writes the packed copy of q without moving atoms.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_pack_fix(Arrays a, Box b, int n) {
   const int i = blockIdx.x * BLOCK + threadIdx.x;
   if (i >= n) return;
   const double4 q = a.q[i];
-  a.qfix[i] = make_int4(fixed_coord(q.x, b.L[0]), fixed_coord(q.y, b.L[1]), fixed_coord(q.z, b.L[2]), 0);
+  pack_position(a.qfix, a.pz, i, q.x, q.y, q.z, b.L);
 }
 
 enum ForceMode { kKick = 0, kForceOut = 1, kKickNoseHoover = 2, kKickLangevin = 3 };
@@ -1864,47 +1894,222 @@ __device__ __forceinline__ void finish_atom(Arrays &a, const Box &b, const Therm
   a.v[i] = v;
 }
 
-// FP64 force kick, one thread per atom over its full row.  Every pair term is
-// the reference's (ForceCalculator::CalculateForceNext, src/fcalculator.cc:
-// 228-290): dx = image(q_j) - q_i, r2 = (dx*dx + dy*dy) + dz*dz, skipped if
-// r2 > rc^2, r6 = (r2*r2)*r2, df = ((24 r6 - 48) / ((r6*r6)*r2) + 8 C2) * dt,
-// term = df * dx, all separately rounded; only the summation order differs.
-template <int BLOCK, int MODE>
-__global__ void __launch_bounds__(BLOCK) k_force_fp64(Arrays a, Box b, int n, Thermo th) {
-  const int i = blockIdx.x * BLOCK + threadIdx.x;
-  double v2 = 0.0, ke = 0.0;
-  if (i < n && !a.st->error) {
-    const double4 qi = a.q[i];
-    const int nn = a.nnbr[i];
-    const double c2x8 = b.c2 * 8.0;
-    const double dt = (MODE == kForceOut) ? 1.0 : b.dt;
-    double fx = 0.0, fy = 0.0, fz = 0.0;
-    const int *row = a.nbr + i;
-    // software pipeline: the next partner's position and the entry after it
-    // are in flight while a pair term is formed
-    int jn = nn > 1 ? row[a.stride] : i;
-    double4 qn = a.q[nn > 0 ? row[0] : i];
-    for (int k = 0; k < nn; k++) {
-      const double4 qj = qn;
-      qn = a.q[jn];
-      jn = (k + 2 < nn) ? row[(size_t)(k + 2) * a.stride] : i;
-      const double dx = dsub(image_of(qj.x, qi.x, b.L[0], b.hL[0]), qi.x);
-      const double dy = dsub(image_of(qj.y, qi.y, b.L[1], b.hL[1]), qi.y);
-      const double dz = dsub(image_of(qj.z, qi.z, b.L[2], b.hL[2]), qi.z);
-      const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-      if (r2 > b.rc2) continue;
-      const double r6 = dmul(dmul(r2, r2), r2);
-      const double df = dmul(dadd(ddiv(dsub(dmul(24.0, r6), 48.0), dmul(dmul(r6, r6), r2)), c2x8), dt);
-      fx = dadd(fx, dmul(df, dx));
-      fy = dadd(fy, dmul(df, dy));
-      fz = dadd(fz, dmul(df, dz));
-    }
-    finish_atom<MODE>(a, b, th, i, fx, fy, fz, v2, ke);
+// The per-atom end of a force pass: the FP64 kick (fx, fy, fz) and, with
+// DRIFT, the second half drift (DRIFT == 2 also this step's first half drift
+// of the atom itself and the pack of the next step's first-drift position).
+template <int MODE, int DRIFT>
+__device__ __forceinline__ void kick_and_drift(Arrays &a, const Box &b, const Thermo &th, int i, double fx, double fy,
+                                               double fz, int4 *next, double *next_z, double &v2, double &ke) {
+  const double dt2 = b.dt * 0.5;
+  double4 q;
+  if (DRIFT) q = a.q[i];
+  if (DRIFT == 2) {
+    // this step's first half drift (the partners' copies already have it)
+    const double4 v0 = a.v[i];
+    q.x = dadd(q.x, dmul(v0.x, dt2));
+    q.y = dadd(q.y, dmul(v0.y, dt2));
+    q.z = dadd(q.z, dmul(v0.z, dt2));
   }
-  if (MODE == kKickLangevin) warp_max_to(&a.st->vmax2_bits, v2);
+  finish_atom<MODE>(a, b, th, i, fx, fy, fz, v2, ke);
+  if (DRIFT) {
+    const double4 v = a.v[i];
+    q.x = dadd(q.x, dmul(v.x, dt2));
+    q.y = dadd(q.y, dmul(v.y, dt2));
+    q.z = dadd(q.z, dmul(v.z, dt2));
+    a.q[i] = q;
+    v2 = dadd(dadd(dmul(v.x, v.x), dmul(v.y, v.y)), dmul(v.z, v.z));
+    if (!isfinite(v2) || !isfinite(q.x + q.y + q.z)) atomicOr(&a.st->error, kErrNonFinite);
+    // the next step's first half drift, packed for its force pass
+    if (DRIFT == 2)
+      pack_position(next, next_z, i, dadd(q.x, dmul(v.x, dt2)), dadd(q.y, dmul(v.y, dt2)), dadd(q.z, dmul(v.z, dt2)),
+                    b.L);
+  }
+}
+
+// ------------------------------------------------ FP64 rows, 1, 4 or 8 lanes per atom
+// Whether some partner of an atom of (local) cell pc sits beyond a periodic
+// face: only atoms of the outermost cells have such partners, since a row
+// reaches one cell out and an atom moves less than the skin between builds.
+// For the others image_of is the identity.
+__device__ __forceinline__ bool row_wraps(const int ms[3], int z0, int pc) {
+  const int cx = pc & 2047, cy = (pc >> 11) & 2047, cz = z0 + (int)((unsigned)pc >> 22);
+  return cx == 0 || cx == ms[0] - 1 || cy == 0 || cy == ms[1] - 1 || cz == 0 || cz == ms[2] - 1;
+}
+
+// FP64 positions as the pair kernels gather them: the state's array, or a
+// packed copy (pack_position).
+struct PosState {
+  const double4 *q;
+  __device__ __forceinline__ double3 at(int j) const {
+    const double4 p = q[j];
+    return make_double3(p.x, p.y, p.z);
+  }
+};
+struct PosSplit {
+  const double2 *xy;
+  const double *z;
+  __device__ __forceinline__ double3 at(int j) const {
+    const double2 p = xy[j];
+    return make_double3(p.x, p.y, z[j]);
+  }
+};
+
+// Blocks of 128 threads an SM that the FP64 pair kernels are held to (72
+// registers, 28 warps).  The fused pass of the 2.05M-atom liquid: 0.464 ms with
+// 7, 0.524 with 6, 0.476 with 8, 0.540 with 9; the serial branching loop over
+// double4 positions that it replaced 0.600 ms and 0.054 ms of drift kernels.
+constexpr int kFp64Blocks = 7;
+
+// Lanes per atom of the FP64 pair kernels (every count gives the same sums,
+// fp64_row).  Few atoms leave the chip to the latency of one row, many are
+// bound by the pair arithmetic and the gathers.  Fused pass with 8, 4 and 1
+// lanes: 4,000 atoms 7.5, 9.0, 24.6 us; 8,788 atoms 9.0, 9.6, 24.3; 16,384
+// atoms 12.8, 11.2, 24.8; 55,296 atoms 33, 24, 28; 118,661 atoms (Nose-Hoover)
+// 63, 45, 40.
+inline int fp64_lanes(int n) { return n <= 10000 ? 8 : (n <= 65536 ? 4 : 1); }
+
+// Sums over an atom's row in FP64, NS of them, in one fixed order whatever
+// the number of lanes that share the row: the row falls into chunks of four
+// entries (the last one shorter), each is summed in row order from 0, and the
+// row's sum is ((0 + c0) + c1) + ...  With TPA lanes per atom (consecutive
+// lanes; all lanes of the warp call together), lane `sub` sums chunks sub, sub
+// + TPA, ..., and after each round every lane adds the round's chunk sums in
+// chunk order, so every lane holds the sums.  pair(p, j, on, s) adds the terms
+// of two partners j at p to s, in order; entries past the row's end arrive as
+// the atom itself with on = false.  Two pairs are formed at once and without
+// branches, so that their latencies overlap, and the next two partners'
+// positions and the next chunk's entries are in flight meanwhile.
+template <int TPA, int NS, typename Pos, typename Pair>
+__device__ __forceinline__ void fp64_row(const Pos &q, const int *__restrict__ nbr, int stride, int nn, int i, int sub,
+                                         double (&out)[NS], Pair pair) {
+  const int chunks = (nn + 3) >> 2;
+  const int rounds = TPA > 1 ? __reduce_max_sync(0xffffffffu, (chunks + TPA - 1) / TPA) : chunks;
+  const int first = (threadIdx.x & 31) & ~(TPA - 1);
+  const size_t hop = (size_t)(4 * TPA) * stride;
+  const int *row = nbr + (size_t)(4 * sub) * stride + i;  // the chunk whose entries are loaded next
+  int c = sub;                                            // its number
+  // entries of a chunk (the row is padded to whole chunks)
+  auto load = [&](int (&j)[4]) {
+    const bool in = c < chunks;
+#pragma unroll
+    for (int u = 0; u < 4; u++) j[u] = in ? row[(size_t)u * stride] : i;
+    row += hop;
+    c += TPA;
+  };
+#pragma unroll
+  for (int k = 0; k < NS; k++) out[k] = 0.0;
+  int jc[4], jn[4];
+  load(jc);
+  double3 p[2] = {q.at(jc[0]), q.at(jc[1])};
+  int k = 4 * sub;  // the chunk's first entry
+#pragma unroll 1
+  for (int r = 0; r < rounds; r++, k += 4 * TPA) {
+    double s[NS];
+#pragma unroll
+    for (int m = 0; m < NS; m++) s[m] = 0.0;
+    load(jn);
+    const double3 p2[2] = {q.at(jc[2]), q.at(jc[3])};
+    {
+      const int j[2] = {jc[0], jc[1]};
+      const bool on[2] = {k < nn, k + 1 < nn};
+      pair(p, j, on, s);
+    }
+    p[0] = q.at(jn[0]);
+    p[1] = q.at(jn[1]);
+    {
+      const int j[2] = {jc[2], jc[3]};
+      const bool on[2] = {k + 2 < nn, k + 3 < nn};
+      pair(p2, j, on, s);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) jc[u] = jn[u];
+#pragma unroll
+    for (int l = 0; l < TPA; l++)
+#pragma unroll
+      for (int m = 0; m < NS; m++) out[m] += TPA > 1 ? __shfl_sync(0xffffffffu, s[m], first + l) : s[m];
+  }
+}
+
+// FP64 force kick, TPA lanes per atom (BLOCK / TPA atoms per block).  Every
+// pair term is the reference's (ForceCalculator::CalculateForceNext,
+// src/fcalculator.cc:228-290): dx = image(q_j) - q_i, r2 = (dx*dx + dy*dy) +
+// dz*dz, 0 if r2 > rc^2, r6 = (r2*r2)*r2, df = ((24 r6 - 48) /
+// ((r6*r6)*r2) + 8 C2) * dt, term = df * dx, all separately rounded; only the
+// summation order differs (fp64_row).
+struct Fp64Pair {
+  const double *L, *hL;  // box and half box, read for partners beyond a face only
+  double rc2, c2x8, dt;
+  double3 qi;
+};
+
+template <bool WRAP>
+__device__ __forceinline__ void lj_pairs_fp64(const Fp64Pair &f, const double3 (&p)[2], const bool (&on)[2],
+                                              double (&s)[3]) {
+  double d[2][3], df[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    d[u][0] = dsub(WRAP ? image_of(p[u].x, f.qi.x, f.L[0], f.hL[0]) : p[u].x, f.qi.x);
+    d[u][1] = dsub(WRAP ? image_of(p[u].y, f.qi.y, f.L[1], f.hL[1]) : p[u].y, f.qi.y);
+    d[u][2] = dsub(WRAP ? image_of(p[u].z, f.qi.z, f.L[2], f.hL[2]) : p[u].z, f.qi.z);
+    double r2 = dadd(dadd(dmul(d[u][0], d[u][0]), dmul(d[u][1], d[u][1])), dmul(d[u][2], d[u][2]));
+    const bool in = on[u] && !(r2 > f.rc2);
+    r2 = in ? r2 : 1.0;  // an ordinary operand for the division
+    const double r6 = dmul(dmul(r2, r2), r2);
+    df[u] = dmul(dadd(quotient(dsub(dmul(24.0, r6), 48.0), dmul(dmul(r6, r6), r2)), f.c2x8), f.dt);
+    df[u] = in ? df[u] : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    s[0] = dadd(s[0], dmul(df[u], d[u][0]));
+    s[1] = dadd(s[1], dmul(df[u], d[u][1]));
+    s[2] = dadd(s[2], dmul(df[u], d[u][2]));
+  }
+}
+
+template <int TPA, typename Pos>
+__device__ __forceinline__ void fp64_force_row(const Pos &q, const int *nbr, int stride, int nn, int i, int sub,
+                                               const Fp64Pair &f, bool wraps, double (&s)[3]) {
+  // one path for the whole warp
+  if (__any_sync(0xffffffffu, (int)wraps))
+    fp64_row<TPA>(q, nbr, stride, nn, i, sub, s,
+                  [&](const double3 (&p)[2], const int (&)[2], const bool (&on)[2], double (&t)[3]) {
+                    lj_pairs_fp64<true>(f, p, on, t);
+                  });
+  else
+    fp64_row<TPA>(q, nbr, stride, nn, i, sub, s,
+                  [&](const double3 (&p)[2], const int (&)[2], const bool (&on)[2], double (&t)[3]) {
+                    lj_pairs_fp64<false>(f, p, on, t);
+                  });
+}
+
+// DRIFT as in k_force_fp32 (the positions come from the packed copy `pos`,
+// so moving q races with no other thread): 1 also makes the second half
+// drift, 2 the whole NVE step, with the next step's first-drift positions
+// packed into next, next_z.
+template <int BLOCK, int MODE, int DRIFT, int TPA, typename Pos>
+__global__ void __launch_bounds__(BLOCK, kFp64Blocks) k_force_fp64(Arrays a, Box b, int n, Thermo th, Pos pos, int4 *next,
+                                                      double *next_z) {
+  const int t = blockIdx.x * BLOCK + threadIdx.x;
+  const int i = t / TPA, sub = t % TPA;
+  double v2 = 0.0, ke = 0.0;
+  if (DRIFT == 2 && t == 0 && !a.st->error) {
+    // the step counter (k_step_done's work): nothing in this pass reads it
+    a.st->steps++;
+    a.st->sim_time += b.dt;
+  }
+  // the lanes of a warp walk together: they agree on the error flag
+  const int err = warp_error(a.st);
+  const bool on = i < n && !err;
+  const int ii = i < n ? i : 0;
+  const Fp64Pair f{b.L, b.hL, b.rc2, b.c2 * 8.0, MODE == kForceOut ? 1.0 : b.dt, pos.at(ii)};
+  double s[3];
+  fp64_force_row<TPA>(pos, a.nbr, a.stride, on ? a.nnbr[ii] : 0, ii, sub, f,
+                      on && row_wraps(b.ms, b.z0, a.cxyz[ii]), s);
+  if (on && sub == 0) kick_and_drift<MODE, DRIFT>(a, b, th, i, s[0], s[1], s[2], next, next_z, v2, ke);
+  if (MODE == kKickLangevin || DRIFT) warp_max_to(&a.st->vmax2_bits, v2);
   if (MODE == kKickNoseHoover) {
-    double s[1] = {ke};
-    block_sum_to<BLOCK, 1>(s, a.partials);
+    double sum[1] = {ke};  // 0 on lanes other than the atom's first
+    block_sum_to<BLOCK, 1>(sum, a.partials);
   }
 }
 
@@ -1936,39 +2141,11 @@ __device__ __forceinline__ void lj_pair_fp32(const int4 &pi, const int4 &pj, flo
   fz = fmaf(df, dz, fz);
 }
 
-// The per-atom end of an FP32-mixed force pass: the FP64 kick and, with
-// DRIFT, the second half drift (DRIFT == 2 also this step's first half
-// drift of the atom itself and the pack of the next step's first-drift
-// position into qf_next).
 template <int MODE, int DRIFT>
 __device__ __forceinline__ void fp32_finish(Arrays &a, const Box &b, const Thermo &th, int i, double Fx, double Fy,
                                             double Fz, int4 *qf_next, double &v2, double &ke) {
   const double dt = (MODE == kForceOut) ? 1.0 : b.dt;
-  const double dt2 = b.dt * 0.5;
-  double4 q = a.q[i];
-  if (DRIFT == 2) {
-    // this step's first half drift (the neighbours' copies in qf already have it)
-    const double4 v0 = a.v[i];
-    q.x = dadd(q.x, dmul(v0.x, dt2));
-    q.y = dadd(q.y, dmul(v0.y, dt2));
-    q.z = dadd(q.z, dmul(v0.z, dt2));
-  }
-  finish_atom<MODE>(a, b, th, i, Fx * dt, Fy * dt, Fz * dt, v2, ke);
-  if (DRIFT) {
-    const double4 v = a.v[i];
-    q.x = dadd(q.x, dmul(v.x, dt2));
-    q.y = dadd(q.y, dmul(v.y, dt2));
-    q.z = dadd(q.z, dmul(v.z, dt2));
-    a.q[i] = q;
-    v2 = dadd(dadd(dmul(v.x, v.x), dmul(v.y, v.y)), dmul(v.z, v.z));
-    if (!isfinite(v2) || !isfinite(q.x + q.y + q.z)) atomicOr(&a.st->error, kErrNonFinite);
-    if (DRIFT == 2) {
-      // the next step's first half drift, packed for its force pass
-      qf_next[i] = make_int4(fixed_coord(dadd(q.x, dmul(v.x, dt2)), b.L[0]),
-                             fixed_coord(dadd(q.y, dmul(v.y, dt2)), b.L[1]),
-                             fixed_coord(dadd(q.z, dmul(v.z, dt2)), b.L[2]), 0);
-    }
-  }
+  kick_and_drift<MODE, DRIFT>(a, b, th, i, Fx * dt, Fy * dt, Fz * dt, qf_next, nullptr, v2, ke);
 }
 
 // ------------------------------------------------ FP32 row sums, 1-4 lanes per atom
@@ -2729,41 +2906,72 @@ __global__ void __launch_bounds__(BLOCK) k_zeta(Arrays a, Box b, int nblocks, in
 // reached through the periodic boundary is a ghost copy refreshed after the
 // first half drift (MDManager::SendBorderParticles, src/mdmanager.cc:165-167),
 // i.e. the partner's position lag = dt/2 earlier, q_j - v_j dt/2.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_observe(Arrays a, Box b, int n, double lag) {
-  const int i = blockIdx.x * BLOCK + threadIdx.x;
-  double ke = 0.0, pe = 0.0, vir = 0.0;
-  if (i < n) {
-    const double4 v = a.v[i];
-    ke = dadd(dadd(dmul(dmul(0.5, v.x), v.x), dmul(dmul(0.5, v.y), v.y)), dmul(dmul(0.5, v.z), v.z));
-    const double4 qi = a.q[i];
-    const double4 *vl = lag_velocities(a);
-    const int nn = a.nnbr[i];
-    for (int k = 0; k < nn; k++) {
-      const int j = a.nbr[(size_t)k * a.stride + i];
-      double4 qj = a.q[j];
-      if (lag > 0.0 && (fabs(qj.x - qi.x) > b.hL[0] || fabs(qj.y - qi.y) > b.hL[1] ||
-                        fabs(qj.z - qi.z) > b.hL[2])) {
-        const double4 vj = vl[j];
-        qj.x = dsub(qj.x, dmul(vj.x, lag));
-        qj.y = dsub(qj.y, dmul(vj.y, lag));
-        qj.z = dsub(qj.z, dmul(vj.z, lag));
-      }
-      const double dx = dsub(qi.x, image_of(qj.x, qi.x, b.L[0], b.hL[0]));
-      const double dy = dsub(qi.y, image_of(qj.y, qi.y, b.L[1], b.hL[1]));
-      const double dz = dsub(qi.z, image_of(qj.z, qi.z, b.L[2], b.hL[2]));
-      const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-      if (r2 > b.rc2) continue;
-      const double r4 = dmul(r2, r2), r6 = dmul(r4, r2), r8 = dmul(r6, r2), r10 = dmul(r8, r2),
-                   r12 = dmul(r10, r2);
-      const double e = dmul(4.0, dadd(dadd(dsub(ddiv(1.0, r12), ddiv(1.0, r6)), dmul(b.c2, r2)), b.c0));
-      pe = dadd(pe, e);
-      const double r6v = dmul(dmul(r2, r2), r2);
-      const double w = dmul(dadd(ddiv(dsub(dmul(24.0, r6v), 48.0), dmul(dmul(r6v, r6v), r2)), b.c2 * 8.0), r2);
-      vir = dadd(vir, w);
-    }
+// Energy and virial terms of the partners at p[0] and p[1] (t[0] and t[1],
+// counted from both ends); WRAP as in lj_pair_fp64.
+template <bool WRAP>
+__device__ __forceinline__ void observe_pairs(const double *L, const double *hL, double rc2, double c0, double c2,
+                                              const double4 &qi, const double3 (&p)[2], const bool (&on)[2],
+                                              double (&t)[2]) {
+  double e[2], w[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const double dx = dsub(qi.x, WRAP ? image_of(p[u].x, qi.x, L[0], hL[0]) : p[u].x);
+    const double dy = dsub(qi.y, WRAP ? image_of(p[u].y, qi.y, L[1], hL[1]) : p[u].y);
+    const double dz = dsub(qi.z, WRAP ? image_of(p[u].z, qi.z, L[2], hL[2]) : p[u].z);
+    double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+    const bool in = on[u] && !(r2 > rc2);
+    r2 = in ? r2 : 1.0;
+    const double r4 = dmul(r2, r2), r6 = dmul(r4, r2), r8 = dmul(r6, r2), r10 = dmul(r8, r2), r12 = dmul(r10, r2);
+    e[u] = dmul(4.0, dadd(dadd(dsub(quotient(1.0, r12), quotient(1.0, r6)), dmul(c2, r2)), c0));
+    w[u] = dmul(dadd(quotient(dsub(dmul(24.0, r6), 48.0), dmul(dmul(r6, r6), r2)), c2 * 8.0), r2);
+    e[u] = in ? e[u] : 0.0;
+    w[u] = in ? w[u] : 0.0;
   }
-  double s[3] = {ke, 0.5 * pe, 0.5 * vir};
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    t[0] = dadd(t[0], e[u]);
+    t[1] = dadd(t[1], w[u]);
+  }
+}
+
+template <int BLOCK, int TPA>
+__global__ void __launch_bounds__(BLOCK, kFp64Blocks) k_observe(Arrays a, Box b, int n, double lag) {
+  const int tid = blockIdx.x * BLOCK + threadIdx.x;
+  const int i = tid / TPA, sub = tid % TPA;
+  const bool on = i < n;
+  const int ii = on ? i : 0;
+  const double4 qi = a.q[ii];
+  const int nn = on ? a.nnbr[ii] : 0;
+  double t[2];
+  if (__any_sync(0xffffffffu, (int)(on && row_wraps(b.ms, b.z0, a.cxyz[ii])))) {
+    const double4 *vl = lag_velocities(a);
+    fp64_row<TPA>(PosState{a.q}, a.nbr, a.stride, nn, ii, sub, t,
+                  [&](const double3 (&p)[2], const int (&j)[2], const bool (&in)[2], double (&u)[2]) {
+                    double3 qj[2] = {p[0], p[1]};
+                    for (int k = 0; k < 2; k++) {
+                      if (lag > 0.0 && (fabs(qj[k].x - qi.x) > b.hL[0] || fabs(qj[k].y - qi.y) > b.hL[1] ||
+                                        fabs(qj[k].z - qi.z) > b.hL[2])) {
+                        const double4 vj = vl[j[k]];
+                        qj[k].x = dsub(qj[k].x, dmul(vj.x, lag));
+                        qj[k].y = dsub(qj[k].y, dmul(vj.y, lag));
+                        qj[k].z = dsub(qj[k].z, dmul(vj.z, lag));
+                      }
+                    }
+                    observe_pairs<true>(b.L, b.hL, b.rc2, b.c0, b.c2, qi, qj, in, u);
+                  });
+  } else {
+    fp64_row<TPA>(PosState{a.q}, a.nbr, a.stride, nn, ii, sub, t,
+                  [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[2]) {
+                    observe_pairs<false>(b.L, b.hL, b.rc2, b.c0, b.c2, qi, p, in, u);
+                  });
+  }
+  double s[3] = {0.0, 0.0, 0.0};
+  if (on && sub == 0) {
+    const double4 v = a.v[i];
+    s[0] = dadd(dadd(dmul(dmul(0.5, v.x), v.x), dmul(dmul(0.5, v.y), v.y)), dmul(dmul(0.5, v.z), v.z));
+    s[1] = 0.5 * t[0];
+    s[2] = 0.5 * t[1];
+  }
   block_sum_to<BLOCK, 3>(s, a.partials);
 }
 
@@ -2789,24 +2997,41 @@ __global__ void __launch_bounds__(BLOCK) k_final_sum(const double *partials, int
 // Directed list entries within the cut-off (the pairs whose force is
 // evaluated), with the reference's r^2 test (src/fcalculator.cc:268), summed
 // into counts[0]; counts[1] gets all list entries.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_count_pairs(Arrays a, Box b, int n, unsigned long long *counts) {
-  const int i = blockIdx.x * BLOCK + threadIdx.x;
-  int within = 0, nn = 0;
-  if (i < n) {
-    const double4 qi = a.q[i];
-    nn = a.nnbr[i];
-    for (int k = 0; k < nn; k++) {
-      const double4 qj = a.q[a.nbr[(size_t)k * a.stride + i]];
-      const double dx = dsub(image_of(qj.x, qi.x, b.L[0], b.hL[0]), qi.x);
-      const double dy = dsub(image_of(qj.y, qi.y, b.L[1], b.hL[1]), qi.y);
-      const double dz = dsub(image_of(qj.z, qi.z, b.L[2], b.hL[2]), qi.z);
-      const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-      within += (r2 > b.rc2) ? 0 : 1;
-    }
+template <bool WRAP>
+__device__ __forceinline__ void count_pairs(const double *L, const double *hL, double rc2, const double4 &qi,
+                                            const double3 (&p)[2], const bool (&on)[2], double (&t)[1]) {
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const double dx = dsub(WRAP ? image_of(p[u].x, qi.x, L[0], hL[0]) : p[u].x, qi.x);
+    const double dy = dsub(WRAP ? image_of(p[u].y, qi.y, L[1], hL[1]) : p[u].y, qi.y);
+    const double dz = dsub(WRAP ? image_of(p[u].z, qi.z, L[2], hL[2]) : p[u].z, qi.z);
+    const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
+    t[0] += on[u] && !(r2 > rc2) ? 1.0 : 0.0;
   }
-  const int ws = __reduce_add_sync(0xffffffffu, within);
-  const int ns = __reduce_add_sync(0xffffffffu, nn);
+}
+
+template <int BLOCK, int TPA>
+__global__ void __launch_bounds__(BLOCK, kFp64Blocks) k_count_pairs(Arrays a, Box b, int n,
+                                                                    unsigned long long *counts) {
+  const int tid = blockIdx.x * BLOCK + threadIdx.x;
+  const int i = tid / TPA, sub = tid % TPA;
+  const bool on = i < n;
+  const int ii = on ? i : 0;
+  const double4 qi = a.q[ii];
+  const int nn = on ? a.nnbr[ii] : 0;
+  double t[1];
+  if (__any_sync(0xffffffffu, (int)(on && row_wraps(b.ms, b.z0, a.cxyz[ii]))))
+    fp64_row<TPA>(PosState{a.q}, a.nbr, a.stride, nn, ii, sub, t,
+                  [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[1]) {
+                    count_pairs<true>(b.L, b.hL, b.rc2, qi, p, in, u);
+                  });
+  else
+    fp64_row<TPA>(PosState{a.q}, a.nbr, a.stride, nn, ii, sub, t,
+                  [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[1]) {
+                    count_pairs<false>(b.L, b.hL, b.rc2, qi, p, in, u);
+                  });
+  const int ws = __reduce_add_sync(0xffffffffu, sub == 0 ? (int)t[0] : 0);
+  const int ns = __reduce_add_sync(0xffffffffu, sub == 0 ? nn : 0);
   if ((threadIdx.x & 31) == 0) {
     atomicAdd(&counts[0], (unsigned long long)ws);
     atomicAdd(&counts[1], (unsigned long long)ns);

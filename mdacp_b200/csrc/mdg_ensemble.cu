@@ -31,7 +31,8 @@ namespace {
 constexpr int kEB = 256;        // streaming kernels
 constexpr int kEF = 128;        // pair kernels
 constexpr int kEStepsPerGraph = 20;
-constexpr int kEPairParts = 8;  // blocks per replica in the candidate-pair test
+constexpr int kEPairParts = 8;    // blocks per replica in the candidate-pair test
+constexpr int kEPairShort = 64;   // candidates up to which one block takes it
 
 struct Rep {
   double L[3], hL[3], inv_cs[3], cs[3];
@@ -73,7 +74,10 @@ struct Ens {
   RepStatus *rs;
   const int *rep_of;  // replica of each atom slot (fixed: atoms move only within their replica)
   double4 *q, *v, *q_old;
-  int4 *qfix;
+  // packed first-drift positions of this step and the next, taking turns
+  // (pack_position; pz and pz2: z of an FP64 ensemble's, else null)
+  int4 *qfix, *qfix2;
+  double *pz, *pz2;
   float4 *qloc;
   int *cxyz, *xsub;  // packed cell coordinates and the list-build trim table (as the single-system arrays)
   int *ids, *cell, *cell_tmp, *nbr, *nnbr, *cell_count, *cell_start, *slot, *perm, *perm2;
@@ -187,12 +191,28 @@ __device__ __forceinline__ int work_find(const int *prefix, int nk, int g) {
   return lo;
 }
 
-// Replica and atom slot of work atom g of list w.
-__device__ __forceinline__ int work_atom(const Ens &e, const WorkList &w, int g, int *r) {
-  const int k = work_find(w.atom_prefix, w.count[0], g);
-  *r = w.rep[k];
-  return e.rep[*r].atom_off + (g - w.atom_prefix[k]);
-}
+// A block's share of a work list's atoms: consecutive items, so that a thread
+// finds the replica of its next item from that of its last one (the binary
+// search of every item was most of the time of the light sweeps: 32 us for
+// ke_disp_collect over 2.5M atoms).
+struct WorkSweep {
+  const WorkList &w;
+  int nk, base, end, k = -1;
+  __device__ __forceinline__ WorkSweep(const WorkList &list, int block) : w(list) {
+    nk = w.count[0];
+    const int total = w.count[1];
+    const int share = ((total + (int)gridDim.x - 1) / (int)gridDim.x + block - 1) / block * block;
+    base = min((long long)blockIdx.x * share, (long long)total);
+    end = min(base + share, total);
+  }
+  // replica and atom slot of work atom g (not below the last one asked for)
+  __device__ __forceinline__ int atom(const Ens &e, int g, int *r) {
+    if (k < 0) k = work_find(w.atom_prefix, nk, g);
+    while (k + 1 < nk && w.atom_prefix[k + 1] <= g) k++;
+    *r = w.rep[k];
+    return e.rep[*r].atom_off + (g - w.atom_prefix[k]);
+  }
+};
 
 // One block, 1024 threads: the work list of the replicas whose disp (WHICH
 // 0) or build (WHICH 1) flag is set.
@@ -283,14 +303,14 @@ __device__ __forceinline__ CopyView ens_view(const Ens &e) { return CopyView{e.q
 // (The atoms of the checked replicas, through the skin-check work list;
 // block-uniform sweeps, so every lane reaches rep_max.)
 __global__ void __launch_bounds__(kEB) ke_disp_max(Ens e) {
-  const int total = e.wd.count[1];
-  for (int base = blockIdx.x * kEB; base < total; base += gridDim.x * kEB) {
+  WorkSweep sweep(e.wd, kEB);
+  for (int base = sweep.base; base < sweep.end; base += kEB) {
     const int g = base + threadIdx.x;
-    const bool active = g < total;
+    const bool active = g < sweep.end;
     int r = 0;
     double d2 = 0.0;
     if (active) {
-      const int i = work_atom(e, e.wd, g, &r);
+      const int i = sweep.atom(e, g, &r);
       for_each_copy(ens_view(e), e.rep[r].L, i, e.lag, [&](int, double x) { d2 = fmax(d2, x); });
       e.disp2[i] = d2;
     }
@@ -299,10 +319,10 @@ __global__ void __launch_bounds__(kEB) ke_disp_max(Ens e) {
 }
 
 __global__ void __launch_bounds__(kEB) ke_disp_collect(Ens e) {
-  const int total = e.wd.count[1];
-  for (int g = blockIdx.x * kEB + threadIdx.x; g < total; g += gridDim.x * kEB) {
+  WorkSweep sweep(e.wd, kEB);
+  for (int g = sweep.base + threadIdx.x; g < sweep.end; g += kEB) {
     int r;
-    const int i = work_atom(e, e.wd, g, &r);
+    const int i = sweep.atom(e, g, &r);
     RepStatus &st = e.rs[r];
     const double c = e.rep[r].buffer_length - sqrt(__longlong_as_double((long long)st.dr2max_bits));
     const double c_d2 = c * c;
@@ -324,7 +344,8 @@ __global__ void __launch_bounds__(kEB) ke_disp_collect(Ens e) {
 __global__ void __launch_bounds__(256) ke_disp_pairs(Ens e) {
   const int r = blockIdx.x;
   RepStatus &st = e.rs[r];
-  if (!st.disp) return;
+  // a short candidate list takes one block (its rows are 256 columns wide)
+  if (!st.disp || (blockIdx.y > 0 && st.cand_n <= kEPairShort)) return;
   __shared__ PairStage sm;
   __shared__ volatile int found;
   if (threadIdx.x == 0) found = 0;
@@ -337,7 +358,7 @@ __global__ void __launch_bounds__(256) ke_disp_pairs(Ens e) {
   } else {
     const int l = min(st.cand_n, e.cll);
     candidate_pair_test<256>(ens_view(e), rep.L, e.cand + (size_t)r * e.cll, l, e.lag, rep.sl2, e.rc2, blockIdx.y,
-                             gridDim.y, sm, &found);
+                             l <= kEPairShort ? 1 : gridDim.y, sm, &found);
   }
   __syncthreads();
   if (threadIdx.x == 0 && found) st.want_build = 1;
@@ -407,10 +428,10 @@ __device__ __forceinline__ void cell_assign_atom(const Ens &e, int r, int i) {
 // Atoms of the rebuilding replicas (rebuild work list) from here to ke_build.
 __global__ void __launch_bounds__(kEB) ke_cell_assign(Ens e) {
   if (*e.error) return;
-  const int total = e.wb.count[1];
-  for (int g = blockIdx.x * kEB + threadIdx.x; g < total; g += gridDim.x * kEB) {
+  WorkSweep sweep(e.wb, kEB);
+  for (int g = sweep.base + threadIdx.x; g < sweep.end; g += kEB) {
     int r;
-    const int i = work_atom(e, e.wb, g, &r);
+    const int i = sweep.atom(e, g, &r);
     cell_assign_atom(e, r, i);
   }
 }
@@ -444,10 +465,10 @@ __global__ void __launch_bounds__(kEB) ke_scan_cells(Ens e) {
 
 __global__ void __launch_bounds__(kEB) ke_scatter(Ens e) {
   if (*e.error) return;
-  const int total = e.wb.count[1];
-  for (int g = blockIdx.x * kEB + threadIdx.x; g < total; g += gridDim.x * kEB) {
+  WorkSweep sweep(e.wb, kEB);
+  for (int g = sweep.base + threadIdx.x; g < sweep.end; g += kEB) {
     int r;
-    const int i = work_atom(e, e.wb, g, &r);
+    const int i = sweep.atom(e, g, &r);
     e.perm[e.cell_start[e.cell[i]] + e.slot[i]] = i;
   }
 }
@@ -474,17 +495,28 @@ __global__ void __launch_bounds__(kEB) ke_sort_cells(Ens e) {
   }
 }
 
+// Packs q + v dt/2 of atom i (the coming step's first half drift).
+__device__ __forceinline__ void pack_half(const Ens &e, const Rep &rep, int i, const double4 &q, const double4 &v,
+                                          int4 *pack, double *pack_z) {
+  const double dt2 = e.dt * 0.5;
+  pack_position(pack, pack_z, i, dadd(q.x, dmul(v.x, dt2)), dadd(q.y, dmul(v.y, dt2)), dadd(q.z, dmul(v.z, dt2)),
+                rep.L);
+}
+
 // Gathers the atom that goes to slot s of replica r into the temporary
 // arrays, snapshots q_old (PairList::Init), its ghost-strip membership and
-// cell-local coordinates; returns its copy count (atom + ghost images).
-__device__ __forceinline__ int permute_atom(const Ens &e, int r, int s) {
+// cell-local coordinates; returns its copy count (atom + ghost images).  pack
+// (may be null): the coming step's first-drift positions.
+__device__ __forceinline__ int permute_atom(const Ens &e, int r, int s, int4 *pack, double *pack_z) {
   const Rep rep = e.rep[r];
   const Box b = box_of(e, rep);
   const int o = e.perm2[s];
   const double4 q = e.q[o];
+  const double4 v = e.v[o];
   e.q_tmp[s] = q;
-  e.v_tmp[s] = e.v[o];
+  e.v_tmp[s] = v;
   e.ids_tmp[s] = e.ids[o];
+  if (pack) pack_half(e, rep, s, q, v, pack, pack_z);
   const int cg = e.cell[o];
   e.cell_tmp[s] = cg;
   e.q_old[s] = q;
@@ -500,16 +532,16 @@ __device__ __forceinline__ int permute_atom(const Ens &e, int r, int s) {
   return m;
 }
 
-__global__ void __launch_bounds__(kEB) ke_permute(Ens e) {
+__global__ void __launch_bounds__(kEB) ke_permute(Ens e, int4 *pack, double *pack_z) {
   const bool err = *e.error != 0;
-  const int total = e.wb.count[1];
-  for (int base = blockIdx.x * kEB; base < total; base += gridDim.x * kEB) {
+  WorkSweep sweep(e.wb, kEB);
+  for (int base = sweep.base; base < sweep.end; base += kEB) {
     const int g = base + threadIdx.x;
-    const bool active = g < total && !err;
+    const bool active = g < sweep.end && !err;
     int r = 0, m = 0;
     if (active) {
-      const int s = work_atom(e, e.wb, g, &r);
-      m = permute_atom(e, r, s);
+      const int s = sweep.atom(e, g, &r);
+      m = permute_atom(e, r, s, pack, pack_z);
     }
     rep_add(&e.rs[0].total_images, sizeof(RepStatus), r, m, active);
   }
@@ -517,10 +549,10 @@ __global__ void __launch_bounds__(kEB) ke_permute(Ens e) {
 
 __global__ void __launch_bounds__(kEB) ke_copy_back(Ens e) {
   if (*e.error) return;
-  const int total = e.wb.count[1];
-  for (int g = blockIdx.x * kEB + threadIdx.x; g < total; g += gridDim.x * kEB) {
+  WorkSweep sweep(e.wb, kEB);
+  for (int g = sweep.base + threadIdx.x; g < sweep.end; g += kEB) {
     int r;
-    const int s = work_atom(e, e.wb, g, &r);
+    const int s = sweep.atom(e, g, &r);
     e.q[s] = e.q_tmp[s];
     e.v[s] = e.v_tmp[s];
     e.ids[s] = e.ids_tmp[s];
@@ -584,17 +616,19 @@ __device__ __forceinline__ int small_row(const Ens &e, const Rep &rep, int i) {
 // single-system build makes them (build_rows_warp; small_row for replicas
 // narrower than three cells); a warp's 32 atoms may belong to several
 // replicas.  Block-uniform sweeps, so every lane reaches the warp's votes.
-__global__ void __launch_bounds__(kEF, 768 / kEF) ke_build(Ens e) {
+__global__ void __launch_bounds__(kEF, 1024 / kEF) ke_build(Ens e) {
   __shared__ WarpRows rows[kEF / 32];
   const int w = threadIdx.x >> 5;
+  if (__shfl_sync(0xffffffffu, *(volatile const int *)e.error, 0)) return;
+  WorkSweep sweep(e.wb, kEF);
   const int total = e.wb.count[1];
-  if (total == 0 || __shfl_sync(0xffffffffu, *(volatile const int *)e.error, 0)) return;
+  // strided, not in shares: rows of dense replicas take longer
   for (int base = blockIdx.x * kEF; base < total; base += gridDim.x * kEF) {
     const int g = base + threadIdx.x;
     if (base + w * 32 >= total) return;  // whole warps leave together
     const bool active = g < total;
     int r = 0;
-    const int i = work_atom(e, e.wb, min(g, total - 1), &r);
+    const int i = sweep.atom(e, min(g, total - 1), &r);
     const Rep &rep = e.rep[r];
     const bool cells = active && !rep.small;
     int cnt = 0;
@@ -625,43 +659,55 @@ __global__ void ke_build_done(Ens e) {
 }
 
 // ------------------------------------------------------------- integrate
-template <bool FIX>
-__global__ void __launch_bounds__(kEB) ke_drift(Ens e, int track_vmax) {
+// Packs every atom's coming first-drift position.
+__global__ void __launch_bounds__(kEB) ke_pack_half(Ens e, int4 *pack, double *pack_z) {
   const int i = blockIdx.x * kEB + threadIdx.x;
-  int r = 0;
-  double v2 = 0.0;
-  const bool active = i < e.ntot && !*e.error;
-  if (active) {
-    r = e.rep_of[i];
-    const double dt2 = e.dt * 0.5;
-    double4 q = e.q[i];
-    const double4 v = e.v[i];
-    q.x = dadd(q.x, dmul(v.x, dt2));
-    q.y = dadd(q.y, dmul(v.y, dt2));
-    q.z = dadd(q.z, dmul(v.z, dt2));
-    e.q[i] = q;
-    if (FIX) {
-      const Rep &rep = e.rep[r];
-      e.qfix[i] = make_int4(fixed_coord(q.x, rep.L[0]), fixed_coord(q.y, rep.L[1]), fixed_coord(q.z, rep.L[2]), 0);
-    }
-    if (track_vmax) {
-      v2 = dadd(dadd(dmul(v.x, v.x), dmul(v.y, v.y)), dmul(v.z, v.z));
-      if (!isfinite(v2) || !isfinite(q.x + q.y + q.z)) atomicOr(e.error, kErrNonFinite);
-    }
-  }
-  if (track_vmax) rep_max(&e.rs[0].vmax2_bits, sizeof(RepStatus), r, v2, active);
+  if (i >= e.ntot || *e.error) return;
+  pack_half(e, e.rep[e.rep_of[i]], i, e.q[i], e.v[i], pack, pack_z);
 }
 
-// FP32-mixed kick with the second half drift fused (the single-system
-// k_force_fp32 loop on the replica's fixed-point scale).
+// End of an atom's NVE step: its own first half drift (the partners' packed
+// copies already have it), the kick (fx, fy, fz), the second half drift and
+// the pack of the next step's first-drift position; returns |v|^2.
+__device__ __forceinline__ double finish_step(const Ens &e, const Rep &rep, int i, double fx, double fy, double fz,
+                                              int4 *next, double *next_z) {
+  const double dt2 = e.dt * 0.5;
+  double4 v = e.v[i], q = e.q[i];
+  q.x = dadd(q.x, dmul(v.x, dt2));
+  q.y = dadd(q.y, dmul(v.y, dt2));
+  q.z = dadd(q.z, dmul(v.z, dt2));
+  v.x = dadd(v.x, fx);
+  v.y = dadd(v.y, fy);
+  v.z = dadd(v.z, fz);
+  e.v[i] = v;
+  q.x = dadd(q.x, dmul(v.x, dt2));
+  q.y = dadd(q.y, dmul(v.y, dt2));
+  q.z = dadd(q.z, dmul(v.z, dt2));
+  e.q[i] = q;
+  const double v2 = dadd(dadd(dmul(v.x, v.x), dmul(v.y, v.y)), dmul(v.z, v.z));
+  if (!isfinite(v2) || !isfinite(q.x + q.y + q.z)) atomicOr(e.error, kErrNonFinite);
+  pack_half(e, rep, i, q, v, next, next_z);
+  return v2;
+}
+
+// The step counters; nothing else in a step's pass reads them.
+__device__ __forceinline__ void count_step(const Ens &e, int err) {
+  if (blockIdx.x == 0 && !err)
+    for (int r = threadIdx.x; r < e.nrep; r += blockDim.x) e.rs[r].steps++;
+}
+
+// The whole FP32-mixed NVE step of every replica (k_force_fp32 with DRIFT 2 on
+// the replica's fixed-point scale).  The separate drift and counter kernels
+// that it replaced took 45 us of the 256-replica step.
 template <int TPA>
-__global__ void __launch_bounds__(kEF) ke_force_fp32(Ens e) {
+__global__ void __launch_bounds__(kEF) ke_force_fp32(Ens e, const int4 *qf, int4 *next) {
   const int t = blockIdx.x * kEF + threadIdx.x;
   const int i = t / TPA, sub = t % TPA;
   int r = 0;
   double v2 = 0.0;
   // the lanes of an atom exchange chunk sums: they agree on the error flag
   const int err = __shfl_sync(0xffffffffu, *(volatile const int *)e.error, 0);
+  count_step(e, err);
   const bool active = i < e.ntot && !err;
   double Fx = 0.0, Fy = 0.0, Fz = 0.0;
   if (active) {
@@ -669,113 +715,98 @@ __global__ void __launch_bounds__(kEF) ke_force_fp32(Ens e) {
     const Rep &rep = e.rep[r];
     // positions not loaded a group ahead: at 64 registers this pass is
     // faster without (0.324 vs 0.353 ms on the 256-replica ensemble)
-    GlobalGroups<false> f{e.nbr + i, e.stride, e.qfix, i};
-    fp32_row<TPA>(f, (e.nnbr[i] + 3) >> 2, sub, e.qfix[i], pair_const(rep.fix_scale, e.rc2f, e.c2x8f), Fx, Fy, Fz);
-  }
-  if (active && sub == 0) {
+    GlobalGroups<false> f{e.nbr + i, e.stride, qf, i};
+    fp32_row<TPA>(f, (e.nnbr[i] + 3) >> 2, sub, qf[i], pair_const(rep.fix_scale, e.rc2f, e.c2x8f), Fx, Fy, Fz);
     const double dt = e.dt;
-    double4 v = e.v[i];
-    v.x = dadd(v.x, Fx * dt);
-    v.y = dadd(v.y, Fy * dt);
-    v.z = dadd(v.z, Fz * dt);
-    e.v[i] = v;
-    double4 q = e.q[i];
-    const double dt2 = dt * 0.5;
-    q.x = dadd(q.x, dmul(v.x, dt2));
-    q.y = dadd(q.y, dmul(v.y, dt2));
-    q.z = dadd(q.z, dmul(v.z, dt2));
-    e.q[i] = q;
-    v2 = dadd(dadd(dmul(v.x, v.x), dmul(v.y, v.y)), dmul(v.z, v.z));
-    if (!isfinite(v2) || !isfinite(q.x + q.y + q.z)) atomicOr(e.error, kErrNonFinite);
+    if (sub == 0) v2 = finish_step(e, rep, i, Fx * dt, Fy * dt, Fz * dt, next, nullptr);
   }
   rep_max(&e.rs[0].vmax2_bits, sizeof(RepStatus), r, v2, active);  // v2 = 0 on lanes other than 0
 }
 
-// FP64 kick (the single-system k_force_fp64 pair terms).
-__global__ void __launch_bounds__(kEF) ke_force_fp64(Ens e) {
-  const int i = blockIdx.x * kEF + threadIdx.x;
-  if (i >= e.ntot || *e.error) return;
-  const Rep &rep = e.rep[e.rep_of[i]];
-  const double4 qi = e.q[i];
-  const int nn = e.nnbr[i];
-  const double c2x8 = e.c2 * 8.0;
-  const double dt = e.dt;
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  const int *row = e.nbr + i;
-  int j = nn > 0 ? row[0] : 0;
-  for (int k = 0; k < nn; k++) {
-    const int jn = (k + 1 < nn) ? row[(size_t)(k + 1) * e.stride] : 0;
-    const double4 qj = e.q[j];
-    const double dx = dsub(image_of(qj.x, qi.x, rep.L[0], rep.hL[0]), qi.x);
-    const double dy = dsub(image_of(qj.y, qi.y, rep.L[1], rep.hL[1]), qi.y);
-    const double dz = dsub(image_of(qj.z, qi.z, rep.L[2], rep.hL[2]), qi.z);
-    const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-    j = jn;
-    if (r2 > e.rc2) continue;
-    const double r6 = dmul(dmul(r2, r2), r2);
-    const double df = dmul(dadd(ddiv(dsub(dmul(24.0, r6), 48.0), dmul(dmul(r6, r6), r2)), c2x8), dt);
-    fx = dadd(fx, dmul(df, dx));
-    fy = dadd(fy, dmul(df, dy));
-    fz = dadd(fz, dmul(df, dz));
-  }
-  double4 v = e.v[i];
-  v.x = dadd(v.x, fx);
-  v.y = dadd(v.y, fy);
-  v.z = dadd(v.z, fz);
-  e.v[i] = v;
+// Whether some partner of an atom sits beyond a face of its replica (row_wraps).
+__device__ __forceinline__ bool ens_wraps(const Ens &e, const Rep &rep, int i) {
+  return rep.small || row_wraps(rep.ms, 0, e.cxyz[i]);
 }
 
-__global__ void ke_step_done(Ens e) {
-  if (*e.error) return;
-  for (int r = threadIdx.x; r < e.nrep; r += blockDim.x) e.rs[r].steps++;
+// The whole FP64 NVE step of every replica (k_force_fp64 with DRIFT 2).
+template <int TPA>
+__global__ void __launch_bounds__(kEF, kFp64Blocks) ke_force_fp64(Ens e, PosSplit pos, int4 *next, double *next_z) {
+  const int t = blockIdx.x * kEF + threadIdx.x;
+  const int i = t / TPA, sub = t % TPA;
+  double v2 = 0.0;
+  const int err = __shfl_sync(0xffffffffu, *(volatile const int *)e.error, 0);
+  count_step(e, err);
+  const bool active = i < e.ntot && !err;
+  const int ii = i < e.ntot ? i : 0;
+  const int r = e.rep_of[ii];
+  const Rep &rep = e.rep[r];
+  const Fp64Pair f{rep.L, rep.hL, e.rc2, e.c2 * 8.0, e.dt, pos.at(ii)};
+  double s[3];
+  fp64_force_row<TPA>(pos, e.nbr, e.stride, active ? e.nnbr[ii] : 0, ii, sub, f, active && ens_wraps(e, rep, ii), s);
+  if (active && sub == 0) v2 = finish_step(e, rep, i, s[0], s[1], s[2], next, next_z);
+  rep_max(&e.rs[0].vmax2_bits, sizeof(RepStatus), r, v2, active);
+}
+
+// A double into the replica's sum, one atomic per warp whose active lanes
+// share one replica, else one per active lane.  All lanes must call.
+__device__ __forceinline__ void rep_sum(double *slot, int r, double v, bool active) {
+  const int rr = active ? r : -1;
+  const int r0 = __shfl_sync(0xffffffffu, rr, 0);
+  if (__all_sync(0xffffffffu, rr == r0 || rr < 0) && r0 >= 0) {
+    v = warp_sum(active ? v : 0.0);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&slot[3 * r0], v);
+  } else if (active) {
+    atomicAdd(&slot[3 * r], v);
+  }
 }
 
 // Observer sums per replica (KE, PE, virial x 3), pair terms as k_observe.
-__global__ void __launch_bounds__(kEB) ke_observe(Ens e) {
-  const int i = blockIdx.x * kEB + threadIdx.x;
-  if (i >= e.ntot) return;
-  const int r = e.rep_of[i];
+// Three atomics an atom to 256 x 3 addresses took 4.1 ms for 2.5M atoms.
+template <int TPA>
+__global__ void __launch_bounds__(kEF, kFp64Blocks) ke_observe(Ens e) {
+  const int t = blockIdx.x * kEF + threadIdx.x;
+  const int i = t / TPA, sub = t % TPA;
+  const bool active = i < e.ntot;
+  const int ii = active ? i : 0;
+  const int r = e.rep_of[ii];
   const Rep &rep = e.rep[r];
-  const double4 v = e.v[i];
+  const double4 qi = e.q[ii];
+  const int nn = active ? e.nnbr[ii] : 0;
+  double s[2];
+  if (__any_sync(0xffffffffu, (int)(active && ens_wraps(e, rep, ii))))
+    fp64_row<TPA>(PosState{e.q}, e.nbr, e.stride, nn, ii, sub, s,
+                  [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[2]) {
+                    observe_pairs<true>(rep.L, rep.hL, e.rc2, e.c0, e.c2, qi, p, in, u);
+                  });
+  else
+    fp64_row<TPA>(PosState{e.q}, e.nbr, e.stride, nn, ii, sub, s,
+                  [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[2]) {
+                    observe_pairs<false>(rep.L, rep.hL, e.rc2, e.c0, e.c2, qi, p, in, u);
+                  });
+  const bool first = active && sub == 0;
+  const double4 v = e.v[ii];
   const double ke = dadd(dadd(dmul(dmul(0.5, v.x), v.x), dmul(dmul(0.5, v.y), v.y)), dmul(dmul(0.5, v.z), v.z));
-  const double4 qi = e.q[i];
-  double pe = 0.0, vir = 0.0;
-  const int nn = e.nnbr[i];
-  for (int k = 0; k < nn; k++) {
-    const double4 qj = e.q[e.nbr[(size_t)k * e.stride + i]];
-    const double dx = dsub(qi.x, image_of(qj.x, qi.x, rep.L[0], rep.hL[0]));
-    const double dy = dsub(qi.y, image_of(qj.y, qi.y, rep.L[1], rep.hL[1]));
-    const double dz = dsub(qi.z, image_of(qj.z, qi.z, rep.L[2], rep.hL[2]));
-    const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-    if (r2 > e.rc2) continue;
-    const double r4 = dmul(r2, r2), r6 = dmul(r4, r2), r8 = dmul(r6, r2), r10 = dmul(r8, r2), r12 = dmul(r10, r2);
-    pe = dadd(pe, dmul(4.0, dadd(dadd(dsub(ddiv(1.0, r12), ddiv(1.0, r6)), dmul(e.c2, r2)), e.c0)));
-    vir = dadd(vir, dmul(dadd(ddiv(dsub(dmul(24.0, r6), 48.0), dmul(dmul(r6, r6), r2)), e.c2 * 8.0), r2));
-  }
-  atomicAdd(&e.sums[3 * r + 0], ke);
-  atomicAdd(&e.sums[3 * r + 1], 0.5 * pe);
-  atomicAdd(&e.sums[3 * r + 2], 0.5 * vir);
+  rep_sum(e.sums + 0, r, first ? ke : 0.0, active);
+  rep_sum(e.sums + 1, r, first ? 0.5 * s[0] : 0.0, active);
+  rep_sum(e.sums + 2, r, first ? 0.5 * s[1] : 0.0, active);
 }
 
 // Ordered pairs with r^2 <= rc^2 over the current lists (the FP64 pair
 // test of the force and observer kernels), summed over all replicas.
-__global__ void __launch_bounds__(kEB) ke_count_pairs(Ens e, unsigned long long *count) {
-  const int i = blockIdx.x * kEB + threadIdx.x;
-  int c = 0;
-  if (i < e.ntot) {
-    const Rep &rep = e.rep[e.rep_of[i]];
-    const double4 qi = e.q[i];
-    const int nn = e.nnbr[i];
-    for (int k = 0; k < nn; k++) {
-      const double4 qj = e.q[e.nbr[(size_t)k * e.stride + i]];
-      const double dx = dsub(image_of(qj.x, qi.x, rep.L[0], rep.hL[0]), qi.x);
-      const double dy = dsub(image_of(qj.y, qi.y, rep.L[1], rep.hL[1]), qi.y);
-      const double dz = dsub(image_of(qj.z, qi.z, rep.L[2], rep.hL[2]), qi.z);
-      const double r2 = dadd(dadd(dmul(dx, dx), dmul(dy, dy)), dmul(dz, dz));
-      c += r2 <= e.rc2;
-    }
-  }
-  const int w = __reduce_add_sync(0xffffffffu, c);
+template <int TPA>
+__global__ void __launch_bounds__(kEF, kFp64Blocks) ke_count_pairs(Ens e, unsigned long long *count) {
+  const int t = blockIdx.x * kEF + threadIdx.x;
+  const int i = t / TPA, sub = t % TPA;
+  const bool active = i < e.ntot;
+  const int ii = active ? i : 0;
+  const Rep &rep = e.rep[e.rep_of[ii]];
+  const double4 qi = e.q[ii];
+  double s[1];
+  fp64_row<TPA>(PosState{e.q}, e.nbr, e.stride, active ? e.nnbr[ii] : 0, ii, sub, s,
+                [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[1]) {
+                  count_pairs<true>(rep.L, rep.hL, e.rc2, qi, p, in, u);
+                });
+  const int w = __reduce_add_sync(0xffffffffu, sub == 0 ? (int)s[0] : 0);
   if ((threadIdx.x & 31) == 0 && w) atomicAdd(count, (unsigned long long)w);
 }
 
@@ -829,6 +860,7 @@ struct mdg_ensemble {
   // step uses); the forces are bit-identical for every choice
   int tpa = 0;
   int tune_lanes = 1;
+  int fix_buf = -1;  // which packed copy (0, 1) holds the coming step's positions; -1: none
   float tune_ms[3] = {0.f, 0.f, 0.f};
 };
 
@@ -846,7 +878,8 @@ cudaError_t edalloc(T **p, size_t count) {
 
 void e_free(mdg_ensemble *x) {
   Ens &e = x->e;
-  void *ptrs[] = {(void *)e.rep, e.rs, (void *)e.rep_of, e.q, e.v, e.q_old, e.qfix, e.qloc, e.cxyz, e.xsub, e.ids, e.cell,
+  void *ptrs[] = {(void *)e.rep, e.rs, (void *)e.rep_of, e.q, e.v, e.q_old, e.qfix, e.qfix2, e.pz, e.pz2, e.qloc, e.cxyz,
+                  e.xsub, e.ids, e.cell,
                   e.cell_tmp, e.nbr, e.nnbr, e.cell_count, e.cell_start, e.slot, e.perm, e.perm2, e.q_tmp,
                   e.v_tmp, e.ids_tmp, e.mult, e.cand, e.disp2, e.error, e.sums, x->d_flags, x->d_count,
                   x->d_lists};
@@ -855,6 +888,11 @@ void e_free(mdg_ensemble *x) {
   if (x->exec) cudaGraphExecDestroy(x->exec);
   x->exec = nullptr;
 }
+
+int lane_blocks(int n, int lanes) { return (int)(((long long)n * lanes + kEF - 1) / kEF); }
+
+int4 *e_pack(const Ens &e, int k) { return k ? e.qfix2 : e.qfix; }
+double *e_pack_z(const Ens &e, int k) { return k ? e.pz2 : e.pz; }
 
 // Kernels launched by one skin-check and one rebuild branch.
 constexpr int kEDispKernels = 4, kEBuildKernels = 10;
@@ -870,7 +908,9 @@ void e_launch_disp(mdg_ensemble *x, cudaStream_t s) {
   ke_disp_pairs<<<dim3(e.nrep, kEPairParts), 256, 0, s>>>(e);
 }
 
-void e_launch_build(mdg_ensemble *x, cudaStream_t s) {
+// pack: the packed copy that the coming step reads (0, 1), refreshed for the
+// rebuilt replicas' atoms; -1: none.
+void e_launch_build(mdg_ensemble *x, cudaStream_t s, int pack) {
   Ens &e = x->e;
   const int gb = std::min(nb(e.ntot, kEB), x->work_blocks);
   const int gf = std::min(nb(e.ntot, kEF), 2 * x->work_blocks);
@@ -881,7 +921,7 @@ void e_launch_build(mdg_ensemble *x, cudaStream_t s) {
   ke_scan_cells<<<e.nrep, kEB, 0, s>>>(e);
   ke_scatter<<<gb, kEB, 0, s>>>(e);
   ke_sort_cells<<<gc, kEB, 0, s>>>(e);
-  ke_permute<<<gb, kEB, 0, s>>>(e);
+  ke_permute<<<gb, kEB, 0, s>>>(e, pack < 0 ? nullptr : e_pack(e, pack), pack < 0 ? nullptr : e_pack_z(e, pack));
   ke_copy_back<<<gb, kEB, 0, s>>>(e);
   ke_build<<<gf, kEF, 0, s>>>(e);
   ke_build_done<<<1, 1024, 0, s>>>(e);
@@ -890,7 +930,8 @@ void e_launch_build(mdg_ensemble *x, cudaStream_t s) {
 // The step after the skin decision; e0/e1 (optional) bracket the force
 // kernel.  Inside a stream capture an event record must be external to be
 // recorded when the graph runs (a plain record only orders the capture).
-int e_launch_tail(mdg_ensemble *x, cudaStream_t s, cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr,
+// parity: the packed copy the step reads (it writes the other).
+int e_launch_tail(mdg_ensemble *x, cudaStream_t s, int parity, cudaEvent_t e0 = nullptr, cudaEvent_t e1 = nullptr,
                   bool capture = false) {
   Ens &e = x->e;
   auto rec = [&](cudaEvent_t ev) {
@@ -898,25 +939,25 @@ int e_launch_tail(mdg_ensemble *x, cudaStream_t s, cudaEvent_t e0 = nullptr, cud
     if (capture) cudaEventRecordWithFlags(ev, s, cudaEventRecordExternal);
     else cudaEventRecord(ev, s);
   };
-  if (x->prm.precision == MDG_FP32_MIXED) {
-    ke_drift<true><<<nb(e.ntot, kEB), kEB, 0, s>>>(e, 0);
-    rec(e0);
-    const int lanes = x->tpa > 0 ? x->tpa : x->tune_lanes;
-    const int blocks = (int)(((long long)e.ntot * lanes + kEF - 1) / kEF);
-    if (lanes == 4) ke_force_fp32<4><<<blocks, kEF, 0, s>>>(e);
-    else if (lanes == 2) ke_force_fp32<2><<<blocks, kEF, 0, s>>>(e);
-    else ke_force_fp32<1><<<blocks, kEF, 0, s>>>(e);
-    rec(e1);
-    ke_step_done<<<1, 1024, 0, s>>>(e);
-    return 3;
-  }
-  ke_drift<false><<<nb(e.ntot, kEB), kEB, 0, s>>>(e, 0);
+  const int4 *now = e_pack(e, parity);
+  int4 *next = e_pack(e, 1 - parity);
   rec(e0);
-  ke_force_fp64<<<nb(e.ntot, kEF), kEF, 0, s>>>(e);
+  if (x->prm.precision == MDG_FP32_MIXED) {
+    const int lanes = x->tpa > 0 ? x->tpa : x->tune_lanes;
+    const int blocks = lane_blocks(e.ntot, lanes);
+    if (lanes == 4) ke_force_fp32<4><<<blocks, kEF, 0, s>>>(e, now, next);
+    else if (lanes == 2) ke_force_fp32<2><<<blocks, kEF, 0, s>>>(e, now, next);
+    else ke_force_fp32<1><<<blocks, kEF, 0, s>>>(e, now, next);
+  } else {
+    const PosSplit pos{reinterpret_cast<const double2 *>(now), e_pack_z(e, parity)};
+    double *next_z = e_pack_z(e, 1 - parity);
+    const int lanes = fp64_lanes(e.ntot), blocks = lane_blocks(e.ntot, lanes);
+    if (lanes == 8) ke_force_fp64<8><<<blocks, kEF, 0, s>>>(e, pos, next, next_z);
+    else if (lanes == 4) ke_force_fp64<4><<<blocks, kEF, 0, s>>>(e, pos, next, next_z);
+    else ke_force_fp64<1><<<blocks, kEF, 0, s>>>(e, pos, next, next_z);
+  }
   rec(e1);
-  ke_drift<false><<<nb(e.ntot, kEB), kEB, 0, s>>>(e, 1);
-  ke_step_done<<<1, 1024, 0, s>>>(e);
-  return 4;
+  return 1;
 }
 
 void e_destroy_events(mdg_ensemble *x) {
@@ -997,11 +1038,11 @@ mdg_status e_build_graph(mdg_ensemble *x) {
     {
       ECapture bc{x->cap_stream, body, {}};
       ECUDA(e_begin(bc));
-      e_launch_build(x, bc.s);
+      e_launch_build(x, bc.s, s & 1);
       ECUDA(e_end(bc));
     }
     ECUDA(e_begin(c));
-    kernels += 2 + e_launch_tail(x, c.s, x->timing ? x->ev[2 * s] : nullptr,
+    kernels += 2 + e_launch_tail(x, c.s, s & 1, x->timing ? x->ev[2 * s] : nullptr,
                                  x->timing ? x->ev[2 * s + 1] : nullptr, true);
     ECUDA(e_end(c));
   }
@@ -1013,8 +1054,17 @@ mdg_status e_build_graph(mdg_ensemble *x) {
   return MDG_OK;
 }
 
+// Packs the coming step's positions into copy 0 (not one of the counted
+// step kernels).
+void e_pack_now(mdg_ensemble *x) {
+  ke_pack_half<<<nb(x->e.ntot, kEB), kEB, 0, x->stream>>>(x->e, x->e.qfix, x->e.pz);
+  x->fix_buf = 0;
+}
+
 mdg_status e_step_eager(mdg_ensemble *x, float *force_ms_out = nullptr) {
   int flags[2] = {0, 0};
+  const int parity = x->fix_buf > 0 ? 1 : 0;
+  if (x->fix_buf < 0) e_pack_now(x);
   ke_expiry<<<1, 1024, 0, x->stream>>>(x->e, 0, 0, x->d_flags);
   ECUDA(cudaMemcpyAsync(flags, x->d_flags, sizeof flags, cudaMemcpyDeviceToHost, x->stream));
   ECUDA(cudaStreamSynchronize(x->stream));
@@ -1024,14 +1074,15 @@ mdg_status e_step_eager(mdg_ensemble *x, float *force_ms_out = nullptr) {
   ECUDA(cudaMemcpyAsync(flags, x->d_flags, sizeof flags, cudaMemcpyDeviceToHost, x->stream));
   ECUDA(cudaStreamSynchronize(x->stream));
   x->kernel_launches++;
-  if (flags[1]) e_launch_build(x, x->stream);  // counted on the device (ke_decide)
+  if (flags[1]) e_launch_build(x, x->stream, parity);  // counted on the device (ke_decide)
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   const bool timed = x->timing || force_ms_out;
   if (timed) {
     ECUDA(cudaEventCreate(&e0));
     ECUDA(cudaEventCreate(&e1));
   }
-  x->kernel_launches += e_launch_tail(x, x->stream, e0, e1);
+  x->kernel_launches += e_launch_tail(x, x->stream, parity, e0, e1);
+  x->fix_buf = 1 - parity;
   ECUDA(cudaGetLastError());
   if (timed) {
     float ms = 0.f;
@@ -1206,6 +1257,9 @@ mdg_status mdg_ensemble_create(const mdg_params *prm, int nrep, const mdg_replic
   if (err == cudaSuccess) err = edalloc(&e.v, n);
   if (err == cudaSuccess) err = edalloc(&e.q_old, n);
   if (err == cudaSuccess) err = edalloc(&e.qfix, n);
+  if (err == cudaSuccess) err = edalloc(&e.qfix2, n);
+  if (err == cudaSuccess && prm->precision == MDG_FP64) err = edalloc(&e.pz, n);
+  if (err == cudaSuccess && prm->precision == MDG_FP64) err = edalloc(&e.pz2, n);
   if (err == cudaSuccess) err = edalloc(&e.qloc, n);
   if (err == cudaSuccess) err = edalloc(&e.cxyz, n);
   if (err == cudaSuccess) err = edalloc(&e.xsub, (size_t)tab_entries);
@@ -1289,6 +1343,7 @@ mdg_status mdg_ensemble_set_state(mdg_ensemble *x, const double *q4, const doubl
   ECUDA(cudaSetDevice(x->prm.device));
   ECUDA(cudaStreamSynchronize(x->stream));
   const int n = e.ntot;
+  x->fix_buf = -1;
   ECUDA(cudaMemcpyAsync(e.q, q4, sizeof(double4) * n, cudaMemcpyHostToDevice, x->stream));
   ECUDA(cudaMemcpyAsync(e.v, v4, sizeof(double4) * n, cudaMemcpyHostToDevice, x->stream));
   std::vector<int> ids(n);
@@ -1373,6 +1428,7 @@ mdg_status mdg_ensemble_calculate(mdg_ensemble *x, int nsteps) {
     if (x->use_graphs && left >= kEStepsPerGraph && x->graph_dirty) {
       if ((r = e_build_graph(x))) return r;
     }
+    if (x->use_graphs && left >= kEStepsPerGraph && x->fix_buf != 0) e_pack_now(x);  // the graph's first step reads copy 0
     while (x->use_graphs && left >= kEStepsPerGraph) {
       ECUDA(cudaGraphLaunch(x->exec, x->stream));
       x->kernel_launches += x->graph_kernels;
@@ -1420,12 +1476,16 @@ mdg_status mdg_ensemble_observe(mdg_ensemble *x, double *ke, double *pe, double 
   if (stale) {
     for (auto &s : rs) s.build = s.list_stale;
     ECUDA(cudaMemcpyAsync(e.rs, rs.data(), sizeof(RepStatus) * e.nrep, cudaMemcpyHostToDevice, x->stream));
-    e_launch_build(x, x->stream);
+    x->fix_buf = -1;  // the rebuild renumbers the atoms
+    e_launch_build(x, x->stream, -1);
     if ((r = e_status(x, &err, &rs))) return r;
     if (err) return e_translate(err);
   }
   ECUDA(cudaMemsetAsync(e.sums, 0, sizeof(double) * 3 * e.nrep, x->stream));
-  ke_observe<<<nb(e.ntot, kEB), kEB, 0, x->stream>>>(e);
+  const int lanes = fp64_lanes(e.ntot), blocks = lane_blocks(e.ntot, lanes);
+  if (lanes == 8) ke_observe<8><<<blocks, kEF, 0, x->stream>>>(e);
+  else if (lanes == 4) ke_observe<4><<<blocks, kEF, 0, x->stream>>>(e);
+  else ke_observe<1><<<blocks, kEF, 0, x->stream>>>(e);
   std::vector<double> sums(3 * e.nrep);
   ECUDA(cudaMemcpyAsync(sums.data(), e.sums, sizeof(double) * 3 * e.nrep, cudaMemcpyDeviceToHost, x->stream));
   ECUDA(cudaStreamSynchronize(x->stream));
@@ -1485,7 +1545,10 @@ mdg_status mdg_ensemble_list_stats(mdg_ensemble *x, int64_t *list_entries, int64
   if (pairs_within_cutoff) {
     unsigned long long h = 0;
     ECUDA(cudaMemsetAsync(x->d_count, 0, sizeof(unsigned long long), x->stream));
-    ke_count_pairs<<<nb(e.ntot, kEB), kEB, 0, x->stream>>>(e, x->d_count);
+    const int lanes = fp64_lanes(e.ntot), blocks = lane_blocks(e.ntot, lanes);
+    if (lanes == 8) ke_count_pairs<8><<<blocks, kEF, 0, x->stream>>>(e, x->d_count);
+    else if (lanes == 4) ke_count_pairs<4><<<blocks, kEF, 0, x->stream>>>(e, x->d_count);
+    else ke_count_pairs<1><<<blocks, kEF, 0, x->stream>>>(e, x->d_count);
     ECUDA(cudaGetLastError());
     ECUDA(cudaMemcpyAsync(&h, x->d_count, sizeof h, cudaMemcpyDeviceToHost, x->stream));
     ECUDA(cudaStreamSynchronize(x->stream));

@@ -358,7 +358,7 @@ mdg_status rebuild(mdg_slabs *x) {
     k_scan_add<kSScan><<<ntiles, kSScan, 0, s>>>(a, sl.ncell, sl.d_tiles);
     k_scatter<kSB><<<sblocks(n, kSB), kSB, 0, s>>>(a, n);
     k_sort_cells<<<sblocks((long long)sl.ncell * 32, kSB), kSB, 0, s>>>(a, sl.box, sl.ncell);
-    k_permute<kSB><<<sblocks(n, kSB), kSB, 0, s>>>(a, sl.box, n, nullptr);
+    k_permute<kSB><<<sblocks(n, kSB), kSB, 0, s>>>(a, sl.box, n, nullptr, nullptr);
     SCUDA(x, cudaMemcpyAsync(a.q, a.q_tmp, sizeof(double4) * n, cudaMemcpyDeviceToDevice, s));
     SCUDA(x, cudaMemcpyAsync(a.v, a.v_tmp, sizeof(double4) * n, cudaMemcpyDeviceToDevice, s));
     SCUDA(x, cudaMemcpyAsync(a.ids, a.ids_tmp, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
@@ -576,7 +576,7 @@ mdg_status slab_step(mdg_slabs *x) {
       else if (x->tpa == 2) k_force_fp32<kSF, kKick, 1, 2><<<nb, kSF, 0, sl.stream>>>(sl.a, sl.box, n, th, sl.a.qfix, nullptr);
       else k_force_fp32<kSF, kKick, 1, 1><<<nb, kSF, 0, sl.stream>>>(sl.a, sl.box, n, th, sl.a.qfix, nullptr);
     } else {
-      k_force_fp64<kSF, kKick><<<sblocks(n, kSF), kSF, 0, sl.stream>>>(sl.a, sl.box, n, th);
+      k_force_fp64<kSF, kKick, 0, 1><<<sblocks(n, kSF), kSF, 0, sl.stream>>>(sl.a, sl.box, n, th, PosState{sl.a.q}, nullptr, nullptr);
       k_drift<kSB, false><<<sblocks(n, kSB), kSB, 0, sl.stream>>>(sl.a, sl.box, n, 1);
     }
   }
@@ -858,8 +858,8 @@ mdg_status mdg_slabs_observe(mdg_slabs *x, double *ke, double *pe, double *viria
   double out[3] = {0.0, 0.0, 0.0};
   for (Slab &sl : x->s) {
     SCUDA(x, cudaSetDevice(sl.dev));
-    const int nb = sblocks(sl.n_own, kSB);
-    k_observe<kSB><<<nb, kSB, 0, sl.stream>>>(sl.a, sl.box, sl.n_own, 0.0);
+    const int nb = sblocks(sl.n_own, kSF);
+    k_observe<kSF, 1><<<nb, kSF, 0, sl.stream>>>(sl.a, sl.box, sl.n_own, 0.0);
     k_final_sum<256, 3><<<1, 256, 0, sl.stream>>>(sl.a.partials, nb, sl.d_sums);
     double part[3];
     SCUDA(x, cudaMemcpyAsync(part, sl.d_sums, sizeof part, cudaMemcpyDeviceToHost, sl.stream));
@@ -888,7 +888,7 @@ mdg_status mdg_slabs_forces(mdg_slabs *x, double *f4, int n) {
     SCUDA(x, cudaSetDevice(sl.dev));
     const int m = sl.n_own;
     if (fp32) k_force_fp32<kSF, kForceOut, 0, 1><<<sblocks(m, kSF), kSF, 0, sl.stream>>>(sl.a, sl.box, m, th, sl.a.qfix, nullptr);
-    else k_force_fp64<kSF, kForceOut><<<sblocks(m, kSF), kSF, 0, sl.stream>>>(sl.a, sl.box, m, th);
+    else k_force_fp64<kSF, kForceOut, 0, 1><<<sblocks(m, kSF), kSF, 0, sl.stream>>>(sl.a, sl.box, m, th, PosState{sl.a.q}, nullptr, nullptr);
     std::vector<double4> hf(m);
     std::vector<int> hid(m);
     SCUDA(x, cudaMemcpyAsync(hf.data(), sl.a.v_tmp, sizeof(double4) * m, cudaMemcpyDeviceToHost, sl.stream));

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 
 import mdacp_b200 as M
+from mdacp_b200 import workloads as W
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +70,23 @@ def test_small_replica_sums(n, L):
     # sums of up to 2 x 10^4 positive and negative terms, each rounded a few times
     assert pe[0] == pytest.approx(np.sum(4 * (x ** -6 - x ** -3 + c2 * x + c0)), rel=1e-11)
     assert vir[0] == pytest.approx(np.sum(((24 * x ** 3 - 48) / x ** 7 + 8 * c2) * x) / 3, rel=1e-11)
+
+
+def test_fp64_sums_do_not_depend_on_the_lane_count():
+    # 864 atoms run with 8 lanes an atom, 11,664 with 4, the ensemble of all
+    # of them with 1 (over 65,536 atoms): the same trajectories bit for bit,
+    # rows short and long, with and without partners beyond a face
+    reps = [W.fcc_liquid(c, rho, 1.0, seed=c, jitter=0.05, rc=2.5, dt=0.005)
+            for c, rho in ((6, 0.3), (6, 0.8), ((18, 18, 9), 0.85), ((23, 24, 27), 0.6))]
+    assert sum(r.n for r in reps) > 65536
+    ens = M.Ensemble([(r.q, r.v, r.L) for r in reps], cutoff=2.5, time_step=0.005, precision=M.FP64)
+    ens.calculate(23)
+    got = ens.states_by_id()
+    ens.close()
+    for k, r in enumerate(reps):
+        s = M.System(r.L, cutoff=2.5, time_step=0.005, capacity=r.n, precision=M.FP64)
+        s.set_state(r.q, r.v)
+        s.calculate(23)
+        q, v = s.state_by_id()
+        s.close()
+        assert np.array_equal(got[k][0], q) and np.array_equal(got[k][1], v), f"replica {k}"
