@@ -25,15 +25,31 @@
 // (keeping q_h and v') before its reverse sweep.
 //
 // Pairs come from a Verlet list of search length r_c + skin (r_c = s_c
-// sigma; skin 0.3 sigma, less where the box is narrow), built from a cell
-// grid (cells at least r_c + skin wide, >= 3 per axis, atoms in each cell
-// ordered by index, rows in cell-walk order, so every sum is deterministic).
-// Before each evaluation every atom's displacement from the list's build
-// positions is checked; the list is rebuilt when one exceeds skin/2, which
-// keeps every pair within r_c in the rows.  This component has no
-// counterpart in the reference, which has no gradients.
+// sigma; skin 0.3 sigma, less where the box is narrow).  The kernel that makes
+// the positions of an evaluation also checks them against the list's build
+// positions, and the evaluation's kernel rebuilds the list first when an atom
+// has moved more than skin/2, which keeps every pair within r_c in the rows.
+// A row is ordered by (hash of the partner, partner): eight buckets of the
+// hash, which the lanes that share an atom divide among them, so that a lane's
+// pairs within r_c and their order are a function of the positions alone,
+// whichever build the row comes from.  This component has no counterpart in
+// the reference, which has no gradients.
+//
+// A gradient of 32,000 atoms x 200 steps takes 31 ms, of 500 atoms x 50 steps
+// 2.1 ms; with one kernel per operation (12 launches a step forward, 19 in
+// reverse), a one-block cell grid (170 us a rebuild, 180 more for the rows; 133
+// us in all here), roots and two divisions a pair and ballots to share out a
+// row they took 86 and 8.9 ms.  Per pass at 32,000 atoms: force 15 us (37),
+// loss with gradient 35 (51), Hessian 35 (47).
+//
+// One launch per evaluation: a step is a force pass (kick and both drifts in
+// its end), a loss pass (forward: the sums; reverse: the loss gradient and the
+// first half of the reverse step) and, in reverse, a Hessian pass (and the
+// second half).  The passes are cooperative launches because a rebuild inside
+// one has grid barriers; without a rebuild no block waits for another.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -43,142 +59,388 @@
 #include <vector>
 
 #include "mdacp_b200.h"
+#include "mdg_device.cuh"
 
 namespace {
 
-constexpr int kAB = 128;  // threads per block
+constexpr int kAB = 128;        // threads per block
+constexpr int kABlocks = 7;     // blocks an SM that the passes are held to (72 registers)
+constexpr int kBuckets = 8;     // hash buckets of a row
+constexpr int kReduceSlots = 32;  // steps whose block partials are kept before they are summed
 
 struct Pot {
-  double eps, sigma, rc2;       // energy scale, length scale, cut-off^2 (absolute)
+  double rc2;                   // cut-off^2 (absolute)
   double c0, c2;                // smoothed-LJ constants in units of sigma
-  double a, b, w;               // shell of the smoothed pair count
-  // reciprocals and quotients of the above, formed once on the host
-  double inv_sigma, inv_w, inv_eps, eps_sigma, eps_sigma2;  // 1/sigma, 1/w, 1/eps, eps/sigma, eps/sigma^2
+  double sigma2, inv_sigma, inv_sigma2, inv_eps;
+  double e4;                    // 4 eps
+  double k4;                    // 4 eps / sigma^2
+  double a, b, inv_w;           // shell of the smoothed pair count
+  double mid, h;                // (a + b) / 2, exp((a - b) / (2 w))
+  int one_exp;                  // the shell's exponents stay in range for every r < r_c: one exp per pair
 };
 
-struct Grid {
-  int ms[3];
-  double L[3], inv_cs[3], inv_L[3];
-  const int *start;   // ncell + 1
-  const int *perm;    // atoms in cell order
-  const double4 *qs;  // their positions in the same order (made with the grid)
+// n points: (x, y) pairs, then z.  24 bytes a gathered partner, spread over
+// all bank columns of the L1 (a 32-byte point leaves half of them unused).
+struct Vec {
+  double *p;
+  size_t ns;  // n rounded up to an even number
+  __device__ __forceinline__ double3 at(int i) const {
+    const double2 a = reinterpret_cast<const double2 *>(p)[i];
+    return make_double3(a.x, a.y, p[2 * ns + i]);
+  }
+  __device__ __forceinline__ void set(int i, const double3 &x) const {
+    reinterpret_cast<double2 *>(p)[i] = make_double2(x.x, x.y);
+    p[2 * ns + i] = x.z;
+  }
 };
 
-// The Verlet list: row of atom i = entries nbr[k * n + i], k < cnt[i].
-struct Rows {
-  const int *nbr;
-  const int *cnt;
-  double inv_L[3], L[3];
+// The cell grid and the Verlet list.  Row of atom i: nbr[i * maxnb + k], the
+// end of bucket b at ends[i * kBuckets + b].
+struct List {
+  int ms[3], ncell, maxnb, n;
+  double L[3], inv_L[3], inv_cs[3];
+  float Lf[3], inv_Lf[3], reach2;  // FP32 search: enlarged by the rounding of box coordinates
+  double half_skin2;
+  int *count, *start, *cell, *rank, *cursor;  // cells: atoms, first place; atoms: cell, place in it
+  float4 *sorted;                             // box coordinates and index in cell order
+  int *nbr;
+  unsigned short *ends;
+  Vec qb;                                     // positions at the last build
+  int *overflow, *timeout;
+  mdg::GridBarrier *bar;
 };
 
-// phi(s) and its first two derivatives; one division (1/s).
-__device__ __forceinline__ void phi_d(double s, const Pot &p, double &phi, double &d1, double &d2) {
-  const double is = 1.0 / s;
-  const double is2 = is * is;
-  const double is6 = is2 * is2 * is2;
-  const double is12 = is6 * is6;
-  phi = 4.0 * (is12 - is6 + p.c2 * s * s + p.c0);
-  d1 = 4.0 * (-12.0 * is12 + 6.0 * is6 + 2.0 * p.c2 * s * s) * is;
-  d2 = 4.0 * (156.0 * is12 - 42.0 * is6 + 2.0 * p.c2 * s * s) * is2;
+__device__ __forceinline__ double3 axpy(double h, const double3 &v, const double3 &q) {
+  return make_double3(fma(v.x, h, q.x), fma(v.y, h, q.y), fma(v.z, h, q.z));
+}
+__device__ __forceinline__ double dist2(const double3 &a, const double3 &b) {
+  const double x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
+  return x * x + y * y + z * z;
 }
 
-// U(r), U'(r), U''(r)
-__device__ __forceinline__ void pair_u(double r, const Pot &p, double &u, double &u1, double &u2) {
-  double f, f1, f2;
-  phi_d(r * p.inv_sigma, p, f, f1, f2);
-  u = p.eps * f;
-  u1 = p.eps_sigma * f1;
-  u2 = p.eps_sigma2 * f2;
+// d - L rint(d / L): the rounding by adding and taking away 1.5 2^52, which
+// leaves the nearest whole number for any |d / L| a trajectory reaches.
+__device__ __forceinline__ double min_image(double d, double L, double inv_L) {
+  const double big = 6755399441055744.0;
+  const double k = fma(d, inv_L, big) - big;
+  return fma(-L, k, d);
 }
 
-__device__ __forceinline__ double logistic(double x) { return 1.0 / (1.0 + exp(-x)); }
-
-// smoothed shell count of one pair and its derivative in r
-__device__ __forceinline__ void shell(double r, const Pot &p, double &s, double &s1) {
-  const double x1 = (r - p.a) * p.inv_w, x2 = (p.b - r) * p.inv_w;
-  const double g1 = logistic(x1), g2 = logistic(x2);
-  s = g1 * g2;
-  s1 = (g1 * (1.0 - g1) * g2 - g1 * g2 * (1.0 - g2)) * p.inv_w;
-}
-
-__device__ __forceinline__ int cell_axis(double x, double L, double inv_cs, int ms) {
+__device__ __forceinline__ int cell_axis(double x, double L, double inv_cs, int ms, float *boxed) {
   x -= L * floor(x / L);
+  *boxed = (float)x;
   int c = (int)(x * inv_cs);
   return c < 0 ? 0 : (c >= ms ? ms - 1 : c);
 }
 
-__device__ __forceinline__ int cell_of(const double4 &q, const Grid &g) {
-  const int cx = cell_axis(q.x, g.L[0], g.inv_cs[0], g.ms[0]);
-  const int cy = cell_axis(q.y, g.L[1], g.inv_cs[1], g.ms[1]);
-  const int cz = cell_axis(q.z, g.L[2], g.inv_cs[2], g.ms[2]);
-  return (cz * g.ms[1] + cy) * g.ms[0] + cx;
-}
+__device__ __forceinline__ int bucket_of(int j) { return (int)(((unsigned)j * 0x9E3779B1u) >> 29); }
 
-// Calls f(j, d, r) for every partner j of i's row with r < r_c, d = minimum
-// image of q_i - q_j, in row order (ascending j).  Rows hold every pair
-// within r_c and more, in ascending j, so the pairs within r_c and their
-// order are a function of q alone, whichever build the row comes from.
-// TPA lanes share one atom: they test TPA entries at a time, number the
-// pairs within r_c in row order, and lane `sub` takes pairs sub, sub + TPA,
-// ... of that numbering (shuffled to it from the lane that tested them); the
-// caller combines the lanes' sums with group_sum.  All TPA lanes of the atom
-// call together.
-template <int TPA, class F>
-__device__ __forceinline__ void for_pairs(const double4 *q, const Rows &w, const Pot &p, int i, int sub, int n,
-                                          F f) {
-  const double4 qi = q[i];
-  const int m = w.cnt[i];
-  auto pair_of = [&](int k, int &j, double (&d)[3]) {
-    j = w.nbr[(size_t)k * n + i];
-    const double4 qj = q[j];
-    d[0] = qi.x - qj.x;
-    d[1] = qi.y - qj.y;
-    d[2] = qi.z - qj.z;
-    for (int a = 0; a < 3; a++) d[a] -= w.L[a] * rint(d[a] * w.inv_L[a]);
-    return d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-  };
-  if (TPA == 1) {
-    for (int k = 0; k < m; k++) {
-      int j;
-      double d[3];
-      const double r2 = pair_of(k, j, d);
-      if (r2 < p.rc2) f(j, d, sqrt(r2));
-    }
-    return;
-  }
-  const int lane = threadIdx.x & 31, first = lane & ~(TPA - 1);
-  const unsigned gmask = (TPA == 32) ? 0xffffffffu : (((1u << TPA) - 1u) << first);
-  int before = 0;  // pairs within r_c in the entries already tested
-  for (int k0 = 0; k0 < m; k0 += TPA) {
-    int j = 0;
-    double d[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
-    bool in = false;
-    if (k0 + sub < m) {
-      r2 = pair_of(k0 + sub, j, d);
-      in = r2 < p.rc2;
-    }
-    const unsigned bal = (__ballot_sync(gmask, in) >> first) & ((1u << TPA) - 1u);
-    const int cnt = __popc(bal);
-    // this lane's pair of the batch: number r of the batch's pairs, the one
-    // with overall number == sub (mod TPA)
-    const int r = (sub - before % TPA + TPA) % TPA;
-    int src = 0;
-#pragma unroll
-    for (int b = 0, c = 0; b < TPA; b++) {
-      if ((bal >> b) & 1u) {
-        if (c == r) src = b;
-        c++;
+// ---------------------------------------------------------- Verlet list
+// Every block of the (resident) grid arrives; false when the wait ran out.
+__device__ __forceinline__ bool meet(const List &l) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    ok = 1;
+    const unsigned gen = mdg::ld_acquire_gpu(&l.bar->gen);
+    __threadfence();
+    if (atomicAdd(&l.bar->count, 1u) + 1u == gridDim.x) {
+      l.bar->count = 0u;
+      __threadfence();
+      atomicAdd(&l.bar->gen, 1u);
+    } else {
+      long long polls = 0;
+      while (mdg::ld_acquire_gpu(&l.bar->gen) == gen) {
+        if (++polls > mdg::kBarrierPolls) {
+          atomicOr(l.timeout, 1);
+          ok = 0;
+          break;
+        }
+        __nanosleep(20);
       }
     }
-    const int jj = __shfl_sync(gmask, j, first + src);
-    double dd[3];
-    dd[0] = __shfl_sync(gmask, d[0], first + src);
-    dd[1] = __shfl_sync(gmask, d[1], first + src);
-    dd[2] = __shfl_sync(gmask, d[2], first + src);
-    const double rr = __shfl_sync(gmask, r2, first + src);
-    if (r < cnt) f(jj, dd, sqrt(rr));
-    before += cnt;
   }
+  __syncthreads();
+  return ok != 0;
+}
+
+// Ascending sort of a warp's 128 values, v[e] = element e * 32 + lane (bitonic
+// network).
+__device__ __forceinline__ void warp_sort(unsigned (&v)[4], int lane) {
+#pragma unroll
+  for (int k = 2; k <= 128; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= 32) {  // partner in the same lane
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const int f = e ^ (j / 32);
+          if (f > e) {
+            const bool up = ((e * 32) & k) == 0;
+            const unsigned x = v[e], y = v[f];
+            v[e] = up ? min(x, y) : max(x, y);
+            v[f] = up ? max(x, y) : min(x, y);
+          }
+        }
+      } else {  // partner in lane ^ j
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+          const unsigned o = __shfl_xor_sync(0xffffffffu, v[e], j);
+          const bool up = ((e * 32 + lane) & k) == 0, lower = (lane & j) == 0;
+          v[e] = lower == up ? min(v[e], o) : max(v[e], o);
+        }
+      }
+    }
+  }
+}
+
+// Row of atom i by one warp: the atoms of the 27 cells around it within the
+// search length (FP32 minimum image on box coordinates; the reach is enlarged
+// by more than its rounding, and rows may hold more than they must), put in
+// (bucket, index) order.  The cells of an x-row are consecutive in `sorted`:
+// the 27 cells are 9 runs, and 9 more of one cell each where x wraps; the next
+// 32 atoms' load is in flight while 32 are tested.  keys: maxnb words of shared
+// memory.
+__device__ __forceinline__ void build_row(const List &l, const Vec &x, int i, unsigned *keys) {
+  const int lane = threadIdx.x & 31;
+  const double3 q = x.at(i);
+  float bx, by, bz;
+  const int cx = cell_axis(q.x, l.L[0], l.inv_cs[0], l.ms[0], &bx);
+  const int cy = cell_axis(q.y, l.L[1], l.inv_cs[1], l.ms[1], &by);
+  const int cz = cell_axis(q.z, l.L[2], l.inv_cs[2], l.ms[2], &bz);
+  if (lane == 0) l.qb.set(i, q);
+  const bool wraps = cx == 0 || cx == l.ms[0] - 1;
+  const int runs = wraps ? 18 : 9;
+  int first = 0, len = 0;  // lane < runs: one of the runs
+  if (lane < runs) {
+    const int r = lane % 9;
+    const int z = (cz + r / 3 - 1 + l.ms[2]) % l.ms[2], y = (cy + r % 3 - 1 + l.ms[1]) % l.ms[1];
+    const int row = (z * l.ms[1] + y) * l.ms[0];
+    int c0 = max(cx - 1, 0), c1 = min(cx + 1, l.ms[0] - 1);
+    if (lane >= 9) c0 = c1 = cx == 0 ? l.ms[0] - 1 : 0;
+    first = __ldcg(&l.start[row + c0]);
+    len = __ldcg(&l.start[row + c1]) + __ldcg(&l.count[row + c1]) - first;
+  }
+  int run = -1, f = 0, left = 0;  // the atoms loaded next: left ones from f on
+  auto next = [&]() {
+    f += 32;
+    left -= 32;
+    while (left <= 0 && ++run < runs) {
+      f = __shfl_sync(0xffffffffu, first, run);
+      left = __shfl_sync(0xffffffffu, len, run);
+    }
+  };
+  next();
+  float4 pn = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (lane < left) pn = __ldcg(&l.sorted[f + lane]);
+  int m = 0;
+  while (run < runs) {
+    const float4 p = pn;
+    const bool in = lane < left;
+    next();
+    if (lane < left) pn = __ldcg(&l.sorted[f + lane]);
+    const int j = __float_as_int(p.w);
+    float dx = p.x - bx, dy = p.y - by, dz = p.z - bz;
+    dx = fmaf(-l.Lf[0], rintf(dx * l.inv_Lf[0]), dx);
+    dy = fmaf(-l.Lf[1], rintf(dy * l.inv_Lf[1]), dy);
+    dz = fmaf(-l.Lf[2], rintf(dz * l.inv_Lf[2]), dz);
+    const bool keep = in && j != i && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= l.reach2;
+    const unsigned bal = __ballot_sync(0xffffffffu, keep);
+    const int at = m + __popc(bal & ((1u << lane) - 1u));
+    if (keep && at < l.maxnb) keys[at] = ((unsigned)bucket_of(j) << 29) | (unsigned)j;
+    m += __popc(bal);
+  }
+  if (m > l.maxnb && lane == 0) atomicOr(l.overflow, 1);
+  m = min(m, l.maxnb);
+  __syncwarp();
+  int *row = l.nbr + (size_t)i * l.maxnb;
+  if (m <= 128) {
+    unsigned v[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) v[e] = e * 32 + lane < m ? keys[e * 32 + lane] : 0xffffffffu;
+    warp_sort(v, lane);
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (e * 32 + lane < m) row[e * 32 + lane] = (int)(v[e] & 0x1fffffffu);
+  } else {
+    for (int e = lane; e < m; e += 32) {  // a long row: count the smaller keys
+      const unsigned key = keys[e];
+      int r = 0;
+      for (int k = 0; k < m; k++) r += keys[k] < key ? 1 : 0;
+      row[r] = (int)(key & 0x1fffffffu);
+    }
+  }
+  // ends of the buckets: entries of each, and their running sum
+  int mine = 0;
+  for (int e = 0; e < m; e += 32) {
+    const int bk = e + lane < m ? (int)(keys[e + lane] >> 29) : -1;
+#pragma unroll
+    for (int c = 0; c < kBuckets; c++) {
+      const int k = __popc(__ballot_sync(0xffffffffu, bk == c));
+      mine += lane >= c ? k : 0;
+    }
+  }
+  if (lane < kBuckets) l.ends[(size_t)i * kBuckets + lane] = (unsigned short)mine;
+  __syncwarp();
+}
+
+// The list at x, by the whole grid; false when a barrier's wait ran out.
+// x-rows of cells get their places in the order in which they ask for them:
+// the list does not depend on it.
+__device__ __noinline__ bool rebuild(const List &l, const Vec &x, unsigned *smem) {
+  if (*(volatile const int *)l.timeout) return false;  // an earlier launch gave up: the run has failed
+  const int t = blockIdx.x * kAB + threadIdx.x, nt = gridDim.x * kAB;
+  for (int c = t; c < l.ncell; c += nt) l.count[c] = 0;
+  if (t == 0) *l.cursor = 0;
+  if (!meet(l)) return false;
+  for (int i = t; i < l.n; i += nt) {
+    const double3 q = x.at(i);
+    float f;
+    const int cx = cell_axis(q.x, l.L[0], l.inv_cs[0], l.ms[0], &f);
+    const int cy = cell_axis(q.y, l.L[1], l.inv_cs[1], l.ms[1], &f);
+    const int cz = cell_axis(q.z, l.L[2], l.inv_cs[2], l.ms[2], &f);
+    const int c = (cz * l.ms[1] + cy) * l.ms[0] + cx;
+    l.cell[i] = c;
+    l.rank[i] = atomicAdd(&l.count[c], 1);
+  }
+  if (!meet(l)) return false;
+  {  // a warp per x-row of cells: its place, and the running sum of its cells
+    const int lane = threadIdx.x & 31, ms0 = l.ms[0], rows = l.ms[1] * l.ms[2];
+    for (int r = t >> 5; r < rows; r += nt >> 5) {
+      int total = 0;
+      for (int c = lane; c < ms0; c += 32) total += __ldcg(&l.count[r * ms0 + c]);
+      total = __reduce_add_sync(0xffffffffu, total);
+      int at = 0;
+      if (lane == 0) at = atomicAdd(l.cursor, total);
+      at = __shfl_sync(0xffffffffu, at, 0);
+      for (int c = 0; c < ms0; c += 32) {
+        const int k = c + lane < ms0 ? __ldcg(&l.count[r * ms0 + c + lane]) : 0;
+        int sum = k;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= o) sum += v;
+        }
+        if (c + lane < ms0) l.start[r * ms0 + c + lane] = at + sum - k;
+        at += __shfl_sync(0xffffffffu, sum, 31);
+      }
+    }
+  }
+  if (!meet(l)) return false;
+  for (int i = t; i < l.n; i += nt) {  // the thread's own cell[i] and rank[i]
+    const double3 q = x.at(i);
+    float4 f;
+    cell_axis(q.x, l.L[0], l.inv_cs[0], l.ms[0], &f.x);
+    cell_axis(q.y, l.L[1], l.inv_cs[1], l.ms[1], &f.y);
+    cell_axis(q.z, l.L[2], l.inv_cs[2], l.ms[2], &f.z);
+    f.w = __int_as_float(i);
+    l.sorted[__ldcg(&l.start[l.cell[i]]) + l.rank[i]] = f;
+  }
+  if (!meet(l)) return false;
+  unsigned *keys = smem + (threadIdx.x >> 5) * l.maxnb;
+  for (int i = t >> 5; i < l.n; i += nt >> 5) build_row(l, x, i, keys);
+  return meet(l);
+}
+
+// ------------------------------------------------------------ evaluations
+enum Kind { kForce, kLoss, kHess };
+
+// One evaluation.  Kind kForce: F at x, then v' = v + F dt (into v_out), q' = x
+// + v' dt/2 and the next step's x' = q' + v' dt/2; kLoss: block sums of PE, S
+// and dPE/dsigma at x, with grad the loss gradient into lq and the first half
+// of the reverse step (lv' = lv + lq dt/2, u = lv' dt); kHess: H(x) u, block
+// sums of u . dF/d(eps, sigma), the second half (lq -= w, lv += lq dt/2), and
+// the positions of the step before.
+struct Eval {
+  Vec x;
+  const int *want;      // rebuild the list at x first
+  int *move, *jump;     // flags of the next evaluation and of the one after it
+  double dt;
+  // kForce
+  Vec v, v_out, q_out, x_out;  // q_out, x_out: p = null where not needed
+  // kLoss, kHess
+  Vec lq, lv, u;
+  double scale;                // dL/d(sums); 0: sums only
+  double *part;                // block sums of this step
+  // kHess: the step before (x_prev.p = null: none); q_out gets its q'
+  Vec x_prev, v_prev;
+};
+
+// Terms of the partners at d[0], d[1] (x_i - x_j, minimum image) into s.
+template <Kind K, bool GRAD>
+struct Terms {
+  static constexpr int N = K == kForce ? 3 : (K == kLoss ? (GRAD ? 6 : 3) : 5);
+};
+
+template <Kind K, bool GRAD>
+__device__ __forceinline__ void pair_terms(const Pot &p, const double3 (&d)[2], const bool (&on)[2],
+                                           const double3 &ui, const double3 (&uj)[2],
+                                           double (&s)[Terms<K, GRAD>::N]) {
+  constexpr int N = Terms<K, GRAD>::N;
+  double t[2][N];
+  bool in[2];
+#pragma unroll
+  for (int e = 0; e < 2; e++) {
+    const double3 &v = d[e];
+    // products that sums follow are written out (fma or rounded), so that the
+    // loss's sums do not depend on what else a pass computes
+    double r2 = fma(v.x, v.x, fma(v.y, v.y, v.z * v.z));
+    in[e] = on[e] && r2 < p.rc2;
+    r2 = in[e] ? r2 : p.sigma2;
+    // powers of sigma / r; U'/r and U'' need no root
+    const double ir2 = mdg::quotient(1.0, r2);
+    const double is2 = p.sigma2 * ir2, is6 = __dmul_rn(is2 * is2, is2);
+    const double is8 = is6 * is2;
+    const double A = p.k4 * fma(is8, fma(-12.0, is6, 6.0), 2.0 * p.c2);  // U'/r
+    if (K == kForce) {
+      t[e][0] = -A * v.x;
+      t[e][1] = -A * v.y;
+      t[e][2] = -A * v.z;
+    } else if (K == kLoss) {
+      const double s2 = r2 * p.inv_sigma2;
+      const double u = p.e4 * fma(is6, is6 - 1.0, fma(p.c2, s2, p.c0));
+      const double ir = rsqrt(r2), r = __dmul_rn(r2, ir);
+      // the smoothed count g1 g2 and its derivative g1 g2 (g2 - g1) / w
+      double g1, g2, g;
+      if (p.one_exp) {
+        const double E = exp(__dmul_rn(r - p.mid, p.inv_w));
+        const double P = E + p.h, Q = fma(p.h, E, 1.0);
+        const double inv = mdg::quotient(1.0, P * Q);
+        g1 = E * Q * inv;
+        g2 = P * inv;
+        g = E * inv;
+      } else {
+        g1 = 1.0 / (1.0 + exp(-__dmul_rn(r - p.a, p.inv_w)));
+        g2 = 1.0 / (1.0 + exp(-__dmul_rn(p.b - r, p.inv_w)));
+        g = g1 * g2;
+      }
+      t[e][0] = 0.5 * u;
+      t[e][1] = 0.5 * g;
+      t[e][2] = -0.5 * (A * r2) * p.inv_sigma;  // dU/dsigma at fixed r
+      if (GRAD) {
+        const double c = A + g * (g2 - g1) * p.inv_w * ir;
+        t[e][N - 3] = c * v.x;
+        t[e][N - 2] = c * v.y;
+        t[e][N - 1] = c * v.z;
+      }
+    } else {
+      const double u2 = p.k4 * fma(is8, fma(156.0, is6, -42.0), 2.0 * p.c2);  // U''
+      const double3 du = make_double3(ui.x - uj[e].x, ui.y - uj[e].y, ui.z - uj[e].z);
+      const double B = (u2 - A) * ir2 * (v.x * du.x + v.y * du.y + v.z * du.z);
+      // K du = U'' e (e.du) + U'/r (du - e (e.du))
+      t[e][0] = fma(B, v.x, A * du.x);
+      t[e][1] = fma(B, v.y, A * du.y);
+      t[e][2] = fma(B, v.z, A * du.z);
+      // F_i = sum_j -U'(r) e: dF_i/deps = -(U'/eps) e, dF_i/dsigma = (U' + r U'')/sigma e
+      const double eu = v.x * ui.x + v.y * ui.y + v.z * ui.z;
+      t[e][N - 2] = -(A * p.inv_eps) * eu;
+      t[e][N - 1] = (A + u2) * p.inv_sigma * eu;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 2; e++)
+#pragma unroll
+    for (int k = 0; k < N; k++) s[k] = __dadd_rn(s[k], in[e] ? t[e][k] : 0.0);
 }
 
 // Sum over the TPA lanes of one atom (fixed butterfly order); every lane of
@@ -209,373 +471,148 @@ __device__ __forceinline__ void block_sums(double (&v)[NS], double *part) {
   }
 }
 
-// ------------------------------------------------------------------ cells
-// The grid kernels run only when the list is to be rebuilt (*want != 0).
-__global__ void a_clear(int *count, int *fill, int ncell, const int *want) {
-  if (!*want) return;
-  for (int c = blockIdx.x * kAB + threadIdx.x; c < ncell; c += gridDim.x * kAB) count[c] = fill[c] = 0;
+// Flags for the evaluations at q (the next) and x (the one after): `move` when
+// the list does not serve both, `jump` when a list made at q would not serve x.
+__device__ __forceinline__ void flag_moves(const List &l, const Eval &e, int i, const double3 &q, const double3 &x) {
+  const double3 b = l.qb.at(i);
+  if (dist2(q, b) > l.half_skin2 || dist2(x, b) > l.half_skin2) atomicOr(e.move, 1);
+  if (dist2(q, x) > l.half_skin2) atomicOr(e.jump, 1);
 }
 
-__global__ void a_count(const double4 *q, int n, Grid g, int *cell, int *count, const int *want) {
-  const int i = blockIdx.x * kAB + threadIdx.x;
-  if (i >= n || !*want) return;
-  const int c = cell_of(q[i], g);
-  cell[i] = c;
-  atomicAdd(&count[c], 1);
-}
-
-// exclusive scan of count into start (one block, ncell of any size)
-__global__ void a_scan(const int *count, int *start, int ncell, const int *want) {
-  if (!*want) return;
-  __shared__ int part[1024];
-  const int t = threadIdx.x;
-  const int chunk = (ncell + 1023) / 1024;
-  const int beg = min(t * chunk, ncell), end = min(beg + chunk, ncell);
-  int s = 0;
-  for (int c = beg; c < end; c++) s += count[c];
-  part[t] = s;
-  __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const int x = t >= o ? part[t - o] : 0;
-    __syncthreads();
-    part[t] += x;
-    __syncthreads();
-  }
-  int run = part[t] - s;
-  for (int c = beg; c < end; c++) {
-    start[c] = run;
-    run += count[c];
-  }
-  if (t == 1023) start[ncell] = part[t];
-}
-
-__global__ void a_fill(int n, const int *cell, const int *start, int *fill, int *perm, const int *want) {
-  const int i = blockIdx.x * kAB + threadIdx.x;
-  if (i >= n || !*want) return;
-  const int c = cell[i];
-  perm[start[c] + atomicAdd(&fill[c], 1)] = i;
-}
-
-// Orders every cell by atom index, one warp per cell: each entry's new
-// place is the count of smaller indices in the cell (indices are distinct).
-// perm_in is the fill order, perm_out the sorted one.
-__global__ void a_sort(int ncell, const int *start, const int *perm_in, int *perm_out, const int *want) {
-  const int c = (blockIdx.x * kAB + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (c >= ncell || !*want) return;
-  const int b = start[c], cnt = start[c + 1] - b;
-  for (int base = 0; base < cnt; base += 32) {
-    const int me = base + lane;
-    const int key = me < cnt ? perm_in[b + me] : 0x7fffffff;
-    int rank = 0;
-    for (int ob = 0; ob < cnt; ob += 32) {
-      const int okey = ob + lane < cnt ? perm_in[b + ob + lane] : 0x7fffffff;
-      for (int k = 0; k < 32; k++) rank += (ob + k < cnt) && (__shfl_sync(0xffffffffu, okey, k) < key);
+template <Kind K, bool GRAD, int TPA>
+__global__ void __launch_bounds__(kAB, kABlocks)
+    a_eval(const __grid_constant__ List l, const __grid_constant__ Pot p, const __grid_constant__ Eval e) {
+  extern __shared__ unsigned smem[];
+  if (*(volatile const int *)e.want && !rebuild(l, e.x, smem)) return;
+  constexpr int N = Terms<K, GRAD>::N, NP = kBuckets / TPA;
+  const long long threads = (long long)l.n * TPA, step = (long long)gridDim.x * kAB;
+  double sums[3] = {0.0, 0.0, 0.0};
+  const double3 zero = make_double3(0.0, 0.0, 0.0);
+  // warps walk whole warps of threads, so the lane shuffles stay converged
+  for (long long base = (long long)blockIdx.x * kAB + (threadIdx.x & ~31); base < threads; base += step) {
+    const long long t = base + (threadIdx.x & 31);
+    const bool on = t < threads;
+    const int i = on ? (int)(t / TPA) : 0, sub = (int)(t % TPA);
+    const double3 xi = e.x.at(i), ui = K == kHess ? e.u.at(i) : zero;
+    // the lane's buckets, one run of the row
+    int k = 0, end = 0;
+    if (on) {
+      const unsigned short *ends = l.ends + (size_t)i * kBuckets + sub * NP;
+      k = sub ? ends[-1] : 0;
+      end = ends[NP - 1];
     }
-    if (me < cnt) perm_out[b + rank] = key;
-  }
-}
-
-// Positions in cell order for the pair kernels.
-__global__ void a_gather(const double4 *x, const int *perm, double4 *xs, int n, const int *want) {
-  const int k = blockIdx.x * kAB + threadIdx.x;
-  if (k < n && *want) xs[k] = x[perm[k]];
-}
-
-// The whole grid (clear, count, scan, fill, per-cell index order, gather)
-// in one block of 1024 threads, for up to kGrid1Atoms atoms.
-constexpr int kGrid1Atoms = 262144;
-__global__ void __launch_bounds__(1024) a_grid1(const double4 *x, int n, Grid g, int ncell, int *cell, int *count,
-                                                int *start, int *fill, int *perm_fill, int *perm, double4 *qs,
-                                                const int *want) {
-  if (!*want) return;
-  __shared__ int part[1024];
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  for (int c = t; c < ncell; c += 1024) count[c] = fill[c] = 0;
-  __syncthreads();
-  for (int i = t; i < n; i += 1024) {
-    const int c = cell_of(x[i], g);
-    cell[i] = c;
-    atomicAdd(&count[c], 1);
-  }
-  __syncthreads();
-  {  // exclusive scan of count into start, 1024 chunks
-    const int chunk = (ncell + 1023) / 1024;
-    const int beg = min(t * chunk, ncell), end = min(beg + chunk, ncell);
-    int sum = 0;
-    for (int c = beg; c < end; c++) sum += count[c];
-    part[t] = sum;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-      const int v = t >= o ? part[t - o] : 0;
-      __syncthreads();
-      part[t] += v;
-      __syncthreads();
+    const int *row = l.nbr + (size_t)i * l.maxnb;
+    double s[N];
+#pragma unroll
+    for (int c = 0; c < N; c++) s[c] = 0.0;
+    // two partners at once; the next two's positions and the list entries of
+    // the two after them are in flight
+    int j[2], jn[2];
+    double3 x[2], u[2] = {zero, zero};
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      j[c] = k + c < end ? row[k + c] : i;
+      jn[c] = k + 2 + c < end ? row[k + 2 + c] : i;
+      x[c] = e.x.at(j[c]);
+      if (K == kHess) u[c] = e.u.at(j[c]);
     }
-    int run = part[t] - sum;
-    for (int c = beg; c < end; c++) {
-      start[c] = run;
-      run += count[c];
-    }
-    if (t == 1023) start[ncell] = part[t];
-  }
-  __syncthreads();
-  for (int i = t; i < n; i += 1024) {
-    const int c = cell[i];
-    perm_fill[start[c] + atomicAdd(&fill[c], 1)] = i;
-  }
-  __syncthreads();
-  for (int c = warp; c < ncell; c += 32) {  // index order inside each cell (as a_sort)
-    const int b = start[c], cnt = start[c + 1] - b;
-    for (int base = 0; base < cnt; base += 32) {
-      const int me = base + lane;
-      const int key = me < cnt ? perm_fill[b + me] : 0x7fffffff;
-      int rank = 0;
-      for (int ob = 0; ob < cnt; ob += 32) {
-        const int okey = ob + lane < cnt ? perm_fill[b + ob + lane] : 0x7fffffff;
-        for (int k = 0; k < 32; k++) rank += (ob + k < cnt) && (__shfl_sync(0xffffffffu, okey, k) < key);
+#pragma unroll 1
+    for (; k < end; k += 2) {
+      double3 d[2], uc[2];
+      const bool in[2] = {true, k + 1 < end};
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        d[c] = make_double3(min_image(xi.x - x[c].x, l.L[0], l.inv_L[0]), min_image(xi.y - x[c].y, l.L[1], l.inv_L[1]),
+                            min_image(xi.z - x[c].z, l.L[2], l.inv_L[2]));
+        uc[c] = u[c];
+        x[c] = e.x.at(jn[c]);
+        if (K == kHess) u[c] = e.u.at(jn[c]);
+        jn[c] = k + 4 + c < end ? row[k + 4 + c] : i;
       }
-      if (me < cnt) perm[b + rank] = key;
+      pair_terms<K, GRAD>(p, d, in, ui, uc, s);
     }
-  }
-  __syncthreads();
-  for (int k = t; k < n; k += 1024) qs[k] = x[perm[k]];
-}
-
-// ---------------------------------------------------------- Verlet list
-// flag[0] = 1 if some atom moved more than skin/2 from the list's build
-// positions qb (minimum image); flag[0] starts at 1 for the first build.
-__global__ void a_check(const double4 *x, const double4 *qb, int n, Rows w, double half_skin2, int *flag) {
-  const int i = blockIdx.x * kAB + threadIdx.x;
-  if (i >= n) return;
-  const double4 a = x[i], b = qb[i];
-  double d[3] = {a.x - b.x, a.y - b.y, a.z - b.z};
-  for (int k = 0; k < 3; k++) d[k] -= w.L[k] * rint(d[k] * w.inv_L[k]);
-  if (d[0] * d[0] + d[1] * d[1] + d[2] * d[2] > half_skin2) atomicOr(flag, 1);
-}
-
-// Ascending sort of the 32 E values of a warp, v[e] = element e * 32 + lane
-// (bitonic network, fully unrolled).
-template <int E>
-__device__ __forceinline__ void warp_sort_asc(int (&v)[E], int lane) {
-  constexpr int N = 32 * E;
-#pragma unroll
-  for (int k = 2; k <= N; k <<= 1) {
-#pragma unroll
-    for (int j = k >> 1; j > 0; j >>= 1) {
-#pragma unroll
-      for (int e = 0; e < E; e++) {
-        if (j < 32) {  // partner in lane ^ j, same e
-          const int g = e * 32 + lane;
-          const int o = __shfl_xor_sync(0xffffffffu, v[e], j);
-          const bool up = (g & k) == 0, lower = (g & j) == 0;
-          v[e] = (lower == up) ? min(v[e], o) : max(v[e], o);
-        } else {  // partner e ^ (j / 32) in the same lane
-          const int f = e ^ (j / 32);
-          if (f > e) {
-            const bool up = ((e * 32) & k) == 0;
-            const int a = v[e], b = v[f];
-            v[e] = up ? min(a, b) : max(a, b);
-            v[f] = up ? max(a, b) : min(a, b);
+    // the atom's end, on its first lane
+    if (K == kForce || K == kHess || GRAD) {
+      constexpr int F = K == kLoss ? N - 3 : 0;
+      const double3 w =
+          make_double3(group_sum<TPA>(s[F]), group_sum<TPA>(s[F + 1]), group_sum<TPA>(s[F + 2]));
+      if (on && sub == 0) {
+        const double half = 0.5 * e.dt;
+        if (K == kForce) {
+          const double3 v = axpy(e.dt, w, e.v.at(i));
+          e.v_out.set(i, v);
+          const double3 q = axpy(half, v, xi), xn = axpy(half, v, q);
+          if (e.q_out.p) e.q_out.set(i, q);
+          if (e.x_out.p) e.x_out.set(i, xn);
+          // the next evaluations: q' and x', or x' alone, or (no x') q' and x
+          flag_moves(l, e, i, e.q_out.p ? q : xn, e.x_out.p ? xn : xi);
+        } else if (K == kLoss) {
+          const double3 a = axpy(e.scale, w, e.lq.at(i));
+          const double3 b = axpy(half, a, e.lv.at(i));
+          e.lq.set(i, a);
+          e.lv.set(i, b);
+          e.u.set(i, make_double3(b.x * e.dt, b.y * e.dt, b.z * e.dt));
+        } else {
+          const double3 a = axpy(-1.0, w, e.lq.at(i));
+          e.lq.set(i, a);
+          e.lv.set(i, axpy(half, a, e.lv.at(i)));
+          if (e.x_prev.p) {
+            const double3 xp = e.x_prev.at(i), q = axpy(half, e.v_prev.at(i), xp);
+            e.q_out.set(i, q);
+            flag_moves(l, e, i, q, xp);
           }
         }
       }
     }
-  }
-}
-
-// Rows of the list at x, one warp per atom i: the partners j != i with
-// |x_i - x_j| <= sl (minimum image), found by walking the 27 cells around
-// i's (the lanes test a cell's atoms 32 at a time and gather the kept ones
-// in a shared buffer), then sorted ascending (warp_sort_asc, rows of up to
-// 32 E entries); x is copied to qb.  Runs only when *want != 0; clears
-// *next, the rebuild flag of the next evaluation.  A row longer than maxnb
-// (<= 32 E) sets *overflow.
-template <int E>
-__global__ void __launch_bounds__(kAB) a_rows(const double4 *x, int n, Grid g, double sl2, int maxnb, int *nbr,
-                                              int *cnt, double4 *qb, const int *want, int *next, int *overflow) {
-  __shared__ int buf[kAB / 32][32 * E];
-  const int i = (int)(((long long)blockIdx.x * kAB + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0;
-  if (i >= n || !*want) return;  // whole warps leave together
-  const double4 qi = x[i];
-  if (lane == 0) qb[i] = qi;
-  const int cx = cell_axis(qi.x, g.L[0], g.inv_cs[0], g.ms[0]);
-  const int cy = cell_axis(qi.y, g.L[1], g.inv_cs[1], g.ms[1]);
-  const int cz = cell_axis(qi.z, g.L[2], g.inv_cs[2], g.ms[2]);
-  // lane l < 27 holds cell l's first slot and the inclusive prefix of the
-  // 27 cells' counts: the candidates are one concatenated range of `total`
-  // (the row is sorted afterwards, so the walk order does not matter)
-  int beg = 0, pre = 0;
-  if (lane < 27) {
-    const int z = (cz + lane / 9 - 1 + g.ms[2]) % g.ms[2];
-    const int y = (cy + (lane / 3) % 3 - 1 + g.ms[1]) % g.ms[1];
-    const int xx = (cx + lane % 3 - 1 + g.ms[0]) % g.ms[0];
-    const int c = (z * g.ms[1] + y) * g.ms[0] + xx;
-    beg = g.start[c];
-    pre = g.start[c + 1] - beg;
-  }
+    if (K == kLoss) {
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, pre, o);
-    if (lane >= o) pre += v;
-  }
-  const int total = __shfl_sync(0xffffffffu, pre, 26);
-  int m = 0;  // partners found (warp-uniform)
-  for (int fb = 0; fb < total; fb += 32) {
-    const int f = fb + lane;
-    // the cell of candidate f: the first cell whose inclusive prefix exceeds f
-    int lo = 0, hi = 26;
-#pragma unroll
-    for (int it = 0; it < 5; it++) {
-      const int mid = (lo + hi) >> 1;
-      const int pm = __shfl_sync(0xffffffffu, pre, mid);
-      if (pm > f) hi = mid;
-      else lo = min(mid + 1, hi);
+      for (int c = 0; c < 3; c++) sums[c] += s[c];
     }
-    const int bq = __shfl_sync(0xffffffffu, beg, lo);
-    const int pp = __shfl_sync(0xffffffffu, pre, lo > 0 ? lo - 1 : 0);
-    const int excl = lo > 0 ? pp : 0;  // candidates in the cells before
-    int j = -1;
-    bool keep = false;
-    if (f < total) {
-      const int k = bq + (f - excl);
-      j = g.perm[k];
-      const double4 qj = g.qs[k];
-      double d[3] = {qi.x - qj.x, qi.y - qj.y, qi.z - qj.z};
-      for (int a = 0; a < 3; a++) d[a] -= g.L[a] * rint(d[a] * g.inv_L[a]);
-      keep = j != i && d[0] * d[0] + d[1] * d[1] + d[2] * d[2] <= sl2;
-    }
-    const unsigned bal = __ballot_sync(0xffffffffu, keep);
-    const int slot = m + __popc(bal & ((1u << lane) - 1u));
-    if (keep && slot < maxnb) buf[wib][slot] = j;
-    m += __popc(bal);
-  }
-  __syncwarp();
-  const int mm = min(m, maxnb);
-  int v[E];
-#pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int s = e * 32 + lane;
-    v[e] = s < mm ? buf[wib][s] : 0x7fffffff;
-  }
-  warp_sort_asc<E>(v, lane);
-#pragma unroll
-  for (int e = 0; e < E; e++) {
-    const int s = e * 32 + lane;
-    if (s < mm) nbr[(size_t)s * n + i] = v[e];
-  }
-  if (lane == 0) {
-    cnt[i] = mm;
-    if (m > maxnb) atomicOr(overflow, 1);
-  }
-}
-
-// --------------------------------------------------------------- physics
-template <int TPA>
-__global__ void __launch_bounds__(kAB) a_force(const double4 *q, int n, Rows g, Pot p, double4 *f) {
-  const int t = blockIdx.x * kAB + threadIdx.x;
-  const int i = t / TPA, sub = t % TPA;
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  if (i < n) {
-    for_pairs<TPA>(q, g, p, i, sub, n, [&](int, const double *d, double r) {
-      double u, u1, u2;
-      pair_u(r, p, u, u1, u2);
-      const double c = -u1 / r;
-      fx += c * d[0];
-      fy += c * d[1];
-      fz += c * d[2];
-    });
-  }
-  fx = group_sum<TPA>(fx);
-  fy = group_sum<TPA>(fy);
-  fz = group_sum<TPA>(fz);
-  if (i < n && sub == 0) f[i] = make_double4(fx, fy, fz, 0.0);
-}
-
-// Loss terms at q: per-block sums of PE, S and dPE/dsigma (pairs counted from
-// both ends, halved); with grad, dL_t/dq_i * scale added into lq.
-template <int TPA>
-__global__ void __launch_bounds__(kAB) a_loss(const double4 *q, int n, Rows g, Pot p, double *part, double4 *lq,
-                                              double scale) {
-  const int t = blockIdx.x * kAB + threadIdx.x;
-  const int i = t / TPA, sub = t % TPA;
-  double v[3] = {0.0, 0.0, 0.0};
-  double gx = 0.0, gy = 0.0, gz = 0.0;
-  if (i < n) {
-    for_pairs<TPA>(q, g, p, i, sub, n, [&](int, const double *d, double r) {
-      double u, u1, u2, s, s1;
-      pair_u(r, p, u, u1, u2);
-      shell(r, p, s, s1);
-      v[0] += 0.5 * u;
-      v[1] += 0.5 * s;
-      v[2] += 0.5 * (-(r * p.inv_sigma) * u1);  // dU/dsigma at fixed r
-      const double c = (u1 + s1) / r;
-      gx += c * d[0];
-      gy += c * d[1];
-      gz += c * d[2];
-    });
-  }
-  if (lq) {
-    gx = group_sum<TPA>(gx);
-    gy = group_sum<TPA>(gy);
-    gz = group_sum<TPA>(gz);
-    if (i < n && sub == 0) {
-      double4 l = lq[i];
-      l.x += scale * gx;
-      l.y += scale * gy;
-      l.z += scale * gz;
-      lq[i] = l;
+    if (K == kHess) {
+      sums[0] += s[N - 2];
+      sums[1] += s[N - 1];
     }
   }
-  block_sums<3>(v, part);
-}
-
-// w = H(q) u (pair energy Hessian times u); per-block sums of
-// sum_i u_i . dF_i/d(eps, sigma).
-template <int TPA>
-__global__ void __launch_bounds__(kAB) a_hvp(const double4 *q, int n, Rows g, Pot p, const double4 *u, double4 *w,
-                                             double *part) {
-  const int t = blockIdx.x * kAB + threadIdx.x;
-  const int i = t / TPA, sub = t % TPA;
-  double v[2] = {0.0, 0.0};
-  double wx = 0.0, wy = 0.0, wz = 0.0;
-  if (i < n) {
-    const double4 ui = u[i];
-    for_pairs<TPA>(q, g, p, i, sub, n, [&](int j, const double *d, double r) {
-      double uu, u1, u2;
-      pair_u(r, p, uu, u1, u2);
-      const double4 uj = u[j];
-      const double ir = 1.0 / r;
-      const double ex = d[0] * ir, ey = d[1] * ir, ez = d[2] * ir;
-      const double dux = ui.x - uj.x, duy = ui.y - uj.y, duz = ui.z - uj.z;
-      const double proj = ex * dux + ey * duy + ez * duz;
-      const double t = u1 * ir;
-      // K du = U'' e (e.du) + U'/r (du - e (e.du))
-      wx += u2 * ex * proj + t * (dux - ex * proj);
-      wy += u2 * ey * proj + t * (duy - ey * proj);
-      wz += u2 * ez * proj + t * (duz - ez * proj);
-      // F_i = sum_j -U'(r) e: dF_i/deps = -(U'/eps) e, dF_i/dsigma = (U' + r U'')/sigma e
-      const double eu = ex * ui.x + ey * ui.y + ez * ui.z;
-      v[0] += -(u1 * p.inv_eps) * eu;
-      v[1] += (u1 + r * u2) * p.inv_sigma * eu;
-    });
+  if (K == kLoss) block_sums<3>(sums, e.part);
+  if (K == kHess) {
+    double two[2] = {sums[0], sums[1]};
+    block_sums<2>(two, e.part);
   }
-  wx = group_sum<TPA>(wx);
-  wy = group_sum<TPA>(wy);
-  wz = group_sum<TPA>(wz);
-  if (i < n && sub == 0) w[i] = make_double4(wx, wy, wz, 0.0);
-  block_sums<2>(v, part);
 }
 
-// Fixed-order sum of nb blocks' ns (<= 3) partials into out[k], one block of
-// kRB threads: thread t sums blocks t, t + kRB, ... in order, then a fixed
-// tree; the per-step sums stay on the device until the end of the run.
+// x = q + v h, and the flag of the evaluation at x.
+__global__ void __launch_bounds__(kAB) a_half(List l, Vec q, Vec v, Vec x, double h, int *move) {
+  const int i = blockIdx.x * kAB + threadIdx.x;
+  if (i >= l.n) return;
+  const double3 a = axpy(h, v.at(i), q.at(i));
+  x.set(i, a);
+  if (dist2(a, l.qb.at(i)) > l.half_skin2) atomicOr(move, 1);
+}
+
+// n x 3 arrays of the caller to points and back.
+__global__ void __launch_bounds__(kAB) a_unpack(const double *in, Vec out, int n) {
+  const int i = blockIdx.x * kAB + threadIdx.x;
+  if (i < n) out.set(i, make_double3(in[3 * (size_t)i], in[3 * (size_t)i + 1], in[3 * (size_t)i + 2]));
+}
+__global__ void __launch_bounds__(kAB) a_pack(Vec in, double *out, int n) {
+  const int i = blockIdx.x * kAB + threadIdx.x;
+  if (i >= n) return;
+  const double3 a = in.at(i);
+  out[3 * (size_t)i] = a.x;
+  out[3 * (size_t)i + 1] = a.y;
+  out[3 * (size_t)i + 2] = a.z;
+}
+
+// Fixed-order sums of nb blocks' ns (<= 3) partials, one block per step:
+// step blockIdx.x's partials at part + blockIdx.x * stride, its sums to out +
+// blockIdx.x * ns (out_step < 0: to earlier places, as the reverse sweep goes).
 constexpr int kRB = 256;
-__global__ void __launch_bounds__(kRB) a_reduce(const double *part, int nb, int ns, double *out) {
+__global__ void __launch_bounds__(kRB) a_reduce(const double *part, size_t stride, int nb, int ns, double *out,
+                                                int out_step) {
   __shared__ double sm[3][kRB];
   const int t = threadIdx.x;
+  part += blockIdx.x * stride;
+  out += (long long)blockIdx.x * out_step;
   for (int k = 0; k < ns; k++) {
     double x = 0.0;
     for (int b = t; b < nb; b += kRB) x += part[(size_t)b * ns + k];
@@ -588,59 +625,6 @@ __global__ void __launch_bounds__(kRB) a_reduce(const double *part, int nb, int 
     __syncthreads();
   }
   if (t < ns) out[t] = sm[t][0];
-}
-
-// --------------------------------------------------------- integration
-__global__ void a_drift(double4 *q, const double4 *v, int n, double h) {
-  const int i = blockIdx.x * kAB + threadIdx.x;
-  if (i >= n) return;
-  double4 a = q[i];
-  const double4 b = v[i];
-  a.x += b.x * h;
-  a.y += b.y * h;
-  a.z += b.z * h;
-  q[i] = a;
-}
-
-__global__ void a_kick(double4 *v, const double4 *f, int n, double dt) {
-  const int i = blockIdx.x * kAB + threadIdx.x;
-  if (i >= n) return;
-  double4 a = v[i];
-  const double4 b = f[i];
-  a.x += b.x * dt;
-  a.y += b.y * dt;
-  a.z += b.z * dt;
-  v[i] = a;
-}
-
-// lv' = lv + lq dt/2 (into lv), u = lv' dt
-__global__ void a_rev1(const double4 *lq, double4 *lv, double4 *u, int n, double dt) {
-  const int i = blockIdx.x * kAB + threadIdx.x;
-  if (i >= n) return;
-  const double4 a = lq[i];
-  double4 b = lv[i];
-  b.x += a.x * dt * 0.5;
-  b.y += a.y * dt * 0.5;
-  b.z += a.z * dt * 0.5;
-  lv[i] = b;
-  u[i] = make_double4(b.x * dt, b.y * dt, b.z * dt, 0.0);
-}
-
-// lq_h = lq - w;  lq = lq_h;  lv += lq_h dt/2
-__global__ void a_rev2(double4 *lq, double4 *lv, const double4 *w, int n, double dt) {
-  const int i = blockIdx.x * kAB + threadIdx.x;
-  if (i >= n) return;
-  double4 a = lq[i];
-  const double4 c = w[i];
-  a.x -= c.x;
-  a.y -= c.y;
-  a.z -= c.z;
-  lq[i] = a;
-  double4 b = lv[i];
-  b.x += a.x * dt * 0.5;
-  b.y += a.y * dt * 0.5;
-  b.z += a.z * dt * 0.5;
-  lv[i] = b;
 }
 
 int nblk(int n) { return n > 0 ? (n + kAB - 1) / kAB : 1; }
@@ -670,28 +654,24 @@ void free_workspace(Workspace &w) {
 struct Run {
   Workspace *ws = nullptr;
   size_t slot = 0;  // next workspace buffer
-  int n = 0, ncell = 0, tpa = 1;
+  int n = 0, tpa = 1, device = 0;
   cudaStream_t s = nullptr;
-  Grid g{};
+  List l{};
   Pot p{};
   double dt = 0.0;
-  double4 *q = nullptr, *v = nullptr, *f = nullptr, *tmp = nullptr;
-  double4 *lq = nullptr, *lv = nullptr, *u = nullptr, *w = nullptr;
-  double4 *ck_q = nullptr, *ck_v = nullptr;    // checkpoints
-  double4 *seg_qh = nullptr, *seg_v = nullptr;  // one segment's q_h and v'
-  int *cell = nullptr, *count = nullptr, *start = nullptr, *fill = nullptr, *perm = nullptr, *perm_fill = nullptr;
-  double4 *qs = nullptr;                        // positions in cell order
-  double *part = nullptr;                       // block partials of the pair kernels
+  size_t ns = 0;                                // n rounded up to an even number
+  Vec q{}, v{}, x[2]{}, lq{}, lv{}, u{};        // q': step end states; x: half-step positions, taking turns
+  double *raw = nullptr;                        // n x 3 transfers
+  double *ck_q = nullptr, *ck_v = nullptr;      // checkpoints
+  double *seg_x = nullptr, *seg_v = nullptr;    // one segment's half-step positions and v'
+  double *part = nullptr;                       // block partials of kReduceSlots steps
   double *loss_sums = nullptr;                  // per step: PE, S, dPE/dsigma
   double *adj_sums = nullptr;                   // per reverse step: u . dF/d(eps, sigma)
-  // Verlet list (a_rows): rows, row lengths, build positions, flags (the
-  // rebuild flags of even and odd evaluations, row overflow) and a host copy
-  Rows rows{};
-  int *nbr = nullptr, *cnt = nullptr, *flag = nullptr, *hflag = nullptr;
-  double4 *qb = nullptr;
-  int maxnb = 0;
-  double sl2 = 0.0, half_skin2 = 0.0;
-  long long evals = 0;  // list preparations so far (picks the flag pair's slot)
+  int *flags = nullptr;                         // rebuild flags, one per evaluation
+  int *state = nullptr;                         // row overflow, barrier timeout
+  int next_flag = 0;
+  int sms = 0, max_blocks = 0;
+  cudaError_t err = cudaSuccess;
 
   template <typename T>
   cudaError_t alloc(T **ptr, size_t count_) {
@@ -704,110 +684,87 @@ struct Run {
       if (ws->buf[slot]) cudaFree(ws->buf[slot]);
       ws->buf[slot] = nullptr;
       ws->bytes[slot] = 0;
-      void *p = nullptr;
-      const cudaError_t e = cudaMalloc(&p, b);
+      void *p_ = nullptr;
+      const cudaError_t e = cudaMalloc(&p_, b);
       if (e != cudaSuccess) return e;
-      ws->buf[slot] = p;
+      ws->buf[slot] = p_;
       ws->bytes[slot] = b;
     }
     *ptr = static_cast<T *>(ws->buf[slot++]);
     return cudaSuccess;
   }
-  int pair_blocks() const { return (int)(((long long)n * tpa + kAB - 1) / kAB); }
+  cudaError_t alloc(Vec *out) {
+    out->ns = ns;
+    return alloc(&out->p, 3 * ns);
+  }
+  Vec at(double *base, size_t k) const { return Vec{base + k * 3 * ns, ns}; }
+  int *flag() { return flags + next_flag++; }
+  void note(cudaError_t e) {
+    if (err == cudaSuccess) err = e;
+  }
+  size_t row_smem() const { return sizeof(unsigned) * (size_t)l.maxnb * (kAB / 32); }
 
-  // cell grid of the positions x, when *want != 0
-  void cells(const double4 *x, const int *want) {
-    if (n <= kGrid1Atoms) {
-      a_grid1<<<1, 1024, 0, s>>>(x, n, g, ncell, cell, count, start, fill, perm_fill, perm, qs, want);
-      return;
+  // Blocks of an evaluation: enough for its lanes and for a warp per row of a
+  // rebuild, at most what is resident at once (a rebuild's barriers need every
+  // block).  Fixed for a lane count, and the same for both loss passes, so that
+  // the block sums are.
+  template <Kind K, bool GRAD, int TPA>
+  int grid() {
+    int per_sm = 0;
+    note(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, a_eval<K, GRAD, TPA>, kAB, row_smem()));
+    if (K == kLoss) {
+      int other = 0;
+      note(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&other, a_eval<kLoss, !GRAD, TPA>, kAB, row_smem()));
+      per_sm = std::min(per_sm, other);
     }
-    a_clear<<<std::min(nblk(ncell), 1024), kAB, 0, s>>>(count, fill, ncell, want);
-    a_count<<<nblk(n), kAB, 0, s>>>(x, n, g, cell, count, want);
-    a_scan<<<1, 1024, 0, s>>>(count, start, ncell, want);
-    a_fill<<<nblk(n), kAB, 0, s>>>(n, cell, start, fill, perm_fill, want);
-    a_sort<<<nblk(ncell * 32), kAB, 0, s>>>(ncell, start, perm_fill, perm, want);
-    a_gather<<<nblk(n), kAB, 0, s>>>(x, perm, qs, n, want);
+    const long long need = ((long long)n * std::max(TPA, 32) + kAB - 1) / kAB;
+    return (int)std::max<long long>(1, std::min<long long>(need, (long long)std::max(per_sm, 1) * sms));
   }
-  // True if a row outgrew maxnb in any build so far (the sums are then
-  // incomplete).
-  bool rows_overflowed() {
-    if (cudaMemcpyAsync(hflag, flag + 2, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) return true;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return true;
-    return hflag[0] != 0;
+  int grids[4][8] = {};  // by kind (a loss with gradients: 3) and lanes, 0: not computed yet
+  template <Kind K, bool GRAD, int TPA>
+  int eval_tpa(Eval &e) {
+    int &g = grids[K == kLoss && GRAD ? 3 : K][TPA - 1];
+    if (g == 0) g = grid<K, GRAD, TPA>();
+    void *args[] = {&l, &p, &e};
+    note(cudaLaunchCooperativeKernel((const void *)a_eval<K, GRAD, TPA>, dim3(g), dim3(kAB), args, row_smem(), s));
+    return g;
   }
-  // Makes the list valid for an evaluation at x, on the device: a_check
-  // raises this evaluation's rebuild flag when an atom has moved more than
-  // skin/2 since the list's build, and the grid and row kernels run only
-  // then (two flags, used by alternate evaluations: a_rows clears the next
-  // one).  No host wait.
-  void prepare(const double4 *x) {
-    int *want = flag + (evals & 1), *next = flag + ((evals + 1) & 1);
-    evals++;
-    a_check<<<nblk(n), kAB, 0, s>>>(x, qb, n, rows, half_skin2, want);
-    cells(x, want);
-    const int wb = (int)(((long long)n * 32 + kAB - 1) / kAB);  // one warp per atom
-    int *ov = flag + 2;
-    if (maxnb <= 32) a_rows<1><<<wb, kAB, 0, s>>>(x, n, g, sl2, maxnb, nbr, cnt, qb, want, next, ov);
-    else if (maxnb <= 64) a_rows<2><<<wb, kAB, 0, s>>>(x, n, g, sl2, maxnb, nbr, cnt, qb, want, next, ov);
-    else if (maxnb <= 128) a_rows<4><<<wb, kAB, 0, s>>>(x, n, g, sl2, maxnb, nbr, cnt, qb, want, next, ov);
-    else if (maxnb <= 256) a_rows<8><<<wb, kAB, 0, s>>>(x, n, g, sl2, maxnb, nbr, cnt, qb, want, next, ov);
-    else if (maxnb <= 512) a_rows<16><<<wb, kAB, 0, s>>>(x, n, g, sl2, maxnb, nbr, cnt, qb, want, next, ov);
-    else a_rows<32><<<wb, kAB, 0, s>>>(x, n, g, sl2, maxnb, nbr, cnt, qb, want, next, ov);
-  }
-  void force(const double4 *x) {
-    const int nb = pair_blocks();
+  // Launches one evaluation; returns its blocks.
+  template <Kind K, bool GRAD>
+  int eval(Eval &e) {
     switch (tpa) {
-      case 1: a_force<1><<<nb, kAB, 0, s>>>(x, n, rows, p, f); break;
-      case 2: a_force<2><<<nb, kAB, 0, s>>>(x, n, rows, p, f); break;
-      case 4: a_force<4><<<nb, kAB, 0, s>>>(x, n, rows, p, f); break;
-      default: a_force<8><<<nb, kAB, 0, s>>>(x, n, rows, p, f); break;
+      case 1: return eval_tpa<K, GRAD, 1>(e);
+      case 2: return eval_tpa<K, GRAD, 2>(e);
+      case 4: return eval_tpa<K, GRAD, 4>(e);
+      default: return eval_tpa<K, GRAD, 8>(e);
     }
   }
-  void loss(const double4 *x, double4 *grad, double scale) {
-    const int nb = pair_blocks();
-    switch (tpa) {
-      case 1: a_loss<1><<<nb, kAB, 0, s>>>(x, n, rows, p, part, grad, scale); break;
-      case 2: a_loss<2><<<nb, kAB, 0, s>>>(x, n, rows, p, part, grad, scale); break;
-      case 4: a_loss<4><<<nb, kAB, 0, s>>>(x, n, rows, p, part, grad, scale); break;
-      default: a_loss<8><<<nb, kAB, 0, s>>>(x, n, rows, p, part, grad, scale); break;
-    }
+  size_t part_stride() const { return (size_t)max_blocks * 3; }
+  void half(const Vec &a, const Vec &b, const Vec &out, int *move) {
+    a_half<<<nblk(n), kAB, 0, s>>>(l, a, b, out, 0.5 * dt, move);
   }
-  void hvp(const double4 *x) {
-    const int nb = pair_blocks();
-    switch (tpa) {
-      case 1: a_hvp<1><<<nb, kAB, 0, s>>>(x, n, rows, p, u, w, part); break;
-      case 2: a_hvp<2><<<nb, kAB, 0, s>>>(x, n, rows, p, u, w, part); break;
-      case 4: a_hvp<4><<<nb, kAB, 0, s>>>(x, n, rows, p, u, w, part); break;
-      default: a_hvp<8><<<nb, kAB, 0, s>>>(x, n, rows, p, u, w, part); break;
-    }
+  void copy(double *to, const double *from) {
+    note(cudaMemcpyAsync(to, from, sizeof(double) * 3 * ns, cudaMemcpyDeviceToDevice, s));
   }
-  // one forward step; keeps q_h and v' when asked
-  void step(double4 *qh_out, double4 *v_out) {
-    a_drift<<<nblk(n), kAB, 0, s>>>(q, v, n, 0.5 * dt);
-    prepare(q);
-    force(q);
-    if (qh_out) cudaMemcpyAsync(qh_out, q, sizeof(double4) * n, cudaMemcpyDeviceToDevice, s);
-    a_kick<<<nblk(n), kAB, 0, s>>>(v, f, n, dt);
-    if (v_out) cudaMemcpyAsync(v_out, v, sizeof(double4) * n, cudaMemcpyDeviceToDevice, s);
-    a_drift<<<nblk(n), kAB, 0, s>>>(q, v, n, 0.5 * dt);
-  }
-  // loss terms at x: sums into out[0..2] (device), gradient into lq when scale != 0
-  void loss_at(const double4 *x, double scale, double *out) {
-    prepare(x);
-    loss(x, scale != 0.0 ? lq : nullptr, scale);
-    if (out) a_reduce<<<1, kRB, 0, s>>>(part, pair_blocks(), 3, out);
+  // Row overflow (the sums are then incomplete) or a barrier that timed out.
+  mdg_status list_status() {
+    if (cudaMemcpyAsync(ws->hflag, state, 2 * sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess)
+      return MDG_ERR_CUDA;
+    if (cudaStreamSynchronize(s) != cudaSuccess) return MDG_ERR_CUDA;
+    if (ws->hflag[1]) return MDG_ERR_TIMEOUT;
+    return ws->hflag[0] ? MDG_ERR_CAPACITY : MDG_OK;
   }
 };
 
-// Lanes per atom of the pair kernels, chosen once per device and problem
-// shape by timing the force kernel with 1, 2, 4 and 8 lanes (the fastest is
-// kept for the process, so repeated runs of one shape use the same lanes and
-// give the same sums).
+// Lanes per atom of the passes, chosen once per device and problem shape by
+// timing the loss pass with 1, 2, 4 and 8 lanes (the fastest is kept for the
+// process, so repeated runs of one shape use the same lanes and give the same
+// sums).  `want`: the list's first build.
 std::mutex g_tune_mutex;
 std::map<std::tuple<int, int, int>, int> g_tune;
 
-int autotune_tpa(Run &R, int device) {
-  const auto key = std::make_tuple(device, R.n, R.ncell);
+int autotune_tpa(Run &R, int device, int *want) {
+  const auto key = std::make_tuple(device, R.n, R.l.ncell);
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
     auto it = g_tune.find(key);
@@ -816,23 +773,33 @@ int autotune_tpa(Run &R, int device) {
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  R.prepare(R.q);
   int best = 1;
   float best_ms = 1e30f;
-  for (int t : {1, 2, 4, 8}) {
-    R.tpa = t;
-    R.force(R.q);  // warm-up
-    cudaEventRecord(e0, R.s);
-    for (int r = 0; r < 3; r++) R.force(R.q);
-    cudaEventRecord(e1, R.s);
-    cudaEventSynchronize(e1);
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, e0, e1);
-    if (ms < best_ms) {
-      best_ms = ms;
-      best = t;
+  Eval e{};
+  e.x = R.x[0];
+  e.dt = R.dt;
+  e.part = R.part;
+  e.want = want;
+  int *never = R.flag();
+  // the best of three rounds, the first of which warms up (and its first
+  // launch builds the list)
+  for (int round = 0; round < 3; round++)
+    for (int t : {1, 2, 4, 8}) {
+      R.tpa = t;
+      cudaEventRecord(e0, R.s);
+      for (int r = 0; r < 3; r++) {
+        R.eval<kLoss, false>(e);
+        e.want = never;
+      }
+      cudaEventRecord(e1, R.s);
+      cudaEventSynchronize(e1);
+      float ms = 0.f;
+      cudaEventElapsedTime(&ms, e0, e1);
+      if (round > 0 && ms < best_ms) {
+        best_ms = ms;
+        best = t;
+      }
     }
-  }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   std::lock_guard<std::mutex> lock(g_tune_mutex);
@@ -886,64 +853,81 @@ mdg_status mdg_adjoint_run(const mdg_adjoint_params *prm, const double *q0, cons
   if (prm->device < 0 || prm->device >= ndev) return MDG_ERR_INVALID_ARGUMENT;
   if (cudaSetDevice(prm->device) != cudaSuccess) return MDG_ERR_CUDA;
 
+  if (n >= 1 << 29) return MDG_ERR_CAPACITY;  // a row key holds 29 bits of index
   Run R;
   R.n = n;
+  R.ns = ((size_t)n + 1) / 2 * 2;
+  R.device = prm->device;
   R.dt = prm->time_step;
+  List &l = R.l;
+  l.n = n;
   const double rc = prm->cutoff * prm->sigma;
   // list skin: 0.3 sigma, less where a box axis holds fewer than three
   // cells of r_c + skin (no skin at all: the list is rebuilt whenever an
   // atom moved)
   double skin = 0.3 * prm->sigma;
+  double longest = 0.0;
   for (int d = 0; d < 3; d++) {
     const double L = prm->L[d];
     if (!(L > 0.0) || !std::isfinite(L)) return MDG_ERR_INVALID_ARGUMENT;
     if ((int)(L / rc) < 3) return MDG_ERR_BOX_TOO_SMALL;
     skin = std::min(skin, L / 3.0 * (1.0 - 1e-9) - rc);  // cells of L/ms >= r_c + skin, ms >= 3
+    longest = std::max(longest, L);
   }
   skin = std::max(skin, 0.0);
   const double sl = rc + skin;
   for (int d = 0; d < 3; d++) {
     const double L = prm->L[d];
-    R.g.ms[d] = std::max(3, (int)(L / sl));
-    R.g.L[d] = L;
-    R.g.inv_cs[d] = R.g.ms[d] / L;
-    R.g.inv_L[d] = 1.0 / L;
-    R.rows.L[d] = L;
-    R.rows.inv_L[d] = 1.0 / L;
+    l.ms[d] = std::max(3, (int)(L / sl));
+    l.L[d] = L;
+    l.inv_cs[d] = l.ms[d] / L;
+    l.inv_L[d] = 1.0 / L;
+    l.Lf[d] = (float)L;
+    l.inv_Lf[d] = (float)(1.0 / L);
   }
-  // rows keep pairs up to sl, a hair wider than the r_c + 2 (skin / 2) that
-  // the displacement bound needs
-  R.sl2 = sl * sl * (1.0 + 1e-9);
-  R.half_skin2 = 0.25 * skin * skin;
+  // rows keep pairs up to sl and, for the FP32 rounding of box coordinates
+  // (each difference is off by less than 4 u L, u = 2^-24; eight times that
+  // here), a little more
+  const double reach = sl * (1.0 + 1e-5) + 32.0 / 16777216.0 * longest;
+  l.reach2 = (float)(reach * reach);
+  l.half_skin2 = 0.25 * skin * skin;
   {
     const double vol = prm->L[0] * prm->L[1] * prm->L[2];
     const double est = 4.0 / 3.0 * M_PI * sl * sl * sl * (double)n / vol;
     // twice the mean density's count plus 64, and at least the count at
     // density 1.3 (above a close-packed LJ solid) plus 32, so that a dense
-    // region of a dilute box fits; at most 1024 (the row sort's width).  A
-    // longer row is MDG_ERR_CAPACITY.
+    // region of a dilute box fits; at most 1024.  A longer row is
+    // MDG_ERR_CAPACITY.
     const double dense = 4.0 / 3.0 * M_PI * sl * sl * sl * 1.3 / (prm->sigma * prm->sigma * prm->sigma);
     const double want = std::max(std::ceil(2.0 * est + 64.0), std::ceil(dense + 32.0));
-    R.maxnb = (int)std::min<double>(std::min(std::max(n - 1, 1), 1024), want);
+    l.maxnb = (int)std::min<double>(std::min(std::max(n - 1, 1), 1024), want);
   }
-  R.ncell = R.g.ms[0] * R.g.ms[1] * R.g.ms[2];
+  l.ncell = l.ms[0] * l.ms[1] * l.ms[2];
   const double sc = prm->cutoff;
-  R.p.eps = prm->epsilon;
-  R.p.sigma = prm->sigma;
-  R.p.rc2 = rc * rc;
-  R.p.c2 = 6.0 * pow(sc, -14.0) - 3.0 * pow(sc, -8.0);
-  R.p.c0 = -pow(sc, -12.0) + pow(sc, -6.0) - R.p.c2 * sc * sc;
-  R.p.a = prm->shell_lo;
-  R.p.b = prm->shell_hi;
-  R.p.w = prm->shell_width;
-  R.p.inv_sigma = 1.0 / R.p.sigma;
-  R.p.inv_w = 1.0 / R.p.w;
-  R.p.inv_eps = 1.0 / R.p.eps;
-  R.p.eps_sigma = R.p.eps / R.p.sigma;
-  R.p.eps_sigma2 = R.p.eps / (R.p.sigma * R.p.sigma);
+  Pot &p = R.p;
+  p.rc2 = rc * rc;
+  p.c2 = 6.0 * pow(sc, -14.0) - 3.0 * pow(sc, -8.0);
+  p.c0 = -pow(sc, -12.0) + pow(sc, -6.0) - p.c2 * sc * sc;
+  p.sigma2 = prm->sigma * prm->sigma;
+  p.inv_sigma = 1.0 / prm->sigma;
+  p.inv_sigma2 = 1.0 / p.sigma2;
+  p.inv_eps = 1.0 / prm->epsilon;
+  p.e4 = 4.0 * prm->epsilon;
+  p.k4 = p.e4 / p.sigma2;
+  p.a = prm->shell_lo;
+  p.b = prm->shell_hi;
+  p.inv_w = 1.0 / prm->shell_width;
+  p.mid = 0.5 * (p.a + p.b);
+  p.h = exp(0.5 * (p.a - p.b) * p.inv_w);
+  {
+    // E = exp((r - mid)/w) and h as factors of a product of four stay finite
+    // and normal
+    const double most = 150.0 * prm->shell_width;
+    p.one_exp = fabs(p.mid) < most && fabs(rc - p.mid) < most && fabs(0.5 * (p.a - p.b)) < most;
+  }
   const int T = prm->steps, k = prm->checkpoint_every;
   const int nck = (T + k - 1) / k + 1;
-  const size_t max_blocks = ((size_t)n * 8 + kAB - 1) / kAB;
+  const int seg = std::min(k, T);
 
   std::lock_guard<std::mutex> ws_lock(g_ws_mutex);
   Workspace &ws = g_ws[prm->device];
@@ -957,134 +941,201 @@ mdg_status mdg_adjoint_run(const mdg_adjoint_params *prm, const double *q0, cons
     }
   }
   R.ws = &ws;
-  cudaError_t e = cudaSuccess;
-  if (!ws.s) e = cudaStreamCreateWithFlags(&ws.s, cudaStreamNonBlocking);
+  cudaError_t e = cudaDeviceGetAttribute(&R.sms, cudaDevAttrMultiProcessorCount, prm->device);
+  R.max_blocks = (int)std::min<long long>(((long long)n * 32 + kAB - 1) / kAB, (long long)R.sms * 16);
+  if (e == cudaSuccess && !ws.s) e = cudaStreamCreateWithFlags(&ws.s, cudaStreamNonBlocking);
   if (e == cudaSuccess && !ws.hflag) e = cudaMallocHost((void **)&ws.hflag, 2 * sizeof(int));
   R.s = ws.s;
-  R.hflag = ws.hflag;
-  if (e == cudaSuccess) e = R.alloc(&R.q, n);
-  if (e == cudaSuccess) e = R.alloc(&R.v, n);
-  if (e == cudaSuccess) e = R.alloc(&R.f, n);
-  if (e == cudaSuccess) e = R.alloc(&R.tmp, n);
-  if (e == cudaSuccess) e = R.alloc(&R.cell, n);
-  if (e == cudaSuccess) e = R.alloc(&R.count, R.ncell);
-  if (e == cudaSuccess) e = R.alloc(&R.fill, R.ncell);
-  if (e == cudaSuccess) e = R.alloc(&R.start, R.ncell + 1);
-  if (e == cudaSuccess) e = R.alloc(&R.perm, n);
-  if (e == cudaSuccess) e = R.alloc(&R.perm_fill, n);
-  if (e == cudaSuccess) e = R.alloc(&R.qs, n);
-  if (e == cudaSuccess) e = R.alloc(&R.part, max_blocks * 3);
+  const size_t nflags = 6 * (size_t)T + 2 * (size_t)nck + 16;
+  if (e == cudaSuccess) e = R.alloc(&R.q);
+  if (e == cudaSuccess) e = R.alloc(&R.v);
+  if (e == cudaSuccess) e = R.alloc(&R.x[0]);
+  if (e == cudaSuccess) e = R.alloc(&R.x[1]);
+  if (e == cudaSuccess) e = R.alloc(&l.qb);
+  if (e == cudaSuccess) e = R.alloc(&R.raw, 3 * (size_t)n);
+  if (e == cudaSuccess) e = R.alloc(&l.cell, n);
+  if (e == cudaSuccess) e = R.alloc(&l.rank, n);
+  if (e == cudaSuccess) e = R.alloc(&l.count, l.ncell);
+  if (e == cudaSuccess) e = R.alloc(&l.start, l.ncell);
+  if (e == cudaSuccess) e = R.alloc(&l.sorted, n);
+  if (e == cudaSuccess) e = R.alloc(&l.nbr, (size_t)l.maxnb * n);
+  if (e == cudaSuccess) e = R.alloc(&l.ends, (size_t)kBuckets * n);
+  if (e == cudaSuccess) e = R.alloc(&R.part, R.part_stride() * kReduceSlots * (grad ? 2 : 1));
   if (e == cudaSuccess) e = R.alloc(&R.loss_sums, (size_t)T * 3);
-  if (e == cudaSuccess) e = R.alloc(&R.nbr, (size_t)R.maxnb * n);
-  if (e == cudaSuccess) e = R.alloc(&R.cnt, n);
-  if (e == cudaSuccess) e = R.alloc(&R.qb, n);
-  if (e == cudaSuccess) e = R.alloc(&R.flag, 3);
-  if (e == cudaSuccess) {
-    const int first[3] = {1, 0, 0};  // the first evaluation builds the list; no overflow
-    e = cudaMemsetAsync(R.qb, 0, sizeof(double4) * n, R.s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(R.flag, first, sizeof(first), cudaMemcpyHostToDevice, R.s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(R.s);
-  }
+  if (e == cudaSuccess) e = R.alloc(&R.flags, nflags);
+  if (e == cudaSuccess) e = R.alloc(&R.state, 8);
   if (grad) {
-    if (e == cudaSuccess) e = R.alloc(&R.lq, n);
-    if (e == cudaSuccess) e = R.alloc(&R.lv, n);
-    if (e == cudaSuccess) e = R.alloc(&R.u, n);
-    if (e == cudaSuccess) e = R.alloc(&R.w, n);
+    if (e == cudaSuccess) e = R.alloc(&R.lq);
+    if (e == cudaSuccess) e = R.alloc(&R.lv);
+    if (e == cudaSuccess) e = R.alloc(&R.u);
     if (e == cudaSuccess) e = R.alloc(&R.adj_sums, (size_t)T * 2);
-    if (e == cudaSuccess) e = R.alloc(&R.ck_q, (size_t)nck * n);
-    if (e == cudaSuccess) e = R.alloc(&R.ck_v, (size_t)nck * n);
-    if (e == cudaSuccess) e = R.alloc(&R.seg_qh, (size_t)k * n);
-    if (e == cudaSuccess) e = R.alloc(&R.seg_v, (size_t)k * n);
+    if (e == cudaSuccess) e = R.alloc(&R.ck_q, (size_t)nck * 3 * R.ns);
+    if (e == cudaSuccess) e = R.alloc(&R.ck_v, (size_t)nck * 3 * R.ns);
+    if (e == cudaSuccess) e = R.alloc(&R.seg_x, (size_t)seg * 3 * R.ns);
+    if (e == cudaSuccess) e = R.alloc(&R.seg_v, (size_t)seg * 3 * R.ns);
   }
   if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? MDG_ERR_CAPACITY : MDG_ERR_CUDA;
-  R.g.start = R.start;
-  R.g.perm = R.perm;
-  R.g.qs = R.qs;
-  R.rows.nbr = R.nbr;
-  R.rows.cnt = R.cnt;
+  l.overflow = R.state;
+  l.timeout = R.state + 1;
+  l.cursor = R.state + 2;
+  l.bar = reinterpret_cast<mdg::GridBarrier *>(R.state + 4);
+  R.note(cudaMemsetAsync(R.flags, 0, sizeof(int) * nflags, R.s));
+  R.note(cudaMemsetAsync(R.state, 0, sizeof(int) * 8, R.s));
+  R.note(cudaMemsetAsync(l.qb.p, 0, sizeof(double) * 3 * R.ns, R.s));
 
-  // upload (n x 3 host arrays -> double4)
-  {
-    std::vector<double4> hq(n), hv(n);
-    for (int i = 0; i < n; i++) {
-      hq[i] = make_double4(q0[3 * i], q0[3 * i + 1], q0[3 * i + 2], 0.0);
-      hv[i] = make_double4(v0[3 * i], v0[3 * i + 1], v0[3 * i + 2], 0.0);
-    }
-    e = cudaMemcpyAsync(R.q, hq.data(), sizeof(double4) * n, cudaMemcpyHostToDevice, R.s);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(R.v, hv.data(), sizeof(double4) * n, cudaMemcpyHostToDevice, R.s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(R.s);
-    if (e != cudaSuccess) return MDG_ERR_CUDA;
+  R.note(cudaMemcpyAsync(R.raw, q0, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, R.s));
+  a_unpack<<<nblk(n), kAB, 0, R.s>>>(R.raw, R.q, n);
+  R.note(cudaMemcpyAsync(R.raw, v0, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, R.s));
+  a_unpack<<<nblk(n), kAB, 0, R.s>>>(R.raw, R.v, n);
+
+  // the first evaluation builds the list
+  int *move = R.flag();
+  R.note(cudaMemsetAsync(move, 1, 1, R.s));
+  R.half(R.q, R.v, R.x[0], move);
+  bool built = false;
+  if (prm->threads_per_atom) {
+    R.tpa = prm->threads_per_atom;
+  } else {
+    const int before = R.next_flag;
+    R.tpa = autotune_tpa(R, prm->device, move);
+    built = R.next_flag != before;
+    if (built) move = R.flag();  // timed: the list is there
   }
-  R.tpa = prm->threads_per_atom ? prm->threads_per_atom : autotune_tpa(R, prm->device);
 
-  // forward pass: loss terms per step, checkpoints every k steps
+  // forward pass.  Without gradients: loss terms per step.  With them:
+  // checkpoints every k steps; the reverse sweep passes every step's end
+  // state again, and its loss passes give the loss terms too.
+  int slots = 0, nb = 0;
   for (int t = 0; t < T; t++) {
     if (grad && t % k == 0) {
-      cudaMemcpyAsync(R.ck_q + (size_t)(t / k) * n, R.q, sizeof(double4) * n, cudaMemcpyDeviceToDevice, R.s);
-      cudaMemcpyAsync(R.ck_v + (size_t)(t / k) * n, R.v, sizeof(double4) * n, cudaMemcpyDeviceToDevice, R.s);
+      R.copy(R.ck_q + (size_t)(t / k) * 3 * R.ns, R.q.p);
+      R.copy(R.ck_v + (size_t)(t / k) * 3 * R.ns, R.v.p);
     }
-    R.step(nullptr, nullptr);
-    R.loss_at(R.q, 0.0, R.loss_sums + (size_t)3 * t);
+    if (grad && t / k == (T - 1) / k) break;  // the sweep runs the last segment itself
+    Eval f{};
+    f.x = R.x[t & 1];
+    f.want = move;
+    f.dt = R.dt;
+    f.v = f.v_out = R.v;
+    if (!grad || (t + 1) % k == 0) f.q_out = R.q;
+    f.x_out = R.x[(t + 1) & 1];
+    int *at_q = f.move = R.flag();
+    f.jump = R.flag();
+    move = grad ? f.move : f.jump;
+    R.eval<kForce, false>(f);
+    built = true;
+    if (grad) continue;
+    Eval o{};
+    o.x = R.q;
+    o.want = at_q;
+    o.dt = R.dt;
+    o.part = R.part + R.part_stride() * slots;
+    nb = R.eval<kLoss, false>(o);
+    if (++slots == kReduceSlots || t == T - 1) {
+      a_reduce<<<slots, kRB, 0, R.s>>>(R.part, R.part_stride(), nb, 3, R.loss_sums + (size_t)3 * (t + 1 - slots), 3);
+      slots = 0;
+    }
   }
   std::vector<double> sums((size_t)T * 3);
-  e = cudaMemcpyAsync(sums.data(), R.loss_sums, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, R.s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(R.s);
-  if (e != cudaSuccess || cudaGetLastError() != cudaSuccess) return MDG_ERR_CUDA;
   const double norm = 1.0 / ((double)T * n);
-  double l = 0.0, dl_deps = 0.0, dl_dsig = 0.0;
-  for (int t = 0; t < T; t++) {
-    l += sums[3 * t] + sums[3 * t + 1];
-    dl_deps += sums[3 * t] / prm->epsilon;  // PE is linear in epsilon
-    dl_dsig += sums[3 * t + 2];
+  double sum = 0.0, dl_deps = 0.0, dl_dsig = 0.0;
+  auto read_loss = [&]() {
+    R.note(cudaMemcpyAsync(sums.data(), R.loss_sums, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, R.s));
+    R.note(cudaStreamSynchronize(R.s));
+    for (int t = 0; t < T; t++) {
+      sum += sums[3 * t] + sums[3 * t + 1];
+      dl_deps += sums[3 * t] / prm->epsilon;  // PE is linear in epsilon
+      dl_dsig += sums[3 * t + 2];
+    }
+    *loss = sum * norm;
+  };
+  if (!grad) {
+    read_loss();
+    if (R.err != cudaSuccess || cudaGetLastError() != cudaSuccess) return MDG_ERR_CUDA;
+    return R.list_status();
   }
-  *loss = l * norm;
-  if (!grad) return R.rows_overflowed() ? MDG_ERR_CAPACITY : MDG_OK;
-  dl_deps *= norm;
-  dl_dsig *= norm;
 
   // reverse sweep, one checkpointed segment at a time
-  cudaMemsetAsync(R.lq, 0, sizeof(double4) * n, R.s);
-  cudaMemsetAsync(R.lv, 0, sizeof(double4) * n, R.s);
-  for (int seg = (T - 1) / k; seg >= 0; seg--) {
-    const int t0 = seg * k, t1 = std::min(T, t0 + k);
-    cudaMemcpyAsync(R.q, R.ck_q + (size_t)seg * n, sizeof(double4) * n, cudaMemcpyDeviceToDevice, R.s);
-    cudaMemcpyAsync(R.v, R.ck_v + (size_t)seg * n, sizeof(double4) * n, cudaMemcpyDeviceToDevice, R.s);
-    for (int t = t0; t < t1; t++) R.step(R.seg_qh + (size_t)(t - t0) * n, R.seg_v + (size_t)(t - t0) * n);
+  R.note(cudaMemsetAsync(R.lq.p, 0, sizeof(double) * 3 * R.ns, R.s));
+  R.note(cudaMemsetAsync(R.lv.p, 0, sizeof(double) * 3 * R.ns, R.s));
+  double *hess_part = R.part + R.part_stride() * kReduceSlots;
+  int nb_loss = 0;
+  for (int sg = (T - 1) / k; sg >= 0; sg--) {
+    const int t0 = sg * k, t1 = std::min(T, t0 + k);
+    // forward again from the checkpoint; the last step leaves q' for the sweep
+    move = R.flag();
+    if (!built) R.note(cudaMemsetAsync(move, 1, 1, R.s));  // no evaluation yet (one segment)
+    built = true;
+    R.half(R.at(R.ck_q, sg), R.at(R.ck_v, sg), R.at(R.seg_x, 0), move);
+    int *jump = nullptr;
+    for (int t = t0; t < t1; t++) {
+      Eval f{};
+      f.x = R.at(R.seg_x, t - t0);
+      f.want = move;
+      f.dt = R.dt;
+      f.v = t == t0 ? R.at(R.ck_v, sg) : R.at(R.seg_v, t - 1 - t0);
+      f.v_out = R.at(R.seg_v, t - t0);
+      if (t == t1 - 1) f.q_out = R.q;
+      else f.x_out = R.at(R.seg_x, t + 1 - t0);
+      move = f.move = R.flag();
+      jump = f.jump = R.flag();
+      R.eval<kForce, false>(f);
+    }
     for (int t = t1 - 1; t >= t0; t--) {
-      const double4 *qh = R.seg_qh + (size_t)(t - t0) * n;
-      const double4 *vp = R.seg_v + (size_t)(t - t0) * n;
-      // q' = q_h + v' dt/2, and this step's loss gradient at q'
-      cudaMemcpyAsync(R.tmp, qh, sizeof(double4) * n, cudaMemcpyDeviceToDevice, R.s);
-      a_drift<<<nblk(n), kAB, 0, R.s>>>(R.tmp, vp, n, 0.5 * R.dt);
-      R.loss_at(R.tmp, norm, nullptr);
-      a_rev1<<<nblk(n), kAB, 0, R.s>>>(R.lq, R.lv, R.u, n, R.dt);
-      R.prepare(qh);
-      R.hvp(qh);
-      a_reduce<<<1, kRB, 0, R.s>>>(R.part, R.pair_blocks(), 2, R.adj_sums + (size_t)2 * t);
-      a_rev2<<<nblk(n), kAB, 0, R.s>>>(R.lq, R.lv, R.w, n, R.dt);
+      Eval g{};
+      g.x = R.q;
+      g.want = move;
+      g.dt = R.dt;
+      g.lq = R.lq;
+      g.lv = R.lv;
+      g.u = R.u;
+      g.scale = norm;
+      g.part = R.part + R.part_stride() * slots;
+      nb_loss = R.eval<kLoss, true>(g);
+      Eval h{};
+      h.x = R.at(R.seg_x, t - t0);
+      h.want = jump;
+      h.dt = R.dt;
+      h.lq = R.lq;
+      h.lv = R.lv;
+      h.u = R.u;
+      h.part = hess_part + R.part_stride() * slots;
+      if (t > t0) {
+        h.x_prev = R.at(R.seg_x, t - 1 - t0);
+        h.v_prev = R.at(R.seg_v, t - 1 - t0);
+        h.q_out = R.q;
+      }
+      move = h.move = R.flag();
+      jump = h.jump = R.flag();
+      nb = R.eval<kHess, false>(h);
+      if (++slots == kReduceSlots || t == 0) {
+        // slot s holds step t + slots - 1 - s
+        a_reduce<<<slots, kRB, 0, R.s>>>(R.part, R.part_stride(), nb_loss, 3,
+                                         R.loss_sums + (size_t)3 * (t + slots - 1), -3);
+        a_reduce<<<slots, kRB, 0, R.s>>>(hess_part, R.part_stride(), nb, 2, R.adj_sums + (size_t)2 * (t + slots - 1),
+                                         -2);
+        slots = 0;
+      }
     }
   }
   std::vector<double> adj((size_t)T * 2);
-  e = cudaMemcpyAsync(adj.data(), R.adj_sums, sizeof(double) * adj.size(), cudaMemcpyDeviceToHost, R.s);
-  std::vector<double4> h(n);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), R.lq, sizeof(double4) * n, cudaMemcpyDeviceToHost, R.s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(R.s);
-  if (e != cudaSuccess || cudaGetLastError() != cudaSuccess) return MDG_ERR_CUDA;
+  R.note(cudaMemcpyAsync(adj.data(), R.adj_sums, sizeof(double) * adj.size(), cudaMemcpyDeviceToHost, R.s));
+  if (dloss_dq0) {
+    a_pack<<<nblk(n), kAB, 0, R.s>>>(R.lq, R.raw, n);
+    R.note(cudaMemcpyAsync(dloss_dq0, R.raw, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, R.s));
+  }
+  read_loss();
+  if (R.err != cudaSuccess || cudaGetLastError() != cudaSuccess) return MDG_ERR_CUDA;
+  dl_deps *= norm;
+  dl_dsig *= norm;
   // dynamics terms summed in reverse-sweep order, as the sweep produced them
   for (int t = T - 1; t >= 0; t--) {
     dl_deps += adj[(size_t)2 * t];
     dl_dsig += adj[(size_t)2 * t + 1];
   }
-  if (dloss_dq0) {
-    for (int i = 0; i < n; i++) {
-      dloss_dq0[3 * i] = h[i].x;
-      dloss_dq0[3 * i + 1] = h[i].y;
-      dloss_dq0[3 * i + 2] = h[i].z;
-    }
-  }
   if (dloss_deps) *dloss_deps = dl_deps;
   if (dloss_dsigma) *dloss_dsigma = dl_dsig;
-  return R.rows_overflowed() ? MDG_ERR_CAPACITY : MDG_OK;
+  return R.list_status();
 }
 
 }  // extern "C"
