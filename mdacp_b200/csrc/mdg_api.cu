@@ -111,6 +111,7 @@ struct mdg_handle {
   int tpa = 0;                        // lanes per atom of the FP32 force pass (0: to be tuned)
   int build_block = 0;                // threads per block of the list build (0: to be tuned)
   int build_tpa = 0;                  // lanes per atom of the list build (0: to be tuned)
+  int sms = 148;                      // multiprocessors of the device
   GridBarrier *d_bar = nullptr;       // persistent pass: grid barrier
   int *d_pout = nullptr;              // persistent pass: block 0's decisions
   int64_t persistent_steps = 0;
@@ -274,7 +275,17 @@ void launch_list_build_block(mdg_handle *h, cudaStream_t s, int lanes) {
   else k_build<BLOCK, false, false, 1><<<nb, BLOCK, 0, s>>>(h->a, h->box, n);
 }
 
+// Few atoms with one lane each: the split walk, whatever the block size.
 void launch_list_build(mdg_handle *h, cudaStream_t s, int block, int lanes) {
+  const int split = lanes == 1 ? build_split(h->n, h->sms) : 1;
+  if (split == 9) {
+    k_build_split<9><<<blocks_for(h->n, 32), 9 * 32, 0, s>>>(h->a, h->box, h->n);
+    return;
+  }
+  if (split == 3) {
+    k_build_split<3><<<blocks_for(h->n, 32), 3 * 32, 0, s>>>(h->a, h->box, h->n);
+    return;
+  }
   if (block == 64) launch_list_build_block<64>(h, s, lanes);
   else if (block == 256) launch_list_build_block<256>(h, s, lanes);
   else launch_list_build_block<128>(h, s, lanes);
@@ -1000,6 +1011,7 @@ mdg_status mdg_create(const mdg_params *prm, mdg_handle **out) {
   h->build_tpa = prm->build_threads_per_atom;
 
   cudaError_t e = cudaSetDevice(prm->device);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, prm->device);
   if (e == cudaSuccess) {
     if (prm->stream) {
       h->stream = (cudaStream_t)prm->stream;

@@ -502,6 +502,9 @@ __global__ void __launch_bounds__(BLOCK) k_disp_collect(Arrays a, Box b, int n, 
   // no copy of this atom moved more than c (k_disp_max's per-atom maximum
   // of the same displacements): nothing to collect
   if (a.disp2 && !(a.disp2[i] > c_d2)) return;
+  // a full list: the number of copies has decided (k_disp_pairs; over several
+  // slabs too), and thousands of atomics to one address would follow
+  if (*(volatile const int *)&a.st->cand_weighted >= cand_cap) return;
   for_each_copy(copy_view(a), b.L, i, lag, [&](int code, double d2) {
     if (d2 > c_d2) {
       atomicAdd(&a.st->cand_weighted, 1);
@@ -522,7 +525,7 @@ struct PairStage {
 };
 
 // The pair test of PairList::CheckByDisplacement (src/pairlist.cc:99-121)
-// over rows a = part, part + parts, ... of the candidate list: sets *found
+// over the candidate list's rows, a warp each, dealt over `parts` blocks: sets *found
 // if a pair of candidate copies (a < b) that was at least SearchLength apart
 // at the last build is now inside the cut-off.  Copies carry their shifts,
 // so the distances are the reference's direct differences.  The result is
@@ -534,10 +537,11 @@ template <int BLOCK>
 __device__ __forceinline__ void candidate_pair_test_global(const CopyView &cv, const double L[3], const int2 *cand,
                                                            int l, double lag, double sl2, double rc2, int part,
                                                            int parts, volatile int *found) {
-  for (int a = part; a < l - 1 && !*found; a += parts) {
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int a = part * (BLOCK / 32) + w; a < l - 1 && !*found; a += parts * (BLOCK / 32)) {
     double o1[3], n1[3];
     copy_positions(cv, L, cand[a].x, cand[a].y, lag, o1, n1);
-    for (int c = a + 1 + threadIdx.x; c < l; c += BLOCK) {
+    for (int c = a + 1 + lane; c < l; c += 32) {
       double o2[3], n2[3];
       copy_positions(cv, L, cand[c].x, cand[c].y, lag, o2, n2);
       if (dist2(o1, o2) < sl2) continue;
@@ -561,10 +565,11 @@ __device__ __forceinline__ void candidate_pair_test(const CopyView &cv, const do
       }
     }
     __syncthreads();
-    for (int a = part; a < l - 1 && !*found; a += parts) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int a = part * (BLOCK / 32) + w; a < l - 1 && !*found; a += parts * (BLOCK / 32)) {
       const double o1[3] = {sm.o[0][a], sm.o[1][a], sm.o[2][a]};
       const double n1[3] = {sm.n[0][a], sm.n[1][a], sm.n[2][a]};
-      for (int c = a + 1 + threadIdx.x; c < l; c += BLOCK) {
+      for (int c = a + 1 + lane; c < l; c += 32) {
         const double o2[3] = {sm.o[0][c], sm.o[1][c], sm.o[2][c]};
         if (dist2(o1, o2) < sl2) continue;
         const double n2[3] = {sm.n[0][c], sm.n[1][c], sm.n[2][c]};
@@ -1230,15 +1235,16 @@ __device__ __forceinline__ float sqrt_approx(float x) {
 
 // Candidates of one run that a warp stages at a time, and words of found
 // partners that a lane keeps before they go to the list.
-constexpr int kRunStage = 128, kRowWords = 16;
+constexpr int kRunStage = 128;
 
 // Shared memory of one warp's row walk.
+template <int WORDS>
 struct WarpRows {
   float4 xy[kRunStage / 2];  // staged candidates in pairs: x0, x1, y0, y1
   float2 zz[kRunStage / 2];  //                             z0, z1
   // column l: lane l's words, 32 candidates each: partners as bits (the first
   // candidate at bit 31) and the first candidate's slot
-  uint2 word[kRowWords][32];
+  uint2 word[WORDS][32];
 };
 
 // The exact test of candidate j of atom i (within_search_exact) through the
@@ -1257,11 +1263,32 @@ static __device__ __noinline__ bool band_test_row(const RowGeom &g, const double
   return within_search_exact(qi, qj, shift_of(xc, 0, g.L), shift_of(yz, 1, g.L), shift_of(yz, 2, g.L), g.sl2);
 }
 
+// Words a lane has room for: nine warps' rows fit a block's 48 KB.
+__host__ __device__ constexpr int row_words(int split) { return split == 9 ? 14 : 16; }
+
+// A lane's atom of a system narrower than three cells an axis (ensembles),
+// whose partners are its system's other atoms [beg, end) in slot order, each
+// through its minimum image (unique: L > 2 SearchLength).
+struct SmallRow {
+  bool on;
+  int beg, end;
+};
+
 // The full Verlet rows of a warp's 32 atoms, one lane each: build_rows' rows
 // entry for entry (the same 9 runs of slots in the same order, the same FP32
 // prefilter, ghost-existence rule and exact test of the band).  All 32 lanes
 // call; lanes without an atom pass active = false and any valid slot i.
-// owner tells lanes of different systems apart.
+// owner tells lanes of different systems apart.  With SMALL, lanes whose
+// small.on is set take that row instead (active = false).
+//
+// SPLIT warps of a block (1, 3 or 9; the block has SPLIT warps when more than
+// 1) share the same 32 atoms: warp `part` walks 9 / SPLIT of the runs, or that
+// share of a small row, and the lanes' entries follow those of the parts
+// before (counts: SPLIT x 32 shared words; all threads of the block call).  A
+// single warp's walk is a chain of nine look-ups, loads and walks; with too few
+// atoms to fill the chip that chain is the build's time.  Before its place is
+// known (pass 0) a part keeps its words; one whose words do not fit walks again.  Returns the
+// row length on the first part's lanes, 0 on the others.
 //
 // build_rows is bound by the L1 data path, its latency and its branches: every
 // lane loads its own candidates (32 addresses a load, two thirds of the lanes
@@ -1288,11 +1315,14 @@ static __device__ __noinline__ bool band_test_row(const RowGeom &g, const double
 // the 2.05M-atom liquid 1.13 ms against 2.05 ms.  64 registers (32 warps an
 // SM, a few spills outside the walk) against 80: 1.13 and 1.17 ms; partners
 // filed one by one in a shared-memory ring instead of words: 1.6 ms.
-template <bool SLAB>
+template <bool SLAB, int SPLIT, bool SMALL>
 __device__ __forceinline__ int build_rows_warp(const RowGeom &g, const float4 *__restrict__ qloc,
                                                const double4 *__restrict__ q, const int *__restrict__ tab, int owner,
-                                               int pc, int i, bool active, WarpRows &sm, int *__restrict__ nbr,
-                                               int stride, int maxnb) {
+                                               int pc, int i, bool active, const SmallRow &small,
+                                               WarpRows<row_words(SPLIT)> &sm,
+                                               int (*counts)[32], int part, int *__restrict__ nbr, int stride,
+                                               int maxnb) {
+  static_assert(SPLIT == 1 || SPLIT == 3 || SPLIT == 9, "whole runs per warp");
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kNoSlot = 1 << 30;  // above every slot; differences with slots stay in range
   const int lane = threadIdx.x & 31;
@@ -1311,203 +1341,314 @@ __device__ __forceinline__ int build_rows_warp(const RowGeom &g, const float4 *_
   const int s1 = active && key == k1 && owner == o1, s2 = active && key == k2 && owner == o2;
   const int s12 = __shfl_xor_sync(kAll, s1, 2);  // the other pair's
   const bool quad = s1 && s2 && s12;
-  int cnt = 0;  // entries in the list
+  int cnt = 0;             // the lane's next entry in the list
+  int nw = 0, fresh = 0;   // the lane's words, and the partners in them
+  bool filing = SPLIT == 1;  // the place of the lane's entries is known: full words may go to the list
+  bool lost = false;         // words did not fit before that (warp-uniform)
 
-  // one turn per x-row of cells among the lanes' atoms
-  for (unsigned left = __ballot_sync(kAll, active); left;) {
-    const int lead = __ffs(left) - 1;
-    const unsigned row = (unsigned)__shfl_sync(kAll, pc, lead) >> 11;
-    const int row_owner = __shfl_sync(kAll, owner, lead);
-    const bool on = active && ((unsigned)pc >> 11) == row && owner == row_owner;
-    left &= ~__ballot_sync(kAll, on);
-    // a candidate is kept when r^2 - hi < 0: never on the other lanes
-    const float2 nhi = on ? make_float2(-g.hi, -g.hi) : make_float2(1.f, 1.f);
-    const float2 nlo = on ? make_float2(-g.lo, -g.lo) : make_float2(1.f, 1.f);
-    const int cy = (int)(row & 2047u), lz = (int)(row >> 11);
-    // the row's geometry, from the turn's own lanes
-    const int ms1 = __shfl_sync(kAll, g.ms[1], lead), ms2 = __shfl_sync(kAll, g.ms[2], lead);
-    const int rmx = __shfl_sync(kAll, mx, lead);
-    const float Lx = __shfl_sync(kAll, (float)g.L[0], lead);
-    const int *rtab = (const int *)__shfl_sync(kAll, (unsigned long long)tab, lead);
-    const int cz = SLAB ? g.z0 + lz : lz;  // global layer
-    int nw = 0, fresh = 0;                 // the lane's words, and the partners in them
-
-    // the words' partners into the list
-    auto flush = [&]() {
-      const int mine = min(fresh, maxnb - cnt), n = __reduce_max_sync(kAll, mine);
-      int *dst = nbr + (size_t)cnt * stride + i;
-      const uint2 *w = &sm.word[0][lane];
-      uint2 m = make_uint2(0u, 0u);
-      for (int t = 0; t < n; t++, dst += stride) {
-        if (t < mine) {
-          if (m.x == 0u) {  // the next word (none is empty)
-            m = *w;
-            w += 32;
-          }
-          const int b = __clz(m.x);
-          *dst = (int)m.y + b;
-          m.x ^= 0x80000000u >> b;
+  // the words' partners into the list
+  auto flush = [&]() {
+    const int mine = min(fresh, maxnb - cnt), n = __reduce_max_sync(kAll, mine);
+    int *dst = nbr + (size_t)cnt * stride + i;
+    const uint2 *w = &sm.word[0][lane];
+    uint2 m = make_uint2(0u, 0u);
+    for (int t = 0; t < n; t++, dst += stride) {
+      if (t < mine) {
+        if (m.x == 0u) {  // the next word (none is empty)
+          m = *w;
+          w += 32;
         }
+        const int b = __clz(m.x);
+        *dst = (int)m.y + b;
+        m.x ^= 0x80000000u >> b;
       }
-      cnt += fresh;
-      nw = fresh = 0;
-    };
+    }
+    cnt += fresh;
+    nw = fresh = 0;
+  };
+  // room for three more words a lane
+  auto make_room = [&]() {
+    if (__any_sync(kAll, nw > row_words(SPLIT) - 3)) {
+      if (filing) {
+        flush();
+      } else {
+        lost = true;
+        nw = 0;
+      }
+    }
+  };
+
+  for (int pass = SPLIT == 1 ? 1 : 0; pass < 2; pass++) {
+    if (SMALL && __any_sync(kAll, small.on)) {
+      // an FP32 minimum image on the prefilter coordinates (box coordinates
+      // here, the system being one cell) drops the far atoms: its band is 1e-4
+      // SL^2 plus the rounding of coordinates up to the box lengths (each
+      // difference is off by less than 4 u L, u = 2^-24, and 2 SL of that
+      // reaches r^2)
+      const float lx = (float)g.L[0], ly = (float)g.L[1], lz = (float)g.L[2];
+      const float ix = 1.f / lx, iy = 1.f / ly, iz = 1.f / lz;
+      const float wide = (float)(16.0 / 16777216.0 * (g.L[0] + g.L[1] + g.L[2]) * sqrt(g.sl2));
+      const float hi = (float)(g.sl2 * 1.0001) + wide, lo = (float)(g.sl2 * 0.9999) - wide;
+      const float round_big = 12582912.f;  // + and - it: the nearest whole number
+      auto whole = [&](float x) { return __fsub_rn(__fadd_rn(x, round_big), round_big); };
+      const int n = small.on ? small.end - small.beg : 0;
+      const int share = ((n + SPLIT - 1) / SPLIT + 31) & ~31;  // whole words
+      const int beg = small.beg + min(n, part * share), end = small.beg + min(n, (part + 1) * share);
+      const int trip = __reduce_max_sync(kAll, small.on ? end - beg : 0);
+      for (int k = 0; k < trip; k += 32) {
+        const int first = beg + k;
+        unsigned m = 0u;
+#pragma unroll 1
+        for (int u = 0; u < 32; u += 4) {
+          float4 l[4];
+#pragma unroll
+          for (int c = 0; c < 4; c++) l[c] = __ldg(qloc + (small.on ? min(first + u + c, small.end - 1) : i));
+#pragma unroll
+          for (int c = 0; c < 4; c++) {
+            float dx = l[c].x - li.x, dy = l[c].y - li.y, dz = l[c].z - li.z;
+            dx = fmaf(-lx, whole(__fmul_rn(dx, ix)), dx);
+            dy = fmaf(-ly, whole(__fmul_rn(dy, iy)), dy);
+            dz = fmaf(-lz, whole(__fmul_rn(dz, iz)), dz);
+            m = __funnelshift_l(__float_as_uint(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) - hi), m, 1);
+          }
+        }
+        const int have = small.on ? min(max(end - first, 0), 32) : 0, self = i - first;
+        m = have == 0 ? 0u : m & (0xffffffffu << (32 - have));
+        if (self >= 0 && self < 32) m &= ~(0x80000000u >> self);
+        for (unsigned rest = m; rest;) {
+          const int b = __clz(rest);
+          rest ^= 0x80000000u >> b;
+          const float4 l = __ldg(qloc + first + b);
+          float dx = l.x - li.x, dy = l.y - li.y, dz = l.z - li.z;
+          const float kx = whole(__fmul_rn(dx, ix)), ky = whole(__fmul_rn(dy, iy)), kz = whole(__fmul_rn(dz, iz));
+          dx = fmaf(-lx, kx, dx);
+          dy = fmaf(-ly, ky, dy);
+          dz = fmaf(-lz, kz, dz);
+          // image shift of the partner (shift_of's code) and the strips it
+          // needs; atoms half a box apart, where FP32 may take the wrong image,
+          // are further than SearchLength and so in the band
+          int code = (kx > 0.f ? 1 : (kx < 0.f ? 2 : 0)) | (ky > 0.f ? 4 : (ky < 0.f ? 8 : 0)) |
+                     (kz > 0.f ? 16 : (kz < 0.f ? 32 : 0));
+          const bool band = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) >= lo;
+          if (band) {
+            const double4 qi = q[i], qj = q[first + b];
+            const double tx = qj.x - qi.x, ty = qj.y - qi.y, tz = qj.z - qi.z;
+            code = (tx > 0.5 * g.L[0] ? 1 : (tx < -0.5 * g.L[0] ? 2 : 0)) |
+                   (ty > 0.5 * g.L[1] ? 4 : (ty < -0.5 * g.L[1] ? 8 : 0)) |
+                   (tz > 0.5 * g.L[2] ? 16 : (tz < -0.5 * g.L[2] ? 32 : 0));
+          }
+          const int need = strips_of(code);
+          bool keep = (__float_as_int(l.w) & need) == need;
+          if (keep && band)
+            keep = within_search_exact(q[i], q[first + b], shift_of(code, 0, g.L), shift_of(code, 1, g.L),
+                                       shift_of(code, 2, g.L), g.sl2);
+          if (!keep) m ^= 0x80000000u >> b;
+        }
+        if (m) sm.word[nw++][lane] = make_uint2(m, (unsigned)first);
+        fresh += __popc(m);
+        make_room();
+      }
+    }
+    // one turn per x-row of cells among the lanes' atoms
+    for (unsigned left = __ballot_sync(kAll, active); left;) {
+      const int lead = __ffs(left) - 1;
+      const unsigned row = (unsigned)__shfl_sync(kAll, pc, lead) >> 11;
+      const int row_owner = __shfl_sync(kAll, owner, lead);
+      const bool on = active && ((unsigned)pc >> 11) == row && owner == row_owner;
+      left &= ~__ballot_sync(kAll, on);
+      // a candidate is kept when r^2 - hi < 0: never on the other lanes
+      const float2 nhi = on ? make_float2(-g.hi, -g.hi) : make_float2(1.f, 1.f);
+      const float2 nlo = on ? make_float2(-g.lo, -g.lo) : make_float2(1.f, 1.f);
+      const int cy = (int)(row & 2047u), lz = (int)(row >> 11);
+      // the row's geometry, from the turn's own lanes
+      const int ms1 = __shfl_sync(kAll, g.ms[1], lead), ms2 = __shfl_sync(kAll, g.ms[2], lead);
+      const int rmx = __shfl_sync(kAll, mx, lead);
+      const float Lx = __shfl_sync(kAll, (float)g.L[0], lead);
+      const int *rtab = (const int *)__shfl_sync(kAll, (unsigned long long)tab, lead);
+      const int cz = SLAB ? g.z0 + lz : lz;  // global layer
 
 #pragma unroll 1
-    for (int r = 0; r < 9; r++) {
-      const int dz = r / 3 - 1, dy = r % 3 - 1;
-      int z = cz + dz, y = cy + dy, yz = 0;  // yz: the run's image shift along y and z (shift_of's code)
-      if (z < 0) { z += ms2; yz = 1 << 4; } else if (z >= ms2) { z -= ms2; yz = 2 << 4; }
-      if (y < 0) { y += ms1; yz |= 1 << 2; } else if (y >= ms1) { y -= ms1; yz |= 2 << 2; }
-      int blk = z;
-      if (SLAB) {
-        const int nl = lz + dz;
-        blk = nl < 0 ? g.nzl : (nl >= g.nzl ? g.nzl + 1 : nl);
-      }
-      // the lane's window [wl, wh) in sub-bins of the 3 kXSub bins of cells
-      // cx - 1 .. cx + 1 (build_rows' windows; empty when out of reach)
-      const float gz = dz == 0 ? 0.f : (dz < 0 ? li.z : g.csz - li.z);
-      const float gy = dy == 0 ? 0.f : (dy < 0 ? li.y : g.csy - li.y);
-      const float g2 = fmaf(gy, gy, gz * gz);
-      const float reach = sqrt_approx(fmaxf(g.hi - g2, 0.f)) * per_binf;
-      const bool out = !on || g2 > g.hi;
-      int wl = out ? 3 * kXSub : max((int)floorf(ubin - reach - 1e-3f), 0);
-      int wh = out ? 0 : min((int)floorf(ubin + reach + 1e-3f) + 1, 3 * kXSub);
+      for (int r = part * (9 / SPLIT); r < (part + 1) * (9 / SPLIT); r++) {
+        const int dz = r / 3 - 1, dy = r % 3 - 1;
+        int z = cz + dz, y = cy + dy, yz = 0;  // yz: the run's image shift along y and z (shift_of's code)
+        if (z < 0) { z += ms2; yz = 1 << 4; } else if (z >= ms2) { z -= ms2; yz = 2 << 4; }
+        if (y < 0) { y += ms1; yz |= 1 << 2; } else if (y >= ms1) { y -= ms1; yz |= 2 << 2; }
+        int blk = z;
+        if (SLAB) {
+          const int nl = lz + dz;
+          blk = nl < 0 ? g.nzl : (nl >= g.nzl ? g.nzl + 1 : nl);
+        }
+        // the lane's window [wl, wh) in sub-bins of the 3 kXSub bins of cells
+        // cx - 1 .. cx + 1 (build_rows' windows; empty when out of reach)
+        const float gz = dz == 0 ? 0.f : (dz < 0 ? li.z : g.csz - li.z);
+        const float gy = dy == 0 ? 0.f : (dy < 0 ? li.y : g.csy - li.y);
+        const float g2 = fmaf(gy, gy, gz * gz);
+        const float reach = sqrt_approx(fmaxf(g.hi - g2, 0.f)) * per_binf;
+        const bool out = !on || g2 > g.hi;
+        int wl = out ? 3 * kXSub : max((int)floorf(ubin - reach - 1e-3f), 0);
+        int wh = out ? 0 : min((int)floorf(ubin + reach + 1e-3f) + 1, 3 * kXSub);
 #pragma unroll
-      for (int o = 1; o <= 2; o <<= 1) {
-        const int lo2 = __shfl_xor_sync(kAll, wl, o), hi2 = __shfl_xor_sync(kAll, wh, o);
-        if (quad) {
-          wl = min(wl, lo2);
-          wh = max(wh, hi2);
-        }
-      }
-      // as slots [e0, e1) of the row continued through its x faces: slots
-      // below x0 are those of the row's end (image shift -L), slots from x1
-      // on those of its start (+L)
-      const int *xr = rtab + (size_t)(blk * ms1 + y) * (rmx + 1);
-      const int x0 = xr[0], x1 = xr[rmx], nrow = x1 - x0;
-      int e0 = kNoSlot, e1 = -kNoSlot;
-      if (wl < wh) {
-        const int b0 = vbase + wl, b1 = vbase + wh;
-        e0 = b0 < 0 ? xr[b0 + rmx] - nrow : xr[b0];
-        e1 = b1 > rmx ? xr[b1 - rmx] + nrow : xr[b1];
-        if (e0 >= e1) {
-          e0 = kNoSlot;
-          e1 = -kNoSlot;
-        }
-      }
-      const int c0 = __reduce_min_sync(kAll, e0), c1 = __reduce_max_sync(kAll, e1);
-      const bool wraps = c0 < x0 || c1 > x1, plain = !wraps && yz == 0;
-      const float byf = (float)dy * g.csy - li.y, bzf = (float)dz * g.csz - li.z;
-      const float2 by = make_float2(byf, byf), bz = make_float2(bzf, bzf);
-      for (int c = c0; c < c1; c += kRunStage) {
-        const int total = min(c1 - c, kRunStage);
-        __syncwarp();  // the last walk has read the stage
-        if (plain) {
-          for (int t = 2 * lane; t < ((total + 3) & ~3); t += 64) {
-            const float4 *p = qloc + c + t;
-            float4 l0 = make_float4(1e18f, 0.f, 0.f, 0.f), l1 = l0;
-            if (t < total) l0 = __ldg(p);
-            if (t + 1 < total) l1 = __ldg(p + 1);
-            sm.xy[t >> 1] = make_float4(l0.x, l1.x, l0.y, l1.y);
-            sm.zz[t >> 1] = make_float2(l0.z, l1.z);
+        for (int o = 1; o <= 2; o <<= 1) {
+          const int lo2 = __shfl_xor_sync(kAll, wl, o), hi2 = __shfl_xor_sync(kAll, wh, o);
+          if (quad) {
+            wl = min(wl, lo2);
+            wh = max(wh, hi2);
           }
-        } else {
-          for (int t = 2 * lane; t < ((total + 3) & ~3); t += 64) {
-            float4 p[2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-              p[u] = make_float4(1e18f, 0.f, 0.f, 0.f);
-              if (t + u < total) {
-                int s = c + t + u, code = yz;
-                float sx = 0.f;
-                if (s < x0) {
-                  s += nrow;
-                  sx = -Lx;
-                  code |= 1;
-                } else if (s >= x1) {
-                  s -= nrow;
-                  sx = Lx;
-                  code |= 2;
-                }
-                const int need = strips_of(code);
-                p[u] = __ldg(qloc + s);
-                p[u].x = (__float_as_int(p[u].w) & need) == need ? p[u].x + sx : 1e18f;
-              }
+        }
+        // as slots [e0, e1) of the row continued through its x faces: slots
+        // below x0 are those of the row's end (image shift -L), slots from x1
+        // on those of its start (+L)
+        const int *xr = rtab + (size_t)(blk * ms1 + y) * (rmx + 1);
+        const int x0 = xr[0], x1 = xr[rmx], nrow = x1 - x0;
+        int e0 = kNoSlot, e1 = -kNoSlot;
+        if (wl < wh) {
+          const int b0 = vbase + wl, b1 = vbase + wh;
+          e0 = b0 < 0 ? xr[b0 + rmx] - nrow : xr[b0];
+          e1 = b1 > rmx ? xr[b1 - rmx] + nrow : xr[b1];
+          if (e0 >= e1) {
+            e0 = kNoSlot;
+            e1 = -kNoSlot;
+          }
+        }
+        const int c0 = __reduce_min_sync(kAll, e0), c1 = __reduce_max_sync(kAll, e1);
+        const bool wraps = c0 < x0 || c1 > x1, plain = !wraps && yz == 0;
+        const float byf = (float)dy * g.csy - li.y, bzf = (float)dz * g.csz - li.z;
+        const float2 by = make_float2(byf, byf), bz = make_float2(bzf, bzf);
+        for (int c = c0; c < c1; c += kRunStage) {
+          const int total = min(c1 - c, kRunStage);
+          __syncwarp();  // the last walk has read the stage
+          if (plain) {
+            for (int t = 2 * lane; t < ((total + 3) & ~3); t += 64) {
+              const float4 *p = qloc + c + t;
+              float4 l0 = make_float4(1e18f, 0.f, 0.f, 0.f), l1 = l0;
+              if (t < total) l0 = __ldg(p);
+              if (t + 1 < total) l1 = __ldg(p + 1);
+              sm.xy[t >> 1] = make_float4(l0.x, l1.x, l0.y, l1.y);
+              sm.zz[t >> 1] = make_float2(l0.z, l1.z);
             }
-            sm.xy[t >> 1] = make_float4(p[0].x, p[1].x, p[0].y, p[1].y);
-            sm.zz[t >> 1] = make_float2(p[0].z, p[1].z);
-          }
-        }
-        __syncwarp();
-        // the lane's part of the stage, from an even candidate; the longest
-        // one sets the warp's walk, and starts move down to end in the stage
-        const int f0 = max(e0, c), f1 = min(e1, c + total);
-        int st = f0 < f1 ? (f0 - c) & ~1 : 0;
-        const int trip = (__reduce_max_sync(kAll, f0 < f1 ? f1 - c - st : 0) + 3) & ~3;
-        st = min(st, ((total + 3) & ~3) - trip);
-        const float4 *pxy = sm.xy + (st >> 1);
-        const float2 *pzz = sm.zz + (st >> 1);
-        for (int k = 0; k < trip; k += 32, st += 32) {
-          unsigned m = 0u, band = 0u;
-          const int kn = min(trip - k, 32);
-#pragma unroll 2
-          for (int u = 0; u < kn; u += 4, pxy += 2, pzz += 2) {
-            const float4 a0 = pxy[0], a1 = pxy[1];
-            const float2 z0 = pzz[0], z1 = pzz[1];
-            const float2 ex0 = __fadd2_rn(make_float2(a0.x, a0.y), bx), ey0 = __fadd2_rn(make_float2(a0.z, a0.w), by);
-            const float2 ex1 = __fadd2_rn(make_float2(a1.x, a1.y), bx), ey1 = __fadd2_rn(make_float2(a1.z, a1.w), by);
-            const float2 ez0 = __fadd2_rn(z0, bz), ez1 = __fadd2_rn(z1, bz);
-            const float2 r0 = __ffma2_rn(ex0, ex0, __ffma2_rn(ey0, ey0, __fmul2_rn(ez0, ez0)));
-            const float2 r1 = __ffma2_rn(ex1, ex1, __ffma2_rn(ey1, ey1, __fmul2_rn(ez1, ez1)));
-            const float2 h0 = __fadd2_rn(r0, nhi), h1 = __fadd2_rn(r1, nhi);
-            const float2 b0 = __fmul2_rn(h0, __fadd2_rn(r0, nlo)), b1 = __fmul2_rn(h1, __fadd2_rn(r1, nlo));
-            m = __funnelshift_l(__float_as_uint(h0.x), m, 1);
-            m = __funnelshift_l(__float_as_uint(h0.y), m, 1);
-            m = __funnelshift_l(__float_as_uint(h1.x), m, 1);
-            m = __funnelshift_l(__float_as_uint(h1.y), m, 1);
-            band |= __float_as_uint(b0.x) | __float_as_uint(b0.y);
-            band |= __float_as_uint(b1.x) | __float_as_uint(b1.y);
-          }
-          m <<= 32 - kn;
-          const int first = c + st;  // virtual slot of bit 31
-          const int self = i - first;
-          if (r == 4 && self >= 0 && self < 32) m &= ~(0x80000000u >> self);
-          if (__any_sync(kAll, (int)(band & 0x80000000u))) {
-            // some candidate of some lane in the band: exact test of that
-            // lane's partners
-            if (band >> 31)
-              for (unsigned left2 = m; left2;) {
-                const int b = __clz(left2);
-                left2 &= ~(0x80000000u >> b);
-                int s = first + b;
-                s += s < x0 ? nrow : (s >= x1 ? -nrow : 0);
-                if (!band_test_row(g, q, i, s, cx, yz)) m &= ~(0x80000000u >> b);
-              }
-          }
-          if (!wraps) {
-            if (m) sm.word[nw++][lane] = make_uint2(m, (unsigned)first);
           } else {
-            // the run wraps: the slots before, in and after the row in words
-            // of their own
-            const int h0 = x0 - first, h1 = x1 - first;
-            const unsigned lt0 = h0 <= 0 ? 0u : (h0 >= 32 ? 0xffffffffu : ~(0xffffffffu >> h0));
-            const unsigned lt1 = h1 <= 0 ? 0u : (h1 >= 32 ? 0xffffffffu : ~(0xffffffffu >> h1));
-            if (m & lt0) sm.word[nw++][lane] = make_uint2(m & lt0, (unsigned)(first + nrow));
-            if (m & lt1 & ~lt0) sm.word[nw++][lane] = make_uint2(m & lt1 & ~lt0, (unsigned)first);
-            if (m & ~lt1) sm.word[nw++][lane] = make_uint2(m & ~lt1, (unsigned)(first - nrow));
+            for (int t = 2 * lane; t < ((total + 3) & ~3); t += 64) {
+              float4 p[2];
+#pragma unroll
+              for (int u = 0; u < 2; u++) {
+                p[u] = make_float4(1e18f, 0.f, 0.f, 0.f);
+                if (t + u < total) {
+                  int s = c + t + u, code = yz;
+                  float sx = 0.f;
+                  if (s < x0) {
+                    s += nrow;
+                    sx = -Lx;
+                    code |= 1;
+                  } else if (s >= x1) {
+                    s -= nrow;
+                    sx = Lx;
+                    code |= 2;
+                  }
+                  const int need = strips_of(code);
+                  p[u] = __ldg(qloc + s);
+                  p[u].x = (__float_as_int(p[u].w) & need) == need ? p[u].x + sx : 1e18f;
+                }
+              }
+              sm.xy[t >> 1] = make_float4(p[0].x, p[1].x, p[0].y, p[1].y);
+              sm.zz[t >> 1] = make_float2(p[0].z, p[1].z);
+            }
           }
-          fresh += __popc(m);
-          if (__any_sync(kAll, nw > kRowWords - 3)) flush();
+          __syncwarp();
+          // the lane's part of the stage, from an even candidate; the longest
+          // one sets the warp's walk, and starts move down to end in the stage
+          const int f0 = max(e0, c), f1 = min(e1, c + total);
+          int st = f0 < f1 ? (f0 - c) & ~1 : 0;
+          const int trip = (__reduce_max_sync(kAll, f0 < f1 ? f1 - c - st : 0) + 3) & ~3;
+          st = min(st, ((total + 3) & ~3) - trip);
+          const float4 *pxy = sm.xy + (st >> 1);
+          const float2 *pzz = sm.zz + (st >> 1);
+          for (int k = 0; k < trip; k += 32, st += 32) {
+            unsigned m = 0u, band = 0u;
+            const int kn = min(trip - k, 32);
+#pragma unroll 2
+            for (int u = 0; u < kn; u += 4, pxy += 2, pzz += 2) {
+              const float4 a0 = pxy[0], a1 = pxy[1];
+              const float2 z0 = pzz[0], z1 = pzz[1];
+              const float2 ex0 = __fadd2_rn(make_float2(a0.x, a0.y), bx), ey0 = __fadd2_rn(make_float2(a0.z, a0.w), by);
+              const float2 ex1 = __fadd2_rn(make_float2(a1.x, a1.y), bx), ey1 = __fadd2_rn(make_float2(a1.z, a1.w), by);
+              const float2 ez0 = __fadd2_rn(z0, bz), ez1 = __fadd2_rn(z1, bz);
+              const float2 r0 = __ffma2_rn(ex0, ex0, __ffma2_rn(ey0, ey0, __fmul2_rn(ez0, ez0)));
+              const float2 r1 = __ffma2_rn(ex1, ex1, __ffma2_rn(ey1, ey1, __fmul2_rn(ez1, ez1)));
+              const float2 h0 = __fadd2_rn(r0, nhi), h1 = __fadd2_rn(r1, nhi);
+              const float2 b0 = __fmul2_rn(h0, __fadd2_rn(r0, nlo)), b1 = __fmul2_rn(h1, __fadd2_rn(r1, nlo));
+              m = __funnelshift_l(__float_as_uint(h0.x), m, 1);
+              m = __funnelshift_l(__float_as_uint(h0.y), m, 1);
+              m = __funnelshift_l(__float_as_uint(h1.x), m, 1);
+              m = __funnelshift_l(__float_as_uint(h1.y), m, 1);
+              band |= __float_as_uint(b0.x) | __float_as_uint(b0.y);
+              band |= __float_as_uint(b1.x) | __float_as_uint(b1.y);
+            }
+            m <<= 32 - kn;
+            const int first = c + st;  // virtual slot of bit 31
+            const int self = i - first;
+            if (r == 4 && self >= 0 && self < 32) m &= ~(0x80000000u >> self);
+            if (__any_sync(kAll, (int)(band & 0x80000000u))) {
+              // some candidate of some lane in the band: exact test of that
+              // lane's partners
+              if (band >> 31)
+                for (unsigned left2 = m; left2;) {
+                  const int b = __clz(left2);
+                  left2 &= ~(0x80000000u >> b);
+                  int s = first + b;
+                  s += s < x0 ? nrow : (s >= x1 ? -nrow : 0);
+                  if (!band_test_row(g, q, i, s, cx, yz)) m &= ~(0x80000000u >> b);
+                }
+            }
+            if (!wraps) {
+              if (m) sm.word[nw++][lane] = make_uint2(m, (unsigned)first);
+            } else {
+              // the run wraps: the slots before, in and after the row in words
+              // of their own
+              const int h0 = x0 - first, h1 = x1 - first;
+              const unsigned lt0 = h0 <= 0 ? 0u : (h0 >= 32 ? 0xffffffffu : ~(0xffffffffu >> h0));
+              const unsigned lt1 = h1 <= 0 ? 0u : (h1 >= 32 ? 0xffffffffu : ~(0xffffffffu >> h1));
+              if (m & lt0) sm.word[nw++][lane] = make_uint2(m & lt0, (unsigned)(first + nrow));
+              if (m & lt1 & ~lt0) sm.word[nw++][lane] = make_uint2(m & lt1 & ~lt0, (unsigned)first);
+              if (m & ~lt1) sm.word[nw++][lane] = make_uint2(m & ~lt1, (unsigned)(first - nrow));
+            }
+            fresh += __popc(m);
+            make_room();
+          }
         }
       }
     }
-    flush();
-    // padded with the atom itself to a multiple of 4
-    if (on)
-      for (int k = cnt; (k & 3) && k < maxnb; k++) nbr[(size_t)k * stride + i] = i;
+    if (SPLIT > 1 && pass == 0) {
+      // the entries' places: after those of the parts before
+      counts[part][lane] = fresh;
+      __syncthreads();
+      int before = 0, all = 0;
+#pragma unroll
+      for (int w = 0; w < SPLIT; w++) {
+        if (w == part) before = all;
+        all += counts[w][lane];
+      }
+      cnt = before;
+      filing = true;
+      if (!lost) {
+        flush();
+        cnt = all;
+        break;
+      }
+      nw = fresh = 0;  // once more, filing as it goes
+    } else {
+      flush();
+      if (SPLIT > 1) {
+        cnt = 0;
+#pragma unroll
+        for (int w = 0; w < SPLIT; w++) cnt += counts[w][lane];
+      }
+    }
   }
-  return cnt;
+  // padded with the atom itself to a multiple of 4
+  const bool mine = part == 0 && (active || (SMALL && small.on));
+  if (mine)
+    for (int k = cnt; (k & 3) && k < maxnb; k++) nbr[(size_t)k * stride + i] = i;
+  return mine ? cnt : 0;
 }
 
 // Stage offset of global slot j: the plan range whose atoms hold j (ranges
@@ -1548,14 +1689,14 @@ __global__ void __launch_bounds__(BLOCK, !STAGE && BTPA == 1 ? 1024 / BLOCK : 0)
   const int i = t / BTPA, sub = t % BTPA;
   int cnt = 0;
   if (!STAGE && BTPA == 1) {
-    __shared__ WarpRows rows[STAGE || BTPA > 1 ? 1 : BLOCK / 32];
+    __shared__ WarpRows<row_words(1)> rows[STAGE || BTPA > 1 ? 1 : BLOCK / 32];
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     // the lanes of a warp walk together: they agree on the error flag
     if (t - l < n && !warp_error(a.st)) {
       const bool active = i < n;
       const int ii = active ? i : n - 1;
-      cnt = build_rows_warp<SLAB>(row_geom(b), a.qloc, a.q, a.xsub, 0, a.cxyz[ii], ii, active, rows[w], a.nbr, a.stride,
-                                  a.maxnb);
+      cnt = build_rows_warp<SLAB, 1, false>(row_geom(b), a.qloc, a.q, a.xsub, 0, a.cxyz[ii], ii, active, SmallRow{},
+                                            rows[w], nullptr, 0, a.nbr, a.stride, a.maxnb);
       if (active) {
         a.nnbr[i] = min(cnt, a.maxnb);
         if (cnt > a.maxnb) atomicOr(&a.st->error, kErrCapacity);
@@ -1628,6 +1769,38 @@ __global__ void __launch_bounds__(BLOCK, !STAGE && BTPA == 1 ? 1024 / BLOCK : 0)
   }
   if (sub != 0) cnt = 0;  // the atom's row is counted once
   count_rows(a.st, cnt);
+}
+
+// The same for few atoms: SPLIT warps share every 32 of them.
+template <int SPLIT>
+__global__ void __launch_bounds__(SPLIT * 32, 27 / SPLIT) k_build_split(Arrays a, Box b, int n) {
+  __shared__ WarpRows<row_words(SPLIT)> rows[SPLIT];
+  __shared__ int counts[SPLIT][32];
+  __shared__ int err;
+  const int w = threadIdx.x >> 5, i = blockIdx.x * 32 + (threadIdx.x & 31);
+  if (threadIdx.x == 0) err = *(volatile const int *)&a.st->error;
+  __syncthreads();
+  if (err) return;
+  const bool active = i < n;
+  const int ii = active ? i : n - 1;
+  const int cnt = build_rows_warp<false, SPLIT, false>(row_geom(b), a.qloc, a.q, a.xsub, 0, a.cxyz[ii], ii, active,
+                                                       SmallRow{}, rows[w], counts, w, a.nbr, a.stride, a.maxnb);
+  if (active && w == 0) {
+    a.nnbr[i] = min(cnt, a.maxnb);
+    if (cnt > a.maxnb) atomicOr(&a.st->error, kErrCapacity);
+  }
+  count_rows(a.st, cnt);
+}
+
+// Warps that share 32 atoms' rows, so that few atoms fill the chip too: nine
+// while that makes up to 64 warps a multiprocessor, then three up to 128 (its
+// 32 warps at a time finish unevenly; more parts even them out).  A rebuild of
+// the liquid with one / three / nine warps, us: 6,912 atoms - / 97 / 94 (109
+// with eight lanes an atom), 32,000 - / 121 / 119 (144), 55,296 152 / 134 /
+// 135, 108,000 175 / 167 / -, 157,216 205 / 196 / -, 340,736 298 / 302 / -.
+inline int build_split(long long atoms, int sms) {
+  const long long warps = atoms / 32;
+  return warps * 9 <= 64LL * sms ? 9 : (warps * 3 <= 128LL * sms ? 3 : 1);
 }
 
 // Before a build: clear the build counters.

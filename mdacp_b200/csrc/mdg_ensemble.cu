@@ -329,6 +329,8 @@ __global__ void __launch_bounds__(kEB) ke_disp_collect(Ens e) {
     // no copy of this atom moved more than c (ke_disp_max's per-atom
     // maximum of the same displacements): nothing to collect
     if (!(e.disp2[i] > c_d2)) continue;
+    // a full list: the number of copies has decided (k_disp_collect)
+    if (*(volatile const int *)&st.cand_weighted >= e.cll) continue;
     for_each_copy(ens_view(e), e.rep[r].L, i, e.lag, [&](int code, double d2) {
       if (d2 > c_d2) {
         atomicAdd(&st.cand_weighted, 1);
@@ -559,92 +561,47 @@ __global__ void __launch_bounds__(kEB) ke_copy_back(Ens e) {
   }
 }
 
-// Row of atom i of a small replica (an axis shorter than three cells): every
-// other atom of the replica in slot order, through its minimum image (unique:
-// L > 2 SearchLength).  An FP32 minimum image on the prefilter coordinates
-// (which are box coordinates here, the replica being one cell) drops the far
-// atoms; its band is 1e-4 SL^2 plus the rounding of coordinates up to the
-// box lengths (each of the three differences is off by less than 4 u L, u =
-// 2^-24, and 2 SL of that reaches r^2).  The others take the exact test.
-// Returns the entries found.  Four candidates are loaded at a time; the FP64
-// test of every candidate that this replaced took 74 us for 24 replicas of up to
-// 3,000 atoms on a B200 (one block's lanes walk 500 candidates each, so the
-// launch waits for that chain).
-__device__ __forceinline__ int small_row(const Ens &e, const Rep &rep, int i) {
-  const int maxnb = e.maxnb, stride = e.stride;
-  const double4 qi = e.q[i];
-  const float4 li = e.qloc[i];
-  const float lx = (float)rep.L[0], ly = (float)rep.L[1], lz = (float)rep.L[2];
-  const float ix = 1.f / lx, iy = 1.f / ly, iz = 1.f / lz;
-  const float hi = (float)(rep.sl2 * 1.0001 + 16.0 / 16777216.0 * (rep.L[0] + rep.L[1] + rep.L[2]) * rep.sl);
-  const int end = rep.atom_off + rep.n;
-  int cnt = 0;
-  for (int j0 = rep.atom_off; j0 < end; j0 += 4) {
-    float4 l[4];
-    bool near[4];
-#pragma unroll
-    for (int u = 0; u < 4; u++) l[u] = e.qloc[min(j0 + u, end - 1)];
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      float dx = l[u].x - li.x, dy = l[u].y - li.y, dz = l[u].z - li.z;
-      dx = fmaf(-lx, rintf(dx * ix), dx);
-      dy = fmaf(-ly, rintf(dy * iy), dy);
-      dz = fmaf(-lz, rintf(dz * iz), dz);
-      near[u] = j0 + u < end && j0 + u != i && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= hi;
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-      if (!near[u]) continue;
-      const int j = j0 + u;
-      const double4 qj = e.q[j];
-      const double tx = qj.x - qi.x, ty = qj.y - qi.y, tz = qj.z - qi.z;
-      const double sx = tx > rep.hL[0] ? -rep.L[0] : (tx < -rep.hL[0] ? rep.L[0] : 0.0);
-      const double sy = ty > rep.hL[1] ? -rep.L[1] : (ty < -rep.hL[1] ? rep.L[1] : 0.0);
-      const double sz = tz > rep.hL[2] ? -rep.L[2] : (tz < -rep.hL[2] ? rep.L[2] : 0.0);
-      const int need = needed_strips(sx, sy, sz);
-      if (need && (e.mult[j] & need) != need) continue;
-      if (!within_search_exact(qi, qj, sx, sy, sz, rep.sl2)) continue;
-      if (cnt < maxnb) e.nbr[(size_t)cnt * stride + i] = j;
-      cnt++;
-    }
-  }
-  for (int k = cnt; k < ((cnt + 3) & ~3) && k < maxnb; k++) e.nbr[(size_t)k * stride + i] = i;
-  return cnt;
-}
-
 // Rows of the rebuilding replicas' atoms (rebuild work list), as the
-// single-system build makes them (build_rows_warp; small_row for replicas
-// narrower than three cells); a warp's 32 atoms may belong to several
-// replicas.  Block-uniform sweeps, so every lane reaches the warp's votes.
-__global__ void __launch_bounds__(kEF, 1024 / kEF) ke_build(Ens e) {
-  __shared__ WarpRows rows[kEF / 32];
-  const int w = threadIdx.x >> 5;
-  if (__shfl_sync(0xffffffffu, *(volatile const int *)e.error, 0)) return;
-  WorkSweep sweep(e.wb, kEF);
+// single-system build makes them (build_rows_warp; replicas narrower than
+// three cells all-pairs); a warp's 32 atoms may belong to several replicas, and
+// SPLIT warps share them.  Block-uniform sweeps, so every thread reaches the
+// votes and barriers.
+template <int SPLIT>
+__global__ void __launch_bounds__(SPLIT == 1 ? kEF : SPLIT * 32, SPLIT == 1 ? 1024 / kEF : 27 / SPLIT) ke_build(Ens e) {
+  constexpr int kWarps = SPLIT == 1 ? kEF / 32 : SPLIT, kAtoms = SPLIT == 1 ? kEF : 32;
+  __shared__ WarpRows<row_words(SPLIT)> rows[kWarps];
+  __shared__ int counts[SPLIT][32];
+  __shared__ int err;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, part = SPLIT == 1 ? 0 : w;
+  if (threadIdx.x == 0) err = *(volatile const int *)e.error;
+  __syncthreads();
+  if (err) return;
+  WorkSweep sweep(e.wb, kAtoms);
   const int total = e.wb.count[1];
   // strided, not in shares: rows of dense replicas take longer
-  for (int base = blockIdx.x * kEF; base < total; base += gridDim.x * kEF) {
-    const int g = base + threadIdx.x;
-    if (base + w * 32 >= total) return;  // whole warps leave together
+  for (int base = blockIdx.x * kAtoms; base < total; base += gridDim.x * kAtoms) {
+    const int g = base + (SPLIT == 1 ? (int)threadIdx.x : lane);
+    if (SPLIT == 1 && base + w * 32 >= total) return;  // whole warps leave together
     const bool active = g < total;
     int r = 0;
     const int i = sweep.atom(e, min(g, total - 1), &r);
     const Rep &rep = e.rep[r];
-    const bool cells = active && !rep.small;
-    int cnt = 0;
-    if (__any_sync(0xffffffffu, cells)) {
-      const RowGeom geom{{rep.L[0], rep.L[1], rep.L[2]}, rep.cs[0], rep.inv_cs[0], rep.sl2, (float)rep.cs[1],
-                         (float)rep.cs[2], rep.sl2_lo, rep.sl2_hi, {rep.ms[0], rep.ms[1], rep.ms[2]}, 0, rep.ms[2]};
-      cnt = build_rows_warp<false>(geom, e.qloc, e.q, e.xsub + rep.tab_off, r, e.cxyz[i], i, cells, rows[w], e.nbr,
-                                   e.stride, e.maxnb);
-    }
-    if (active && rep.small) cnt = small_row(e, rep, i);
-    if (active) {
+    const RowGeom geom{{rep.L[0], rep.L[1], rep.L[2]}, rep.cs[0], rep.inv_cs[0], rep.sl2, (float)rep.cs[1],
+                       (float)rep.cs[2], rep.sl2_lo, rep.sl2_hi, {rep.ms[0], rep.ms[1], rep.ms[2]}, 0, rep.ms[2]};
+    const SmallRow small{active && rep.small, rep.atom_off, rep.atom_off + rep.n};
+    if (SPLIT > 1) __syncthreads();  // the counts of the last 32 atoms have been read
+    const int cnt = build_rows_warp<false, SPLIT, true>(geom, e.qloc, e.q, e.xsub + rep.tab_off, r, e.cxyz[i], i,
+                                                        active && !rep.small, small, rows[w], counts, part, e.nbr,
+                                                        e.stride, e.maxnb);
+    const bool mine = active && part == 0;
+    if (mine) {
       e.nnbr[i] = min(cnt, e.maxnb);
       if (cnt > e.maxnb) atomicOr(e.error, kErrCapacity);
     }
-    rep_max_row(e, r, cnt, active);
-    rep_add(&e.rs[0].list_entries, sizeof(RepStatus), r, min(cnt, e.maxnb), active);
+    if (part == 0) {
+      rep_max_row(e, r, cnt, active);
+      rep_add(&e.rs[0].list_entries, sizeof(RepStatus), r, min(cnt, e.maxnb), active);
+    }
   }
 }
 
@@ -913,7 +870,6 @@ void e_launch_disp(mdg_ensemble *x, cudaStream_t s) {
 void e_launch_build(mdg_ensemble *x, cudaStream_t s, int pack) {
   Ens &e = x->e;
   const int gb = std::min(nb(e.ntot, kEB), x->work_blocks);
-  const int gf = std::min(nb(e.ntot, kEF), 2 * x->work_blocks);
   const int gc = std::min(nb(x->ncell_tot * 32, kEB), x->work_blocks);
   ke_make_list<1><<<1, 1024, 0, s>>>(e);
   ke_clear_cells<<<e.nrep, kEB, 0, s>>>(e);
@@ -923,7 +879,14 @@ void e_launch_build(mdg_ensemble *x, cudaStream_t s, int pack) {
   ke_sort_cells<<<gc, kEB, 0, s>>>(e);
   ke_permute<<<gb, kEB, 0, s>>>(e, pack < 0 ? nullptr : e_pack(e, pack), pack < 0 ? nullptr : e_pack_z(e, pack));
   ke_copy_back<<<gb, kEB, 0, s>>>(e);
-  ke_build<<<gf, kEF, 0, s>>>(e);
+  // a list lives some eight steps, so about one replica in eight rebuilds at a
+  // time (24 replicas of 40,000 atoms in all: 60 us with one warp per 32 atoms,
+  // 23 us with nine)
+  switch (build_split(e.ntot / 8, x->work_blocks / 8)) {
+    case 9: ke_build<9><<<std::min(nb(e.ntot, 32), x->work_blocks), 9 * 32, 0, s>>>(e); break;
+    case 3: ke_build<3><<<std::min(nb(e.ntot, 32), 2 * x->work_blocks), 3 * 32, 0, s>>>(e); break;
+    default: ke_build<1><<<std::min(nb(e.ntot, kEF), 2 * x->work_blocks), kEF, 0, s>>>(e);
+  }
   ke_build_done<<<1, 1024, 0, s>>>(e);
 }
 

@@ -33,6 +33,10 @@ def _rows(q, L, rc, lanes):
     (700, (60.0, 9.0, 9.0), 2.5),     # long rows
     (257, (9.0, 40.0, 40.0), 2.5),    # a few atoms a row, empty cells
     (2500, (23.1, 14.0, 17.3), 3.0),
+    (6000, (11.1, 11.1, 11.1), 2.5),  # nine warps per 32 atoms, more words than fit
+    (34001, (40.0, 35.0, 37.0), 2.5),  # three warps (from 33,700 atoms on 148 multiprocessors)
+    (34001, (18.0, 18.0, 18.0), 2.5),  # the same, more words than fit
+    (203001, (64.0, 63.0, 62.0), 2.5),  # one warp (from 202,100)
 ])
 def test_rows_equal_the_general_walk(n, L, rc):
     rng = np.random.Generator(np.random.Philox(n))
@@ -46,7 +50,8 @@ def test_rows_equal_the_general_walk(n, L, rc):
             assert np.array_equal(x, y)
 
 
-@pytest.mark.parametrize("n,L", [(500, (8.2, 8.2, 8.2)), (37, (5.7, 30.0, 8.6)), (130, (6.0, 6.0, 90.0))])
+@pytest.mark.parametrize("n,L", [(500, (8.2, 8.2, 8.2)), (37, (5.7, 30.0, 8.6)), (130, (6.0, 6.0, 90.0)),
+                                 (4700, (8.2, 8.2, 8.2))])
 def test_small_replica_sums(n, L):
     # an axis shorter than three cells: every pair through its minimum image
     rng = np.random.Generator(np.random.Philox(n))
@@ -70,6 +75,35 @@ def test_small_replica_sums(n, L):
     # sums of up to 2 x 10^4 positive and negative terms, each rounded a few times
     assert pe[0] == pytest.approx(np.sum(4 * (x ** -6 - x ** -3 + c2 * x + c0)), rel=1e-11)
     assert vir[0] == pytest.approx(np.sum(((24 * x ** 3 - 48) / x ** 7 + 8 * c2) * x) / 3, rel=1e-11)
+
+
+@pytest.mark.parametrize("cells", [16, 45, 60])
+def test_replica_rows_equal_a_systems(cells):
+    # 33,000, 729,000 and 1,728,000 atoms in all: nine, three and one warp per
+    # 32 atoms, all of whose replicas rebuild; one replica is all-pairs
+    reps = [W.fcc_liquid((cells,) * 3, 0.8, 1.0, seed=1, jitter=0.05, rc=2.5, dt=0.005),
+            W.fcc_liquid((4, 4, 4), 0.8, 1.0, seed=2, jitter=0.05, rc=2.5, dt=0.005),
+            W.fcc_liquid((cells,) * 3, 0.7, 1.0, seed=3, jitter=0.05, rc=2.5, dt=0.005)]
+    ens = M.Ensemble([(r.q, r.v, r.L) for r in reps], cutoff=2.5, time_step=0.005)
+    ens.observe()  # builds the lists
+    got = ens.list_stats()
+    ens.close()
+    entries = within = 0
+    for r in reps:
+        if min(r.L) < 3 * 2.8:
+            d = r.q[:, None] - r.q[None]
+            d -= np.array(r.L) * np.round(d / np.array(r.L))
+            r2 = (d * d).sum(2)[np.triu_indices(r.n, 1)]
+            entries += 2 * int((r2 <= 2.8 ** 2).sum())
+            within += int((r2 <= 2.5 ** 2).sum())
+            continue
+        s = M.System(r.L, cutoff=2.5, time_step=0.005, capacity=r.n, build_block=128, build_threads_per_atom=2)
+        s.set_state(r.q, r.v)
+        s.make_pairlist()
+        w, e = s.pair_counts()
+        entries, within = entries + e, within + w // 2
+        s.close()
+    assert got == (entries, within)
 
 
 def test_fp64_sums_do_not_depend_on_the_lane_count():
