@@ -85,7 +85,7 @@ struct mdg_handle {
   cudaStream_t stream = nullptr;      // work stream (user's or owned)
   bool own_stream = false;
   cudaStream_t cap_stream = nullptr;  // capture stream (always owned)
-  int *d_flags = nullptr;             // eager-mode conditional values
+  int *d_flags = nullptr;             // [0, 1] eager-mode conditional values, [2] k_drift's ticket
   double *d_sums = nullptr;           // reduction outputs
   int *d_tiles = nullptr;             // tile totals of the cell-count scan
   size_t partial_cap = 0;
@@ -396,10 +396,9 @@ void launch_fp64(mdg_handle *h, cudaStream_t s, const Thermo &th, int drift, con
 }
 
 // drift: 1 also applies the second half drift in the same pass, 2 the whole
-// fused NVE step reading qf and packing into qf_next; returns whether the
-// second drift was made.
+// fused NVE step reading qf and packing into qf_next.
 template <int MODE>
-bool launch_force_mode(mdg_handle *h, cudaStream_t s, const Thermo &th, int drift = 0, const int4 *qf = nullptr,
+void launch_force_mode(mdg_handle *h, cudaStream_t s, const Thermo &th, int drift = 0, const int4 *qf = nullptr,
                        int4 *qf_next = nullptr) {
   const int n = h->n;
   const int nb = blocks_for(n, kForceBlock);
@@ -412,21 +411,20 @@ bool launch_force_mode(mdg_handle *h, cudaStream_t s, const Thermo &th, int drif
       k_force_fp32_staged<kForceBlock, MODE, 1><<<nb, kForceBlock, smem, s>>>(h->a, h->box, n, th, qf, nullptr);
     else
       k_force_fp32_staged<kForceBlock, MODE, 0><<<nb, kForceBlock, smem, s>>>(h->a, h->box, n, th, qf, nullptr);
-    return drift != 0;
+    return;
   }
   if (h->prm.precision == MDG_FP32_MIXED) {
     const int tpa = h->tpa > 0 ? h->tpa : 1;
     if (tpa == 4) launch_fp32<MODE, 4>(h, s, th, drift, qf, qf_next);
     else if (tpa == 2) launch_fp32<MODE, 2>(h, s, th, drift, qf, qf_next);
     else launch_fp32<MODE, 1>(h, s, th, drift, qf, qf_next);
-    return drift != 0;
+    return;
   }
   switch (fp64_lanes(n)) {
     case 8: launch_fp64<MODE, 8>(h, s, th, drift, qf, qf_next); break;
     case 4: launch_fp64<MODE, 4>(h, s, th, drift, qf, qf_next); break;
     default: launch_fp64<MODE, 1>(h, s, th, drift, qf, qf_next);
   }
-  return drift != 0;
 }
 
 Thermo thermo_of(const mdg_handle *h) {
@@ -437,20 +435,19 @@ Thermo thermo_of(const mdg_handle *h) {
   return th;
 }
 
-void launch_drift(mdg_handle *h, cudaStream_t s, bool pack_fix, int track_vmax) {
-  const int nb = blocks_for(h->n, kBlock);
-  if (pack_fix)
-    k_drift<kBlock, true><<<nb, kBlock, 0, s>>>(h->a, h->box, h->n, track_vmax);
-  else
-    k_drift<kBlock, false><<<nb, kBlock, 0, s>>>(h->a, h->box, h->n, track_vmax);
+// The first half drift, packing the positions that the force pass reads.
+void launch_drift(mdg_handle *h, cudaStream_t s) {
+  k_drift<kBlock, true><<<blocks_for(h->n, kBlock), kBlock, 0, s>>>(h->a, h->box, h->n, 0);
 }
 
 // Everything of MDManager::Calculate after the rebuild decision; returns the
 // number of kernels launched.  ev_start/ev_stop bracket the force kernel.
 // parity: the fixed-point buffer the fused NVE step reads (it writes the
 // other one).
+// end: the next step's expiry decision, where a kernel of this one can make it
+// (ends_step).
 int launch_step_tail(mdg_handle *h, cudaStream_t s, cudaEvent_t ev_start, cudaEvent_t ev_stop,
-                     bool capture, int parity) {
+                     bool capture, int parity, const StepEnd &end = StepEnd{}) {
   const bool fix = h->prm.precision == MDG_FP32_MIXED;
   const Thermo th = thermo_of(h);
   const int n = h->n;
@@ -467,39 +464,31 @@ int launch_step_tail(mdg_handle *h, cudaStream_t s, cudaEvent_t ev_start, cudaEv
     rec(ev_stop);
     return 1;
   }
-  launch_drift(h, s, true, 0);
-  launches++;
   if (h->prm.thermostat == MDG_NOSE_HOOVER) {
-    const int nbk = blocks_for(n, kBlock);
-    k_ke_partial<kBlock><<<nbk, kBlock, 0, s>>>(h->a, n);
-    k_zeta<1024><<<1, 1024, 0, s>>>(h->a, h->box, nbk, n, h->prm.aimed_temperature, h->prm.heatbath_tau);
+    k_drift<kBlock, true, true><<<blocks_for(n, kBlock), kBlock, 0, s>>>(
+        h->a, h->box, n, 0, DriftZeta{h->d_flags + 2, h->prm.aimed_temperature, h->prm.heatbath_tau});
     rec(ev_start);
     // the second drift does not read zeta, so it may precede the zeta update
-    const bool drifted = launch_force_mode<kKickNoseHoover>(h, s, th, 1);
+    launch_force_mode<kKickNoseHoover>(h, s, th, 1);
     rec(ev_stop);
     k_zeta<1024><<<1, 1024, 0, s>>>(h->a, h->box, fix ? blocks_for(n, kForceBlock) : fp64_blocks(n), n,
-                                     h->prm.aimed_temperature, h->prm.heatbath_tau);
-    launches += 4;
-    if (!drifted) {
-      launch_drift(h, s, false, 1);
-      launches++;
-    }
-  } else if (h->prm.thermostat == MDG_LANGEVIN) {
+                                     h->prm.aimed_temperature, h->prm.heatbath_tau, end);
+    return launches + 3 + launch_external(h, s);
+  }
+  launch_drift(h, s);
+  launches++;
+  if (h->prm.thermostat == MDG_LANGEVIN) {
     rec(ev_start);
     launch_force_mode<kKickLangevin>(h, s, th);
     rec(ev_stop);
     launches += 1;
   } else {
     rec(ev_start);
-    const bool drifted = launch_force_mode<kKick>(h, s, th, 1);
+    launch_force_mode<kKick>(h, s, th, 1);
     rec(ev_stop);
     launches += 1;
-    if (!drifted) {
-      launch_drift(h, s, false, 1);
-      launches++;
-    }
   }
-  k_step_done<<<1, 32, 0, s>>>(h->a, h->box);
+  k_step_done<<<1, 32, 0, s>>>(h->a, h->box, end);
   return launches + 1 + launch_external(h, s);
 }
 
@@ -555,32 +544,40 @@ mdg_status build_graph(mdg_handle *h) {
   }
   Capture c{h->cap_stream, g, {}};
   int kernels = 0;
+  // a step whose last kernel counts it decides the next one's branch too
+  const bool ends_step = !fused_step(h) && h->ext.kind == 0;
+  cudaGraphConditionalHandle h_any[kStepsPerGraph];
+  for (auto &x : h_any) CUDA_TRY(h, cudaGraphConditionalHandleCreate(&x, g, 0, cudaGraphCondAssignDefault));
   for (int s = 0; s < kStepsPerGraph; s++) {
-    cudaGraphConditionalHandle hd, hb;
-    CUDA_TRY(h, cudaGraphConditionalHandleCreate(&hd, g, 0, cudaGraphCondAssignDefault));
-    CUDA_TRY(h, cudaGraphConditionalHandleCreate(&hb, g, 0, cudaGraphCondAssignDefault));
-    CUDA_TRY(h, begin_capture(c));
-    k_expiry<<<1, 32, 0, c.s>>>(h->a, h->box, hd, hb, 1, h->d_flags);
-    CUDA_TRY(h, end_capture(c));
-    cudaGraph_t body;
-    CUDA_TRY(h, add_if(c, hd, &body));
+    if (s == 0 || !ends_step) {
+      CUDA_TRY(h, begin_capture(c));
+      k_expiry<<<1, 32, 0, c.s>>>(h->a, h->box, h_any[s], 1, nullptr);
+      kernels++;
+      CUDA_TRY(h, end_capture(c));
+    }
+    cudaGraph_t branch, body;
+    CUDA_TRY(h, add_if(c, h_any[s], &branch));
     {
-      Capture bc{h->cap_stream, body, {}};
+      cudaGraphConditionalHandle hb;
+      CUDA_TRY(h, cudaGraphConditionalHandleCreate(&hb, branch, 0, cudaGraphCondAssignDefault));
+      Capture bc{h->cap_stream, branch, {}};
       CUDA_TRY(h, begin_capture(bc));
       launch_disp(h, bc.s, step_lag(h));
-      k_decide<<<1, 32, 0, bc.s>>>(h->a, hb, 1, h->d_flags);
+      k_decide<<<1, 32, 0, bc.s>>>(h->a, hb, 1, nullptr);
       CUDA_TRY(h, end_capture(bc));
+      CUDA_TRY(h, add_if(bc, hb, &body));
     }
-    CUDA_TRY(h, add_if(c, hb, &body));
     {
       Capture bc{h->cap_stream, body, {}};
       CUDA_TRY(h, begin_capture(bc));
       launch_build(h, bc.s, fused_step(h) ? fix_buffer(h, s & 1) : nullptr);
       CUDA_TRY(h, end_capture(bc));
     }
+    StepEnd end{};
+    if (ends_step && s + 1 < kStepsPerGraph) end = StepEnd{1, h_any[s + 1]};
     CUDA_TRY(h, begin_capture(c));
-    kernels += 1 + launch_step_tail(h, c.s, h->timing ? h->ev[2 * s] : nullptr,
-                                    h->timing ? h->ev[2 * s + 1] : nullptr, true, s & 1);
+    kernels += launch_step_tail(h, c.s, h->timing ? h->ev[2 * s] : nullptr,
+                                h->timing ? h->ev[2 * s + 1] : nullptr, true, s & 1, end);
     CUDA_TRY(h, end_capture(c));
   }
   cudaError_t e = cudaGraphInstantiate(&h->exec, g, 0);
@@ -595,7 +592,7 @@ mdg_status build_graph(mdg_handle *h) {
 // fine-grained entry points).
 mdg_status step_eager(mdg_handle *h) {
   int flags[2] = {0, 0};
-  k_expiry<<<1, 32, 0, h->stream>>>(h->a, h->box, 0, 0, 0, h->d_flags);
+  k_expiry<<<1, 32, 0, h->stream>>>(h->a, h->box, 0, 0, h->d_flags);
   CUDA_TRY(h, cudaMemcpyAsync(flags, h->d_flags, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   h->kernel_launches++;
@@ -1057,6 +1054,7 @@ mdg_status mdg_create(const mdg_params *prm, mdg_handle **out) {
   if (e == cudaSuccess) e = dalloc(&a.partials, h->partial_cap);
   if (e == cudaSuccess) e = dalloc(&a.st, 1);
   if (e == cudaSuccess) e = dalloc(&h->d_flags, 4);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->d_flags, 0, 4 * sizeof(int), h->stream);
   if (e == cudaSuccess) e = dalloc(&h->d_sums, 8);
   if (e == cudaSuccess) e = dalloc(&h->d_tiles, (size_t)blocks_for(h->ncell, kScanBlock) + 1);
   if (e == cudaSuccess) e = dalloc(&h->d_bar, 1);
@@ -1239,7 +1237,7 @@ mdg_status mdg_check_expired(mdg_handle *h, int *expired) {
   if (h->n == 0) return MDG_OK;
   k_vmax<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->n);
   int flags[2] = {0, 0};
-  k_expiry<<<1, 32, 0, h->stream>>>(h->a, h->box, 0, 0, 0, h->d_flags);
+  k_expiry<<<1, 32, 0, h->stream>>>(h->a, h->box, 0, 0, h->d_flags);
   CUDA_TRY(h, cudaMemcpyAsync(flags, h->d_flags, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   if (flags[0]) launch_disp(h, h->stream, h->obs_lag);
@@ -1260,7 +1258,7 @@ mdg_status mdg_update_position_half(mdg_handle *h) {
   h->fix_buf = -1;  // q, v or the fixed-point copy change outside the fused step
   h->obs_lag = 0.0;
   if (h->n == 0) return MDG_OK;
-  launch_drift(h, h->stream, true, 0);
+  launch_drift(h, h->stream);
   CUDA_TRY(h, cudaGetLastError());
   return MDG_OK;
 }

@@ -366,24 +366,31 @@ __device__ __forceinline__ int expiry_decide(Status *st, const Box &b, int *disp
   return build;
 }
 
-// expiry_decide as a kernel: sets the two conditional handles of this
-// step's graph (or device flags in eager mode).
-static __global__ void k_expiry(Arrays a, Box b, cudaGraphConditionalHandle h_disp,
-                                cudaGraphConditionalHandle h_build, int in_graph, int *eager_flags) {
+// expiry_decide in a graph: the step's conditional branch (skin check, then
+// rebuild) runs if either may be due.  One thread.  A conditional node costs
+// 6.5 us where its branch is not taken (a rate every step pays), so a step has
+// one, and the rebuild's is inside its branch.
+__device__ __forceinline__ void expiry_in_graph(Status *st, const Box &b, cudaGraphConditionalHandle h_any) {
+  int disp = 0;
+  const int build = expiry_decide(st, b, &disp);
+  cudaGraphSetConditional(h_any, disp || (st->error == 0 && build));
+}
+
+// expiry_decide as a kernel: for a graph, or setting device flags in eager
+// mode (there the check and the rebuild are launched apart).
+static __global__ void k_expiry(Arrays a, Box b, cudaGraphConditionalHandle h_any, int in_graph, int *eager_flags) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   Status *st = a.st;
+  if (in_graph) {
+    expiry_in_graph(st, b, h_any);
+    return;
+  }
   int disp = 0;
   const int build = expiry_decide(st, b, &disp);
   // the rebuild decision when no displacement check runs; otherwise k_decide,
   // after the check, sets it again
-  const int build_now = st->error == 0 && build;
-  if (in_graph) {
-    cudaGraphSetConditional(h_disp, disp);
-    cudaGraphSetConditional(h_build, build_now);
-  } else {
-    eager_flags[0] = disp;
-    eager_flags[1] = build_now;
-  }
+  eager_flags[0] = disp;
+  eager_flags[1] = st->error == 0 && build;
 }
 
 // Sets the rebuild condition of this step from the expiry and displacement
@@ -486,6 +493,7 @@ template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_disp_max(Arrays a, Box b, int n, double lag) {
   const int i = blockIdx.x * BLOCK + threadIdx.x;
   double d2 = 0.0;
+  if (a.st->list_stale) return;  // a graph's branch that only rebuilds
   if (i < n) for_each_copy(copy_view(a), b.L, i, lag, [&](int, double x) { d2 = fmax(d2, x); });
   if (a.disp2 && i < n) a.disp2[i] = d2;
   block_max_to<BLOCK>(&a.st->dr2max_bits, d2);
@@ -496,7 +504,7 @@ __global__ void __launch_bounds__(BLOCK) k_disp_max(Arrays a, Box b, int n, doub
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_disp_collect(Arrays a, Box b, int n, int cand_cap, double lag) {
   const int i = blockIdx.x * BLOCK + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || a.st->list_stale) return;
   const double c = b.buffer_length - sqrt(__longlong_as_double((long long)a.st->dr2max_bits));
   const double c_d2 = c * c;
   // no copy of this atom moved more than c (k_disp_max's per-atom maximum
@@ -593,6 +601,7 @@ __global__ void __launch_bounds__(BLOCK) k_disp_pairs(Arrays a, Box b, double la
   if (threadIdx.x == 0) found = 0;
   __syncthreads();
   Status *st = a.st;
+  if (st->list_stale) return;
   const long long tn = st->total_images;
   const int nl = (int)((tn > b.check_list_length) ? b.check_list_length : tn);
   if (st->cand_weighted >= nl) {
@@ -1845,12 +1854,50 @@ static __global__ void k_build_done(Arrays a, Box b) {
   st->rebuilds++;
 }
 
+// Nose-Hoover: T = KE/N/1.5 from the blocks' partial sums, zeta += (T -
+// T0)/tau^2 * dt/2 (ForceCalculator::HeatbathZeta, src/fcalculator.cc:979-985).
+// All threads of one block; the sum has the same order for every block size.
+template <int BLOCK>
+__device__ __forceinline__ void add_zeta(const Arrays &a, const Box &b, int nblocks, int n, double aimed_t,
+                                         double tau) {
+  constexpr int kTerms = 1024;
+  __shared__ double sm[kTerms];
+  for (int t = threadIdx.x; t < kTerms; t += BLOCK) {
+    double s = 0.0;
+    for (int k = t; k < nblocks; k += kTerms) s += __ldcg(a.partials + k);  // other blocks' stores
+    sm[t] = s;
+  }
+  for (int off = kTerms / 2; off >= 32; off >>= 1) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < off; t += BLOCK) sm[t] += sm[t + off];
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  double s = sm[threadIdx.x];
+  for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+  if (threadIdx.x == 0 && !a.st->error) {
+    const double t = s / (double)n / 1.5;
+    const double t1 = (t - aimed_t) / (tau * tau);
+    a.st->zeta += t1 * (b.dt * 0.5);
+  }
+}
+
+// First zeta update of a Nose-Hoover step, made by k_drift's last block (of
+// the kinetic energy that the drift leaves alone): ticket counts the blocks.
+struct DriftZeta {
+  int *ticket;
+  double aimed_t, tau;
+};
+
 // q += v dt/2 (ForceCalculator::UpdatePositionHalf, src/fcalculator.cc:17-30);
-// FIX also writes the packed copy that the force pass reads.
-template <int BLOCK, bool FIX>
-__global__ void __launch_bounds__(BLOCK) k_drift(Arrays a, Box b, int n, int track_vmax) {
+// FIX also writes the packed copy that the force pass reads.  ZETA: with the
+// kinetic energy partials (KineticEnergyObserver, src/observer.cc:4-15) and the
+// zeta update in the pass; as kernels of their own they took 2.0 + 2.9 us of a
+// 118,661-atom step besides the drift's 3.0.
+template <int BLOCK, bool FIX, bool ZETA = false>
+__global__ void __launch_bounds__(BLOCK) k_drift(Arrays a, Box b, int n, int track_vmax, DriftZeta zeta = DriftZeta{}) {
   const int i = blockIdx.x * BLOCK + threadIdx.x;
-  double v2 = 0.0;
+  double v2 = 0.0, ke[1] = {0.0};
   if (i < n && !a.st->error) {
     const double dt2 = b.dt * 0.5;
     double4 q = a.q[i];
@@ -1864,8 +1911,23 @@ __global__ void __launch_bounds__(BLOCK) k_drift(Arrays a, Box b, int n, int tra
       v2 = dadd(dadd(dmul(v.x, v.x), dmul(v.y, v.y)), dmul(v.z, v.z));
       if (!isfinite(v2) || !isfinite(q.x + q.y + q.z)) atomicOr(&a.st->error, kErrNonFinite);
     }
+    if (ZETA)
+      ke[0] = dadd(dadd(dmul(dmul(0.5, v.x), v.x), dmul(dmul(0.5, v.y), v.y)), dmul(dmul(0.5, v.z), v.z));
   }
   if (track_vmax) block_max_to<BLOCK>(&a.st->vmax2_bits, v2);
+  if constexpr (ZETA) {
+    __shared__ bool last;
+    block_sum_to<BLOCK, 1>(ke, a.partials);
+    if (threadIdx.x == 0) {
+      __threadfence();  // the partial before the ticket
+      last = atomicAdd(zeta.ticket, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    add_zeta<BLOCK>(a, b, gridDim.x, n, zeta.aimed_t, zeta.tau);
+    if (threadIdx.x == 0) *zeta.ticket = 0;
+  }
 }
 
 // ------------------------------------------------------------ executors
@@ -3038,38 +3100,28 @@ static __global__ void k_set_target(Arrays a, long long target, int parity) {
   a.st->fix_parity = parity;
 }
 
-// Kinetic energy partials (KineticEnergyObserver, src/observer.cc:4-15).
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_ke_partial(Arrays a, int n) {
-  const int i = blockIdx.x * BLOCK + threadIdx.x;
-  double ke = 0.0;
-  if (i < n) {
-    const double4 v = a.v[i];
-    ke = dadd(dadd(dmul(dmul(0.5, v.x), v.x), dmul(dmul(0.5, v.y), v.y)), dmul(dmul(0.5, v.z), v.z));
+// What a step's last kernel does besides its own work: counts the step and, in
+// a graph, decides the next step's branch (expiry_in_graph).
+struct StepEnd {
+  int expiry;
+  cudaGraphConditionalHandle h_any;
+};
+
+// One thread.
+__device__ __forceinline__ void end_step(Status *st, const Box &b, const StepEnd &end) {
+  if (!st->error) {
+    st->steps++;
+    st->sim_time += b.dt;
   }
-  double s[1] = {ke};
-  block_sum_to<BLOCK, 1>(s, a.partials);
+  if (end.expiry) expiry_in_graph(st, b, end.h_any);
 }
 
-// Sums nblocks partials in a fixed order; Nose-Hoover: T = KE/N/1.5,
-// zeta += (T - T0)/tau^2 * dt/2 (ForceCalculator::HeatbathZeta, src/fcalculator.cc:979-985).
+// The second zeta update of a Nose-Hoover step, and the step's end.
 template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_zeta(Arrays a, Box b, int nblocks, int n, double aimed_t,
-                                                double tau) {
-  __shared__ double sm[BLOCK];
-  double s = 0.0;
-  for (int k = threadIdx.x; k < nblocks; k += BLOCK) s += a.partials[k];
-  sm[threadIdx.x] = s;
-  __syncthreads();
-  for (int off = BLOCK / 2; off > 0; off >>= 1) {
-    if (threadIdx.x < off) sm[threadIdx.x] += sm[threadIdx.x + off];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0 && !a.st->error) {
-    const double t = sm[0] / (double)n / 1.5;
-    const double t1 = (t - aimed_t) / (tau * tau);
-    a.st->zeta += t1 * (b.dt * 0.5);
-  }
+__global__ void __launch_bounds__(BLOCK) k_zeta(Arrays a, Box b, int nblocks, int n, double aimed_t, double tau,
+                                                StepEnd end) {
+  add_zeta<BLOCK>(a, b, nblocks, n, aimed_t, tau);
+  if (threadIdx.x == 0) end_step(a.st, b, end);
 }
 
 // Observers: KE, PE, virial per atom over the full list, x 1/2 for pair sums
@@ -3212,11 +3264,8 @@ __global__ void __launch_bounds__(BLOCK, kFp64Blocks) k_count_pairs(Arrays a, Bo
 }
 
 // End of step bookkeeping (MDManager::Calculate: s_time += TimeStep).
-static __global__ void k_step_done(Arrays a, Box b) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (a.st->error) return;
-  a.st->steps++;
-  a.st->sim_time += b.dt;
+static __global__ void k_step_done(Arrays a, Box b, StepEnd end) {
+  if (threadIdx.x == 0 && blockIdx.x == 0) end_step(a.st, b, end);
 }
 
 // Langevin alone (ForceCalculator::Langevin, src/fcalculator.cc:1001-1017),

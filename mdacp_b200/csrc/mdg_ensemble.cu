@@ -59,7 +59,7 @@ struct RepStatus {
 };
 
 // The replicas a skin check or a rebuild acts on, compacted in replica order
-// (ke_make_list), with the prefix sums that map a work index to an atom or
+// (make_list), with the prefix sums that map a work index to an atom or
 // a cell: the per-atom and per-cell kernels of those branches sweep only
 // these atoms and cells.
 struct WorkList {
@@ -217,7 +217,7 @@ struct WorkSweep {
 // One block, 1024 threads: the work list of the replicas whose disp (WHICH
 // 0) or build (WHICH 1) flag is set.
 template <int WHICH>
-__global__ void __launch_bounds__(1024) ke_make_list(Ens e) {
+__device__ __forceinline__ void make_list(const Ens &e) {
   const WorkList w = WHICH ? e.wb : e.wd;
   __shared__ int base_k, base_a, base_c, tk, ta, tc;
   if (threadIdx.x == 0) base_k = base_a = base_c = 0;
@@ -259,7 +259,12 @@ __global__ void __launch_bounds__(1024) ke_make_list(Ens e) {
 }
 
 // --------------------------------------------------------------- step kernels
-__global__ void ke_expiry(Ens e, cudaGraphConditionalHandle h_disp, int in_graph, int *flags) {
+// What ke_expiry and ke_decide do with their verdicts over all replicas.
+enum { kVerdictFlags = 0, kVerdictGraph = 1, kVerdictNone = 2 };
+
+// One block: every replica's expiry decision (expiry_decide's arithmetic) and
+// the check's work list.
+__global__ void __launch_bounds__(1024) ke_expiry(Ens e, cudaGraphConditionalHandle h_any, int verdict, int *flags) {
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
@@ -287,14 +292,15 @@ __global__ void ke_expiry(Ens e, cudaGraphConditionalHandle h_disp, int in_graph
     st.disp = disp;
     st.want_build = build;
     st.vmax2_bits = 0ull;
-    if (disp) any = 1;
+    if (disp || build) any = 1;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (in_graph) cudaGraphSetConditional(h_disp, any);
+  if (threadIdx.x == 0 && verdict != kVerdictNone) {
+    if (verdict == kVerdictGraph) cudaGraphSetConditional(h_any, any);
     else flags[0] = any;
     if (any) flags[2]++;  // steps that launch the skin-check branch
   }
+  make_list<0>(e);
 }
 
 __device__ __forceinline__ CopyView ens_view(const Ens &e) { return CopyView{e.q_old, e.q, e.v, e.mult}; }
@@ -342,11 +348,15 @@ __global__ void __launch_bounds__(kEB) ke_disp_collect(Ens e) {
 }
 
 // kEPairParts blocks per replica (blockIdx.y) share the rows of the
-// candidate-pair test of PairList::CheckByDisplacement.
+// candidate-pair test of PairList::CheckByDisplacement, and clear the cell
+// counts of every replica that may rebuild.
 __global__ void __launch_bounds__(256) ke_disp_pairs(Ens e) {
   const int r = blockIdx.x;
   RepStatus &st = e.rs[r];
-  // a short candidate list takes one block (its rows are 256 columns wide)
+  if (!st.disp && !st.want_build) return;  // want_build alone: a stale list
+  const int ncell = e.rep[r].ncell;
+  for (int c = blockIdx.y * 256 + threadIdx.x; c < ncell; c += gridDim.y * 256) e.cell_count[e.rep[r].cell_off + c] = 0;
+  // a short candidate list takes one block
   if (!st.disp || (blockIdx.y > 0 && st.cand_n <= kEPairShort)) return;
   __shared__ PairStage sm;
   __shared__ volatile int found;
@@ -366,7 +376,8 @@ __global__ void __launch_bounds__(256) ke_disp_pairs(Ens e) {
   if (threadIdx.x == 0 && found) st.want_build = 1;
 }
 
-__global__ void ke_decide(Ens e, cudaGraphConditionalHandle h_build, int in_graph, int *flags) {
+// One block: the rebuilding replicas and their work list.
+__global__ void __launch_bounds__(1024) ke_decide(Ens e, cudaGraphConditionalHandle h_build, int verdict, int *flags) {
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
@@ -383,21 +394,15 @@ __global__ void ke_decide(Ens e, cudaGraphConditionalHandle h_build, int in_grap
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (in_graph) cudaGraphSetConditional(h_build, any);
+  if (threadIdx.x == 0 && verdict != kVerdictNone) {
+    if (verdict == kVerdictGraph) cudaGraphSetConditional(h_build, any);
     else flags[1] = any;
     if (any) flags[3]++;  // steps that launch the rebuild branch
   }
+  make_list<1>(e);
 }
 
 // ---------------------------------------------------------- rebuild kernels
-__global__ void __launch_bounds__(kEB) ke_clear_cells(Ens e) {
-  const int r = blockIdx.x;
-  if (!e.rs[r].build) return;
-  const Rep rep = e.rep[r];
-  for (int c = threadIdx.x; c < rep.ncell; c += kEB) e.cell_count[rep.cell_off + c] = 0;
-}
-
 // Wraps atom i of replica r into its box (Variables::AdjustPeriodicBoundary,
 // src/variables.cc:63-84), checks it, and files it in its cell.
 __device__ __forceinline__ void cell_assign_atom(const Ens &e, int r, int i) {
@@ -851,18 +856,26 @@ int lane_blocks(int n, int lanes) { return (int)(((long long)n * lanes + kEF - 1
 int4 *e_pack(const Ens &e, int k) { return k ? e.qfix2 : e.qfix; }
 double *e_pack_z(const Ens &e, int k) { return k ? e.pz2 : e.pz; }
 
-// Kernels launched by one skin-check and one rebuild branch.
-constexpr int kEDispKernels = 4, kEBuildKernels = 10;
+// Kernels launched by one skin check (with its decision) and one rebuild.
+constexpr int kEDispKernels = 4, kEBuildKernels = 8;
+
+// From this many replicas the check's and the rebuild's kernels are launched
+// every step, and sweep empty work lists where nothing is due.  A list lives
+// some eight steps, so with eight replicas most steps rebuild one; a
+// conditional branch costs 6.5 us to pass by and about 12 to take, twice a step
+// (and two waits by the host outside graphs), twelve empty launches about 20.
+constexpr int kEAlways = 8;
 
 // The per-atom and per-cell kernels of the branches sweep the work list with
 // a grid of at most x->work_blocks blocks (full occupancy of every SM).
-void e_launch_disp(mdg_ensemble *x, cudaStream_t s) {
+// The verdict's arguments go to ke_decide.
+void e_launch_disp(mdg_ensemble *x, cudaStream_t s, cudaGraphConditionalHandle h_build, int verdict) {
   Ens &e = x->e;
   const int gb = std::min(nb(e.ntot, kEB), x->work_blocks);
-  ke_make_list<0><<<1, 1024, 0, s>>>(e);
   ke_disp_max<<<gb, kEB, 0, s>>>(e);
   ke_disp_collect<<<gb, kEB, 0, s>>>(e);
   ke_disp_pairs<<<dim3(e.nrep, kEPairParts), 256, 0, s>>>(e);
+  ke_decide<<<1, 1024, 0, s>>>(e, h_build, verdict, x->d_flags);
 }
 
 // pack: the packed copy that the coming step reads (0, 1), refreshed for the
@@ -871,8 +884,6 @@ void e_launch_build(mdg_ensemble *x, cudaStream_t s, int pack) {
   Ens &e = x->e;
   const int gb = std::min(nb(e.ntot, kEB), x->work_blocks);
   const int gc = std::min(nb(x->ncell_tot * 32, kEB), x->work_blocks);
-  ke_make_list<1><<<1, 1024, 0, s>>>(e);
-  ke_clear_cells<<<e.nrep, kEB, 0, s>>>(e);
   ke_cell_assign<<<gb, kEB, 0, s>>>(e);
   ke_scan_cells<<<e.nrep, kEB, 0, s>>>(e);
   ke_scatter<<<gb, kEB, 0, s>>>(e);
@@ -921,6 +932,14 @@ int e_launch_tail(mdg_ensemble *x, cudaStream_t s, int parity, cudaEvent_t e0 = 
   }
   rec(e1);
   return 1;
+}
+
+// A step without branches (kEAlways); returns its kernels.
+int e_launch_step(mdg_ensemble *x, cudaStream_t s, int parity, cudaEvent_t e0, cudaEvent_t e1, bool capture) {
+  ke_expiry<<<1, 1024, 0, s>>>(x->e, 0, kVerdictNone, nullptr);
+  e_launch_disp(x, s, 0, kVerdictNone);
+  e_launch_build(x, s, parity);
+  return 1 + kEDispKernels + kEBuildKernels + e_launch_tail(x, s, parity, e0, e1, capture);
 }
 
 void e_destroy_events(mdg_ensemble *x) {
@@ -980,24 +999,28 @@ mdg_status e_build_graph(mdg_ensemble *x) {
   ECapture c{x->cap_stream, g, {}};
   int kernels = 0;
   for (int s = 0; s < kEStepsPerGraph; s++) {
-    cudaGraphConditionalHandle hd, hb;
-    ECUDA(cudaGraphConditionalHandleCreate(&hd, g, 0, cudaGraphCondAssignDefault));
-    ECUDA(cudaGraphConditionalHandleCreate(&hb, g, 0, cudaGraphCondAssignDefault));
-    ECUDA(e_begin(c));
-    ke_expiry<<<1, 1024, 0, c.s>>>(x->e, hd, 1, x->d_flags);
-    ECUDA(e_end(c));
-    cudaGraph_t body;
-    ECUDA(e_add_if(c, hd, &body));
-    {
-      ECapture bc{x->cap_stream, body, {}};
-      ECUDA(e_begin(bc));
-      e_launch_disp(x, bc.s);
-      ECUDA(e_end(bc));
+    cudaEvent_t e0 = x->timing ? x->ev[2 * s] : nullptr, e1 = x->timing ? x->ev[2 * s + 1] : nullptr;
+    if (x->e.nrep >= kEAlways) {
+      ECUDA(e_begin(c));
+      kernels += e_launch_step(x, c.s, s & 1, e0, e1, true);
+      ECUDA(e_end(c));
+      continue;
     }
+    cudaGraphConditionalHandle ha, hb;
+    ECUDA(cudaGraphConditionalHandleCreate(&ha, g, 0, cudaGraphCondAssignDefault));
     ECUDA(e_begin(c));
-    ke_decide<<<1, 1024, 0, c.s>>>(x->e, hb, 1, x->d_flags);
+    ke_expiry<<<1, 1024, 0, c.s>>>(x->e, ha, kVerdictGraph, x->d_flags);
     ECUDA(e_end(c));
-    ECUDA(e_add_if(c, hb, &body));
+    cudaGraph_t branch, body;
+    ECUDA(e_add_if(c, ha, &branch));
+    {
+      ECUDA(cudaGraphConditionalHandleCreate(&hb, branch, 0, cudaGraphCondAssignDefault));
+      ECapture bc{x->cap_stream, branch, {}};
+      ECUDA(e_begin(bc));
+      e_launch_disp(x, bc.s, hb, kVerdictGraph);
+      ECUDA(e_end(bc));
+      ECUDA(e_add_if(bc, hb, &body));
+    }
     {
       ECapture bc{x->cap_stream, body, {}};
       ECUDA(e_begin(bc));
@@ -1005,8 +1028,7 @@ mdg_status e_build_graph(mdg_ensemble *x) {
       ECUDA(e_end(bc));
     }
     ECUDA(e_begin(c));
-    kernels += 2 + e_launch_tail(x, c.s, s & 1, x->timing ? x->ev[2 * s] : nullptr,
-                                 x->timing ? x->ev[2 * s + 1] : nullptr, true);
+    kernels += 1 + e_launch_tail(x, c.s, s & 1, e0, e1, true);
     ECUDA(e_end(c));
   }
   cudaError_t err = cudaGraphInstantiate(&x->exec, g, 0);
@@ -1028,23 +1050,27 @@ mdg_status e_step_eager(mdg_ensemble *x, float *force_ms_out = nullptr) {
   int flags[2] = {0, 0};
   const int parity = x->fix_buf > 0 ? 1 : 0;
   if (x->fix_buf < 0) e_pack_now(x);
-  ke_expiry<<<1, 1024, 0, x->stream>>>(x->e, 0, 0, x->d_flags);
-  ECUDA(cudaMemcpyAsync(flags, x->d_flags, sizeof flags, cudaMemcpyDeviceToHost, x->stream));
-  ECUDA(cudaStreamSynchronize(x->stream));
-  x->kernel_launches++;
-  if (flags[0]) e_launch_disp(x, x->stream);  // counted on the device (ke_expiry)
-  ke_decide<<<1, 1024, 0, x->stream>>>(x->e, 0, 0, x->d_flags);
-  ECUDA(cudaMemcpyAsync(flags, x->d_flags, sizeof flags, cudaMemcpyDeviceToHost, x->stream));
-  ECUDA(cudaStreamSynchronize(x->stream));
-  x->kernel_launches++;
-  if (flags[1]) e_launch_build(x, x->stream, parity);  // counted on the device (ke_decide)
+  const bool always = x->e.nrep >= kEAlways;
+  if (!always) {
+    ke_expiry<<<1, 1024, 0, x->stream>>>(x->e, 0, kVerdictFlags, x->d_flags);
+    x->kernel_launches++;
+    ECUDA(cudaMemcpyAsync(flags, x->d_flags, sizeof flags, cudaMemcpyDeviceToHost, x->stream));
+    ECUDA(cudaStreamSynchronize(x->stream));
+    if (flags[0]) {  // counted on the device (ke_expiry)
+      e_launch_disp(x, x->stream, 0, kVerdictFlags);
+      ECUDA(cudaMemcpyAsync(flags, x->d_flags, sizeof flags, cudaMemcpyDeviceToHost, x->stream));
+      ECUDA(cudaStreamSynchronize(x->stream));
+      if (flags[1]) e_launch_build(x, x->stream, parity);  // counted on the device (ke_decide)
+    }
+  }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   const bool timed = x->timing || force_ms_out;
   if (timed) {
     ECUDA(cudaEventCreate(&e0));
     ECUDA(cudaEventCreate(&e1));
   }
-  x->kernel_launches += e_launch_tail(x, x->stream, parity, e0, e1);
+  x->kernel_launches += always ? e_launch_step(x, x->stream, parity, e0, e1, false)
+                               : e_launch_tail(x, x->stream, parity, e0, e1);
   x->fix_buf = 1 - parity;
   ECUDA(cudaGetLastError());
   if (timed) {
@@ -1437,9 +1463,14 @@ mdg_status mdg_ensemble_observe(mdg_ensemble *x, double *ke, double *pe, double 
   bool stale = false;
   for (auto &s : rs) stale |= s.list_stale != 0;
   if (stale) {
-    for (auto &s : rs) s.build = s.list_stale;
+    for (auto &s : rs) {
+      s.want_build = s.list_stale;
+      s.disp = 0;
+    }
     ECUDA(cudaMemcpyAsync(e.rs, rs.data(), sizeof(RepStatus) * e.nrep, cudaMemcpyHostToDevice, x->stream));
     x->fix_buf = -1;  // the rebuild renumbers the atoms
+    ke_disp_pairs<<<dim3(e.nrep, kEPairParts), 256, 0, x->stream>>>(e);  // clears their cells
+    ke_decide<<<1, 1024, 0, x->stream>>>(e, 0, kVerdictNone, nullptr);
     e_launch_build(x, x->stream, -1);
     if ((r = e_status(x, &err, &rs))) return r;
     if (err) return e_translate(err);

@@ -539,7 +539,7 @@ mdg_status slab_step(mdg_slabs *x) {
   for (Slab &sl : x->s) {
     SCUDA(x, cudaSetDevice(sl.dev));
     SCUDA(x, cudaMemcpyAsync(&sl.a.st->vmax2_bits, &vmax, sizeof vmax, cudaMemcpyHostToDevice, sl.stream));
-    k_expiry<<<1, 32, 0, sl.stream>>>(sl.a, sl.box, 0, 0, 0, sl.d_flags);
+    k_expiry<<<1, 32, 0, sl.stream>>>(sl.a, sl.box, 0, 0, sl.d_flags);
   }
   int flags[2] = {0, 0};
   {

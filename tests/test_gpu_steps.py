@@ -1,0 +1,48 @@
+"""Steps through graphs and step by step, and ensembles with and without
+conditional branches, give the same trajectories bit for bit."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import mdacp_b200 as M
+from mdacp_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+# one block, a block and an atom, and several blocks of the drift's sums
+@pytest.mark.parametrize("cut", [256, 257, 3000])
+@pytest.mark.parametrize("precision", [M.FP64, M.FP32_MIXED])
+@pytest.mark.parametrize("thermostat", [M.NVE, M.NOSE_HOOVER, M.LANGEVIN])
+def test_graph_steps_equal_single_steps(cut, precision, thermostat):
+    w = W.fcc_liquid(5 if cut < 500 else 10, 0.6, 1.0, seed=cut, jitter=0.05, rc=2.5, dt=0.005)
+    out = []
+    for chunks in ([63], [1] * 63):
+        s = M.System(w.L, cutoff=2.5, time_step=0.005, capacity=w.n, precision=precision, thermostat=thermostat,
+                     aimed_temperature=1.2, seed=3)
+        s.set_state(w.q[:cut], w.v[:cut])
+        for k in chunks:
+            s.calculate(k)
+        info = s.info()
+        out.append((*s.state_by_id(), s.zeta(), info["steps"], info["rebuilds"], info["displacement_checks"]))
+        s.close()
+    a, b = out
+    assert a[4] > 1 and a[5] > 1  # the steps rebuilt and checked
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2:] == b[2:]
+
+
+@pytest.mark.parametrize("precision", [M.FP64, M.FP32_MIXED])
+def test_few_replicas_equal_many(precision):
+    # from eight replicas the check's and rebuild's kernels run every step
+    reps = [W.fcc_liquid(4 + k % 3, 0.5 + 0.04 * k, 1.0, seed=k, jitter=0.05, rc=2.5, dt=0.005) for k in range(9)]
+    out = []
+    for n, chunks in ((9, [67]), (9, [20] + [1] * 47), (8, [67]), (7, [67]), (1, [67])):
+        ens = M.Ensemble([(r.q, r.v, r.L) for r in reps[:n]], cutoff=2.5, time_step=0.005, precision=precision)
+        for k in chunks:
+            ens.calculate(k)
+        out.append(ens.states_by_id())
+        ens.close()
+    for other in out[1:]:
+        for (q, v), (q1, v1) in zip(out[0], other):
+            assert np.array_equal(q, q1) and np.array_equal(v, v1)
