@@ -2576,13 +2576,12 @@ __device__ __forceinline__ void fp32_row(Groups &f, int G, int sub, const int4 &
 // 0.282 ms per fused pass on the 2.05M-atom liquid against 0.304 ms for
 // fp32_row<1> over GlobalGroups (whose per-group selects the compiler
 // schedules worse).
-__device__ __forceinline__ void fp32_row_global(const Arrays &a, const Box &b, const int4 *qf, int i,
-                                                const int4 &pi, int nn4, double &Fx, double &Fy, double &Fz) {
-  const float sx = b.fix_scale[0], sy = b.fix_scale[1], sz = b.fix_scale[2];
-  const unsigned rc2_bits = __float_as_uint(b.rc2f);
-  const float c2x8 = b.c2x8f;
-  const int *row = a.nbr + i;
-  const int st = a.stride;
+__device__ __forceinline__ void fp32_row_global(const int *nbr, int st, const int4 *qf, int i, const int4 &pi, int nn4,
+                                                const PairConst &c, double &Fx, double &Fy, double &Fz) {
+  const float sx = c.sx, sy = c.sy, sz = c.sz;
+  const unsigned rc2_bits = c.rc2_bits;
+  const float c2x8 = c.c2x8;
+  const int *row = nbr + i;
   float fx = 0.f, fy = 0.f, fz = 0.f;
   int n0 = i, n1 = i, n2 = i, n3 = i;
   int m0 = i, m1 = i, m2 = i, m3 = i;
@@ -2690,7 +2689,7 @@ __global__ void __launch_bounds__(BLOCK) k_force_fp32(Arrays a, Box b, int n, Th
     double Fx, Fy, Fz;
     const PairConst k = pair_const(b.fix_scale, b.rc2f, b.c2x8f);
     if (TPA == 1) {
-      fp32_row_global(a, b, qf, i, pi, (a.nnbr[i] + 3) & ~3, Fx, Fy, Fz);
+      fp32_row_global(a.nbr, a.stride, qf, i, pi, (a.nnbr[i] + 3) & ~3, k, Fx, Fy, Fz);
     } else {
       GlobalGroups<> f{a.nbr + i, a.stride, qf, i};
       fp32_row<TPA>(f, (a.nnbr[i] + 3) >> 2, sub, pi, k, Fx, Fy, Fz);

@@ -675,10 +675,15 @@ __global__ void __launch_bounds__(kEF) ke_force_fp32(Ens e, const int4 *qf, int4
   if (active) {
     r = e.rep_of[i];
     const Rep &rep = e.rep[r];
-    // positions not loaded a group ahead: at 64 registers this pass is
-    // faster without (0.324 vs 0.353 ms on the 256-replica ensemble)
-    GlobalGroups<false> f{e.nbr + i, e.stride, qf, i};
-    fp32_row<TPA>(f, (e.nnbr[i] + 3) >> 2, sub, qf[i], pair_const(rep.fix_scale, e.rc2f, e.c2x8f), Fx, Fy, Fz);
+    const PairConst k = pair_const(rep.fix_scale, e.rc2f, e.c2x8f);
+    if (TPA == 1) {
+      fp32_row_global(e.nbr, e.stride, qf, i, qf[i], (e.nnbr[i] + 3) & ~3, k, Fx, Fy, Fz);
+    } else {
+      // positions not loaded a group ahead: at 64 registers this pass is
+      // faster without (0.324 vs 0.353 ms on the 256-replica ensemble)
+      GlobalGroups<false> f{e.nbr + i, e.stride, qf, i};
+      fp32_row<TPA>(f, (e.nnbr[i] + 3) >> 2, sub, qf[i], k, Fx, Fy, Fz);
+    }
     const double dt = e.dt;
     if (sub == 0) v2 = finish_step(e, rep, i, Fx * dt, Fy * dt, Fz * dt, next, nullptr);
   }
