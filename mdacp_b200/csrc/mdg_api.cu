@@ -75,6 +75,14 @@ size_t trim_table_size(const mdg::Box &b) { return (size_t)b.ms[1] * b.ms[2] * (
 
 }  // namespace
 
+// A handle's small answers from the device, in pinned memory: a copy to the
+// stack goes through the driver's staging and takes twice as long.
+struct HostLanding {
+  Status st;
+  int flags[2];
+  double sums[3];
+};
+
 struct mdg_handle {
   mdg_params prm{};
   Box box{};
@@ -85,6 +93,11 @@ struct mdg_handle {
   cudaStream_t stream = nullptr;      // work stream (user's or owned)
   bool own_stream = false;
   cudaStream_t cap_stream = nullptr;  // capture stream (always owned)
+  HostLanding *pin = nullptr;         // pinned: what the device's small answers are copied to
+  // the device's status after mdg_calculate's last wait; dropped by every call
+  // that may change it (check_ready), kept by those that only read the state
+  Status seen;
+  bool seen_ok = false;
   int *d_flags = nullptr;             // [0, 1] eager-mode conditional values, [2] k_drift's ticket
   double *d_sums = nullptr;           // reduction outputs
   int *d_tiles = nullptr;             // tile totals of the cell-count scan
@@ -185,8 +198,9 @@ mdg_status translate_device_error(mdg_handle *h, const Status &st) {
 }
 
 mdg_status read_status(mdg_handle *h, Status *st) {
-  CUDA_TRY(h, cudaMemcpyAsync(st, h->a.st, sizeof(Status), cudaMemcpyDeviceToHost, h->stream));
+  CUDA_TRY(h, cudaMemcpyAsync(&h->pin->st, h->a.st, sizeof(Status), cudaMemcpyDeviceToHost, h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  *st = h->pin->st;
   return MDG_OK;
 }
 
@@ -588,18 +602,33 @@ mdg_status build_graph(mdg_handle *h) {
   return MDG_OK;
 }
 
+// Whether the step after status st neither checks nor rebuilds, whatever the
+// last bits of the budget: the device's decision (expiry_decide) without
+// asking it.
+bool quiet_step(const mdg_handle *h, const Status &st) {
+  if (st.error || st.list_stale || !(st.budget > 0.0)) return false;
+  double v2;
+  memcpy(&v2, &st.vmax2_bits, sizeof v2);
+  const double left = st.budget - 2.0 * std::sqrt(v2) * h->box.dt;
+  return left > 1e-9 * h->box.buffer_length;
+}
+
 // One step with host-side decisions (used for partial chunks and by the
-// fine-grained entry points).
-mdg_status step_eager(mdg_handle *h) {
-  int flags[2] = {0, 0};
+// fine-grained entry points); quiet: the step's decisions are known
+// (quiet_step), so nothing is waited for.
+mdg_status step_eager(mdg_handle *h, bool quiet = false) {
+  int *flags = h->pin->flags;
+  flags[0] = flags[1] = 0;
   k_expiry<<<1, 32, 0, h->stream>>>(h->a, h->box, 0, 0, h->d_flags);
-  CUDA_TRY(h, cudaMemcpyAsync(flags, h->d_flags, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
-  CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   h->kernel_launches++;
+  if (!quiet) {
+    CUDA_TRY(h, cudaMemcpyAsync(flags, h->d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+  }
   if (flags[0]) {
     launch_disp(h, h->stream, step_lag(h));
     k_decide<<<1, 32, 0, h->stream>>>(h->a, 0, 0, h->d_flags);
-    CUDA_TRY(h, cudaMemcpyAsync(flags, h->d_flags, sizeof flags, cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(h, cudaMemcpyAsync(flags, h->d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     h->kernel_launches += 4;
   }
@@ -628,14 +657,18 @@ mdg_status step_eager(mdg_handle *h) {
   return MDG_OK;
 }
 
-mdg_status check_ready(mdg_handle *h) {
+// reads: the call leaves the device's status as it is (or renews h->seen itself).
+mdg_status check_ready(mdg_handle *h, bool reads = false) {
   if (!h) return MDG_ERR_INVALID_ARGUMENT;
+  if (!reads) h->seen_ok = false;
   if (!h->state_set) return fail(h, MDG_ERR_STATE, "no state uploaded (mdg_set_state)");
   return MDG_OK;
 }
 
 // Builds the list now if it is stale (forces / observers need a valid list).
 mdg_status ensure_list(mdg_handle *h) {
+  if (h->seen_ok && !h->seen.error && !h->seen.list_stale) return MDG_OK;
+  h->seen_ok = false;
   Status st;
   mdg_status r = read_status(h, &st);
   if (r) return r;
@@ -724,6 +757,7 @@ mdg_status autotune(mdg_handle *h) {
   // the first step without spending the skin budget) gets its status back
   // afterwards, so that the first step behaves the same whether the shapes
   // were timed, cached or pinned
+  h->seen_ok = false;
   Status before;
   mdg_status r = read_status(h, &before);
   if (r) return r;
@@ -1053,6 +1087,7 @@ mdg_status mdg_create(const mdg_params *prm, mdg_handle **out) {
   if (e == cudaSuccess) e = dalloc(&a.cand, prm->check_list_length);
   if (e == cudaSuccess) e = dalloc(&a.partials, h->partial_cap);
   if (e == cudaSuccess) e = dalloc(&a.st, 1);
+  if (e == cudaSuccess) e = cudaHostAlloc((void **)&h->pin, sizeof(HostLanding), cudaHostAllocDefault);
   if (e == cudaSuccess) e = dalloc(&h->d_flags, 4);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->d_flags, 0, 4 * sizeof(int), h->stream);
   if (e == cudaSuccess) e = dalloc(&h->d_sums, 8);
@@ -1097,6 +1132,7 @@ mdg_status mdg_destroy(mdg_handle *h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   destroy_graph(h);
   free_arrays(h->a);
+  if (h->pin) cudaFreeHost(h->pin);
   if (h->d_flags) cudaFree(h->d_flags);
   if (h->d_sums) cudaFree(h->d_sums);
   if (h->d_tiles) cudaFree(h->d_tiles);
@@ -1110,6 +1146,7 @@ mdg_status mdg_destroy(mdg_handle *h) {
 
 mdg_status mdg_set_state(mdg_handle *h, const double *q4, const double *v4, const int *type, int n) {
   if (!h || n < 0 || (n > 0 && (!q4 || !v4))) return MDG_ERR_INVALID_ARGUMENT;
+  h->seen_ok = false;
   if (n > h->cap) return fail(h, MDG_ERR_CAPACITY, "more atoms than the handle's capacity");
   h->fix_buf = -1;
   CUDA_TRY(h, cudaSetDevice(h->prm.device));
@@ -1162,7 +1199,7 @@ mdg_status mdg_set_state(mdg_handle *h, const double *q4, const double *v4, cons
 }
 
 mdg_status mdg_get_state(mdg_handle *h, double *q4, double *v4, int *type, int n) {
-  mdg_status r = check_ready(h);
+  mdg_status r = check_ready(h, true);
   if (r) return r;
   if (n != h->n) return fail(h, MDG_ERR_INVALID_ARGUMENT, "n differs from the handle's atom count");
   if (n == 0) return MDG_OK;
@@ -1204,7 +1241,7 @@ mdg_status mdg_set_velocities(mdg_handle *h, const double *v4, int n) {
 }
 
 mdg_status mdg_get_ids(mdg_handle *h, int *ids, int n) {
-  mdg_status r = check_ready(h);
+  mdg_status r = check_ready(h, true);
   if (r) return r;
   if (n != h->n || (n > 0 && !ids)) return fail(h, MDG_ERR_INVALID_ARGUMENT, "bad ids buffer");
   if (n == 0) return MDG_OK;
@@ -1314,6 +1351,7 @@ mdg_status mdg_langevin(mdg_handle *h) {
 mdg_status mdg_set_control(mdg_handle *h, int thermostat, double aimed_temperature, double heatbath_tau,
                            double heatbath_gamma) {
   if (!h || thermostat < MDG_NVE || thermostat > MDG_LANGEVIN) return MDG_ERR_INVALID_ARGUMENT;
+  h->seen_ok = false;
   if (thermostat != h->prm.thermostat || aimed_temperature != h->prm.aimed_temperature ||
       heatbath_tau != h->prm.heatbath_tau || heatbath_gamma != h->prm.heatbath_gamma) {
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
@@ -1329,6 +1367,7 @@ mdg_status mdg_set_control(mdg_handle *h, int thermostat, double aimed_temperatu
 
 mdg_status mdg_set_external(mdg_handle *h, const mdg_external *x) {
   if (!h) return MDG_ERR_INVALID_ARGUMENT;
+  h->seen_ok = false;
   External e{};
   if (x && x->kind != MDG_EXTERNAL_NONE) {
     if (x->kind < MDG_EXTERNAL_GRAVITY || x->kind > MDG_EXTERNAL_SHELL || x->axis < 0 || x->axis > 2 ||
@@ -1475,26 +1514,31 @@ mdg_status mdg_get_zeta(mdg_handle *h, double *zeta) {
 
 mdg_status mdg_set_zeta(mdg_handle *h, double zeta) {
   if (!h) return MDG_ERR_INVALID_ARGUMENT;
+  h->seen_ok = false;
   CUDA_TRY(h, cudaMemcpyAsync(&h->a.st->zeta, &zeta, sizeof(double), cudaMemcpyHostToDevice, h->stream));
   CUDA_TRY(h, cudaStreamSynchronize(h->stream));
   return MDG_OK;
 }
 
 mdg_status mdg_calculate(mdg_handle *h, int nsteps) {
-  mdg_status r = check_ready(h);
+  mdg_status r = check_ready(h, true);
   if (r) return r;
   if (nsteps < 0) return MDG_ERR_INVALID_ARGUMENT;
   if (h->n == 0 || nsteps == 0) return MDG_OK;
   CUDA_TRY(h, cudaSetDevice(h->prm.device));
   if ((r = autotune(h))) return r;
   Status st;
-  if ((r = read_status(h, &st))) return r;
+  bool known = h->seen_ok;
+  if (known) st = h->seen;
+  else if ((r = read_status(h, &st))) return r;
+  h->seen_ok = false;
   if (st.error) return translate_device_error(h, st);
   long long target = st.steps + nsteps;
   for (int attempt = 0; attempt < 8; attempt++) {
     long long left = target - st.steps;
     if (left <= 0) break;
-    if (fused_step(h) && h->fix_buf != 0) {
+    const bool eager = !h->use_graphs || (left < kStepsPerGraph && !use_persistent(h));
+    if (fused_step(h) && (h->fix_buf < 0 || (h->fix_buf != 0 && !eager))) {
       // the graph's first step reads buffer 0
       k_pack_half<kBlock><<<blocks_for(h->n, kBlock), kBlock, 0, h->stream>>>(h->a, h->box, h->n, h->a.qfix, h->a.pz);
       h->kernel_launches++;
@@ -1507,6 +1551,7 @@ mdg_status mdg_calculate(mdg_handle *h, int nsteps) {
     if (h->use_graphs && left >= kStepsPerGraph && h->graph_dirty) {
       if ((r = build_graph(h))) return r;
     }
+    if (!eager) known = false;  // st is the status before the steps below
     while (h->use_graphs && left >= kStepsPerGraph) {
       CUDA_TRY(h, cudaGraphLaunch(h->exec, h->stream));
       h->kernel_launches += h->graph_kernel_count;
@@ -1522,7 +1567,8 @@ mdg_status mdg_calculate(mdg_handle *h, int nsteps) {
       }
     }
     while (left > 0) {
-      if ((r = step_eager(h))) return r;
+      if ((r = step_eager(h, known && quiet_step(h, st)))) return r;
+      known = false;  // st is the status before this step
       left--;
     }
     if ((r = read_status(h, &st))) return r;
@@ -1540,6 +1586,8 @@ mdg_status mdg_calculate(mdg_handle *h, int nsteps) {
   // after a full step the reference's ghost copies date from the first half
   // drift; the Langevin branch has no second drift (src/mdmanager.cc:289-315)
   h->obs_lag = h->prm.thermostat == MDG_LANGEVIN ? 0.0 : 0.5 * h->prm.time_step;
+  h->seen = st;
+  h->seen_ok = true;
   return MDG_OK;
 }
 
@@ -1559,7 +1607,7 @@ mdg_status mdg_forces(mdg_handle *h, double *f4) {
 }
 
 mdg_status mdg_observe(mdg_handle *h, double *ke, double *pe, double *virial) {
-  mdg_status r = check_ready(h);
+  mdg_status r = check_ready(h, true);
   if (r) return r;
   double out[3] = {0.0, 0.0, 0.0};
   if (h->n > 0) {
@@ -1573,8 +1621,9 @@ mdg_status mdg_observe(mdg_handle *h, double *ke, double *pe, double *virial) {
     }
     k_final_sum<256, 3><<<1, 256, 0, h->stream>>>(h->a.partials, nb, h->d_sums);
     CUDA_TRY(h, cudaGetLastError());
-    CUDA_TRY(h, cudaMemcpyAsync(out, h->d_sums, sizeof out, cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(h, cudaMemcpyAsync(h->pin->sums, h->d_sums, sizeof out, cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    memcpy(out, h->pin->sums, sizeof out);
   }
   if (ke) *ke = out[0];
   if (pe) *pe = out[1];
@@ -1788,6 +1837,7 @@ mdg_status mdg_save_checkpoint(mdg_handle *h, const char *path) {
 
 mdg_status mdg_load_checkpoint(mdg_handle *h, const char *path) {
   if (!h || !path) return MDG_ERR_INVALID_ARGUMENT;
+  h->seen_ok = false;
   std::ifstream f(path, std::ios::binary);
   if (!f) return fail(h, MDG_ERR_IO, std::string("cannot read ") + path);
   CkptHeader hd{};

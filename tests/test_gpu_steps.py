@@ -46,3 +46,41 @@ def test_few_replicas_equal_many(precision):
     for other in out[1:]:
         for (q, v), (q1, v1) in zip(out[0], other):
             assert np.array_equal(q, q1) and np.array_equal(v, v1)
+
+
+@pytest.mark.parametrize("precision", [M.FP64, M.FP32_MIXED])
+def test_single_steps_between_other_calls(precision):
+    # the status kept from the last step is dropped by whatever may change it:
+    # the same calls with it dropped before every step (set_control drops it)
+    w = W.fcc_liquid(6, 0.7, 1.0, seed=4, jitter=0.05, rc=2.5, dt=0.005)
+    out = []
+    for drop in (False, True):
+        s = M.System(w.L, cutoff=2.5, time_step=0.005, capacity=w.n, precision=precision)
+        sums = []
+
+        def steps(n, s=s, sums=sums, drop=drop):
+            for _ in range(n):
+                if drop:
+                    s.set_control(M.NVE)
+                s.calculate(1)
+                sums.append(s.observe())
+
+        s.set_state(w.q, w.v)
+        steps(12)
+        q, v = s.state_by_id()
+        s.set_state(q, 3.0 * v)  # faster atoms, a stale list
+        steps(9)
+        s.make_pairlist()
+        steps(3)
+        s.set_external(kind=M.EXTERNAL_GRAVITY, axis=1, strength=0.3, time_step=0.005)
+        steps(5)
+        s.set_external()
+        s.calculate(21)
+        steps(8)
+        s.change_scale(1.01)
+        steps(6)
+        info = s.info()
+        out.append((sums, *s.state_by_id(), info["steps"], info["rebuilds"], info["displacement_checks"]))
+        s.close()
+    a, b = out
+    assert a[0] == b[0] and np.array_equal(a[1], b[1]) and np.array_equal(a[2], b[2]) and a[3:] == b[3:]
