@@ -94,6 +94,11 @@ struct Vec {
   }
 };
 
+// A grid barrier's arrivals and generation (meet).
+struct Meeting {
+  unsigned count, gen;
+};
+
 // The cell grid and the Verlet list.  Row of atom i: nbr[i * maxnb + k], the
 // end of bucket b at ends[i * kBuckets + b].
 struct List {
@@ -107,7 +112,7 @@ struct List {
   unsigned short *ends;
   Vec qb;                                     // positions at the last build
   int *overflow, *timeout;
-  mdg::GridBarrier *bar;
+  Meeting *bar;
 };
 
 __device__ __forceinline__ double3 axpy(double h, const double3 &v, const double3 &q) {
@@ -978,7 +983,7 @@ mdg_status mdg_adjoint_run(const mdg_adjoint_params *prm, const double *q0, cons
   l.overflow = R.state;
   l.timeout = R.state + 1;
   l.cursor = R.state + 2;
-  l.bar = reinterpret_cast<mdg::GridBarrier *>(R.state + 4);
+  l.bar = reinterpret_cast<Meeting *>(R.state + 4);
   R.note(cudaMemsetAsync(R.flags, 0, sizeof(int) * nflags, R.s));
   R.note(cudaMemsetAsync(R.state, 0, sizeof(int) * 8, R.s));
   R.note(cudaMemsetAsync(l.qb.p, 0, sizeof(double) * 3 * R.ns, R.s));

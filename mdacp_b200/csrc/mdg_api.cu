@@ -129,6 +129,7 @@ struct mdg_handle {
   int *d_pout = nullptr;              // persistent pass: block 0's decisions
   int64_t persistent_steps = 0;
   int persist_grid = -1;              // blocks of the persistent pass (-1: not computed yet)
+  bool persist_deep = false;          // its threads cover every atom's lanes (k_nve_persistent, DEEP)
   double steps_per_cycle = 4.0;       // persistent pipeline: steps per queued launch pair, as last seen
   External ext{};                     // executor applied after every step (kind 0: none)
   // snapshots: one set of pinned buffers per handle, at most one pending writer
@@ -828,28 +829,38 @@ mdg_status autotune(mdg_handle *h) {
 // Blocks of the persistent pass for this handle: enough for every atom's
 // lanes, at most what the device keeps resident at once (a cooperative
 // launch needs all of them resident); 0 if the kernel cannot be resident.
-template <int TPA>
-int persistent_grid_of(mdg_handle *h) {
-  int per_sm = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nve_persistent<kPersistBlock, TPA>, kPersistBlock, 0) !=
-          cudaSuccess ||
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->prm.device) != cudaSuccess)
+template <int TPA, bool DEEP>
+int persistent_grid_of(const mdg_handle *h) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_nve_persistent<kPersistBlock, TPA, DEEP>, kPersistBlock,
+                                                    0) != cudaSuccess)
     return 0;
   const long long need = ((long long)h->n * TPA + kPersistBlock - 1) / kPersistBlock;
-  return (int)std::min<long long>(need, (long long)per_sm * sms);
+  return (int)std::min<long long>(need, (long long)per_sm * h->sms);
+}
+
+template <int TPA>
+void persistent_shape(mdg_handle *h) {
+  h->persist_grid = persistent_grid_of<TPA, true>(h);
+  h->persist_deep = (long long)h->persist_grid * kPersistBlock >= (long long)h->n * TPA;
+  if (!h->persist_deep) h->persist_grid = persistent_grid_of<TPA, false>(h);
 }
 
 // Lanes per atom of the persistent pass.  Its steps end in a grid barrier
-// whose cost grows with the block count, so it takes fewer lanes than the
-// graph path's tuned force pass: one per atom from 16,384 atoms (measured
-// on the 32,000-atom liquid: 31 us per step with one lane, 35-40 with two),
-// more for smaller systems.  Every lane count gives the same forces.
-int persistent_tpa(const mdg_handle *h) { return h->n >= 16384 ? 1 : (h->n >= 8192 ? 2 : 4); }
+// whose cost grows with the block count, and more lanes walk more masked
+// entries, so it takes fewer lanes than the graph path's tuned force pass.  us
+// per step, rebuilds included, with 1, 2 and 4 lanes: 2,048 atoms 19.7, 16.0,
+// 14.8; 8,788 atoms 19.3, 16.5, 16.6; 19,652 atoms 21.2, 20.2, 25.6; 23,328
+// atoms 22.7, 21.4, 26.3 (at half the density 21.2, 21.3, 28.0); 32,000 atoms
+// 23.7, 26.2, 32.8.  Every lane count gives the same forces.
+int persistent_tpa(const mdg_handle *h) { return h->n >= 24000 ? 1 : (h->n >= 8192 ? 2 : 4); }
 
 int persistent_grid(mdg_handle *h) {
   if (h->persist_grid < 0) {
     const int tpa = persistent_tpa(h);
-    h->persist_grid = tpa == 4 ? persistent_grid_of<4>(h) : (tpa == 2 ? persistent_grid_of<2>(h) : persistent_grid_of<1>(h));
+    if (tpa == 4) persistent_shape<4>(h);
+    else if (tpa == 2) persistent_shape<2>(h);
+    else persistent_shape<1>(h);
   }
   return h->persist_grid;
 }
@@ -879,8 +890,9 @@ mdg_status enqueue_persistent_tpa(mdg_handle *h) {
   int4 *q0 = h->a.qfix, *q1 = h->a.qfix2;
   double lag = step_lag(h);  // the ghost copies' age at a step's displacement check
   void *args[] = {&h->a, &h->box, &n, &q0, &q1, &lag, &h->d_bar};
-  CUDA_TRY(h, cudaLaunchCooperativeKernel((const void *)k_nve_persistent<kPersistBlock, TPA>, dim3(grid),
-                                          dim3(kPersistBlock), args, 0, h->stream));
+  const void *kernel = h->persist_deep ? (const void *)k_nve_persistent<kPersistBlock, TPA, true>
+                                       : (const void *)k_nve_persistent<kPersistBlock, TPA, false>;
+  CUDA_TRY(h, cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kPersistBlock), args, 0, h->stream));
   h->kernel_launches++;
   return MDG_OK;
 }

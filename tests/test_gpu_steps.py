@@ -84,3 +84,22 @@ def test_single_steps_between_other_calls(precision):
         s.close()
     a, b = out
     assert a[0] == b[0] and np.array_equal(a[1], b[1]) and np.array_equal(a[2], b[2]) and a[3:] == b[3:]
+
+
+# lanes per atom change at 8,192 and 24,000 atoms; 148 multiprocessors hold
+# the lanes of 75,776 atoms with the row's head in registers
+@pytest.mark.parametrize("n", [2, 33, 257, 8191, 8192, 23999, 24000, 75776, 75777])
+def test_persistent_steps_equal_graphs_at_the_edges(n):
+    w = W.fcc_liquid(max(5, int(np.ceil((n / 3.6) ** (1 / 3)))), 0.7, 1.0, seed=n, jitter=0.05, rc=2.5, dt=0.005)
+    keep = np.sort(np.random.Generator(np.random.Philox(n)).permutation(w.n)[:n])
+    out = []
+    for mode in (1, 2):  # graphs, persistent
+        s = M.System(w.L, cutoff=2.5, time_step=0.005, capacity=n, precision=M.FP32_MIXED, step_mode=mode)
+        s.set_state(w.q[keep], w.v[keep])
+        s.calculate(45)
+        info = s.info()
+        out.append((*s.state_by_id(), info["rebuilds"], info["displacement_checks"], info["persistent_steps"]))
+        s.close()
+    a, b = out
+    assert a[4] == 0 and b[4] > 0
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1]) and a[2:4] == b[2:4]
