@@ -439,8 +439,8 @@ mdg_status mdg_external_state(mdg_handle *h, double *position, double *impulse);
  * [PE + sum over pairs g((r-lo)/w) g((hi-r)/w)], g the logistic function.
  * Pairs come from a Verlet list of search length cutoff + 0.3 sigma (less in
  * boxes narrower than three such lengths), rebuilt when an atom has moved
- * half the skin; its rows are in ascending partner order, so the sums are a
- * function of the positions alone (and of threads_per_atom). */
+ * half the skin; its rows are in an order of the partner indices alone, so the
+ * sums are a function of the positions (and of threads_per_atom). */
 typedef struct mdg_adjoint_params {
   double L[3];
   double cutoff;          /* in units of sigma (CUTOFF_LENGTH, include/mdconfig.h:31) */

@@ -5,8 +5,9 @@
 // (box, cell grid, cell and atom offsets), and skin budgets, displacement
 // checks and pairlist rebuilds are per replica -- a rebuild pass only
 // touches the replicas whose lists expired.  Steps are captured in CUDA
-// graphs with IF conditional nodes on "some replica needs a displacement
-// check / a rebuild", exactly like the single-system handle.
+// graphs; with few replicas the check and the rebuild are conditional
+// branches ("some replica needs one"), as in the single-system handle, with
+// many they run every step over work lists that may be empty (kEAlways).
 //
 // The arithmetic of every kernel is the single-system kernels' (shared
 // device helpers from mdg_device.cuh), and rows are built in the same order,
@@ -677,10 +678,11 @@ __global__ void __launch_bounds__(kEF) ke_force_fp32(Ens e, const int4 *qf, int4
     const Rep &rep = e.rep[r];
     const PairConst k = pair_const(rep.fix_scale, e.rc2f, e.c2x8f);
     if (TPA == 1) {
+      // 338 us for 256 replicas of 2.6M atoms; through the groups below 378
       fp32_row_global(e.nbr, e.stride, qf, i, qf[i], (e.nnbr[i] + 3) & ~3, k, Fx, Fy, Fz);
     } else {
       // positions not loaded a group ahead: at 64 registers this pass is
-      // faster without (0.324 vs 0.353 ms on the 256-replica ensemble)
+      // faster without
       GlobalGroups<false> f{e.nbr + i, e.stride, qf, i};
       fp32_row<TPA>(f, (e.nnbr[i] + 3) >> 2, sub, qf[i], k, Fx, Fy, Fz);
     }
