@@ -499,6 +499,24 @@ __global__ void __launch_bounds__(BLOCK) k_disp_max(Arrays a, Box b, int n, doub
   block_max_to<BLOCK>(&a.st->dr2max_bits, d2);
 }
 
+// Files atom i's copies that moved further than sqrt(c_d2) as candidates
+// (slot, image code): counted first, so that an atom waits for one atomic
+// instead of one per copy (24 replicas' collection 8.9 -> 5.3 us, 256
+// replicas' 23 -> 18).  weighted counts them all, stored those with a
+// place offered.
+__device__ __forceinline__ void collect_copies(const CopyView &cv, const double L[3], int i, double lag, double c_d2,
+                                               int *weighted, int *stored, int2 *cand, int cand_cap) {
+  unsigned long long codes = 0ull;  // 6 bits a copy, at most 8 copies
+  int k = 0;
+  for_each_copy(cv, L, i, lag, [&](int code, double d2) {
+    if (d2 > c_d2) codes |= (unsigned long long)code << (6 * k++);
+  });
+  if (k == 0) return;
+  atomicAdd(weighted, k);
+  const int at = atomicAdd(stored, k);
+  for (int u = 0; u < k && at + u < cand_cap; u++, codes >>= 6) cand[at + u] = make_int2(i, (int)(codes & 63ull));
+}
+
 // Second pass: copies that moved more than BufferLength - sqrt(dr2_max)
 // (src/pairlist.cc:86-97); each is stored as (slot, image code).
 template <int BLOCK>
@@ -513,13 +531,7 @@ __global__ void __launch_bounds__(BLOCK) k_disp_collect(Arrays a, Box b, int n, 
   // a full list: the number of copies has decided (k_disp_pairs; over several
   // slabs too), and thousands of atomics to one address would follow
   if (*(volatile const int *)&a.st->cand_weighted >= cand_cap) return;
-  for_each_copy(copy_view(a), b.L, i, lag, [&](int code, double d2) {
-    if (d2 > c_d2) {
-      atomicAdd(&a.st->cand_weighted, 1);
-      const int k = atomicAdd(&a.st->cand_n, 1);
-      if (k < cand_cap) a.cand[k] = make_int2(i, code);
-    }
-  });
+  collect_copies(copy_view(a), b.L, i, lag, c_d2, &a.st->cand_weighted, &a.st->cand_n, a.cand, cand_cap);
 }
 
 // Candidate copies staged in shared memory for the pair test: old and
@@ -3104,13 +3116,8 @@ __global__ void __launch_bounds__(BLOCK, DEEP ? 512 / BLOCK : 0) k_nve_persisten
       if (lead) bar->dr2[(checks + 1) & 1] = 0ull;
       if (dr2max > c_d2) {
         for (int i = gtid; i < n; i += gthreads)
-          for_each_copy(copy_view(a), b.L, i, lag, [&](int code, double x) {
-            if (x > c_d2) {
-              atomicAdd(&st->cand_weighted, 1);
-              const int kk = atomicAdd(&st->cand_n, 1);
-              if (kk < b.check_list_length) a.cand[kk] = make_int2(i, code);
-            }
-          });
+          collect_copies(copy_view(a), b.L, i, lag, c_d2, &st->cand_weighted, &st->cand_n, a.cand,
+                         b.check_list_length);
         if (!grid_barrier(bar, st, kBarrierPolls, goal)) break;
         if (threadIdx.x == 0) found = 0;
         __syncthreads();

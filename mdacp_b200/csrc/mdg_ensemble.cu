@@ -338,13 +338,8 @@ __global__ void __launch_bounds__(kEB) ke_disp_collect(Ens e) {
     if (!(e.disp2[i] > c_d2)) continue;
     // a full list: the number of copies has decided (k_disp_collect)
     if (*(volatile const int *)&st.cand_weighted >= e.cll) continue;
-    for_each_copy(ens_view(e), e.rep[r].L, i, e.lag, [&](int code, double d2) {
-      if (d2 > c_d2) {
-        atomicAdd(&st.cand_weighted, 1);
-        const int k = atomicAdd(&st.cand_n, 1);
-        if (k < e.cll) e.cand[(size_t)r * e.cll + k] = make_int2(i, code);
-      }
-    });
+    collect_copies(ens_view(e), e.rep[r].L, i, e.lag, c_d2, &st.cand_weighted, &st.cand_n,
+                   e.cand + (size_t)r * e.cll, e.cll);
   }
 }
 
