@@ -461,8 +461,10 @@ void mdg_adjoint_default_params(mdg_adjoint_params *p);
  * 4 B per row entry, rows of up to 1024 entries) is kept per device after
  * the call and reused by later calls whose buffers fit, so repeated calls of
  * one shape allocate nothing; one run at a time per process.
- * MDG_ERR_CAPACITY if a row outgrows its capacity (three times the mean
- * density's count within the search length, plus 64). */
+ * MDG_ERR_CAPACITY if a row outgrows its capacity (the larger of twice the
+ * mean density's count within the search length plus 64 and the count at
+ * density 1.3 sigma^-3 plus 32, at most 1024); MDG_ERR_TIMEOUT if a bounded
+ * device wait inside a list rebuild ran out. */
 mdg_status mdg_adjoint_run(const mdg_adjoint_params *p, const double *q0, const double *v0, int n, double *loss,
                            double *dloss_deps, double *dloss_dsigma, double *dloss_dq0);
 /* Frees the device memory, stream and pinned buffer that mdg_adjoint_run
