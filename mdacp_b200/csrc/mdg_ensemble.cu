@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kEF) ke_force_fp32(Ens e, const int4 *qf, int4
   rep_max(&e.rs[0].vmax2_bits, sizeof(RepStatus), r, v2, active);  // v2 = 0 on lanes other than 0
 }
 
-// Whether some partner of an atom sits beyond a face of its replica (row_wraps).
+// Whether some partner of an atom sat beyond a face of its replica at the build (row_wraps).
 __device__ __forceinline__ bool ens_wraps(const Ens &e, const Rep &rep, int i) {
   return rep.small || row_wraps(rep.ms, 0, e.cxyz[i]);
 }
@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(kEF, kFp64Blocks) ke_force_fp64(Ens e, PosSpli
   const int ii = i < e.ntot ? i : 0;
   const int r = e.rep_of[ii];
   const Rep &rep = e.rep[r];
-  const Fp64Pair f{rep.L, rep.hL, e.rc2, e.c2 * 8.0, e.dt, pos.at(ii)};
+  const Fp64Pair f{edges_of(rep.L, rep.hL), e.rc2, e.c2 * 8.0, e.dt, pos.at(ii)};
   double s[3];
   fp64_force_row<TPA>(pos, e.nbr, e.stride, active ? e.nnbr[ii] : 0, ii, sub, f, active && ens_wraps(e, rep, ii), s);
   if (active && sub == 0) v2 = finish_step(e, rep, i, s[0], s[1], s[2], next, next_z);
@@ -734,18 +734,20 @@ __global__ void __launch_bounds__(kEF, kFp64Blocks) ke_observe(Ens e) {
   const int ii = active ? i : 0;
   const int r = e.rep_of[ii];
   const Rep &rep = e.rep[r];
-  const double4 qi = e.q[ii];
+  const PosState pos{e.q};
+  const double3 qi = pos.at(ii);
+  const Edges box = edges_of(rep.L, rep.hL);
   const int nn = active ? e.nnbr[ii] : 0;
   double s[2];
   if (__any_sync(0xffffffffu, (int)(active && ens_wraps(e, rep, ii))))
-    fp64_row<TPA>(PosState{e.q}, e.nbr, e.stride, nn, ii, sub, s,
+    fp64_row<TPA>(pos, e.nbr, e.stride, nn, ii, sub, s,
                   [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[2]) {
-                    observe_pairs<true>(rep.L, rep.hL, e.rc2, e.c0, e.c2, qi, p, in, u);
+                    observe_pairs<true>(box, e.rc2, e.c0, e.c2, qi, p, in, u);
                   });
   else
-    fp64_row<TPA>(PosState{e.q}, e.nbr, e.stride, nn, ii, sub, s,
+    fp64_row<TPA>(pos, e.nbr, e.stride, nn, ii, sub, s,
                   [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[2]) {
-                    observe_pairs<false>(rep.L, rep.hL, e.rc2, e.c0, e.c2, qi, p, in, u);
+                    observe_pairs<false>(box, e.rc2, e.c0, e.c2, qi, p, in, u);
                   });
   const bool first = active && sub == 0;
   const double4 v = e.v[ii];
@@ -764,11 +766,13 @@ __global__ void __launch_bounds__(kEF, kFp64Blocks) ke_count_pairs(Ens e, unsign
   const bool active = i < e.ntot;
   const int ii = active ? i : 0;
   const Rep &rep = e.rep[e.rep_of[ii]];
-  const double4 qi = e.q[ii];
+  const PosState pos{e.q};
+  const double3 qi = pos.at(ii);
+  const Edges box = edges_of(rep.L, rep.hL);
   double s[1];
-  fp64_row<TPA>(PosState{e.q}, e.nbr, e.stride, active ? e.nnbr[ii] : 0, ii, sub, s,
+  fp64_row<TPA>(pos, e.nbr, e.stride, active ? e.nnbr[ii] : 0, ii, sub, s,
                 [&](const double3 (&p)[2], const int (&)[2], const bool (&in)[2], double (&u)[1]) {
-                  count_pairs<true>(rep.L, rep.hL, e.rc2, qi, p, in, u);
+                  count_pairs<true>(box, e.rc2, qi, p, in, u);
                 });
   const int w = __reduce_add_sync(0xffffffffu, sub == 0 ? (int)s[0] : 0);
   if ((threadIdx.x & 31) == 0 && w) atomicAdd(count, (unsigned long long)w);
