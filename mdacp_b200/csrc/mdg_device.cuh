@@ -2450,13 +2450,21 @@ __device__ __forceinline__ void fp32_finish(Arrays &a, const Box &b, const Therm
 // order, so every lane holds S at the end.  Chunks past the row's end add
 // +0.0, which leaves S unchanged (S starts at +0.0 and is never -0.0).
 
+// A packed position.  LIVE: the copy changes while the kernel runs (the
+// persistent pass), so the load is an ordinary one: the read-only path promises
+// nothing for such data, and the compiler may move its loads across a barrier.
+template <bool LIVE>
+__device__ __forceinline__ int4 packed_at(const int4 *qf, int i) {
+  return LIVE ? qf[i] : __ldg(qf + i);
+}
+
 // Partner positions of a lane's groups from the global fixed-point copy.
 // The list entries of the group after the next are in flight while a group
 // is summed (the list is the pass's one stream from HBM); with AHEAD the
 // next group's positions are too (software pipeline: the gathers are the
 // pass's long-latency loads; four more int4 registers).  Group -1 is none:
 // its entries are the atom itself.
-template <bool AHEAD = true>
+template <bool AHEAD = true, bool LIVE = false>
 struct GlobalGroups {
   const int *row;  // nbr + atom
   int st;          // list stride
@@ -2480,10 +2488,10 @@ struct GlobalGroups {
   __device__ __forceinline__ void start(int ga, int gb) {
     load(ga, n0, n1, n2, n3);
     if (AHEAD) {
-      c0 = __ldg(qf + n0);
-      c1 = __ldg(qf + n1);
-      c2 = __ldg(qf + n2);
-      c3 = __ldg(qf + n3);
+      c0 = packed_at<LIVE>(qf, n0);
+      c1 = packed_at<LIVE>(qf, n1);
+      c2 = packed_at<LIVE>(qf, n2);
+      c3 = packed_at<LIVE>(qf, n3);
     }
     load(gb, m0, m1, m2, m3);
   }
@@ -2495,15 +2503,15 @@ struct GlobalGroups {
       p1 = c1;
       p2 = c2;
       p3 = c3;
-      c0 = __ldg(qf + m0);
-      c1 = __ldg(qf + m1);
-      c2 = __ldg(qf + m2);
-      c3 = __ldg(qf + m3);
+      c0 = packed_at<LIVE>(qf, m0);
+      c1 = packed_at<LIVE>(qf, m1);
+      c2 = packed_at<LIVE>(qf, m2);
+      c3 = packed_at<LIVE>(qf, m3);
     } else {
-      p0 = __ldg(qf + n0);
-      p1 = __ldg(qf + n1);
-      p2 = __ldg(qf + n2);
-      p3 = __ldg(qf + n3);
+      p0 = packed_at<LIVE>(qf, n0);
+      p1 = packed_at<LIVE>(qf, n1);
+      p2 = packed_at<LIVE>(qf, n2);
+      p3 = packed_at<LIVE>(qf, n3);
       n0 = m0;
       n1 = m1;
       n2 = m2;
@@ -3000,7 +3008,7 @@ __device__ __forceinline__ void fp32_row_deep(const Arrays &a, const int4 *qf, i
   int e[8];
 #pragma unroll
   for (int u = 0; u < 8; u++) {
-    p[u] = __ldg(qf + h.first[u]);
+    p[u] = packed_at<true>(qf, h.first[u]);
     e[u] = h.second[u];
   }
   Fx = Fy = Fz = 0.0;
@@ -3008,7 +3016,7 @@ __device__ __forceinline__ void fp32_row_deep(const Arrays &a, const int4 *qf, i
   for (int r = 0; r < rounds; r++) {
     int4 pn[8];
 #pragma unroll
-    for (int u = 0; u < 8; u++) pn[u] = __ldg(qf + e[u]);
+    for (int u = 0; u < 8; u++) pn[u] = packed_at<true>(qf, e[u]);
     row_chunk<TPA>(a, i, h.groups, sub + (r + 2) * TPA, e);
     float fx = 0.f, fy = 0.f, fz = 0.f;
 #pragma unroll
@@ -3222,7 +3230,7 @@ __global__ void __launch_bounds__(BLOCK, DEEP ? 512 / BLOCK : 0) k_nve_persisten
         if (t < nthreads && !err) {
           const int4 pi = qf[i];
           double Fx, Fy, Fz;
-          GlobalGroups<> f{a.nbr + i, a.stride, qf, i};
+          GlobalGroups<true, true> f{a.nbr + i, a.stride, qf, i};
           fp32_row<TPA>(f, (a.nnbr[i] + 3) >> 2, sub, pi, k, Fx, Fy, Fz);
           if (sub == 0) fp32_finish<kKick, 2>(a, b, th, i, Fx, Fy, Fz, qf_next, v2, ke);
         }
