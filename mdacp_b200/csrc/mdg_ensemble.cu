@@ -857,7 +857,7 @@ void e_free(mdg_ensemble *x) {
   x->exec = nullptr;
 }
 
-int lane_blocks(int n, int lanes) { return (int)(((long long)n * lanes + kEF - 1) / kEF); }
+int lane_blocks(int n, int lanes) { return (int)std::max(1LL, ((long long)n * lanes + kEF - 1) / kEF); }
 
 int4 *e_pack(const Ens &e, int k) { return k ? e.qfix2 : e.qfix; }
 double *e_pack_z(const Ens &e, int k) { return k ? e.pz2 : e.pz; }
