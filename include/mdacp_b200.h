@@ -302,7 +302,8 @@ mdg_status mdg_ensemble_set_kernel_timing(mdg_ensemble *e, int on);
 mdg_status mdg_ensemble_kernel_time(mdg_ensemble *e, double *force_ms, int64_t *force_launches,
                                     int64_t *kernel_launches);
 /* Over all replicas: neighbour-list entries of the current lists and the
-   unordered pairs closer than the cut-off at the current positions. */
+   unordered pairs closer than the cut-off at the current positions.  Lists
+   that an upload made stale are built first, as mdg_ensemble_observe does. */
 mdg_status mdg_ensemble_list_stats(mdg_ensemble *e, int64_t *list_entries, int64_t *pairs_within_cutoff);
 void *mdg_ensemble_stream(mdg_ensemble *e);
 

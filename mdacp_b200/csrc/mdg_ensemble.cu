@@ -1146,6 +1146,34 @@ mdg_status e_mark_all_stale(mdg_ensemble *x) {
   return MDG_OK;
 }
 
+// Builds the stale lists (fresh upload): observers and counts walk the rows.
+// *st (may be null) gets every replica's status.
+mdg_status e_current_lists(mdg_ensemble *x, std::vector<RepStatus> *st = nullptr) {
+  Ens &e = x->e;
+  std::vector<RepStatus> rs;
+  int err = 0;
+  mdg_status r = e_status(x, &err, &rs);
+  if (r) return r;
+  if (err) return e_translate(err);
+  bool stale = false;
+  for (auto &s : rs) stale |= s.list_stale != 0;
+  if (stale) {
+    for (auto &s : rs) {
+      s.want_build = s.list_stale;
+      s.disp = 0;
+    }
+    ECUDA(cudaMemcpyAsync(e.rs, rs.data(), sizeof(RepStatus) * e.nrep, cudaMemcpyHostToDevice, x->stream));
+    x->fix_buf = -1;  // the rebuild renumbers the atoms
+    ke_disp_pairs<<<dim3(e.nrep, kEPairParts), 256, 0, x->stream>>>(e);  // clears their cells
+    ke_decide<<<1, 1024, 0, x->stream>>>(e, 0, kVerdictNone, nullptr);
+    e_launch_build(x, x->stream, -1);
+    if ((r = e_status(x, &err, &rs))) return r;
+    if (err) return e_translate(err);
+  }
+  if (st) *st = std::move(rs);
+  return MDG_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1460,27 +1488,8 @@ mdg_status mdg_ensemble_calculate(mdg_ensemble *x, int nsteps) {
 mdg_status mdg_ensemble_observe(mdg_ensemble *x, double *ke, double *pe, double *virial) {
   if (!x || !x->state_set) return MDG_ERR_STATE;
   Ens &e = x->e;
-  // a stale list (fresh upload) is built first
-  std::vector<RepStatus> rs;
-  int err = 0;
-  mdg_status r = e_status(x, &err, &rs);
+  mdg_status r = e_current_lists(x);
   if (r) return r;
-  if (err) return e_translate(err);
-  bool stale = false;
-  for (auto &s : rs) stale |= s.list_stale != 0;
-  if (stale) {
-    for (auto &s : rs) {
-      s.want_build = s.list_stale;
-      s.disp = 0;
-    }
-    ECUDA(cudaMemcpyAsync(e.rs, rs.data(), sizeof(RepStatus) * e.nrep, cudaMemcpyHostToDevice, x->stream));
-    x->fix_buf = -1;  // the rebuild renumbers the atoms
-    ke_disp_pairs<<<dim3(e.nrep, kEPairParts), 256, 0, x->stream>>>(e);  // clears their cells
-    ke_decide<<<1, 1024, 0, x->stream>>>(e, 0, kVerdictNone, nullptr);
-    e_launch_build(x, x->stream, -1);
-    if ((r = e_status(x, &err, &rs))) return r;
-    if (err) return e_translate(err);
-  }
   ECUDA(cudaMemsetAsync(e.sums, 0, sizeof(double) * 3 * e.nrep, x->stream));
   const int lanes = fp64_lanes(e.ntot), blocks = lane_blocks(e.ntot, lanes);
   if (lanes == 8) ke_observe<8><<<blocks, kEF, 0, x->stream>>>(e);
@@ -1535,10 +1544,8 @@ mdg_status mdg_ensemble_list_stats(mdg_ensemble *x, int64_t *list_entries, int64
   if (!x || !x->state_set) return MDG_ERR_STATE;
   Ens &e = x->e;
   std::vector<RepStatus> rs;
-  int err = 0;
-  mdg_status r = e_status(x, &err, &rs);
+  mdg_status r = e_current_lists(x, &rs);
   if (r) return r;
-  if (err) return e_translate(err);
   long long entries = 0;
   for (auto &st : rs) entries += st.list_entries;
   if (list_entries) *list_entries = entries;
