@@ -1163,7 +1163,7 @@ __device__ __forceinline__ int build_rows(const Box &b, const float4 *__restrict
                                           const double4 *__restrict__ q, const unsigned char *__restrict__ mult,
                                           const int *__restrict__ tab, int pc, int i, Emit &emit) {
   const float4 li = qloc[i];
-  const int cx = pc & 2047, cy = (pc >> 11) & 2047, cz = pc >> 22;
+  const int cx = pc & 2047, cy = (pc >> 11) & 2047, cz = (int)((unsigned)pc >> 22);  // layers from 512 on use the sign bit
   const int ms0 = b.ms[0], ms1 = b.ms[1], ms2 = b.ms[2];
   const float hi = b.sl2_hi;
   const int mx = ms0 * kXSub;
