@@ -290,9 +290,14 @@ void launch_list_build_block(mdg_handle *h, cudaStream_t s, int lanes) {
   else k_build<BLOCK, false, false, 1><<<nb, BLOCK, 0, s>>>(h->a, h->box, n);
 }
 
+// Warps that share 32 atoms' rows when each atom has one lane.
+int list_split(const mdg_handle *h) {
+  return build_split(h->n, h->sms, (double)h->n / h->ncell, (double)h->n / (h->box.ms[1] * h->box.ms[2]));
+}
+
 // Few atoms with one lane each: the split walk, whatever the block size.
 void launch_list_build(mdg_handle *h, cudaStream_t s, int block, int lanes) {
-  const int split = lanes == 1 ? build_split(h->n, h->sms) : 1;
+  const int split = lanes == 1 ? list_split(h) : 1;
   if (split == 9) {
     k_build_split<9><<<blocks_for(h->n, 32), 9 * 32, 0, s>>>(h->a, h->box, h->n);
     return;

@@ -1284,6 +1284,107 @@ static __device__ __noinline__ bool band_test_row(const RowGeom &g, const double
   return within_search_exact(qi, qj, shift_of(xc, 0, g.L), shift_of(yz, 1, g.L), shift_of(yz, 2, g.L), g.sl2);
 }
 
+// Entries of atom i's row from runs [first, last) of the nine, walked by one lane
+// (rows as build_rows', entry for entry); filed from entry cnt on, or only
+// counted (nbr null).  Returns the next entry.  For atoms that lie thin: see
+// build_rows_warp.
+template <bool SLAB>
+__device__ __forceinline__ int walk_own_runs(const RowGeom &g, const float4 *__restrict__ qloc,
+                                          const double4 *__restrict__ q, const int *__restrict__ tab, int pc, int i,
+                                          int first, int last, int cnt, int *__restrict__ nbr, int stride, int maxnb) {
+  const float4 li = qloc[i];
+  const int cx = pc & 2047, cy = (pc >> 11) & 2047, lz = (int)((unsigned)pc >> 22);
+  const int cz = SLAB ? g.z0 + lz : lz;
+  const int mx = g.ms[0] * kXSub, vbase = (cx - 1) * kXSub;
+  const double qx = q[i].x;
+  const double per_bin = kXSub / g.cs0;
+  const float ubin = (float)((qx - (cx - 1) * g.cs0) * per_bin), per_binf = (float)per_bin;
+#pragma unroll 1
+  for (int r = first; r < last; r++) {
+    const int dz = r / 3 - 1, dy = r % 3 - 1;
+    const float gz = dz == 0 ? 0.f : (dz < 0 ? li.z : g.csz - li.z);
+    const float gy = dy == 0 ? 0.f : (dy < 0 ? li.y : g.csy - li.y);
+    const float g2 = fmaf(gy, gy, gz * gz);
+    if (g2 > g.hi) continue;
+    const float reach = sqrt_approx(g.hi - g2) * per_binf;
+    const int lo = vbase + max((int)floorf(ubin - reach - 1e-3f), 0);
+    const int hi = vbase + min((int)floorf(ubin + reach + 1e-3f) + 1, 3 * kXSub);
+    int z = cz + dz, y = cy + dy, yz = 0;
+    if (z < 0) { z += g.ms[2]; yz = 1 << 4; } else if (z >= g.ms[2]) { z -= g.ms[2]; yz = 2 << 4; }
+    if (y < 0) { y += g.ms[1]; yz |= 1 << 2; } else if (y >= g.ms[1]) { y -= g.ms[1]; yz |= 2 << 2; }
+    int blk = z;
+    if (SLAB) {
+      const int nl = lz + dz;
+      blk = nl < 0 ? g.nzl : (nl >= g.nzl ? g.nzl + 1 : nl);
+    }
+    const int *xr = tab + (size_t)(blk * g.ms[1] + y) * (mx + 1);
+    const float byf = (float)dy * g.csy - li.y, bzf = (float)dz * g.csz - li.z;
+    // the run's pieces: through the -x face, inside the row, through the +x face
+#pragma unroll 1
+    for (int xc = lo < 0 ? 1 : 0; xc <= 2; xc = xc == 1 ? 0 : (xc == 0 && hi > mx ? 2 : 3)) {
+      const int b0 = xc == 1 ? lo + mx : (xc == 2 ? 0 : max(lo, 0));
+      const int b1 = xc == 1 ? mx : (xc == 2 ? hi - mx : min(hi, mx));
+      const int code = yz | xc, need = strips_of(code);
+      const float bx = (float)(shift_of(xc, 0, g.L) - qx);
+      const int end = xr[b1];
+      for (int j = xr[b0]; j < end; j++) {
+        const float4 l = __ldg(qloc + j);
+        const float ex = l.x + bx, ey = l.y + byf, ez = l.z + bzf;
+        const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+        if (r2 > g.hi || (__float_as_int(l.w) & need) != need || (j == i && code == 0)) continue;
+        if (r2 >= g.lo && !within_search_exact(q[i], q[j], shift_of(code, 0, g.L), shift_of(code, 1, g.L),
+                                               shift_of(code, 2, g.L), g.sl2))
+          continue;
+        if (nbr && cnt < maxnb) nbr[(size_t)cnt * stride + i] = j;
+        cnt++;
+      }
+    }
+  }
+  return cnt;
+}
+
+// Whether a warp's atoms lie thin: many x-rows of cells among them and few atoms
+// a cell that has any (the rule's figures: build_rows_warp); shared: the lanes
+// would walk their runs twice.  All lanes call.
+__device__ __forceinline__ bool rows_lie_thin(int owner, int pc, bool active, bool all_pairs, bool shared) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int key = active ? pc : -1;  // no packed cell is -1
+  const int before_key = __shfl_up_sync(kAll, key, 1), before_owner = __shfl_up_sync(kAll, owner, 1);
+  const bool first = (threadIdx.x & 31) == 0 || owner != before_owner;
+  const int atoms = __popc(__ballot_sync(kAll, active));
+  const int cells = __popc(__ballot_sync(kAll, active && (first || key != before_key)));
+  const int turns = __popc(__ballot_sync(kAll, active && (first || (unsigned)key >> 11 != (unsigned)before_key >> 11)));
+  const bool others = __any_sync(kAll, (int)all_pairs);
+  return !others && turns * (5 * cells + atoms) * 25 > (15 * cells + 27 * atoms) * (shared ? 8 : 5);
+}
+
+// build_rows_warp for atoms that lie thin.
+template <bool SLAB, int SPLIT>
+static __device__ __noinline__ int rows_alone(const RowGeom &g, const float4 *__restrict__ qloc,
+                                              const double4 *__restrict__ q, const int *__restrict__ tab, int pc, int i,
+                                              bool active, int (*counts)[32], int part, int *__restrict__ nbr, int stride,
+                                              int maxnb) {
+  const int lane = threadIdx.x & 31, first = part * (9 / SPLIT), last = first + 9 / SPLIT;
+  int cnt = 0;
+  for (int pass = SPLIT == 1 ? 1 : 0; pass < 2; pass++) {
+    // pass 0 counts, so that the entries of the parts have their places
+    const int at = cnt;
+    if (active) cnt = walk_own_runs<SLAB>(g, qloc, q, tab, pc, i, first, last, cnt, pass ? nbr : nullptr, stride, maxnb);
+    if (SPLIT > 1) {
+      if (pass == 0) {
+        counts[part][lane] = cnt - at;
+        __syncthreads();
+      }
+      cnt = 0;
+      for (int w = 0; w < (pass ? SPLIT : part); w++) cnt += counts[w][lane];
+    }
+  }
+  const bool mine = part == 0 && active;
+  if (mine)
+    for (int k = cnt; (k & 3) && k < maxnb; k++) nbr[(size_t)k * stride + i] = i;
+  return mine ? cnt : 0;
+}
+
 // Words a lane has room for: nine warps' rows fit a block's 48 KB.
 __host__ __device__ constexpr int row_words(int split) { return split == 9 ? 14 : 16; }
 
@@ -1336,6 +1437,17 @@ struct SmallRow {
 // the 2.05M-atom liquid 1.13 ms against 2.05 ms.  64 registers (32 warps an
 // SM, a few spills outside the walk) against 80: 1.13 and 1.17 ms; partners
 // filed one by one in a shared-memory ring instead of words: 1.6 ms.
+//
+// Turns cost about the same however little there is to walk, so where atoms lie
+// thin (many x-rows among 32, few candidates a run) every lane walks alone
+// (rows_alone).  With T turns a warp and p atoms in a cell that has any, turns
+// pay up to T (5 + p) = 3 + 5.4 p, and up to 1.6 times that T where the lanes
+// alone would walk twice (count, then file) because warps share their atoms.  In
+// turns, alone, and by build_rows with one lane an atom, us: 400,000 atoms, p =
+// 1, T = 4.4: 226, 115, 101; p = 1.4, T = 1.5: 111, 102, 110; p = 2.6, T = 1.9:
+// 133, 153, 153; T = 3: 199, 166, 173; p = 4.7, T = 2: 158, 218, 212; T = 3.2:
+// 238, 233, 231; 30,000 atoms, nine warps, p = 1, T = 9: 44, 18, 16; p = 1.4, T =
+// 3.9: 27, 23, 25; p = 2.6, T = 5.4: 36, 31, 37; T = 2.9: 25, 29, 35.
 template <bool SLAB, int SPLIT, bool SMALL>
 __device__ __forceinline__ int build_rows_warp(const RowGeom &g, const float4 *__restrict__ qloc,
                                                const double4 *__restrict__ q, const int *__restrict__ tab, int owner,
@@ -1347,6 +1459,8 @@ __device__ __forceinline__ int build_rows_warp(const RowGeom &g, const float4 *_
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int kNoSlot = 1 << 30;  // above every slot; differences with slots stay in range
   const int lane = threadIdx.x & 31;
+  if (rows_lie_thin(owner, pc, active, SMALL && small.on, SPLIT > 1))
+    return rows_alone<SLAB, SPLIT>(g, qloc, q, tab, pc, i, active, counts, part, nbr, stride, maxnb);
   const float4 li = qloc[i];
   const int cx = pc & 2047;
   const int mx = g.ms[0] * kXSub, vbase = (cx - 1) * kXSub;
@@ -1819,9 +1933,14 @@ __global__ void __launch_bounds__(SPLIT * 32, 27 / SPLIT) k_build_split(Arrays a
 // the liquid with one / three / nine warps, us: 6,912 atoms - / 97 / 94 (109
 // with eight lanes an atom), 32,000 - / 121 / 119 (144), 55,296 152 / 134 /
 // 135, 108,000 175 / 167 / -, 157,216 205 / 196 / -, 340,736 298 / 302 / -.
-inline int build_split(long long atoms, int sms) {
+// Three warps that would all walk alone (a system whose atoms lie thin on
+// average) are one: 100,000 atoms, T = 20: 41 us with three, 35 with one.
+inline int build_split(long long atoms, int sms, double per_cell, double per_row) {
   const long long warps = atoms / 32;
-  return warps * 9 <= 64LL * sms ? 9 : (warps * 3 <= 128LL * sms ? 3 : 1);
+  if (warps * 9 <= 64LL * sms) return 9;
+  const double p = fmax(per_cell / -expm1(-per_cell), 1.0);  // atoms in a cell that has any, scattered at random
+  const double turns = 1.0 + 31.0 / fmax(per_row, 1.0);
+  return warps * 3 <= 128LL * sms && turns * (5.0 + p) <= 3.0 + 5.4 * p ? 3 : 1;
 }
 
 // Before a build: clear the build counters.

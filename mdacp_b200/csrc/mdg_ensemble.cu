@@ -806,7 +806,7 @@ struct mdg_ensemble {
   mdg_params prm{};
   Ens e{};
   std::vector<Rep> reps;
-  int ncell_tot = 0;
+  int ncell_tot = 0, nrow_tot = 0;  // cells and x-rows of cells
   int *d_flags = nullptr;
   unsigned long long *d_count = nullptr;  // ke_count_pairs
   int *d_lists = nullptr;                 // storage of the two work lists
@@ -899,7 +899,7 @@ void e_launch_build(mdg_ensemble *x, cudaStream_t s, int pack) {
   // a list lives some eight steps, so about one replica in eight rebuilds at a
   // time (24 replicas of 40,000 atoms in all: 60 us with one warp per 32 atoms,
   // 23 us with nine)
-  switch (build_split(e.ntot / 8, x->work_blocks / 8)) {
+  switch (build_split(e.ntot / 8, x->work_blocks / 8, (double)e.ntot / x->ncell_tot, (double)e.ntot / x->nrow_tot)) {
     case 9: ke_build<9><<<std::min(nb(e.ntot, 32), x->work_blocks), 9 * 32, 0, s>>>(e); break;
     case 3: ke_build<3><<<std::min(nb(e.ntot, 32), 2 * x->work_blocks), 3 * 32, 0, s>>>(e); break;
     default: ke_build<1><<<std::min(nb(e.ntot, kEF), 2 * x->work_blocks), kEF, 0, s>>>(e);
@@ -1199,7 +1199,7 @@ mdg_status mdg_ensemble_create(const mdg_params *prm, int nrep, const mdg_replic
   x->tpa = prm->threads_per_atom;
   x->reps.resize(nrep);
   long long atoms = 0, tab_entries = 0;
-  int cells = 0;
+  int cells = 0, rows = 0;
   for (int r = 0; r < nrep; r++) {
     Rep &rp = x->reps[r];
     memset(&rp, 0, sizeof rp);
@@ -1243,6 +1243,7 @@ mdg_status mdg_ensemble_create(const mdg_params *prm, int nrep, const mdg_replic
     rp.atom_off = (int)atoms;
     rp.n = replicas[r].n;
     cells += rp.ncell;
+    rows += rp.ms[1] * rp.ms[2];
     atoms += replicas[r].n;
   }
   if (atoms > (1LL << 30)) {
@@ -1266,6 +1267,7 @@ mdg_status mdg_ensemble_create(const mdg_params *prm, int nrep, const mdg_replic
   e.rc2f = (float)e.rc2;
   e.c2x8f = (float)(e.c2 * 8.0);
   x->ncell_tot = cells;
+  x->nrow_tot = rows;
   const size_t n = (size_t)std::max<long long>(atoms, 1);
   cudaError_t err = cudaStreamCreateWithFlags(&x->stream, cudaStreamNonBlocking);
   if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&x->cap_stream, cudaStreamNonBlocking);
