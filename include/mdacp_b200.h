@@ -459,12 +459,12 @@ void mdg_adjoint_default_params(mdg_adjoint_params *p);
 /* q0, v0: n x 3 doubles.  loss is required; with all three gradient
  * pointers NULL only the forward pass runs.  dloss_dq0: n x 3 doubles.
  * Device memory (checkpoints: 2 x 32 B per atom per checkpoint; the list:
- * 4 B per row entry, rows of up to 1024 entries) is kept per device after
+ * 4 B per row entry, rows of up to 1056 entries) is kept per device after
  * the call and reused by later calls whose buffers fit, so repeated calls of
  * one shape allocate nothing; one run at a time per process.
  * MDG_ERR_CAPACITY if a row outgrows its capacity (the larger of twice the
  * mean density's count within the search length plus 64 and the count at
- * density 1.3 sigma^-3 plus 32, at most 1024); MDG_ERR_TIMEOUT if a bounded
+ * density 1.3 sigma^-3 plus 32, at most 1056); MDG_ERR_TIMEOUT if a bounded
  * device wait inside a list rebuild ran out. */
 mdg_status mdg_adjoint_run(const mdg_adjoint_params *p, const double *q0, const double *v0, int n, double *loss,
                            double *dloss_deps, double *dloss_dsigma, double *dloss_dq0);

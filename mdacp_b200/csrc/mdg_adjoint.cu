@@ -104,7 +104,9 @@ struct Meeting {
 struct List {
   int ms[3], ncell, maxnb, n;
   double L[3], inv_L[3], inv_cs[3];
-  float Lf[3], inv_Lf[3], reach2;  // FP32 search: enlarged by the rounding of box coordinates
+  // search length^2: enlarged by the rounding of box coordinates for an FP32
+  // search; negative for an FP64 one (boxes too long for FP32)
+  float Lf[3], inv_Lf[3], reach2;
   double half_skin2;
   int *count, *start, *cell, *rank, *cursor;  // cells: atoms, first place; atoms: cell, place in it
   float4 *sorted;                             // box coordinates and index in cell order
@@ -201,11 +203,13 @@ __device__ __forceinline__ void warp_sort(unsigned (&v)[4], int lane) {
 
 // Row of atom i by one warp: the atoms of the 27 cells around it within the
 // search length (FP32 minimum image on box coordinates; the reach is enlarged
-// by more than its rounding, and rows may hold more than they must), put in
+// by more than its rounding, and rows may hold more than they must; FP64 where
+// that would be more than a hundredth of the search length), put in
 // (bucket, index) order.  The cells of an x-row are consecutive in `sorted`:
 // the 27 cells are 9 runs, and 9 more of one cell each where x wraps; the next
 // 32 atoms' load is in flight while 32 are tested.  keys: maxnb words of shared
 // memory.
+template <bool EXACT>
 __device__ __forceinline__ void build_row(const List &l, const Vec &x, int i, unsigned *keys) {
   const int lane = threadIdx.x & 31;
   const double3 q = x.at(i);
@@ -249,7 +253,13 @@ __device__ __forceinline__ void build_row(const List &l, const Vec &x, int i, un
     dx = fmaf(-l.Lf[0], rintf(dx * l.inv_Lf[0]), dx);
     dy = fmaf(-l.Lf[1], rintf(dy * l.inv_Lf[1]), dy);
     dz = fmaf(-l.Lf[2], rintf(dz * l.inv_Lf[2]), dz);
-    const bool keep = in && j != i && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= l.reach2;
+    bool keep = in && j != i && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= l.reach2;
+    if (EXACT) {
+      const double3 o = x.at(j);
+      const double ex = min_image(q.x - o.x, l.L[0], l.inv_L[0]), ey = min_image(q.y - o.y, l.L[1], l.inv_L[1]),
+                   ez = min_image(q.z - o.z, l.L[2], l.inv_L[2]);
+      keep = in && j != i && ex * ex + ey * ey + ez * ez <= -(double)l.reach2;
+    }
     const unsigned bal = __ballot_sync(0xffffffffu, keep);
     const int at = m + __popc(bal & ((1u << lane) - 1u));
     if (keep && at < l.maxnb) keys[at] = ((unsigned)bucket_of(j) << 29) | (unsigned)j;
@@ -343,7 +353,10 @@ __device__ __noinline__ bool rebuild(const List &l, const Vec &x, unsigned *smem
   }
   if (!meet(l)) return false;
   unsigned *keys = smem + (threadIdx.x >> 5) * l.maxnb;
-  for (int i = t >> 5; i < l.n; i += nt >> 5) build_row(l, x, i, keys);
+  if (l.reach2 < 0.f)
+    for (int i = t >> 5; i < l.n; i += nt >> 5) build_row<true>(l, x, i, keys);
+  else
+    for (int i = t >> 5; i < l.n; i += nt >> 5) build_row<false>(l, x, i, keys);
   return meet(l);
 }
 
@@ -892,20 +905,24 @@ mdg_status mdg_adjoint_run(const mdg_adjoint_params *prm, const double *q0, cons
   }
   // rows keep pairs up to sl and, for the FP32 rounding of box coordinates
   // (each difference is off by less than 4 u L, u = 2^-24; eight times that
-  // here), a little more
-  const double reach = sl * (1.0 + 1e-5) + 32.0 / 16777216.0 * longest;
-  l.reach2 = (float)(reach * reach);
+  // here), a little more; where that is much, FP64 decides
+  const double margin = 32.0 / 16777216.0 * longest;
+  const double wide = sl * (1.0 + 1e-5) + margin;
+  const bool exact = margin > 0.01 * sl;
+  l.reach2 = (float)(exact ? -sl * sl * (1.0 + 1e-6) : wide * wide);
   l.half_skin2 = 0.25 * skin * skin;
   {
+    const double reach = exact ? sl : wide;
     const double vol = prm->L[0] * prm->L[1] * prm->L[2];
-    const double est = 4.0 / 3.0 * M_PI * sl * sl * sl * (double)n / vol;
+    const double sphere = 4.0 / 3.0 * M_PI * reach * reach * reach;
+    const double est = sphere * (double)n / vol;
     // twice the mean density's count plus 64, and at least the count at
     // density 1.3 (above a close-packed LJ solid) plus 32, so that a dense
-    // region of a dilute box fits; at most 1024.  A longer row is
-    // MDG_ERR_CAPACITY.
-    const double dense = 4.0 / 3.0 * M_PI * sl * sl * sl * 1.3 / (prm->sigma * prm->sigma * prm->sigma);
+    // region of a dilute box fits; at most 1024 within sl, which is 1056 within
+    // a reach a hundredth longer.  A longer row is MDG_ERR_CAPACITY.
+    const double dense = sphere * 1.3 / (prm->sigma * prm->sigma * prm->sigma);
     const double want = std::max(std::ceil(2.0 * est + 64.0), std::ceil(dense + 32.0));
-    l.maxnb = (int)std::min<double>(std::min(std::max(n - 1, 1), 1024), want);
+    l.maxnb = (int)std::min<double>(std::min(std::max(n - 1, 1), 1056), want);
   }
   l.ncell = l.ms[0] * l.ms[1] * l.ms[2];
   const double sc = prm->cutoff;
