@@ -269,19 +269,35 @@ __device__ __forceinline__ void build_row(const List &l, const Vec &x, int i, un
   m = min(m, l.maxnb);
   __syncwarp();
   int *row = l.nbr + (size_t)i * l.maxnb;
-  if (m <= 128) {
+  // in parts of 128, sorted in registers; an entry of a longer row comes after
+  // the smaller ones of every part (a binary search each)
+  for (int part = 0; part < m; part += 128) {
     unsigned v[4];
 #pragma unroll
-    for (int e = 0; e < 4; e++) v[e] = e * 32 + lane < m ? keys[e * 32 + lane] : 0xffffffffu;
+    for (int e = 0; e < 4; e++) v[e] = part + e * 32 + lane < m ? keys[part + e * 32 + lane] : 0xffffffffu;
     warp_sort(v, lane);
 #pragma unroll
     for (int e = 0; e < 4; e++)
-      if (e * 32 + lane < m) row[e * 32 + lane] = (int)(v[e] & 0x1fffffffu);
-  } else {
-    for (int e = lane; e < m; e += 32) {  // a long row: count the smaller keys
+      if (part + e * 32 + lane < m) {
+        if (m <= 128) row[e * 32 + lane] = (int)(v[e] & 0x1fffffffu);
+        else keys[part + e * 32 + lane] = v[e];
+      }
+  }
+  if (m > 128) {
+    __syncwarp();
+    for (int e = lane; e < m; e += 32) {
       const unsigned key = keys[e];
-      int r = 0;
-      for (int k = 0; k < m; k++) r += keys[k] < key ? 1 : 0;
+      int r = e & 127;
+      for (int part = 0; part < m; part += 128) {
+        if (part == (e & ~127)) continue;
+        int lo = part, hi = min(part + 128, m);  // the first key of the part above this one
+        while (lo < hi) {
+          const int mid = (lo + hi) >> 1;
+          if (keys[mid] < key) lo = mid + 1;
+          else hi = mid;
+        }
+        r += lo - part;
+      }
       row[r] = (int)(key & 0x1fffffffu);
     }
   }

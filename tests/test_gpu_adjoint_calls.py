@@ -32,3 +32,15 @@ def test_a_dense_block_in_a_long_box(length):
     # the rows have room for): beyond some 1.47e4 FP64 decides
     st = W.fcc_liquid(5, 0.8442, 1.0, 12, jitter=0.05, rc=2.5, dt=0.005)
     _check(st.q, st.v, np.array([9.0, 9.0, length]), 6, 2.5)
+
+
+@pytest.mark.parametrize("cells,cut,drop", [
+    (8, 3.0, 0),   # rows of about 128, some on either side
+    (8, 3.9, 1),   # two parts and a little more
+    (9, 4.9, 2),   # four parts
+    (11, 6.1, 0),  # eight parts: rows of about 925
+])
+def test_long_rows(cells, cut, drop):
+    # rows longer than the 128 entries that a warp sorts at a time
+    st = W.fcc_liquid(cells, 0.8442, 1.0, 20 + cells, jitter=0.05, rc=2.5, dt=0.005)
+    _check(st.q[: st.n - drop], st.v[: st.n - drop], st.L, 3, cut)
