@@ -73,15 +73,56 @@ bool cells_packable(const mdg::Box &b) { return b.ms[0] < 2048 && b.ms[1] < 2048
 // Entries of the list build's trim table: one block of 8 ms_x + 1 per x-row.
 size_t trim_table_size(const mdg::Box &b) { return (size_t)b.ms[1] * b.ms[2] * (b.ms[0] * kXSub + 1); }
 
-}  // namespace
-
-// A handle's small answers from the device, in pinned memory: a copy to the
-// stack goes through the driver's staging and takes twice as long.
+// A handle's small answers from the device.
 struct HostLanding {
   Status st;
   int flags[2];
   double sums[3];
 };
+
+// Places for them in page-locked memory, where a copy takes half as long as
+// through the driver's staging.  One block for the process, locked at its first
+// use (0.5 ms): page-locked memory of each handle's own took 3 ms to allocate
+// and free.  A handle that finds every place taken keeps its answers in
+// ordinary memory.
+constexpr int kLandings = 64;
+struct alignas(4096) LandingBlock {
+  HostLanding place[kLandings];
+};
+LandingBlock g_landing;
+bool g_landing_used[kLandings], g_landing_locked = false;
+std::mutex g_landing_mutex;
+
+class Landing {
+ public:
+  Landing() = default;
+  Landing(const Landing &) = delete;
+  Landing &operator=(const Landing &) = delete;
+  ~Landing() {
+    if (at_ == &own_) return;
+    std::lock_guard<std::mutex> lock(g_landing_mutex);
+    g_landing_used[at_ - g_landing.place] = false;
+  }
+  void take() {
+    std::lock_guard<std::mutex> lock(g_landing_mutex);
+    if (!g_landing_locked) {
+      g_landing_locked = true;
+      if (cudaHostRegister(&g_landing, sizeof g_landing, cudaHostRegisterPortable) != cudaSuccess) cudaGetLastError();
+    }
+    for (int k = 0; k < kLandings && at_ == &own_; k++)
+      if (!g_landing_used[k]) {
+        g_landing_used[k] = true;
+        at_ = &g_landing.place[k];
+      }
+  }
+  HostLanding *operator->() const { return at_; }
+
+ private:
+  HostLanding own_{};
+  HostLanding *at_ = &own_;
+};
+
+}  // namespace
 
 struct mdg_handle {
   mdg_params prm{};
@@ -93,7 +134,7 @@ struct mdg_handle {
   cudaStream_t stream = nullptr;      // work stream (user's or owned)
   bool own_stream = false;
   cudaStream_t cap_stream = nullptr;  // capture stream (always owned)
-  HostLanding *pin = nullptr;         // pinned: what the device's small answers are copied to
+  Landing pin;                        // what the device's small answers are copied to
   // the device's status after mdg_calculate's last wait; dropped by every call
   // that may change it (check_ready), kept by those that only read the state
   Status seen;
@@ -163,7 +204,7 @@ cudaError_t dalloc(T **p, size_t count) {
 }
 
 void free_arrays(Arrays &a) {
-  void *ptrs[] = {a.q, a.v, a.q_old, a.qfix, a.qfix2, a.pz, a.pz2, a.qloc, a.cxyz, a.xsub, a.ids, a.type, a.cell, a.nbr, a.nnbr, a.cell_count,
+  void *ptrs[] = {a.q, a.v, a.q_old, a.qfix, a.qloc, a.cxyz, a.xsub, a.ids, a.type, a.cell, a.nbr, a.nnbr, a.cell_count,
                   a.cell_start, a.slot, a.perm, a.perm2, a.q_tmp, a.v_tmp, a.v_lag, a.ids_tmp, a.type_tmp,
                   a.cell_tmp, a.mult, a.cand, a.partials, a.st, a.stage_rng, a.stage_n, a.nbr16, a.disp2};
   for (void *p : ptrs)
@@ -1077,10 +1118,15 @@ mdg_status mdg_create(const mdg_params *prm, mdg_handle **out) {
   if (e == cudaSuccess) e = dalloc(&a.q, cap);
   if (e == cudaSuccess) e = dalloc(&a.v, cap);
   if (e == cudaSuccess) e = dalloc(&a.q_old, cap);
-  if (e == cudaSuccess) e = dalloc(&a.qfix, cap);
-  if (e == cudaSuccess) e = dalloc(&a.qfix2, cap);
-  if (e == cudaSuccess && prm->precision == MDG_FP64) e = dalloc(&a.pz, cap);
-  if (e == cudaSuccess && prm->precision == MDG_FP64) e = dalloc(&a.pz2, cap);
+  {  // both packed copies in one allocation
+    const bool split = prm->precision == MDG_FP64;
+    if (e == cudaSuccess) e = dalloc(&a.qfix, (size_t)cap * (split ? 3 : 2));
+    a.qfix2 = a.qfix + cap;
+    if (split) {
+      a.pz = reinterpret_cast<double *>(a.qfix2 + cap);
+      a.pz2 = a.pz + cap;
+    }
+  }
   if (e == cudaSuccess) e = dalloc(&a.qloc, cap);
   if (e == cudaSuccess) e = dalloc(&a.cxyz, cap);
   if (e == cudaSuccess) e = dalloc(&a.xsub, trim_table_size(b));
@@ -1104,7 +1150,7 @@ mdg_status mdg_create(const mdg_params *prm, mdg_handle **out) {
   if (e == cudaSuccess) e = dalloc(&a.cand, prm->check_list_length);
   if (e == cudaSuccess) e = dalloc(&a.partials, h->partial_cap);
   if (e == cudaSuccess) e = dalloc(&a.st, 1);
-  if (e == cudaSuccess) e = cudaHostAlloc((void **)&h->pin, sizeof(HostLanding), cudaHostAllocDefault);
+  if (e == cudaSuccess) h->pin.take();
   if (e == cudaSuccess) e = dalloc(&h->d_flags, 4);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->d_flags, 0, 4 * sizeof(int), h->stream);
   if (e == cudaSuccess) e = dalloc(&h->d_sums, 8);
@@ -1149,7 +1195,6 @@ mdg_status mdg_destroy(mdg_handle *h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   destroy_graph(h);
   free_arrays(h->a);
-  if (h->pin) cudaFreeHost(h->pin);
   if (h->d_flags) cudaFree(h->d_flags);
   if (h->d_sums) cudaFree(h->d_sums);
   if (h->d_tiles) cudaFree(h->d_tiles);

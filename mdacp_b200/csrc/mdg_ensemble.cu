@@ -846,7 +846,7 @@ cudaError_t edalloc(T **p, size_t count) {
 
 void e_free(mdg_ensemble *x) {
   Ens &e = x->e;
-  void *ptrs[] = {(void *)e.rep, e.rs, (void *)e.rep_of, e.q, e.v, e.q_old, e.qfix, e.qfix2, e.pz, e.pz2, e.qloc, e.cxyz,
+  void *ptrs[] = {(void *)e.rep, e.rs, (void *)e.rep_of, e.q, e.v, e.q_old, e.qfix, e.qloc, e.cxyz,
                   e.xsub, e.ids, e.cell,
                   e.cell_tmp, e.nbr, e.nnbr, e.cell_count, e.cell_start, e.slot, e.perm, e.perm2, e.q_tmp,
                   e.v_tmp, e.ids_tmp, e.mult, e.cand, e.disp2, e.error, e.sums, x->d_flags, x->d_count,
@@ -1281,10 +1281,15 @@ mdg_status mdg_ensemble_create(const mdg_params *prm, int nrep, const mdg_replic
   if (err == cudaSuccess) err = edalloc(&e.q, n);
   if (err == cudaSuccess) err = edalloc(&e.v, n);
   if (err == cudaSuccess) err = edalloc(&e.q_old, n);
-  if (err == cudaSuccess) err = edalloc(&e.qfix, n);
-  if (err == cudaSuccess) err = edalloc(&e.qfix2, n);
-  if (err == cudaSuccess && prm->precision == MDG_FP64) err = edalloc(&e.pz, n);
-  if (err == cudaSuccess && prm->precision == MDG_FP64) err = edalloc(&e.pz2, n);
+  {  // both packed copies in one allocation
+    const bool split = prm->precision == MDG_FP64;
+    if (err == cudaSuccess) err = edalloc(&e.qfix, n * (split ? 3 : 2));
+    e.qfix2 = e.qfix + n;
+    if (split) {
+      e.pz = reinterpret_cast<double *>(e.qfix2 + n);
+      e.pz2 = e.pz + n;
+    }
+  }
   if (err == cudaSuccess) err = edalloc(&e.qloc, n);
   if (err == cudaSuccess) err = edalloc(&e.cxyz, n);
   if (err == cudaSuccess) err = edalloc(&e.xsub, (size_t)tab_entries);
