@@ -79,7 +79,10 @@ typedef struct {
                                0 (default) = chosen by timing the three once per device
                                and problem shape, at the first step */
   int build_block;          /* list build: threads per block, 64, 128 or 256; 0
-                               (default) = chosen by timing, as threads_per_atom */
+                               (default) = chosen by timing, as threads_per_atom.  With
+                               one lane per atom and few atoms (below some 200,000)
+                               several warps share 32 atoms' rows, in blocks of a size of
+                               their own; chosen by timing it is then 128 */
   int build_threads_per_atom; /* list build: lanes per atom, 1, 2, 4 or 8 (the rows are the
                                same for every choice); 0 (default) = chosen by timing
                                together with build_block */

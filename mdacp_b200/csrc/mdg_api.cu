@@ -781,7 +781,7 @@ static __global__ void k_list_counters_reset(Arrays a) {
 
 mdg_status autotune(mdg_handle *h) {
   const bool fp32 = h->prm.precision == MDG_FP32_MIXED;
-  if (!fp32 && h->tpa == 0) h->tpa = 1;            // the FP64 pass has one lane per atom
+  if (!fp32 && h->tpa == 0) h->tpa = 1;  // not tuned: the FP64 pass takes its lanes by size (fp64_lanes)
   if (h->a.stage_cap > 0) {  // stage rows per 128 atoms, one lane per atom
     if (h->build_block == 0) h->build_block = kForceBlock;
     if (h->build_tpa == 0) h->build_tpa = 1;
@@ -840,6 +840,8 @@ mdg_status autotune(mdg_handle *h) {
       if (bb != 0 && cb != bb) continue;
       for (int cl : lanes) {
         if (bl != 0 && cl != bl) continue;
+        // the split walk has a block size of its own: timed once
+        if (cl == 1 && list_split(h) > 1 && cb != (bb != 0 ? bb : kForceBlock)) continue;
         const float ms = time_launches(s, [&]() { launch_list_build(h, s, cb, cl); }, 3);
         if (ms < 0.f) return fail(h, MDG_ERR_CUDA, "autotune: build timing failed");
         if (best < 0.f || ms < best) {
