@@ -180,8 +180,11 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 // IBM RISC System/6000 processor", 1990).  The reciprocal is good to about
 // 2^-40, so the quotient before its last rounding is to about 2^-80: the
 // correctly rounded one but for some 10^-8 of the operands, where it is its
-// neighbour.  Unlike the operator it has no branch for unusual operands, so
-// the quotients of several pairs overlap.
+// neighbour (tests/test_gpu_quotient.py: none differs from the IEEE quotient in
+// 10^5 pairs of the force and observer terms from 1e-12 to the cut-off).  Unlike
+// the operator it has no branch for unusual operands, so the quotients of several
+// pairs overlap; one that overflows, or whose denominator is zero or subnormal
+// (pairs nearer than 1e-22), is NaN where the operator gives an infinity.
 __device__ __forceinline__ double quotient(double a, double b) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
@@ -2443,8 +2446,9 @@ __device__ __forceinline__ void pair_displacements(const Edges &e, const double3
 // pair term is the reference's (ForceCalculator::CalculateForceNext,
 // src/fcalculator.cc:228-290): dx = image(q_j) - q_i, r2 = (dx*dx + dy*dy) +
 // dz*dz, 0 if r2 > rc^2, r6 = (r2*r2)*r2, df = ((24 r6 - 48) /
-// ((r6*r6)*r2) + 8 C2) * dt, term = df * dx, all separately rounded; only the
-// summation order differs (fp64_row).
+// ((r6*r6)*r2) + 8 C2) * dt, term = df * dx, all separately rounded but for the
+// division's last bit in some 10^-8 of pairs (quotient); and the summation order
+// differs (fp64_row).
 struct Fp64Pair {
   Edges e;
   double rc2, c2x8, dt;
