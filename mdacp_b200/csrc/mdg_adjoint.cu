@@ -1012,7 +1012,10 @@ mdg_status mdg_adjoint_run(const mdg_adjoint_params *prm, const double *q0, cons
     if (e == cudaSuccess) e = R.alloc(&R.seg_x, (size_t)seg * 3 * R.ns);
     if (e == cudaSuccess) e = R.alloc(&R.seg_v, (size_t)seg * 3 * R.ns);
   }
-  if (e != cudaSuccess) return e == cudaErrorMemoryAllocation ? MDG_ERR_CAPACITY : MDG_ERR_CUDA;
+  if (e != cudaSuccess) {
+    cudaGetLastError();  // reported here, not by the next call
+    return e == cudaErrorMemoryAllocation ? MDG_ERR_CAPACITY : MDG_ERR_CUDA;
+  }
   l.overflow = R.state;
   l.timeout = R.state + 1;
   l.cursor = R.state + 2;

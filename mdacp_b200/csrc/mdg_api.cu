@@ -194,6 +194,7 @@ mdg_status fail(mdg_handle *h, mdg_status s, const std::string &msg) {
   do {                                                                                     \
     cudaError_t e_ = (expr);                                                               \
     if (e_ != cudaSuccess) {                                                               \
+      cudaGetLastError(); /* reported here, not again by the next call */                  \
       return fail((h), MDG_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
     }                                                                                      \
   } while (0)
@@ -1170,15 +1171,14 @@ mdg_status mdg_create(const mdg_params *prm, mdg_handle **out) {
   if (e == cudaSuccess) e = cudaMemsetAsync(a.st, 0, sizeof(Status), h->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
   if (e != cudaSuccess) {
-    free_arrays(a);
-    delete h;
+    cudaGetLastError();
+    mdg_destroy(h);
     return MDG_ERR_CUDA;
   }
   if (prm->max_neighbors > 0) {
     mdg_status r = alloc_neighbors(h, prm->max_neighbors);
     if (r) {
-      free_arrays(a);
-      delete h;
+      mdg_destroy(h);
       return r;
     }
   }

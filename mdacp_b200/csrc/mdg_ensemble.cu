@@ -834,9 +834,12 @@ struct mdg_ensemble {
 
 namespace {
 
-#define ECUDA(expr)                      \
-  do {                                   \
-    if ((expr) != cudaSuccess) return MDG_ERR_CUDA; \
+#define ECUDA(expr)                                                  \
+  do {                                                               \
+    if ((expr) != cudaSuccess) {                                     \
+      cudaGetLastError(); /* reported here, not by the next call */  \
+      return MDG_ERR_CUDA;                                           \
+    }                                                                \
   } while (0)
 
 template <typename T>
@@ -1347,8 +1350,8 @@ mdg_status mdg_ensemble_create(const mdg_params *prm, int nrep, const mdg_replic
     if (err == cudaSuccess) err = cudaMemset(e.error, 0, sizeof(int));
   }
   if (err != cudaSuccess) {
-    e_free(x);
-    delete x;
+    cudaGetLastError();
+    mdg_ensemble_destroy(x);
     return MDG_ERR_CUDA;
   }
   *out = x;

@@ -194,7 +194,10 @@ mdg_status sfail(mdg_slabs *x, mdg_status st, const std::string &msg) {
 #define SCUDA(x, expr)                                                                         \
   do {                                                                                         \
     cudaError_t e_ = (expr);                                                                   \
-    if (e_ != cudaSuccess) return sfail((x), MDG_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                                   \
+      cudaGetLastError(); /* reported here, not again by the next call */                      \
+      return sfail((x), MDG_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_));     \
+    }                                                                                          \
   } while (0)
 
 template <typename T>
@@ -743,6 +746,7 @@ mdg_status mdg_slabs_create(const mdg_params *prm, int nslabs, const int *device
   for (Slab &sl : x->s)
     if (e == cudaSuccess) e = cudaStreamSynchronize(sl.stream);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     for (Slab &sl : x->s) free_slab(sl);
     delete x;
     return MDG_ERR_CUDA;
