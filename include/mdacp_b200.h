@@ -92,7 +92,7 @@ typedef struct {
                                MDG_STEPS_GRAPHS: CUDA graphs with conditional rebuild nodes;
                                MDG_STEPS_PERSISTENT: cooperative launches run the steps
                                back to back, displacement checks included (one lane per
-                               atom from 16,384 atoms, 2 or 4 below); each stops at a step
+                               atom from 24,000 atoms, 2 from 8,192, 4 below); each stops at a step
                                that needs a rebuild, which a queued graph takes, and the
                                next launch follows without a host wait.  Same results. */
   long long stage_wait_cycles; /* staged FP32-mixed pass (stage_atoms != 0): clock cycles a
@@ -223,7 +223,8 @@ typedef struct {
   int64_t displacement_checks;
   double simulation_time;
   double buffer_left;     /* skin budget (PairList::buffer_length) */
-  int threads_per_atom;   /* lanes per atom of the FP32-mixed force pass (0: not chosen yet) */
+  int threads_per_atom;   /* lanes per atom of the FP32-mixed force pass (0: not chosen yet;
+                             FP64 handles say 1, their passes take 1, 4 or 8 by size) */
   int build_block;        /* threads per block of the list build (0: not chosen yet) */
   int build_threads_per_atom; /* lanes per atom of the list build (0: not chosen yet) */
   int64_t persistent_steps;   /* steps taken by the persistent pass (step_mode) */
@@ -461,7 +462,7 @@ typedef struct mdg_adjoint_params {
 void mdg_adjoint_default_params(mdg_adjoint_params *p);
 /* q0, v0: n x 3 doubles.  loss is required; with all three gradient
  * pointers NULL only the forward pass runs.  dloss_dq0: n x 3 doubles.
- * Device memory (checkpoints: 2 x 32 B per atom per checkpoint; the list:
+ * Device memory (checkpoints: 2 x 24 B per atom per checkpoint; the list:
  * 4 B per row entry, rows of up to 1056 entries) is kept per device after
  * the call and reused by later calls whose buffers fit, so repeated calls of
  * one shape allocate nothing; one run at a time per process.

@@ -39,8 +39,9 @@
 // 2.1 ms; with one kernel per operation (12 launches a step forward, 19 in
 // reverse), a one-block cell grid (170 us a rebuild, 180 more for the rows; 133
 // us in all here), roots and two divisions a pair and ballots to share out a
-// row they took 86 and 8.9 ms.  Per pass at 32,000 atoms: force 15 us (37),
-// loss with gradient 35 (51), Hessian 35 (47).
+// row they took 86 and 8.9 ms.  Per pass at 32,000 atoms, four lanes an atom:
+// force 15 us (37), loss with gradient 34 (51), Hessian 35 (47); of the 29 ms
+// of kernels in that run 19.5 are 780 passes and 9.5 are 71 rebuilds.
 //
 // One launch per evaluation: a step is a force pass (kick and both drifts in
 // its end), a loss pass (forward: the sums; reverse: the loss gradient and the
@@ -64,7 +65,10 @@
 namespace {
 
 constexpr int kAB = 128;        // threads per block
-constexpr int kABlocks = 7;     // blocks an SM that the passes are held to (72 registers)
+// Blocks an SM that the passes are held to: 72 registers, which the force and
+// loss sums keep to; the loss with its gradient and the Hessian spill some 110
+// and 150 bytes a thread.  Other caps have not been measured.
+constexpr int kABlocks = 7;
 constexpr int kBuckets = 8;     // hash buckets of a row
 constexpr int kReduceSlots = 32;  // steps whose block partials are kept before they are summed
 

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <atomic>
 #include <fstream>
@@ -83,14 +84,12 @@ struct HostLanding {
 // Places for them in page-locked memory, where a copy takes half as long as
 // through the driver's staging.  One block for the process, locked at its first
 // use (0.5 ms): page-locked memory of each handle's own took 3 ms to allocate
-// and free.  A handle that finds every place taken keeps its answers in
-// ordinary memory.
+// and free.  It is ordinary memory that is never freed, so that a device reset
+// only unlocks it and unloading the library leaves no locked address behind for
+// others.  A handle that finds every place taken keeps its answers in itself.
 constexpr int kLandings = 64;
-struct alignas(4096) LandingBlock {
-  HostLanding place[kLandings];
-};
-LandingBlock g_landing;
-bool g_landing_used[kLandings], g_landing_locked = false;
+HostLanding *g_landing = nullptr;
+bool g_landing_used[kLandings];
 std::mutex g_landing_mutex;
 
 class Landing {
@@ -101,18 +100,19 @@ class Landing {
   ~Landing() {
     if (at_ == &own_) return;
     std::lock_guard<std::mutex> lock(g_landing_mutex);
-    g_landing_used[at_ - g_landing.place] = false;
+    g_landing_used[at_ - g_landing] = false;
   }
   void take() {
     std::lock_guard<std::mutex> lock(g_landing_mutex);
-    if (!g_landing_locked) {
-      g_landing_locked = true;
-      if (cudaHostRegister(&g_landing, sizeof g_landing, cudaHostRegisterPortable) != cudaSuccess) cudaGetLastError();
+    if (!g_landing) {
+      const size_t bytes = (kLandings * sizeof(HostLanding) + 4095) / 4096 * 4096;
+      g_landing = static_cast<HostLanding *>(std::aligned_alloc(4096, bytes));
+      if (g_landing && cudaHostRegister(g_landing, bytes, cudaHostRegisterPortable) != cudaSuccess) cudaGetLastError();
     }
-    for (int k = 0; k < kLandings && at_ == &own_; k++)
+    for (int k = 0; g_landing && k < kLandings && at_ == &own_; k++)
       if (!g_landing_used[k]) {
         g_landing_used[k] = true;
-        at_ = &g_landing.place[k];
+        at_ = &g_landing[k];
       }
   }
   HostLanding *operator->() const { return at_; }
@@ -158,8 +158,8 @@ struct mdg_handle {
   int64_t force_launches = 0;
   int64_t kernel_launches = 0;
   int graph_kernel_count = 0;         // kernels per graph launch outside conditionals
-  // fused FP32 NVE step: which fixed-point buffer (0: qfix, 1: qfix2) holds
-  // every atom's position after the coming step's first half drift; -1: none
+  // fused NVE step: which packed copy (0: qfix, 1: qfix2) holds every atom's
+  // position after the coming step's first half drift; -1: none
   int fix_buf = -1;
   int cell_cap = 0;                   // cells the cell tables hold
   int tpa = 0;                        // lanes per atom of the FP32 force pass (0: to be tuned)
@@ -310,9 +310,7 @@ double step_lag(const mdg_handle *h) {
   return h->prm.thermostat == MDG_LANGEVIN ? 0.0 : 0.5 * h->prm.time_step;
 }
 
-// Pairlist rebuild (MDManager::MakePairList).
-// pack: where to put the coming step's first-drift positions after the
-// rebuild (the fused FP32 NVE step), or nullptr.
+// The packed copies that the fused NVE steps take turns with.
 int4 *fix_buffer(mdg_handle *h, int k) { return k ? h->a.qfix2 : h->a.qfix; }
 // The z array of a packed copy (null: fixed-point).
 double *fix_z(const mdg_handle *h, const int4 *buf) { return buf == h->a.qfix2 ? h->a.pz2 : h->a.pz; }
@@ -353,6 +351,9 @@ void launch_list_build(mdg_handle *h, cudaStream_t s, int block, int lanes) {
   else launch_list_build_block<128>(h, s, lanes);
 }
 
+// Pairlist rebuild (MDManager::MakePairList).
+// pack: where to put the coming step's first-drift positions after the
+// rebuild (the fused NVE step), or nullptr.
 void launch_build(mdg_handle *h, cudaStream_t s, int4 *pack = nullptr) {
   const int n = h->n;
   Arrays &a = h->a;
@@ -504,8 +505,7 @@ void launch_drift(mdg_handle *h, cudaStream_t s) {
 
 // Everything of MDManager::Calculate after the rebuild decision; returns the
 // number of kernels launched.  ev_start/ev_stop bracket the force kernel.
-// parity: the fixed-point buffer the fused NVE step reads (it writes the
-// other one).
+// parity: the packed copy the fused NVE step reads (it writes the other one).
 // end: the next step's expiry decision, where a kernel of this one can make it
 // (ends_step).
 int launch_step_tail(mdg_handle *h, cudaStream_t s, cudaEvent_t ev_start, cudaEvent_t ev_stop,

@@ -547,15 +547,8 @@ struct PairStage {
   double o[3][kPairStage], n[3][kPairStage];
 };
 
-// The pair test of PairList::CheckByDisplacement (src/pairlist.cc:99-121)
-// over the candidate list's rows, a warp each, dealt over `parts` blocks: sets *found
-// if a pair of candidate copies (a < b) that was at least SearchLength apart
-// at the last build is now inside the cut-off.  Copies carry their shifts,
-// so the distances are the reference's direct differences.  The result is
-// an "any" over the pairs, so splitting the rows over blocks and the columns
-// over threads changes only the time.  l must be the same for every thread
-// of the block (the staging pass ends in a barrier).
-// The same reading the copies' positions from global memory (any l).
+// candidate_pair_test reading the copies' positions from global memory (any l,
+// no barrier).
 template <int BLOCK>
 __device__ __forceinline__ void candidate_pair_test_global(const CopyView &cv, const double L[3], const int2 *cand,
                                                            int l, double lag, double sl2, double rc2, int part,
@@ -573,6 +566,14 @@ __device__ __forceinline__ void candidate_pair_test_global(const CopyView &cv, c
   }
 }
 
+// The pair test of PairList::CheckByDisplacement (src/pairlist.cc:99-121)
+// over the candidate list's rows, a warp each, dealt over `parts` blocks: sets *found
+// if a pair of candidate copies (a < b) that was at least SearchLength apart
+// at the last build is now inside the cut-off.  Copies carry their shifts,
+// so the distances are the reference's direct differences.  The result is
+// an "any" over the pairs, so splitting the rows over blocks and the columns
+// over threads changes only the time.  l must be the same for every thread
+// of the block (the staging pass ends in a barrier).
 template <int BLOCK>
 __device__ __forceinline__ void candidate_pair_test(const CopyView &cv, const double L[3], const int2 *cand, int l,
                                                     double lag, double sl2, double rc2, int part, int parts,
@@ -1812,8 +1813,8 @@ __device__ __forceinline__ void count_rows(Status *st, int cnt) {
   }
 }
 
-// Rebuild 6/6: full Verlet list, one thread per atom (build_rows_warp) or
-// BTPA of them (build_rows; also the rows that carry stage indices).  Each
+// Rebuild 6/6: full Verlet list, one thread per atom (build_rows_warp, which
+// walks thin atoms' rows alone) or BTPA of them (build_rows; also the rows that carry stage indices).  Each
 // candidate is first tested in FP32; only candidates whose FP32 r^2 falls in
 // a band around SearchLength^2 -- wider than the FP32 error bound, which
 // mdg_create derives from the box -- are decided by the exact FP64 test, so

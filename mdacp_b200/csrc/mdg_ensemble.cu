@@ -869,10 +869,15 @@ double *e_pack_z(const Ens &e, int k) { return k ? e.pz2 : e.pz; }
 constexpr int kEDispKernels = 4, kEBuildKernels = 8;
 
 // From this many replicas the check's and the rebuild's kernels are launched
-// every step, and sweep empty work lists where nothing is due.  A list lives
-// some eight steps, so with eight replicas most steps rebuild one; a
-// conditional branch costs 6.5 us to pass by and about 12 to take, twice a step
+// every step, and sweep empty work lists where nothing is due.  The list of a hot
+// replica lives some eight steps, so with eight of them most steps rebuild one;
+// a conditional branch costs 6.5 us to pass by and about 12 to take, twice a step
 // (and two waits by the host outside graphs), twelve empty launches about 20.
+// 100 FP32 steps of replicas of 860 to 2,900 atoms with the nested nodes and with
+// none, ms: eight hot ones 7.0 and 5.9, 24 10.1 and 8.2, 256 21.3 and 18.6; cold
+// ones 6.1 and 5.3, 9.3 and 7.7, 21.8 and 19.1; margins of 0.8 6.0 and 5.4, 9.2
+// and 8.0, 29.7 and 27.0; four with nodes 5.6.  Equal copies, which rebuild
+// together, are the exception: eight 3.8 and 4.7.
 constexpr int kEAlways = 8;
 
 // The per-atom and per-cell kernels of the branches sweep the work list with

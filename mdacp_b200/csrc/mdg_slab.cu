@@ -579,6 +579,9 @@ mdg_status slab_step(mdg_slabs *x) {
       else if (x->tpa == 2) k_force_fp32<kSF, kKick, 1, 2><<<nb, kSF, 0, sl.stream>>>(sl.a, sl.box, n, th, sl.a.qfix, nullptr);
       else k_force_fp32<kSF, kKick, 1, 1><<<nb, kSF, 0, sl.stream>>>(sl.a, sl.box, n, th, sl.a.qfix, nullptr);
     } else {
+      // unpacked positions: the ghost layers are pushed as they lie in q, and a
+      // step's host waits (about 200 us on one device) outweigh what the split
+      // copy and the fused drifts would give the pass
       k_force_fp64<kSF, kKick, 0, 1><<<sblocks(n, kSF), kSF, 0, sl.stream>>>(sl.a, sl.box, n, th, PosState{sl.a.q}, nullptr, nullptr);
       k_drift<kSB, false><<<sblocks(n, kSB), kSB, 0, sl.stream>>>(sl.a, sl.box, n, 1);
     }
