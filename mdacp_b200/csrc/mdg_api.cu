@@ -321,13 +321,13 @@ int build_kernels(const mdg_handle *h) { return (h->ncell <= kScanSingleCells ? 
 // The list build alone (the rows of the atoms' current cell order), with
 // `block` threads per block and `lanes` threads per atom.
 template <int BLOCK>
-void launch_list_build_block(mdg_handle *h, cudaStream_t s, int lanes) {
+void launch_list_build_block(mdg_handle *h, const Arrays &a, cudaStream_t s, int lanes) {
   const int n = h->n;
   const int nb = (int)std::max<long long>(1, ((long long)n * lanes + BLOCK - 1) / BLOCK);
-  if (lanes == 8) k_build<BLOCK, false, false, 8><<<nb, BLOCK, 0, s>>>(h->a, h->box, n);
-  else if (lanes == 4) k_build<BLOCK, false, false, 4><<<nb, BLOCK, 0, s>>>(h->a, h->box, n);
-  else if (lanes == 2) k_build<BLOCK, false, false, 2><<<nb, BLOCK, 0, s>>>(h->a, h->box, n);
-  else k_build<BLOCK, false, false, 1><<<nb, BLOCK, 0, s>>>(h->a, h->box, n);
+  if (lanes == 8) k_build<BLOCK, false, false, 8><<<nb, BLOCK, 0, s>>>(a, h->box, n);
+  else if (lanes == 4) k_build<BLOCK, false, false, 4><<<nb, BLOCK, 0, s>>>(a, h->box, n);
+  else if (lanes == 2) k_build<BLOCK, false, false, 2><<<nb, BLOCK, 0, s>>>(a, h->box, n);
+  else k_build<BLOCK, false, false, 1><<<nb, BLOCK, 0, s>>>(a, h->box, n);
 }
 
 // Warps that share 32 atoms' rows when each atom has one lane.
@@ -335,20 +335,21 @@ int list_split(const mdg_handle *h) {
   return build_split(h->n, h->sms, (double)h->n / h->ncell, (double)h->n / (h->box.ms[1] * h->box.ms[2]));
 }
 
-// Few atoms with one lane each: the split walk, whatever the block size.
-void launch_list_build(mdg_handle *h, cudaStream_t s, int block, int lanes) {
+// Few atoms with one lane each: the split walk, whatever the block size.  a:
+// the handle's arrays with q as it was when the atoms were put in cell order.
+void launch_list_build(mdg_handle *h, const Arrays &a, cudaStream_t s, int block, int lanes) {
   const int split = lanes == 1 ? list_split(h) : 1;
   if (split == 9) {
-    k_build_split<9><<<blocks_for(h->n, 32), 9 * 32, 0, s>>>(h->a, h->box, h->n);
+    k_build_split<9><<<blocks_for(h->n, 32), 9 * 32, 0, s>>>(a, h->box, h->n);
     return;
   }
   if (split == 3) {
-    k_build_split<3><<<blocks_for(h->n, 32), 3 * 32, 0, s>>>(h->a, h->box, h->n);
+    k_build_split<3><<<blocks_for(h->n, 32), 3 * 32, 0, s>>>(a, h->box, h->n);
     return;
   }
-  if (block == 64) launch_list_build_block<64>(h, s, lanes);
-  else if (block == 256) launch_list_build_block<256>(h, s, lanes);
-  else launch_list_build_block<128>(h, s, lanes);
+  if (block == 64) launch_list_build_block<64>(h, a, s, lanes);
+  else if (block == 256) launch_list_build_block<256>(h, a, s, lanes);
+  else launch_list_build_block<128>(h, a, s, lanes);
 }
 
 // Pairlist rebuild (MDManager::MakePairList).
@@ -376,7 +377,7 @@ void launch_build(mdg_handle *h, cudaStream_t s, int4 *pack = nullptr) {
     k_stage_plan<kBlock><<<blocks_for(blocks_for(n, kStageBlock), kBlock), kBlock, 0, s>>>(a, h->box, n);
     k_build<kForceBlock, true><<<blocks_for(n, kForceBlock), kForceBlock, 0, s>>>(a, h->box, n);
   } else {
-    launch_list_build(h, s, h->build_block > 0 ? h->build_block : kForceBlock, h->build_tpa > 0 ? h->build_tpa : 1);
+    launch_list_build(h, a, s, h->build_block > 0 ? h->build_block : kForceBlock, h->build_tpa > 0 ? h->build_tpa : 1);
   }
   k_build_done<<<1, 32, 0, s>>>(a, h->box);
 }
@@ -749,8 +750,9 @@ mdg_status ensure_list(mdg_handle *h) {
 // and remembered per device and problem shape (atoms, cells, precision)
 // for the rest of the process.  The force candidates run force-only (the
 // forces go to scratch, the state is untouched); the build candidates
-// rebuild the same rows from the same cell order, and a last build with the
-// chosen block leaves the list counters as a normal build does.
+// rebuild the same rows from the same cell order and the positions of the last
+// build, and a last build with the chosen block leaves the list counters as a
+// normal build does.
 std::mutex g_tune_mutex;
 std::map<std::tuple<int, int, int, int>, std::tuple<int, int, int>> g_tuned;
 
@@ -836,6 +838,9 @@ mdg_status autotune(mdg_handle *h) {
   if (bb == 0 || bl == 0) {
     float best = -1.f;
     int bb_best = 0, bl_best = 0;
+    // the rows of the list's own positions: the atoms may have moved since
+    Arrays a = h->a;
+    a.q = a.q_old;
     const int blocks[3] = {64, 128, 256}, lanes[4] = {1, 2, 4, 8};
     for (int cb : blocks) {
       if (bb != 0 && cb != bb) continue;
@@ -843,7 +848,7 @@ mdg_status autotune(mdg_handle *h) {
         if (bl != 0 && cl != bl) continue;
         // the split walk has a block size of its own: timed once
         if (cl == 1 && list_split(h) > 1 && cb != (bb != 0 ? bb : kForceBlock)) continue;
-        const float ms = time_launches(s, [&]() { launch_list_build(h, s, cb, cl); }, 3);
+        const float ms = time_launches(s, [&]() { launch_list_build(h, a, s, cb, cl); }, 3);
         if (ms < 0.f) return fail(h, MDG_ERR_CUDA, "autotune: build timing failed");
         if (best < 0.f || ms < best) {
           best = ms;
@@ -855,7 +860,7 @@ mdg_status autotune(mdg_handle *h) {
     bb = bb_best;
     bl = bl_best;
     k_list_counters_reset<<<1, 32, 0, s>>>(h->a);
-    launch_list_build(h, s, bb, bl);
+    launch_list_build(h, a, s, bb, bl);
   }
   CUDA_TRY(h, cudaGetLastError());
   Status st;
