@@ -1970,7 +1970,7 @@ __global__ void __launch_bounds__(BLOCK) k_build_begin_clear(Arrays a, int ncell
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_copy_back(Arrays a, int n) {
   const int i = blockIdx.x * BLOCK + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || a.st->error) return;  // nothing was permuted: the atoms stay
   a.q[i] = a.q_tmp[i];
   a.v[i] = a.v_tmp[i];
   a.ids[i] = a.ids_tmp[i];

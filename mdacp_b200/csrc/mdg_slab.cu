@@ -362,10 +362,7 @@ mdg_status rebuild(mdg_slabs *x) {
     k_scatter<kSB><<<sblocks(n, kSB), kSB, 0, s>>>(a, n);
     k_sort_cells<<<sblocks((long long)sl.ncell * 32, kSB), kSB, 0, s>>>(a, sl.box, sl.ncell);
     k_permute<kSB><<<sblocks(n, kSB), kSB, 0, s>>>(a, sl.box, n, nullptr, nullptr);
-    SCUDA(x, cudaMemcpyAsync(a.q, a.q_tmp, sizeof(double4) * n, cudaMemcpyDeviceToDevice, s));
-    SCUDA(x, cudaMemcpyAsync(a.v, a.v_tmp, sizeof(double4) * n, cudaMemcpyDeviceToDevice, s));
-    SCUDA(x, cudaMemcpyAsync(a.ids, a.ids_tmp, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
-    SCUDA(x, cudaMemcpyAsync(a.type, a.type_tmp, sizeof(int) * n, cudaMemcpyDeviceToDevice, s));
+    k_copy_back<kSB><<<sblocks(n, kSB), kSB, 0, s>>>(a, n);
   }
   SCUDA(x, cudaGetLastError());
   // border layer sizes: the own bottom layer ends at the start of layer 1,
