@@ -377,9 +377,11 @@ __global__ void __launch_bounds__(1024) ke_decide(Ens e, cudaGraphConditionalHan
   __shared__ int any;
   if (threadIdx.x == 0) any = 0;
   __syncthreads();
-  for (int r = threadIdx.x; r < e.nrep; r += blockDim.x) {
+  // after an error the flags of the step that met it stay: a build whose rows
+  // outgrew their capacity is made again for the replicas that it was made for
+  for (int r = threadIdx.x; r < e.nrep && *e.error == 0; r += blockDim.x) {
     RepStatus &st = e.rs[r];
-    const int b = (*e.error == 0) && st.want_build;
+    const int b = st.want_build;
     st.build = b;
     st.disp = 0;
     if (b) {
@@ -1121,13 +1123,31 @@ mdg_status e_translate(int err) {
   return err ? MDG_ERR_CUDA : MDG_OK;
 }
 
-mdg_status e_alloc_neighbors(mdg_ensemble *x, int maxnb) {
+// Rows of up to maxnb partners.  *kept (may be null: not asked for): whether the
+// rows that there were are still there.
+mdg_status e_alloc_neighbors(mdg_ensemble *x, int maxnb, bool *kept = nullptr) {
   maxnb = std::max(8, (maxnb + 7) / 8 * 8);
+  if (kept) *kept = x->e.nbr != nullptr;
   if (x->e.nbr && maxnb <= x->e.maxnb) return MDG_OK;
   ECUDA(cudaStreamSynchronize(x->stream));
-  if (x->e.nbr) cudaFree(x->e.nbr);
+  int *old = x->e.nbr;
   x->e.nbr = nullptr;
-  ECUDA(edalloc(&x->e.nbr, (size_t)maxnb * x->e.stride));
+  if (old && kept) {
+    // entry k of every row lies at k * stride: the old rows are the new table's first part
+    cudaError_t err = edalloc(&x->e.nbr, (size_t)maxnb * x->e.stride);
+    if (err == cudaSuccess)
+      err = cudaMemcpyAsync(x->e.nbr, old, sizeof(int) * (size_t)x->e.maxnb * x->e.stride, cudaMemcpyDeviceToDevice,
+                            x->stream);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(x->stream);
+    if (err != cudaSuccess) {  // no room for both
+      cudaGetLastError();
+      if (x->e.nbr) cudaFree(x->e.nbr);
+      x->e.nbr = nullptr;
+      *kept = false;
+    }
+  }
+  if (old) cudaFree(old);
+  if (!x->e.nbr) ECUDA(edalloc(&x->e.nbr, (size_t)maxnb * x->e.stride));
   x->e.maxnb = maxnb;
   if (x->exec) cudaGraphExecDestroy(x->exec);
   x->exec = nullptr;
@@ -1135,14 +1155,15 @@ mdg_status e_alloc_neighbors(mdg_ensemble *x, int maxnb) {
   return MDG_OK;
 }
 
-// Marks every replica stale and clears the device error.
-mdg_status e_mark_all_stale(mdg_ensemble *x) {
+// Marks the replicas stale whose build met the error, or all of them, and clears
+// the error.
+mdg_status e_mark_stale(mdg_ensemble *x, bool all) {
   std::vector<RepStatus> rs;
   int err = 0;
   mdg_status r = e_status(x, &err, &rs);
   if (r) return r;
   for (auto &s : rs) {
-    s.list_stale = 1;
+    if (all || s.build) s.list_stale = 1;
     s.build = 0;
     s.want_build = 0;
     s.disp = 0;
@@ -1489,8 +1510,12 @@ mdg_status mdg_ensemble_calculate(mdg_ensemble *x, int nsteps) {
     if (err == kErrCapacity) {
       int need = 0;
       for (auto &s : rs) need = std::max(need, s.max_row);
-      if ((r = e_alloc_neighbors(x, (int)(need * 1.25) + 8))) return r;
-      if ((r = e_mark_all_stale(x))) return r;
+      bool kept = false;
+      if ((r = e_alloc_neighbors(x, (int)(need * 1.25) + 8, &kept))) return r;
+      // the others keep their lists and budgets, as each would alone; the coming
+      // step's positions lie in the copy that the failed step was to read
+      if ((r = e_mark_stale(x, !kept))) return r;
+      x->fix_buf = -1;
       if ((r = e_status(x, &err, &rs))) return r;
       continue;
     }
