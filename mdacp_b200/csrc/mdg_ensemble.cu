@@ -1175,8 +1175,9 @@ mdg_status e_mark_stale(mdg_ensemble *x, bool all) {
   return MDG_OK;
 }
 
-// Builds the stale lists (fresh upload): observers and counts walk the rows.
-// *st (may be null) gets every replica's status.
+// Builds the stale lists (fresh upload), with longer rows where they do not fit:
+// observers and counts walk the rows.  *st (may be null) gets every replica's
+// status.
 mdg_status e_current_lists(mdg_ensemble *x, std::vector<RepStatus> *st = nullptr) {
   Ens &e = x->e;
   std::vector<RepStatus> rs;
@@ -1184,9 +1185,21 @@ mdg_status e_current_lists(mdg_ensemble *x, std::vector<RepStatus> *st = nullptr
   mdg_status r = e_status(x, &err, &rs);
   if (r) return r;
   if (err) return e_translate(err);
-  bool stale = false;
-  for (auto &s : rs) stale |= s.list_stale != 0;
-  if (stale) {
+  for (int attempt = 0; attempt < 4; attempt++) {
+    bool stale = false;
+    int need = 0;
+    for (auto &s : rs) {
+      stale |= s.list_stale != 0;
+      need = std::max(need, s.max_row);
+    }
+    if (err == kErrCapacity) {  // the last attempt's rows did not fit
+      bool kept = false;
+      if ((r = e_alloc_neighbors(x, (int)(need * 1.25) + 8, &kept))) return r;
+      if ((r = e_mark_stale(x, !kept))) return r;
+      if ((r = e_status(x, &err, &rs))) return r;
+    } else if (err || !stale) {
+      break;
+    }
     for (auto &s : rs) {
       s.want_build = s.list_stale;
       s.disp = 0;
@@ -1197,8 +1210,8 @@ mdg_status e_current_lists(mdg_ensemble *x, std::vector<RepStatus> *st = nullptr
     ke_decide<<<1, 1024, 0, x->stream>>>(e, 0, kVerdictNone, nullptr);
     e_launch_build(x, x->stream, -1);
     if ((r = e_status(x, &err, &rs))) return r;
-    if (err) return e_translate(err);
   }
+  if (err) return e_translate(err);
   if (st) *st = std::move(rs);
   return MDG_OK;
 }

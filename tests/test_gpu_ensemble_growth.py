@@ -46,3 +46,32 @@ def test_the_others_go_on(precision, liquids, chunks):
         assert info["rebuilds"] == r
         assert np.array_equal(sq, gq) and np.array_equal(sv, gv)
     assert longest > capacity  # the rows did outgrow it
+
+
+@pytest.mark.parametrize("precision", [M.FP64, M.FP32_MIXED])
+@pytest.mark.parametrize("first", ["observe", "list_stats"])
+def test_sums_before_the_first_step(precision, first):
+    # a dense drop in a wide box: the first build's rows outgrow the capacity
+    # that the mean density gives, and a call that only reads builds them longer
+    w = W.fcc_liquid(6, 0.95, 1.0, seed=4, jitter=0.05, rc=2.5, dt=0.005)
+    L = np.array([40.0, 41.0, 42.0])
+    q = w.q + (L - w.L) / 2
+    gas = W.fcc_liquid(5, 0.2, 1.0, seed=5, jitter=0.05, rc=2.5, dt=0.005)
+    ens = M.Ensemble([(gas.q, gas.v, gas.L), (q, w.v, L)], cutoff=2.5, time_step=0.005, precision=precision)
+    getattr(ens, first)()
+    sums, (entries, within) = ens.observe(), ens.list_stats()
+    ens.calculate(10)
+    got = ens.states_by_id()
+    ens.close()
+    total = pairs = 0
+    for k, (x, v, box) in enumerate(((gas.q, gas.v, gas.L), (q, w.v, L))):
+        s = M.System(box, cutoff=2.5, time_step=0.005, capacity=len(x), precision=precision)
+        s.set_state(x, v)
+        assert [a[k] for a in sums] == pytest.approx(s.observe(), rel=1e-12)
+        n, e = s.pair_counts()
+        total, pairs = total + e, pairs + n // 2
+        s.calculate(10)
+        sq, sv = s.state_by_id()
+        s.close()
+        assert np.array_equal(sq, got[k][0]) and np.array_equal(sv, got[k][1])
+    assert (entries, within) == (total, pairs)
